@@ -228,6 +228,7 @@ sl::LuWork make_work() {
   w.status = g_dev.dsmall + 2;
   w.info_col = g_dev.dsmall + 3;
   w.cand = g_dev.dcand;
+  w.cand_launches = &g_dev.cand_launches;
   w.swap_plan = g_dev.dplan;
   w.perm = g_dev.dperm;
   w.bswap = g_dev.dbswap;

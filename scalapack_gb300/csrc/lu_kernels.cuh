@@ -42,17 +42,17 @@ inline cudaError_t smem_attr_once(const void* kern, int bytes) {
 }  // namespace
 
 constexpr int PW = 32;       // sub-panel width held in shared memory (<= 64)
-constexpr int PMAXG = 224;   // max CTAs of the panel kernel (warp 7 reads the diagonal row)
-// Exchange area of the panel kernel, in 8-byte tagged words: the diagonal
-// rows [2 parities][2*PW], the candidate keys [2 parities][PMAXG][4] (|x| key
-// lo, key hi, row, spare: one 32-byte sector per CTA, so that CTAs do not
-// write into each other's sectors) and the candidate rows
-// [PMAXG][2 parities][2*PW].
-constexpr int PX_DIAG = 0;
-constexpr int PX_KEYS = 4 * PW;
+constexpr int PMAXG = 224;   // max CTAs of the panel kernel
+// Exchange area of the panel kernel, in 8-byte tagged words: the candidate
+// keys [2 parities][PMAXG][4] (|x| key lo, key hi, label, spare: one 32-byte
+// sector per CTA, so that CTAs do not write into each other's sectors) and the
+// candidate rows [PMAXG][2 parities][2*PW].
+constexpr int PX_KEYS = 0;
 constexpr int PX_VALS = PX_KEYS + 8 * PMAXG;
 constexpr int PX_WORDS = PX_VALS + PMAXG * 2 * 2 * PW;
-constexpr int PT = 256;      // threads per panel CTA
+constexpr int PTR = 256;     // row threads per panel CTA
+constexpr int PT = PTR + 32; // and the exchange warp
+constexpr int PCH = 16;       // columns a row thread copies at a time
 constexpr int PLD = PW + 1;  // shared row stride: conflict-free row and column walks
 
 // Factor rows [r0, m) x columns [c0, c0+w) (w <= 32) of A in place (the
@@ -91,8 +91,9 @@ __device__ __forceinline__ void st_value(unsigned long long* p, int j, T v, uint
     st_tagged(p + j, __float_as_uint(v), tag);
   } else {
     const unsigned long long b = (unsigned long long)__double_as_longlong(v);
-    st_tagged(p + 2 * j, (uint32_t)b, tag);
-    st_tagged(p + 2 * j + 1, (uint32_t)(b >> 32), tag);
+    const unsigned long long t = (unsigned long long)tag << 32;
+    asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p + 2 * j), "l"(t | (uint32_t)b),
+                 "l"(t | (b >> 32)) : "memory");
   }
 }
 
@@ -129,68 +130,125 @@ __device__ __forceinline__ long long amax_ikey(float v) {
 __device__ __forceinline__ void ikey_combine(long long& k, int& r, long long k2, int r2) {
   if (k2 > k || (k2 == k && r2 < r)) { k = k2; r = r2; }
 }
+// The warp's best (key, row) on every lane, by three integer warp reductions
+// (high half, low half among its ties, lowest row among theirs) instead of
+// five shuffle rounds of a 64-bit key and a row: about 100 cycles instead of
+// 400, three times on every panel column's critical path.
 __device__ __forceinline__ void warp_ikey(long long& k, int& r) {
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
-    const long long k2 = __shfl_xor_sync(0xffffffffu, k, off);
-    const int r2 = __shfl_xor_sync(0xffffffffu, r, off);
-    ikey_combine(k, r, k2, r2);
-  }
+  const int h = (int)(k >> 32), hm = __reduce_max_sync(0xffffffffu, h);
+  const unsigned l = h == hm ? (unsigned)k : 0u, lm = __reduce_max_sync(0xffffffffu, l);
+  const unsigned c = (h == hm && l == lm) ? (unsigned)r : 0xffffffffu;
+  r = (int)__reduce_min_sync(0xffffffffu, c);
+  k = ((long long)hm << 32) | lm;
+}
+
+// 1/x for a positive finite x, rounded to nearest, from its bit pattern. The
+// FP64 pipe of this GPU takes 64 cycles per warp instruction, so a division
+// there (a chain of them, beside the other warps' updates) would cost more
+// than the L2 round trip it can hide behind; this one runs on the integer
+// pipe: Newton's iteration for the reciprocal of the 53-bit significand in
+// 64-bit fixed point from a 23-bit seed, then one exact comparison that picks
+// the nearest of two neighbours. Subnormal operands or results divide.
+__device__ __forceinline__ double recip_bits(unsigned long long bits) {
+  const int bexp = (int)(bits >> 52);
+  if (bexp == 0 || bexp >= 2045) return 1.0 / __longlong_as_double((long long)bits);
+  const unsigned long long frac = bits & 0xfffffffffffffULL;
+  if (frac == 0) return __longlong_as_double((long long)((unsigned long long)(2046 - bexp) << 52));
+  const unsigned long long m = frac | (1ULL << 52);
+  const unsigned long long d = m << 11;                       // D = d / 2^64 in (1/2, 1)
+  const float rf = __frcp_rn((float)(unsigned)(d >> 40));     // in (2^-24, 2^-23]
+  const float sf = rf * 36028797018963968.0f;                 // 2^55: Y = 1/D in units of 2^-31
+  const unsigned y0 = sf >= 4294967040.0f ? 4294967040u : (unsigned)sf;
+  // Y <- Y (2 - D Y), twice; e = 2^63 (1 - D Y)
+  unsigned long long y = (unsigned long long)y0 << 32;
+  long long e = (long long)((1ULL << 63) - __umul64hi(d, y));
+  y += (unsigned long long)(((long long)y0 * (e >> 12)) >> 19);
+  e = (long long)((1ULL << 63) - __umul64hi(d, y));
+  y += (unsigned long long)(((long long)(y >> 32) * e) >> 31);
+  // y is within a few units of 2^64 / (2 D): 16 units below the rounding
+  // boundary the lower neighbour is q, and q + 1 is nearer exactly when
+  // m (2q + 1) < 2^106
+  unsigned long long q = (y + 1024 - 16) >> 11;
+  if (__umul64hi(m, 2 * q + 1) < (1ULL << 42)) ++q;
+  return __longlong_as_double((long long)(((unsigned long long)(2045 - bexp) << 52) + (q - (1ULL << 52))));
 }
 
 // Cooperative unblocked LU of a sub-panel (PDGETF2, SRC/pdgetf2.f:206-237)
 // over rows r0..m-1 and columns c0..c0+w-1 of A, w <= PW. CTA b owns rows
-// r0 + b*rpc .. +rpc-1 in shared memory. Per column k:
-//   1. each CTA's IDAMAX candidate (first max, NaN never wins --
-//      PBLAS/SRC/pdamax_.c:414-486 through idamax_) is published as tagged
-//      words: its key and row, and the candidate row itself; the owner of the
-//      diagonal row publishes that row too;
-//   2. every CTA polls all keys (thread q reads CTA q's sector) until the
-//      tags match, reduces to the global winner (largest |x|, lowest row on
-//      ties) and then reads the pivot row from the winner's slot;
-//   3. rows d and piv are exchanged inside the sub-panel, the column is scaled
-//      by the reciprocal of the pivot and the rank-1 update is applied
-//      (PDSWAP/PDSCAL/PDGER, pdgetf2.f:218-233) with one thread per row, which
-//      also forms the next column's IDAMAX key.
-// Column k's words carry tag k+1 and the launch zeroes the area first. A word
-// of parity k&1 is rewritten only at column k+2, after every CTA has read
-// column k+1 -- which it can only do after finishing column k -- so two
-// parities suffice. Every poll is bounded (at most spin_limit polls); a CTA
-// that gives up records kFlagTimeout and returns, and block 0 then writes the
-// identity for the pivots it has not chosen, so the interchanges launched
-// after it stay inside the matrix.
+// r0 + b*rpc .. +rpc-1 in shared memory; rows are never moved: each has a
+// label, the row of the sub-panel where its content stands after the
+// interchanges so far (negative, ~k, once it is pivot row k), and goes back to
+// that row of A at the end. PTR row threads update the rows (thread t owns rows
+// t, t + PTR, ...); one more warp runs the exchange. Per column k:
+//   1. barrier; every warp reduces the row warps' IDAMAX candidates (first max
+//      by label, NaN never wins unless it stands in the diagonal row --
+//      PBLAS/SRC/pdamax_.c:414-486 through idamax_). The exchange warp
+//      publishes the CTA's key and label as tagged words; the row warp that
+//      holds the candidate publishes that row as it is, before column k-1's
+//      update of its columns beyond k, and then all row warps apply that
+//      update while the exchange is under way;
+//   2. the exchange warp polls all CTAs' keys (lane q reads CTAs q, q+32, ..)
+//      until the tags match, reduces them to the winner (largest |x|, lowest
+//      label on ties), reads the winner's row, forms 1/|pivot| from the key
+//      while that row is on its way, and applies column k-1's update to it:
+//      U(k, :), the diagonal row's swap being a change of label;
+//   3. barrier; the row threads scale column k by the reciprocal of the pivot
+//      and update column k+1 (PDSWAP/PDSCAL/PDGER, pdgetf2.f:218-233), which
+//      gives the next column's IDAMAX keys.
+// Every element receives the updates of columns 0, 1, ... in order, as one
+// fma each.
+//
+// Bound: the two L2 round trips of a column's exchange (publish and poll the
+// keys, read the winner's row; about 0.9 us together) plus two barriers and
+// two dependent FP64 instructions per row; the rest of the rank-1 update (half a
+// lane per cycle and sub-partition on this GPU's FP64 pipe) hides behind them
+// up to about 256 rows per SM. Measured, per column: 2.50 us over PDGESV
+// N = 4096 (3.74 with the rows swapped in place, the diagonal row published
+// too and the reciprocal divided on the FP64 pipe), 2.3 us at N = 600 (3.75).
+//
+// Column k's words carry tag tag0 + k, where tag0 differs from launch to
+// launch, so nothing is cleared between launches. A word of parity k&1 is
+// rewritten only at column k+2, after every CTA has read column k+1 -- which
+// it can only do after finishing column k -- so two parities suffice. Every
+// poll is bounded (at most spin_limit polls); a CTA that gives up records
+// kFlagTimeout and returns, and block 0 then writes the identity for the
+// pivots it has not chosen, so the interchanges launched after it stay inside
+// the matrix.
 //
 // GTILE: for panels taller than the CTAs' shared memory holds (more than 768
 // FP64 rows per CTA on every SM), each CTA's rows live in a global buffer
 // instead (gtile, column-major per CTA: rpc rows x PW columns, so a warp's
-// row walk is one coalesced access); the algorithm is unchanged.
+// row walk is one coalesced access; the labels follow all rows); the algorithm
+// is unchanged.
 template <typename T, bool GTILE = false>
-__global__ void __launch_bounds__(PT)
+__global__ void __launch_bounds__(PT, 3)
 panel_kernel(T* A, long long lda, int m, int r0, int c0, int w, int rpc, int* ipiv,
-             int* info_col, double* cand, int* status, long long spin_limit, T* gtile) {
+             int* info_col, double* cand, int* status, long long spin_limit, T* gtile,
+             uint32_t tag0) {
   extern __shared__ __align__(16) unsigned char panel_smem[];
   // element (r, c) of this CTA's rows: [rpc][PLD] in shared memory, or
   // column-major rpc x PW in the global buffer
   T* tile = GTILE ? gtile + (size_t)blockIdx.x * (size_t)rpc * PW : reinterpret_cast<T*>(panel_smem);
+  int* lab = GTILE ? reinterpret_cast<int*>(gtile + (size_t)gridDim.x * (size_t)rpc * PW) + (size_t)blockIdx.x * rpc
+                   : reinterpret_cast<int*>(reinterpret_cast<T*>(panel_smem) + (size_t)rpc * PLD);
   auto tix = [&](int r, int c) -> size_t {
     return GTILE ? (size_t)c * (size_t)rpc + (size_t)r : (size_t)r * PLD + (size_t)c;
   };
-  __shared__ T s_U[PW];
-  __shared__ T s_D[PW];
-  __shared__ long long s_wk[PT / 32];
-  __shared__ int s_wr[PT / 32];
-  __shared__ int s_lrow, s_row, s_fail, s_scale;
-  __shared__ long long s_lkey, s_gkey;
+  constexpr int NW = PTR / 32;  // row warps
+  __shared__ T s_U[2][PW];      // U(k, :) by column parity
+  __shared__ long long s_wk[NW];  // row warps' candidates: key, label, local row
+  __shared__ int s_wr[NW], s_wl[NW];
+  __shared__ int s_piv, s_own, s_fail, s_scale;
   __shared__ T s_rinv;
 
   const int G = gridDim.x, b = blockIdx.x, tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
+  const bool exch = warp == NW;
   const int R = m - r0;
   const int kw = min(w, R);
   const int lo = b * rpc;                   // first local row (relative to r0)
   const int nr = max(0, min(rpc, R - lo));  // rows owned
   unsigned long long* words = reinterpret_cast<unsigned long long*>(cand);
-  unsigned long long* diagw = words + PX_DIAG;
   unsigned long long* keyw = words + PX_KEYS;
   unsigned long long* valw = words + PX_VALS;
   // block 0 on a timeout at column k: pivots k.. become the diagonal rows
@@ -198,183 +256,214 @@ panel_kernel(T* A, long long lda, int m, int r0, int c0, int w, int rpc, int* ip
     if (b == 0)
       for (int q = k + tid; q < kw; q += PT) ipiv[c0 + q] = r0 + q;
   };
+  // a row's IDAMAX key for column k: a NaN in the diagonal row stays (IDAMAX
+  // keeps the first element when it is NaN), elsewhere it never wins
+  auto row_key = [&](T v, int label, int k) -> long long {
+    const long long key = amax_ikey(v);
+    return (key < 0 && label == k) ? LLONG_MAX : key;
+  };
+  auto put_candidate = [&](long long key, int label, int lrow) {
+    const long long mk = key;
+    const int ml = label;
+    warp_ikey(key, label);
+    const unsigned hit = __ballot_sync(0xffffffffu, mk == key && ml == label);
+    if (lane == __ffs(hit) - 1) {
+      s_wk[warp] = key;
+      s_wr[warp] = label;
+      s_wl[warp] = lrow;
+    }
+  };
 
-  // Sub-panel rows into shared memory, all w columns' loads in flight at once.
-  for (int r = tid; r < nr; r += PT) {
-    const T* src = A + (long long)(r0 + lo + r) + (long long)c0 * lda;
-    T v[PW];
+  if (!exch) {
+    // Sub-panel rows into shared memory, PCH columns' loads in flight at
+    // once, and the row warps' IDAMAX candidates of column 0; those of column
+    // k+1 come out of column k's rank-1 update.
+    long long key = -2;
+    int label = INT_MAX, lrow = 0;
+    for (int r = tid; r < nr; r += PTR) {
+      const T* src = A + (long long)(r0 + lo + r) + (long long)c0 * lda;
 #pragma unroll
-    for (int c = 0; c < PW; ++c) v[c] = (c < w) ? src[(long long)c * lda] : (T)0;
+      for (int cb = 0; cb < PW; cb += PCH) {
+        T v[PCH];
 #pragma unroll
-    for (int c = 0; c < PW; ++c)
-      if (c < w) tile[tix(r, c)] = v[c];
+        for (int c = 0; c < PCH; ++c) v[c] = (cb + c < w) ? src[(long long)(cb + c) * lda] : (T)0;
+#pragma unroll
+        for (int c = 0; c < PCH; ++c)
+          if (cb + c < w) tile[tix(r, cb + c)] = v[c];
+      }
+      lab[r] = lo + r;
+      const long long k2 = row_key(tile[tix(r, 0)], lo + r, 0);
+      if (k2 > key) { key = k2; label = lo + r; lrow = r; }
+    }
+    put_candidate(key, label, lrow);
   }
   if (tid == 0) s_fail = 0;
 
-  // Per-warp IDAMAX candidates of column 0; those of column k+1 come out of
-  // column k's rank-1 update.
-  {
-    long long key = -2;
-    int row = INT_MAX;
-    for (int r = tid; r < nr; r += PT) ikey_combine(key, row, amax_ikey(tile[tix(r, 0)]), lo + r);  // own rows
-    warp_ikey(key, row);
-    if (lane == 0) { s_wk[warp] = key; s_wr[warp] = row; }
-  }
-  __syncthreads();
-
-  // Column k's rank-1 update is applied in two parts: right after its pivot,
-  // only column k+1 (which gives the next pivot search its keys); the rest
-  // (columns k+2..) after column k+1's key has been published, while the
-  // other CTAs' keys are on their way. Every element still receives the
-  // updates of columns 0, 1, ... in order, as one fma each.
-  auto finish_update = [&](int kp) {  // columns kp+2 .. w-1 of the rows below kp
-    for (int r = max(0, kp + 1 - lo) + tid; r < nr; r += PT) {
+  auto finish_update = [&](int kp) {  // columns kp+2 .. w-1 of the active rows
+    const T* U = s_U[kp & 1];
+    for (int r = tid; r < nr; r += PTR) {
+      if (lab[r] < 0) continue;
       const T l = tile[tix(r, kp)];
 #pragma unroll 4
-      for (int j = kp + 2; j < w; ++j) tile[tix(r, j)] = fma(-l, s_U[j], tile[tix(r, j)]);
+      for (int j = kp + 2; j < w; ++j) tile[tix(r, j)] = fma(-l, U[j], tile[tix(r, j)]);
     }
   };
 
   for (int k = 0; k < kw; ++k) {
-    const int d = k;  // diagonal row relative to r0
     const int par = k & 1;
-    const uint32_t tag = (uint32_t)(k + 1);
-    // --- this CTA's candidate: IDAMAX over its rows >= d; its key goes out
-    //     at once ---
-    if (warp == 0) {
-      long long key = lane < PT / 32 ? s_wk[lane] : -2;
-      int row = lane < PT / 32 ? s_wr[lane] : INT_MAX;
-      warp_ikey(key, row);
-      if (lane == 0) {
-        s_lrow = row;
-        s_lkey = key;
-        const unsigned long long kb = (unsigned long long)key;
-        unsigned long long* kw4 = keyw + ((size_t)par * PMAXG + b) * 4;
-        st_tagged(kw4 + 0, (uint32_t)kb, tag);
-        st_tagged(kw4 + 1, (uint32_t)(kb >> 32), tag);
-        st_tagged(kw4 + 2, (uint32_t)row, tag);
-      }
-    }
+    const uint32_t tag = tag0 + (uint32_t)k;
     __syncthreads();
-    {
-      // the rest of column k-1's update, then the candidate row and the
-      // diagonal row (if owned), each published by its owner warp
-      if (k > 0) finish_update(k - 1);
-      // finish_update(k-1) hands row r (of this CTA) to thread (r - st) % PT
-      const int st = max(0, k - lo);
-      const int lr = s_lrow;
-      if (lr != INT_MAX && lr - lo >= st && lr - lo < nr && (((lr - lo - st) % PT) >> 5) == warp) {
+    // --- this CTA's candidate ---
+    long long key = lane < NW ? s_wk[lane] : -2;
+    int label = lane < NW ? s_wr[lane] : INT_MAX;
+    const long long mk = key;
+    const int ml = label;
+    warp_ikey(key, label);
+    const unsigned hit = __ballot_sync(0xffffffffu, lane < NW && mk == key && ml == label);
+    const int cw = __ffs(hit) - 1;  // row warp that holds it
+    const int lrow = s_wl[cw];
+    if (!exch) {
+      if (warp == cw && label != INT_MAX) {
+        // the candidate row before column k-1's update of its columns beyond k
         __syncwarp();
         for (int c = lane; c < w; c += 32)
-          st_value<T>(valw + ((size_t)b * 2 + par) * 2 * PW, c, tile[tix(lr - lo, c)], tag);
-      }
-      if (d - lo >= st && d - lo < nr && (((d - lo - st) % PT) >> 5) == warp) {
+          st_value<T>(valw + ((size_t)b * 2 + par) * 2 * PW, c, tile[tix(lrow, c)], tag);
         __syncwarp();
-        for (int c = lane; c < w; c += 32) st_value<T>(diagw + par * 2 * PW, c, tile[tix(d - lo, c)], tag);
       }
-    }
-
-    // --- poll every CTA's key (thread q <- CTA q) and the diagonal row (warp 7);
-    //     the polls spin without sleeping (a sleep costs more than it saves
-    //     here), bounded by spin_limit ---
-    long long key = -2;
-    int row = INT_MAX;
-    if (tid < G) {
-      long long spins = 0;
-      for (;;) {
-        if (spins++ >= spin_limit) { atomicExch(status, (int)kFlagTimeout); s_fail = 1; break; }
-        unsigned long long w0, w1, w2, w3;
-        ld_tagged2(keyw + ((size_t)tid + (size_t)par * PMAXG) * 4, w0, w1);
-        ld_tagged2(keyw + ((size_t)tid + (size_t)par * PMAXG) * 4 + 2, w2, w3);
-        if (tag_ok(w0, tag) && tag_ok(w1, tag) && tag_ok(w2, tag)) {
-          key = (long long)join(w0, w1);
-          const uint32_t rr = payload(w2);
-          row = rr >= (uint32_t)INT_MAX ? INT_MAX : (int)rr;
-          break;
+      if (k > 0) finish_update(k - 1);
+    } else {
+      if (lane < 3) {
+        const unsigned long long kb = (unsigned long long)key;
+        const uint32_t pay = lane == 0 ? (uint32_t)kb : (lane == 1 ? (uint32_t)(kb >> 32) : (uint32_t)label);
+        st_tagged(keyw + ((size_t)par * PMAXG + b) * 4 + lane, pay, tag);
+      }
+      // --- poll every CTA's key; the polls spin without sleeping (a sleep
+      //     costs more than it saves here), bounded by spin_limit ---
+      bool fail = false;
+      key = -2;
+      label = INT_MAX;
+      int own = 0;  // CTA of this lane's best key
+      for (int q = lane; q < G; q += 32) {
+        const unsigned long long* kq = keyw + ((size_t)q + (size_t)par * PMAXG) * 4;
+        for (long long spins = 0;;) {
+          if (spins++ >= spin_limit) { fail = true; break; }
+          unsigned long long w0, w1, w2, w3;
+          ld_tagged2(kq, w0, w1);
+          ld_tagged2(kq + 2, w2, w3);
+          if (tag_ok(w0, tag) && tag_ok(w1, tag) && tag_ok(w2, tag)) {
+            const long long k2 = (long long)join(w0, w1);
+            const int l2 = (int)payload(w2);
+            if (k2 > key || (k2 == key && l2 < label)) { key = k2; label = l2; own = q; }
+            break;
+          }
+        }
+        if (fail) break;
+      }
+      const long long lk = key;
+      const int ll = label;
+      warp_ikey(key, label);
+      const unsigned win = __ballot_sync(0xffffffffu, lk == key && ll == label);
+      own = __shfl_sync(0xffffffffu, own, __ffs(win) - 1);
+      fail = __any_sync(0xffffffffu, fail);
+      // --- the winner's row: U(k, :), and 1/|pivot| meanwhile ---
+      T v = (T)0, ra = (T)0;
+      if (!fail) {
+        const unsigned long long* vq = valw + ((size_t)own * 2 + par) * 2 * PW;
+        if constexpr (sizeof(T) == 8) {
+          // first look at the row, the reciprocal while it is in flight
+          unsigned long long a0 = 0, a1 = 0;
+          if (lane < w) ld_tagged2(vq + 2 * lane, a0, a1);
+          const unsigned long long kb = (unsigned long long)key;
+          if (kb - 1ULL < 0x7FEFFFFFFFFFFFFFULL) ra = recip_bits(kb);
+          if (tag_ok(a0, tag) && tag_ok(a1, tag)) v = __longlong_as_double((long long)join(a0, a1));
+          else if (lane < w && !ld_value<T>(vq, lane, tag, v, spin_limit)) fail = true;
+        } else {
+          if (lane < w && !ld_value<T>(vq, lane, tag, v, spin_limit)) fail = true;
         }
       }
-    } else if (warp == PT / 32 - 1) {
-      for (int c = lane; c < w; c += 32) {
-        T v;
-        if (ld_value<T>(diagw + par * 2 * PW, c, tag, v, spin_limit)) s_D[c] = v;
-        else { atomicExch(status, (int)kFlagTimeout); s_fail = 1; }
-      }
-    }
-    warp_ikey(key, row);
-    if (lane == 0) { s_wk[warp] = key; s_wr[warp] = row; }
-    __syncthreads();
-    if (s_fail) { give_up(k); return; }
-    if (warp == 0) {
-      key = lane < PT / 32 ? s_wk[lane] : -2;
-      row = lane < PT / 32 ? s_wr[lane] : INT_MAX;
-      warp_ikey(key, row);
-      if (lane == 0) { s_row = row; s_gkey = key; }
-    }
-    __syncthreads();
-    // IDAMAX keeps the first element when it is NaN; AMAX == 0 selects the
-    // diagonal row (PBLAS/SRC/pdamax_.c:486).
-    const int piv = (amax_ikey(s_D[k]) < 0 || s_gkey == 0) ? d : s_row;
-    // U = the pivot row: the diagonal row, or the winner's published row
-    if (tid < w) {
-      if (piv == d) {
-        s_U[tid] = s_D[tid];
+      fail = __any_sync(0xffffffffu, fail);
+      if (fail) {
+        if (lane == 0) {
+          atomicExch(status, (int)kFlagTimeout);
+          s_fail = 1;
+        }
       } else {
-        T v;
-        if (ld_value<T>(valw + ((size_t)(piv / rpc) * 2 + par) * 2 * PW, tid, tag, v, spin_limit)) s_U[tid] = v;
-        else { atomicExch(status, (int)kFlagTimeout); s_fail = 1; }
+        if (k > 0) {
+          const T l = __shfl_sync(0xffffffffu, v, k - 1);
+          if (lane > k && lane < w) v = fma(-l, s_U[par ^ 1][lane], v);
+        }
+        if (lane < w) s_U[par][lane] = v;
+        if (lane == k) {  // ONE/GMAX (pdgetf2.f:224)
+          T rinv;
+          if constexpr (sizeof(T) == 8) {
+            const unsigned long long kb = (unsigned long long)key;
+            rinv = (kb - 1ULL < 0x7FEFFFFFFFFFFFFFULL) ? (v < 0 ? -ra : ra) : (v != (T)0 ? (T)1 / v : (T)0);
+          } else {
+            rinv = v != (T)0 ? (T)1 / v : (T)0;
+          }
+          s_rinv = rinv;
+          s_scale = v != (T)0;
+          s_piv = label;
+          s_own = own;
+          if (b == 0) {
+            ipiv[c0 + k] = r0 + label;
+            if (v == (T)0) atomicMin(info_col, c0 + k);
+          }
+        }
       }
     }
     __syncthreads();
     if (s_fail) { give_up(k); return; }
-    // --- row interchange inside the sub-panel (PDSWAP, pdgetf2.f:218) ---
-    if (piv != d && tid < w) {
-      if (d >= lo && d < lo + nr) tile[tix(d - lo, tid)] = s_U[tid];
-      if (piv >= lo && piv < lo + nr) tile[tix(piv - lo, tid)] = s_D[tid];
-    }
-    if (tid == 0) {
-      const T gmax = s_U[k];
-      s_scale = (gmax != (T)0);
-      s_rinv = (gmax != (T)0) ? (T)1 / gmax : (T)0;  // ONE/GMAX (pdgetf2.f:224)
-      if (b == 0) {
-        ipiv[c0 + k] = r0 + piv;
-        if (gmax == (T)0) atomicMin(info_col, c0 + k);
+    // --- labels (PDSWAP), scale (PDSCAL) and the first column of the rank-1
+    //     update (PDGER); the row's next-column entry gives its IDAMAX key for
+    //     column k+1 ---
+    if (!exch) {
+      const bool scale = s_scale != 0;
+      const T rinv = s_rinv;
+      const int piv = s_piv, mine = s_own == b ? lrow : -1;
+      const int kn = k + 1;
+      const T un = kn < w ? s_U[par][kn] : (T)0;
+      long long nkey = -2;
+      int nlab = INT_MAX, nrow = 0;
+      for (int r = tid; r < nr; r += PTR) {
+        int lb = lab[r];
+        if (lb < 0) continue;
+        if (r == mine) {  // pivot row k
+          lab[r] = ~k;
+          continue;
+        }
+        if (lb == k) lab[r] = lb = piv;  // the diagonal row goes where the pivot row stood
+        T l = tile[tix(r, k)];
+        if (scale) l *= rinv;
+        tile[tix(r, k)] = l;
+        if (kn < w) {
+          const T v = fma(-l, un, tile[tix(r, kn)]);
+          tile[tix(r, kn)] = v;
+          if (kn < kw) {
+            const long long k2 = row_key(v, lb, kn);
+            if (k2 > nkey || (k2 == nkey && lb < nlab)) { nkey = k2; nlab = lb; nrow = r; }
+          }
+        }
       }
+      if (kn < kw) put_candidate(nkey, nlab, nrow);
     }
-    __syncthreads();
-    // --- scale (PDSCAL) and the first column of the rank-1 update (PDGER),
-    //     one thread per row; the row's next-column entry gives its IDAMAX
-    //     key for column k+1 ---
-    const bool scale = s_scale != 0;
-    const T rinv = s_rinv;
-    const int kn = k + 1;
-    long long nkey = -2;
-    int nrow = INT_MAX;
-    for (int r = max(0, d + 1 - lo) + tid; r < nr; r += PT) {
-      T l = tile[tix(r, k)];
-      if (scale) l *= rinv;
-      tile[tix(r, k)] = l;
-      if (kn < w) tile[tix(r, kn)] = fma(-l, s_U[kn], tile[tix(r, kn)]);
-      if (kn < kw) ikey_combine(nkey, nrow, amax_ikey(tile[tix(r, kn)]), lo + r);
-    }
-    if (kn < kw) {
-      warp_ikey(nkey, nrow);
-      if (lane == 0) { s_wk[warp] = nkey; s_wr[warp] = nrow; }
-    }
-    __syncthreads();
   }
   // the last column's remaining update (columns beyond kw when the panel has
-  // fewer rows than columns)
+  // fewer rows than columns), then every row to where its content stands
+  if (exch) return;
   if (kw > 0) finish_update(kw - 1);
-  __syncthreads();
-
-  for (int r = tid; r < nr; r += PT) {
-    T* dst = A + (long long)(r0 + lo + r) + (long long)c0 * lda;
-    T v[PW];
+  for (int r = tid; r < nr; r += PTR) {
+    const int lb = lab[r];
+    T* dst = A + (long long)(r0 + (lb < 0 ? ~lb : lb)) + (long long)c0 * lda;
 #pragma unroll
-    for (int c = 0; c < PW; ++c) v[c] = (c < w) ? tile[tix(r, c)] : (T)0;
+    for (int cb = 0; cb < PW; cb += PCH) {
+      T v[PCH];
 #pragma unroll
-    for (int c = 0; c < PW; ++c)
-      if (c < w) dst[(long long)c * lda] = v[c];
+      for (int c = 0; c < PCH; ++c) v[c] = (cb + c < w) ? tile[tix(r, cb + c)] : (T)0;
+#pragma unroll
+      for (int c = 0; c < PCH; ++c)
+        if (cb + c < w) dst[(long long)(cb + c) * lda] = v[c];
+    }
   }
 }
 
@@ -1059,8 +1148,9 @@ inline cudaError_t launch_panel(T* A, long long lda, int m, int r0, int c0, int 
   if (rpc > rpc_max) rpc = (R + num_sms() - 1) / num_sms();
   rpc = (rpc + 7) & ~7;
   int G = (R + rpc - 1) / rpc;
-  size_t smem = sizeof(T) * (size_t)rpc * PLD;
+  size_t smem = sizeof(T) * (size_t)rpc * PLD;  // and the labels
   const bool global_tile = smem > 200 * 1024 || G > PMAXG;
+  smem += sizeof(int) * (size_t)rpc;
   T* gtile = nullptr;
   if (global_tile) {
     if constexpr (sizeof(T) != 8) {
@@ -1069,18 +1159,27 @@ inline cudaError_t launch_panel(T* A, long long lda, int m, int r0, int c0, int 
       G = std::min(PMAXG, num_sms());
       rpc = ((R + G - 1) / G + 7) & ~7;
       G = (R + rpc - 1) / rpc;
-      if (!ws.ptile || ws.ptile_len < (size_t)G * rpc * PW) return cudaErrorInvalidValue;
+      if (!ws.ptile || ws.ptile_len < (size_t)G * rpc * PW + ((size_t)G * rpc + 1) / 2)
+        return cudaErrorInvalidValue;
       gtile = ws.ptile;
       smem = 0;
     }
   }
-  if (!global_tile) SL_TRY(smem_attr_once((const void*)panel_kernel<T, false>, 200 * 1024));
-  // zero the diagonal rows and the G slots used (stale tags must not match)
-  cudaError_t e = cudaMemsetAsync(ws.cand, 0, sizeof(unsigned long long) * ((size_t)PX_VALS + (size_t)G * 2 * 2 * PW), s);
-  if (e != cudaSuccess) return e;
+  if (!global_tile) SL_TRY(smem_attr_once((const void*)panel_kernel<T, false>, 212 * 1024));
+  // Tags of this launch's words: 64 per launch, never used before in this
+  // area since it was cleared (when new and when the launch count wraps).
+  // Without a launch count the words are cleared for every launch.
+  constexpr unsigned kLaunches = 1u << 26;
+  unsigned id = 1;
+  if (!ws.cand_launches || *ws.cand_launches == 0 || *ws.cand_launches + 1 >= kLaunches) {
+    SL_TRY(cudaMemsetAsync(ws.cand, 0, sizeof(unsigned long long) * (size_t)PX_WORDS, s));
+    if (ws.cand_launches) *ws.cand_launches = 0;
+  }
+  if (ws.cand_launches) id = ++*ws.cand_launches;
+  uint32_t tag0 = id * 64u;
   long long limit = spin_limit();
   void* args[] = {&A, &lda, &m, &r0, &c0, &w, (void*)&rpc, &ipiv, (void*)&ws.info_col,
-                  (void*)&ws.cand, (void*)&ws.status, (void*)&limit, (void*)&gtile};
+                  (void*)&ws.cand, (void*)&ws.status, (void*)&limit, (void*)&gtile, (void*)&tag0};
   count_launches(1);
   if (global_tile)
     return cudaLaunchCooperativeKernel((void*)panel_kernel<T, true>, dim3(G), dim3(PT), args, 0, s);

@@ -112,6 +112,10 @@ struct LuWork {
   int* status;       // 1 int: device status word (DevStatus)
   int* info_col;     // 1 int: first zero-pivot column (0-based), INT_MAX if none
   double* cand;      // exchange area of the panel kernel (kPanelCandDoubles words)
+  // Launches that have used `cand` (host counter, 0 for a new area): their
+  // tags tell each launch's words from all earlier ones. Null: `cand` is
+  // cleared before every launch.
+  unsigned* cand_launches = nullptr;
   int* swap_plan = nullptr;  // kSwapPlanInts: composite form of a panel's interchanges
   int* perm;         // n ints: composed row permutation (solve)
   double* bswap;     // n * nrhs doubles: gathered right-hand sides (solve)
@@ -170,10 +174,9 @@ inline size_t kSolveInvDoubles(int n) {
 constexpr size_t kDinv64Doubles = (size_t)16 * 64 * 64;
 
 size_t panel_cand_doubles();
-// 8-byte words of the panel kernel's exchange area (2 diagonal rows of 2 x 32
-// words, 2 x 224 x 4 key words, 224 CTAs x 2 parities x 64 row words);
-// panel_cand_doubles() returns it.
-constexpr size_t kPanelCandDoubles = (size_t)4 * 32 + (size_t)8 * 224 + (size_t)224 * 2 * 2 * 32;
+// 8-byte words of the panel kernel's exchange area (2 x 224 x 4 key words, 224
+// CTAs x 2 parities x 64 row words); panel_cand_doubles() returns it.
+constexpr size_t kPanelCandDoubles = (size_t)8 * 224 + (size_t)224 * 2 * 2 * 32;
 // Ints of a panel's interchange plan (count + 2 x 512 (row, src) pairs).
 constexpr size_t kSwapPlanInts = 1 + 4 * 256 + 15;
 // Largest M whose FP64 panel rows fit the SMs' shared memory on this device;

@@ -169,3 +169,73 @@ def test_interchange_plan_walk_matches_replay():
         m = k1 + npiv + int(rng.integers(0, 60))
         piv = [int(rng.integers(k1 + i, m)) for i in range(npiv)]
         assert _plan_walk(k1, k1 + npiv, piv) == _plan_replay(k1, k1 + npiv, piv)
+
+
+def _recip_model(bits):
+    """The panel kernel's 1/x for a normal positive x: Newton's iteration on the
+    significand in 64-bit fixed point, then one exact comparison."""
+    bexp, frac = bits >> 52, bits & ((1 << 52) - 1)
+    if frac == 0:
+        return (2046 - bexp) << 52
+    m = frac | (1 << 52)
+    d = m << 11
+    sf = np.float32(1) / np.float32(d >> 40) * np.float32(2.0**55)
+    y = (4294967040 if sf >= np.float32(4294967040.0) else int(sf)) << 32
+    for sh in (12, 0):
+        e = (1 << 63) - ((d * y) >> 64)
+        t = (y >> 32) * (e >> sh)
+        assert -(1 << 63) <= t < (1 << 63)  # the device's 64-bit product
+        y += t >> (31 - sh)
+        assert y < 1 << 64
+    q = (y + 1024 - 16) >> 11
+    if ((m * (2 * q + 1)) >> 64) < (1 << 42):
+        q += 1
+    return ((2045 - bexp) << 52) + (q - (1 << 52))
+
+
+def test_panel_reciprocal_is_correctly_rounded():
+    rng = np.random.default_rng(3)
+    fr = np.concatenate([rng.integers(0, 1 << 52, 20000), np.arange(200), (1 << 52) - 1 - np.arange(200)])
+    ex = rng.integers(1, 2045, fr.size)
+    for f, e in zip(fr, ex):
+        bits = (int(e) << 52) | int(f)
+        x = np.uint64(bits).view(np.float64)
+        assert np.uint64(_recip_model(bits)).view(np.float64) == 1.0 / x
+
+
+@pytest.mark.parametrize("rows,w", [(1, 1), (5, 5), (33, 32), (40, 32), (3, 8)])
+def test_panel_row_labels_follow_the_interchanges(rows, w):
+    """The panel kernel never moves a row: it relabels the diagonal row and
+    retires the pivot row. Against the interchanges themselves, with ties, a
+    zero column and NaNs in and off the diagonal."""
+    rng = np.random.default_rng(rows * 100 + w)
+    for trial in range(30):
+        vals = rng.integers(-3, 4, (min(rows, w), rows)).astype(float)  # column k's values by content
+        if trial % 3 == 1:
+            vals[rng.random(vals.shape) < 0.2] = np.nan
+        if trial % 5 == 2:
+            vals[:] = 0.0
+        content = list(range(rows))  # sequential: content standing in each row
+        lab, done = list(range(rows)), [False] * rows
+        for k in range(min(rows, w)):
+            col = [vals[k][content[r]] for r in range(rows)]
+            p = k  # IDAMAX from row k: a leading NaN stays, a later one never wins
+            if not np.isnan(col[k]):
+                for r in range(k + 1, rows):
+                    if abs(col[r]) > abs(col[p]):
+                        p = r
+            best = None
+            for c in range(rows):
+                if done[c]:
+                    continue
+                v = vals[k][c]
+                key = (np.inf if lab[c] == k else -1.0) if np.isnan(v) else abs(v)
+                if best is None or key > best[0] or (key == best[0] and lab[c] < best[1]):
+                    best = (key, lab[c], c)
+            assert best[1] == p
+            for c in range(rows):
+                if c != best[2] and not done[c] and lab[c] == k:
+                    lab[c] = p
+            lab[best[2]], done[best[2]] = k, True
+            content[k], content[p] = content[p], content[k]
+            assert all(content[lab[c]] == c for c in range(rows))
