@@ -337,9 +337,9 @@ void sl1x1_debug_set_spin_limit(long long polls);
  * column's pivot exchange but a longer rank-1 update per CTA. Changes only the
  * speed, not the results. */
 void sl1x1_set_panel_rows(int rows);
-/* CTAs (8..224, default 64) that the cooperative panel kernel spreads a tall
- * panel's rows over, before the minimum slice above applies. Changes only the
- * speed, not the results. */
+/* CTAs (8..224, default 64; at most 160 are used) that the cooperative panel
+ * kernel spreads a tall panel's rows over, before the minimum slice above
+ * applies. Changes only the speed, not the results. */
 void sl1x1_set_panel_ctas(int ctas);
 /* 32-column sub-panels per in-panel block of the FP64 panel factorization
  * (1..8, default 2): inside a block only the next sub-panel's columns are

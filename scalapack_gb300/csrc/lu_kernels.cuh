@@ -42,16 +42,17 @@ inline cudaError_t smem_attr_once(const void* kern, int bytes) {
 }  // namespace
 
 constexpr int PW = 32;       // sub-panel width held in shared memory (<= 64)
-constexpr int PMAXG = 224;   // max CTAs of the panel kernel
-// Exchange area of the panel kernel, in 8-byte tagged words: the candidate
-// keys [2 parities][PMAXG][4] (|x| key lo, key hi, label, spare: one 32-byte
-// sector per CTA, so that CTAs do not write into each other's sectors) and the
-// candidate rows [PMAXG][2 parities][2*PW].
+constexpr int PMAXG = 160;   // max CTAs of the panel kernel
+// Exchange area of the panel kernel, in 8-byte words: the candidate keys
+// [2 parities][PMAXG readers][PMAXG writers], each {key, label | tag << 32} in
+// one 16-byte word, so that a CTA polls lines that no other CTA reads, and the
+// candidate rows [PMAXG][2 parities][2*PW] in tagged 8-byte words.
 constexpr int PX_KEYS = 0;
-constexpr int PX_VALS = PX_KEYS + 8 * PMAXG;
+constexpr int PX_VALS = PX_KEYS + 2 * PMAXG * PMAXG * 2;
 constexpr int PX_WORDS = PX_VALS + PMAXG * 2 * 2 * PW;
 constexpr int PTR = 256;     // row threads per panel CTA
 constexpr int PT = PTR + 32; // and the exchange warp
+constexpr int PKP = 2;        // key polls a lane keeps in flight (64 CTAs)
 constexpr int PCH = 16;       // columns a row thread copies at a time
 constexpr int PLD = PW + 1;  // shared row stride: conflict-free row and column walks
 
@@ -82,6 +83,20 @@ __device__ __forceinline__ bool tag_ok(unsigned long long wd, uint32_t tag) {
 __device__ __forceinline__ uint32_t payload(unsigned long long wd) { return (uint32_t)wd; }
 __device__ __forceinline__ unsigned long long join(unsigned long long lo, unsigned long long hi) {
   return ((unsigned long long)payload(hi) << 32) | payload(lo);
+}
+
+// A candidate key with its label and tag, one single-copy atomic 16-byte word.
+__device__ __forceinline__ void st_key(unsigned long long* p, long long key, int label, uint32_t tag) {
+  const unsigned long long hi = ((unsigned long long)tag << 32) | (uint32_t)label;
+  asm volatile("{ .reg .b128 t;\n mov.b128 t, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], t; }" ::"l"(p),
+               "l"((unsigned long long)key), "l"(hi)
+               : "memory");
+}
+__device__ __forceinline__ void ld_key(const unsigned long long* p, unsigned long long& key, unsigned long long& hi) {
+  asm volatile("{ .reg .b128 t;\n ld.relaxed.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t; }"
+               : "=l"(key), "=l"(hi)
+               : "l"(p)
+               : "memory");
 }
 
 // Value v of a row as tagged words (FP32: one word, FP64: two).
@@ -116,30 +131,36 @@ __device__ __forceinline__ bool ld_value(const unsigned long long* p, int j, uin
 }
 
 // IDAMAX key of a value: the bit pattern of |x| as an integer (monotonic in
-// |x| for IEEE formats, +0 and -0 equal), -1 for NaN so that NaN never wins.
-// Integer keys keep the pivot search off the FP64 pipe.
+// |x| for IEEE formats, +0 and -0 equal; an FP32 pattern in the high half), -1
+// for NaN so that NaN never wins. Integer keys keep the pivot search off the
+// FP64 pipe.
 __device__ __forceinline__ long long amax_ikey(double v) {
   const long long b = __double_as_longlong(v) & 0x7FFFFFFFFFFFFFFFLL;
   return b > 0x7FF0000000000000LL ? -1LL : b;
 }
 __device__ __forceinline__ long long amax_ikey(float v) {
   const int b = __float_as_int(v) & 0x7FFFFFFF;
-  return b > 0x7F800000 ? -1LL : (long long)b;
+  return b > 0x7F800000 ? -1LL : (long long)b << 32;
 }
-// Larger key wins, ties go to the lower row (IDAMAX returns the first max).
-__device__ __forceinline__ void ikey_combine(long long& k, int& r, long long k2, int r2) {
-  if (k2 > k || (k2 == k && r2 < r)) { k = k2; r = r2; }
-}
-// The warp's best (key, row) on every lane, by three integer warp reductions
-// (high half, low half among its ties, lowest row among theirs) instead of
-// five shuffle rounds of a 64-bit key and a row: about 100 cycles instead of
-// 400, three times on every panel column's critical path.
-__device__ __forceinline__ void warp_ikey(long long& k, int& r) {
-  const int h = (int)(k >> 32), hm = __reduce_max_sync(0xffffffffu, h);
-  const unsigned l = h == hm ? (unsigned)k : 0u, lm = __reduce_max_sync(0xffffffffu, l);
-  const unsigned c = (h == hm && l == lm) ? (unsigned)r : 0xffffffffu;
-  r = (int)__reduce_min_sync(0xffffffffu, c);
-  k = ((long long)hm << 32) | lm;
+// The lane that holds the warp's best (key, row): largest key, lowest row among
+// ties. One integer warp reduction (28 cycles) over the keys' high halves decides
+// unless two lanes tie there (two more then, over the low halves and the rows),
+// instead of five rounds of three dependent shuffles (42 cycles each), three
+// times on every panel column's critical path.
+__device__ __forceinline__ int warp_best(long long key, int row) {
+  const int h = (int)(key >> 32);
+  const int hm = __reduce_max_sync(0xffffffffu, h);
+  unsigned hit = __ballot_sync(0xffffffffu, h == hm);
+  if (hit & (hit - 1)) {  // (the same on every lane: all take part in what follows)
+    const bool t0 = (hit >> (threadIdx.x & 31)) & 1u;
+    const unsigned l = t0 ? (unsigned)key : 0u;
+    const unsigned lm = __reduce_max_sync(0xffffffffu, l);
+    const bool t1 = t0 && l == lm;
+    const unsigned r = t1 ? (unsigned)row : 0xffffffffu;
+    const unsigned rm = __reduce_min_sync(0xffffffffu, r);
+    hit = __ballot_sync(0xffffffffu, t1 && r == rm);
+  }
+  return __ffs(hit) - 1;
 }
 
 // 1/x for a positive finite x, rounded to nearest, from its bit pattern. The
@@ -178,33 +199,39 @@ __device__ __forceinline__ double recip_bits(unsigned long long bits) {
 // r0 + b*rpc .. +rpc-1 in shared memory; rows are never moved: each has a
 // label, the row of the sub-panel where its content stands after the
 // interchanges so far (negative, ~k, once it is pivot row k), and goes back to
-// that row of A at the end. PTR row threads update the rows (thread t owns rows
-// t, t + PTR, ...); one more warp runs the exchange. Per column k:
+// that row of A at the end. PTR row threads update the rows: tpr of them, lanes
+// of one warp, share a row (4, 2 or 1, so that a CTA's rows keep four warps
+// busy: the FP64 unit is one per SM, takes a warp instruction every 20 cycles
+// whatever lanes are active, and has one of a warp's in flight at a time, for 64
+// cycles), the first of them owns it. One more warp runs the exchange. Per
+// column k:
 //   1. barrier; every warp reduces the row warps' IDAMAX candidates (first max
 //      by label, NaN never wins unless it stands in the diagonal row --
 //      PBLAS/SRC/pdamax_.c:414-486 through idamax_). The exchange warp
 //      publishes the CTA's key and label as tagged words; the row warp that
-//      holds the candidate publishes that row as it is, before column k-1's
-//      update of its columns beyond k, and then all row warps apply that
-//      update while the exchange is under way;
-//   2. the exchange warp polls all CTAs' keys (lane q reads CTAs q, q+32, ..)
-//      until the tags match, reduces them to the winner (largest |x|, lowest
-//      label on ties), reads the winner's row, forms 1/|pivot| from the key
-//      while that row is on its way, and applies column k-1's update to it:
-//      U(k, :), the diagonal row's swap being a change of label;
+//      holds the candidate publishes that row with column k-1's update applied
+//      (a lane per column), and then all row warps apply that update to their
+//      rows while the exchange is under way;
+//   2. the exchange warp polls all CTAs' keys (lane q reads CTAs q, q+32, ..,
+//      PKP in flight) until the tags match, reduces them to the winner
+//      (largest |x|, lowest label on ties), reads the winner's row -- U(k, :),
+//      the diagonal row's swap being a change of label -- and forms 1/|pivot|
+//      from the key while that row is on its way;
 //   3. barrier; the row threads scale column k by the reciprocal of the pivot
 //      and update column k+1 (PDSWAP/PDSCAL/PDGER, pdgetf2.f:218-233), which
 //      gives the next column's IDAMAX keys.
 // Every element receives the updates of columns 0, 1, ... in order, as one
 // fma each.
 //
-// Bound: the two L2 round trips of a column's exchange (publish and poll the
-// keys, read the winner's row; about 0.9 us together) plus two barriers and
-// two dependent FP64 instructions per row; the rest of the rank-1 update (half a
-// lane per cycle and sub-partition on this GPU's FP64 pipe) hides behind them
-// up to about 256 rows per SM. Measured, per column: 2.50 us over PDGESV
-// N = 4096 (3.74 with the rows swapped in place, the diagonal row published
-// too and the reciprocal divided on the FP64 pipe), 2.3 us at N = 600 (3.75).
+// Bound: the L2 round trips of a column's exchange (publish and poll the keys,
+// about 950 cycles between two CTAs, 1900 over 64 CTAs on both dies; read the
+// winner's row, 600), two barriers, and a chain of dependent FP64 and warp
+// reductions (about 1200); the rest of the rank-1 update hides behind them up to
+// about 256 rows per SM. Keys are pushed to each reader's own lines: 64 CTAs
+// polling the same 64 sectors cost 1200 cycles more. Measured, per column: 2.4
+// us over 32 CTAs (R = 4096), 2.6 over 64 (R = 8192), 2.2 with two; 3.74 with
+// shuffle reductions, rows swapped in place, the diagonal row published too and
+// the reciprocal divided on the FP64 pipe. PDGESV N = 4096 28.0 -> 22.3 ms.
 //
 // Column k's words carry tag tag0 + k, where tag0 differs from launch to
 // launch, so nothing is cleared between launches. A word of parity k&1 is
@@ -221,10 +248,10 @@ __device__ __forceinline__ double recip_bits(unsigned long long bits) {
 // row walk is one coalesced access; the labels follow all rows); the algorithm
 // is unchanged.
 template <typename T, bool GTILE = false>
-__global__ void __launch_bounds__(PT, 3)
+__global__ void __launch_bounds__(PT, GTILE ? 1 : 3)
 panel_kernel(T* A, long long lda, int m, int r0, int c0, int w, int rpc, int* ipiv,
              int* info_col, double* cand, int* status, long long spin_limit, T* gtile,
-             uint32_t tag0) {
+             uint32_t tag0, int tpr) {
   extern __shared__ __align__(16) unsigned char panel_smem[];
   // element (r, c) of this CTA's rows: [rpc][PLD] in shared memory, or
   // column-major rpc x PW in the global buffer
@@ -238,7 +265,7 @@ panel_kernel(T* A, long long lda, int m, int r0, int c0, int w, int rpc, int* ip
   __shared__ T s_U[2][PW];      // U(k, :) by column parity
   __shared__ long long s_wk[NW];  // row warps' candidates: key, label, local row
   __shared__ int s_wr[NW], s_wl[NW];
-  __shared__ int s_piv, s_own, s_fail, s_scale;
+  __shared__ int s_piv, s_own, s_fail;
   __shared__ T s_rinv;
 
   const int G = gridDim.x, b = blockIdx.x, tid = threadIdx.x;
@@ -263,16 +290,14 @@ panel_kernel(T* A, long long lda, int m, int r0, int c0, int w, int rpc, int* ip
     return (key < 0 && label == k) ? LLONG_MAX : key;
   };
   auto put_candidate = [&](long long key, int label, int lrow) {
-    const long long mk = key;
-    const int ml = label;
-    warp_ikey(key, label);
-    const unsigned hit = __ballot_sync(0xffffffffu, mk == key && ml == label);
-    if (lane == __ffs(hit) - 1) {
+    if (lane == warp_best(key, label)) {
       s_wk[warp] = key;
       s_wr[warp] = label;
       s_wl[warp] = lrow;
     }
   };
+  // row thread tid: part `part` of rows row0, row0 + rstep, ...
+  const int part = tid & (tpr - 1), row0 = tid / tpr, rstep = PTR / tpr;
 
   if (!exch) {
     // Sub-panel rows into shared memory, PCH columns' loads in flight at
@@ -292,20 +317,35 @@ panel_kernel(T* A, long long lda, int m, int r0, int c0, int w, int rpc, int* ip
           if (cb + c < w) tile[tix(r, cb + c)] = v[c];
       }
       lab[r] = lo + r;
-      const long long k2 = row_key(tile[tix(r, 0)], lo + r, 0);
-      if (k2 > key) { key = k2; label = lo + r; lrow = r; }
     }
+    asm volatile("bar.sync 1, %0;" ::"n"(PTR) : "memory");  // the rows' owners differ from their loaders
+    if (part == 0)
+      for (int r = row0; r < nr; r += rstep) {
+        const long long k2 = row_key(tile[tix(r, 0)], lo + r, 0);
+        if (k2 > key) { key = k2; label = lo + r; lrow = r; }
+      }
     put_candidate(key, label, lrow);
   }
   if (tid == 0) s_fail = 0;
 
-  auto finish_update = [&](int kp) {  // columns kp+2 .. w-1 of the active rows
+  // columns kp+2 .. w-1 of the active rows, column by column in turn among a
+  // row's threads; the next column's operands are read while one is updated
+  auto finish_update = [&](int kp) {
     const T* U = s_U[kp & 1];
-    for (int r = tid; r < nr; r += PTR) {
+    for (int r = row0; r < nr; r += rstep) {
       if (lab[r] < 0) continue;
       const T l = tile[tix(r, kp)];
-#pragma unroll 4
-      for (int j = kp + 2; j < w; ++j) tile[tix(r, j)] = fma(-l, U[j], tile[tix(r, j)]);
+      int j = kp + 2 + part;
+      if (j >= w) continue;
+      T v = tile[tix(r, j)], u = U[j];
+#pragma unroll 2
+      for (; j + tpr < w; j += tpr) {
+        const T vn = tile[tix(r, j + tpr)], un = U[j + tpr];
+        tile[tix(r, j)] = fma(-l, u, v);
+        v = vn;
+        u = un;
+      }
+      tile[tix(r, j)] = fma(-l, u, v);
     }
   };
 
@@ -314,57 +354,62 @@ panel_kernel(T* A, long long lda, int m, int r0, int c0, int w, int rpc, int* ip
     const uint32_t tag = tag0 + (uint32_t)k;
     __syncthreads();
     // --- this CTA's candidate ---
-    long long key = lane < NW ? s_wk[lane] : -2;
+    long long key = lane < NW ? s_wk[lane] : -3;
     int label = lane < NW ? s_wr[lane] : INT_MAX;
-    const long long mk = key;
-    const int ml = label;
-    warp_ikey(key, label);
-    const unsigned hit = __ballot_sync(0xffffffffu, lane < NW && mk == key && ml == label);
-    const int cw = __ffs(hit) - 1;  // row warp that holds it
+    const int cw = warp_best(key, label);  // row warp that holds it
     const int lrow = s_wl[cw];
     if (!exch) {
-      if (warp == cw && label != INT_MAX) {
-        // the candidate row before column k-1's update of its columns beyond k
-        __syncwarp();
-        for (int c = lane; c < w; c += 32)
-          st_value<T>(valw + ((size_t)b * 2 + par) * 2 * PW, c, tile[tix(lrow, c)], tag);
+      if (warp == cw && s_wr[cw] != INT_MAX) {
+        // the candidate row, its columns beyond k with column k-1's update
+        const T l = k > 0 ? tile[tix(lrow, k - 1)] : (T)0;
+        for (int c = lane; c < w; c += 32) {
+          T v = tile[tix(lrow, c)];
+          if (k > 0 && c > k) v = fma(-l, s_U[par ^ 1][c], v);
+          st_value<T>(valw + ((size_t)b * 2 + par) * 2 * PW, c, v, tag);
+        }
         __syncwarp();
       }
       if (k > 0) finish_update(k - 1);
     } else {
-      if (lane < 3) {
-        const unsigned long long kb = (unsigned long long)key;
-        const uint32_t pay = lane == 0 ? (uint32_t)kb : (lane == 1 ? (uint32_t)(kb >> 32) : (uint32_t)label);
-        st_tagged(keyw + ((size_t)par * PMAXG + b) * 4 + lane, pay, tag);
-      }
+      key = __shfl_sync(0xffffffffu, key, cw);
+      label = __shfl_sync(0xffffffffu, label, cw);
+      for (int q = lane; q < G; q += 32)
+        st_key(keyw + (((size_t)par * PMAXG + q) * PMAXG + b) * 2, key, label, tag);
       // --- poll every CTA's key; the polls spin without sleeping (a sleep
       //     costs more than it saves here), bounded by spin_limit ---
       bool fail = false;
-      key = -2;
+      key = -3;
       label = INT_MAX;
       int own = 0;  // CTA of this lane's best key
-      for (int q = lane; q < G; q += 32) {
-        const unsigned long long* kq = keyw + ((size_t)q + (size_t)par * PMAXG) * 4;
-        for (long long spins = 0;;) {
-          if (spins++ >= spin_limit) { fail = true; break; }
-          unsigned long long w0, w1, w2, w3;
-          ld_tagged2(kq, w0, w1);
-          ld_tagged2(kq + 2, w2, w3);
-          if (tag_ok(w0, tag) && tag_ok(w1, tag) && tag_ok(w2, tag)) {
-            const long long k2 = (long long)join(w0, w1);
-            const int l2 = (int)payload(w2);
-            if (k2 > key || (k2 == key && l2 < label)) { key = k2; label = l2; own = q; }
-            break;
-          }
+      const unsigned long long* kq = keyw + ((size_t)par * PMAXG + b) * PMAXG * 2;
+      for (int q0 = lane; q0 < G; q0 += 32 * PKP) {
+        for (long long spins = 0;; ++spins) {
+          unsigned long long kk[PKP], hi[PKP];
+          bool all = true;
+#pragma unroll
+          for (int i = 0; i < PKP; ++i)
+            if (q0 + 32 * i < G) ld_key(kq + 2 * (q0 + 32 * i), kk[i], hi[i]);
+#pragma unroll
+          for (int i = 0; i < PKP; ++i)
+            if (q0 + 32 * i < G) all = all && tag_ok(hi[i], tag);
+          if (spins >= spin_limit) { fail = true; break; }
+          if (!all) continue;
+#pragma unroll
+          for (int i = 0; i < PKP; ++i)
+            if (q0 + 32 * i < G) {
+              const long long k2 = (long long)kk[i];
+              const int l2 = (int)payload(hi[i]);
+              if (k2 > key || (k2 == key && l2 < label)) { key = k2; label = l2; own = q0 + 32 * i; }
+            }
+          break;
         }
         if (fail) break;
       }
-      const long long lk = key;
-      const int ll = label;
-      warp_ikey(key, label);
-      const unsigned win = __ballot_sync(0xffffffffu, lk == key && ll == label);
-      own = __shfl_sync(0xffffffffu, own, __ffs(win) - 1);
       fail = __any_sync(0xffffffffu, fail);
+      const int wl = warp_best(key, label);
+      key = __shfl_sync(0xffffffffu, key, wl);
+      label = __shfl_sync(0xffffffffu, label, wl);
+      own = __shfl_sync(0xffffffffu, own, wl);
       // --- the winner's row: U(k, :), and 1/|pivot| meanwhile ---
       T v = (T)0, ra = (T)0;
       if (!fail) {
@@ -375,6 +420,7 @@ panel_kernel(T* A, long long lda, int m, int r0, int c0, int w, int rpc, int* ip
           if (lane < w) ld_tagged2(vq + 2 * lane, a0, a1);
           const unsigned long long kb = (unsigned long long)key;
           if (kb - 1ULL < 0x7FEFFFFFFFFFFFFFULL) ra = recip_bits(kb);
+          asm volatile("" ::"d"(ra));  // (here, not after the row's arrival)
           if (tag_ok(a0, tag) && tag_ok(a1, tag)) v = __longlong_as_double((long long)join(a0, a1));
           else if (lane < w && !ld_value<T>(vq, lane, tag, v, spin_limit)) fail = true;
         } else {
@@ -388,26 +434,28 @@ panel_kernel(T* A, long long lda, int m, int r0, int c0, int w, int rpc, int* ip
           s_fail = 1;
         }
       } else {
-        if (k > 0) {
-          const T l = __shfl_sync(0xffffffffu, v, k - 1);
-          if (lane > k && lane < w) v = fma(-l, s_U[par ^ 1][lane], v);
-        }
         if (lane < w) s_U[par][lane] = v;
         if (lane == k) {  // ONE/GMAX (pdgetf2.f:224)
+          // (its zero test and sign on the integer pipe, see recip_bits)
           T rinv;
+          bool zero;
           if constexpr (sizeof(T) == 8) {
-            const unsigned long long kb = (unsigned long long)key;
-            rinv = (kb - 1ULL < 0x7FEFFFFFFFFFFFFFULL) ? (v < 0 ? -ra : ra) : (v != (T)0 ? (T)1 / v : (T)0);
+            const unsigned long long kb = (unsigned long long)key, vb = (unsigned long long)__double_as_longlong(v);
+            zero = (vb << 1) == 0;
+            if (kb - 1ULL < 0x7FEFFFFFFFFFFFFFULL)
+              rinv = __longlong_as_double(__double_as_longlong(ra) | (long long)(vb & (1ULL << 63)));
+            else
+              rinv = zero ? (T)1 : (T)1 / v;
           } else {
-            rinv = v != (T)0 ? (T)1 / v : (T)0;
+            zero = v == (T)0;
+            rinv = zero ? (T)1 : (T)1 / v;
           }
           s_rinv = rinv;
-          s_scale = v != (T)0;
           s_piv = label;
           s_own = own;
           if (b == 0) {
             ipiv[c0 + k] = r0 + label;
-            if (v == (T)0) atomicMin(info_col, c0 + k);
+            if (zero) atomicMin(info_col, c0 + k);
           }
         }
       }
@@ -418,32 +466,27 @@ panel_kernel(T* A, long long lda, int m, int r0, int c0, int w, int rpc, int* ip
     //     update (PDGER); the row's next-column entry gives its IDAMAX key for
     //     column k+1 ---
     if (!exch) {
-      const bool scale = s_scale != 0;
-      const T rinv = s_rinv;
+      const T rinv = s_rinv;  // 1 for a zero pivot: its column is not scaled
       const int piv = s_piv, mine = s_own == b ? lrow : -1;
       const int kn = k + 1;
-      const T un = kn < w ? s_U[par][kn] : (T)0;
+      const T un = s_U[par][kn < w ? kn : k];
       long long nkey = -2;
       int nlab = INT_MAX, nrow = 0;
-      for (int r = tid; r < nr; r += PTR) {
-        int lb = lab[r];
-        if (lb < 0) continue;
-        if (r == mine) {  // pivot row k
-          lab[r] = ~k;
-          continue;
-        }
-        if (lb == k) lab[r] = lb = piv;  // the diagonal row goes where the pivot row stood
+      for (int r = part == 0 ? row0 : nr; r < nr; r += rstep) {
+        // straight-line: all of a row's operands at once, stores where it counts
+        const int lb = lab[r];
         T l = tile[tix(r, k)];
-        if (scale) l *= rinv;
-        tile[tix(r, k)] = l;
-        if (kn < w) {
-          const T v = fma(-l, un, tile[tix(r, kn)]);
-          tile[tix(r, kn)] = v;
-          if (kn < kw) {
-            const long long k2 = row_key(v, lb, kn);
-            if (k2 > nkey || (k2 == nkey && lb < nlab)) { nkey = k2; nlab = lb; nrow = r; }
-          }
-        }
+        const T a = tile[tix(r, kn < w ? kn : k)];
+        l *= rinv;
+        const T v = fma(-l, un, a);
+        const bool act = lb >= 0 && r != mine;
+        const int ln = lb == k ? piv : lb;  // the diagonal row goes where the pivot row stood
+        if (act) tile[tix(r, k)] = l;
+        if (act && kn < w) tile[tix(r, kn)] = v;
+        if (r == mine) lab[r] = ~k;  // pivot row k
+        else if (lb == k) lab[r] = ln;
+        const long long k2 = act ? row_key(v, ln, kn) : -2LL;
+        if (k2 > nkey || (k2 == nkey && act && ln < nlab)) { nkey = k2; nlab = ln; nrow = r; }
       }
       if (kn < kw) put_candidate(nkey, nlab, nrow);
     }
@@ -452,6 +495,7 @@ panel_kernel(T* A, long long lda, int m, int r0, int c0, int w, int rpc, int* ip
   // fewer rows than columns), then every row to where its content stands
   if (exch) return;
   if (kw > 0) finish_update(kw - 1);
+  asm volatile("bar.sync 1, %0;" ::"n"(PTR) : "memory");
   for (int r = tid; r < nr; r += PTR) {
     const int lb = lab[r];
     T* dst = A + (long long)(r0 + (lb < 0 ? ~lb : lb)) + (long long)c0 * lda;
@@ -1142,7 +1186,8 @@ inline cudaError_t launch_panel(T* A, long long lda, int m, int r0, int c0, int 
   // Tall panels beyond 64 CTAs' shared memory spread over every SM instead;
   // beyond every SM's shared memory the rows go to the global buffer ws.ptile.
   const int rpc_max = (int)((200 * 1024) / (sizeof(T) * PLD)) & ~7;
-  int rpc = (R + panel_ctas() - 1) / panel_ctas();
+  const int ctas = std::min(panel_ctas(), PMAXG);
+  int rpc = (R + ctas - 1) / ctas;
   const int lo_rows = panel_min_rows() > 0 ? panel_min_rows() : (sizeof(T) == 4 ? 256 : 128);
   if (rpc < lo_rows) rpc = lo_rows;
   if (rpc > rpc_max) rpc = (R + num_sms() - 1) / num_sms();
@@ -1177,9 +1222,10 @@ inline cudaError_t launch_panel(T* A, long long lda, int m, int r0, int c0, int 
   }
   if (ws.cand_launches) id = ++*ws.cand_launches;
   uint32_t tag0 = id * 64u;
+  int tpr = global_tile || rpc > PTR / 4 ? 1 : (rpc > PTR / 8 ? 2 : 4);  // threads per row
   long long limit = spin_limit();
   void* args[] = {&A, &lda, &m, &r0, &c0, &w, (void*)&rpc, &ipiv, (void*)&ws.info_col,
-                  (void*)&ws.cand, (void*)&ws.status, (void*)&limit, (void*)&gtile, (void*)&tag0};
+                  (void*)&ws.cand, (void*)&ws.status, (void*)&limit, (void*)&gtile, (void*)&tag0, (void*)&tpr};
   count_launches(1);
   if (global_tile)
     return cudaLaunchCooperativeKernel((void*)panel_kernel<T, true>, dim3(G), dim3(PT), args, 0, s);

@@ -174,9 +174,9 @@ inline size_t kSolveInvDoubles(int n) {
 constexpr size_t kDinv64Doubles = (size_t)16 * 64 * 64;
 
 size_t panel_cand_doubles();
-// 8-byte words of the panel kernel's exchange area (2 x 224 x 4 key words, 224
-// CTAs x 2 parities x 64 row words); panel_cand_doubles() returns it.
-constexpr size_t kPanelCandDoubles = (size_t)8 * 224 + (size_t)224 * 2 * 2 * 32;
+// 8-byte words of the panel kernel's exchange area (2 x 160 x 160 16-byte keys,
+// 160 CTAs x 2 parities x 64 row words); panel_cand_doubles() returns it.
+constexpr size_t kPanelCandDoubles = (size_t)2 * 160 * 160 * 2 + (size_t)160 * 2 * 2 * 32;
 // Ints of a panel's interchange plan (count + 2 x 512 (row, src) pairs).
 constexpr size_t kSwapPlanInts = 1 + 4 * 256 + 15;
 // Largest M whose FP64 panel rows fit the SMs' shared memory on this device;
