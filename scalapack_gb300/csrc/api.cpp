@@ -179,6 +179,7 @@ void release_all() {
   cudaFree(g_dev.dA2); cudaFree(g_dev.dX); cudaFree(g_dev.drw); cudaFree(g_dev.drc);
   cudaFree(g_dev.dipiv2); cudaFree(g_dev.doz); cudaFree(g_dev.doz2); cudaFree(g_dev.ddinv64);
   cudaFree(g_dev.ddinvs);
+  cudaFree(g_dev.dchain64);
   cudaFree(g_dev.dptile);
   sl::splitk_scratch() = sl::SplitKScratch();
   if (g_dev.stream) cudaStreamDestroy(g_dev.stream);
@@ -244,6 +245,9 @@ sl::LuWork make_work() {
   w.swap_plan_alt = g_split_step ? g_dev.dplan + sl::kSwapPlanInts : nullptr;
   w.dinv_solve = g_dev.ddinvs;
   w.dinv_solve_len = g_dev.ddinvs ? g_dev.capDinvs : 0;
+  w.chain = g_dev.dchain64;
+  w.chain_values = g_dev.dchain64 ? (g_dev.capChain64 - 16) / 4 : 0;
+  w.chain_epoch = &g_dev.chain64_epoch;
   w.ptile = g_dev.dptile;
   w.ptile_len = g_dev.dptile ? g_dev.capPtile : 0;
   if (g_lookahead) {
@@ -264,6 +268,11 @@ cudaError_t ensure_solve_ws(int n, int nrhs) {
     // without them the substitution solves run)
     ensure_oz(n, nrhs, 128);
     if (grow(&g_dev.ddinvs, &g_dev.capDinvs, sl::kSolveInvDoubles(n)) != cudaSuccess) cudaGetLastError();
+    if (nrhs <= sl::kChainRhs) {
+      const int* old = g_dev.dchain64;
+      if (grow(&g_dev.dchain64, &g_dev.capChain64, 16 + 4 * (size_t)n * nrhs) != cudaSuccess) cudaGetLastError();
+      else if (g_dev.dchain64 != old) g_dev.chain64_epoch = 0;  // new words: cleared before their first use
+    }
   }
   return cudaSuccess;
 }
@@ -451,9 +460,11 @@ static int solve_host(char trans, int n, int nrhs, long long ldda, double* B, in
   if (e != cudaSuccess) return cuda_info(e);
   e = cudaMemcpy2DAsync(hb, lldb * sizeof(double), g_dev.dB, lddb * sizeof(double),
                         (size_t)n * sizeof(double), nrhs, cudaMemcpyDeviceToHost, s);
+  int st = 0;
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&st, g_dev.dsmall + 2, sizeof(int), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return cuda_info(e);
-  return 0;
+  return st ? -20000 - st : 0;
 }
 
 void pdgetrs_(const char* TRANS, const int* N, const int* NRHS, const double* A, const int* IA,
@@ -677,9 +688,11 @@ int sl1x1_dgetrs_dev(char trans, int n, int nrhs, const double* dA, long long ld
   if (e != cudaSuccess) return cuda_info(e);
   sl::LuWork w = make_work();
   e = sl::dgetrs_device(trans, n, nrhs, dA, ldda, g_dev.dipiv, dB, lddb, w, s);
+  int st = 0;
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&st, g_dev.dsmall + 2, sizeof(int), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return cuda_info(e);
-  return 0;
+  return st ? -20000 - st : 0;
 }
 
 int sl1x1_dgesv_dev(int n, int nrhs, double* dA, long long ldda, int* dipiv, double* dB,

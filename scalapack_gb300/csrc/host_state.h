@@ -61,6 +61,8 @@ struct DevState {
   double* dptile = nullptr; size_t capPtile = 0;  // rows of panels taller than shared memory holds
   double* ddinvs = nullptr; size_t capDinvs = 0;      // solve: inverses of the diagonal blocks
   int chain_epoch = 0;
+  int* dchain64 = nullptr; size_t capChain64 = 0;  // FP64 chained solves: tickets, then solution words
+  unsigned chain64_epoch = 0;
   unsigned short* dA16 = nullptr; size_t capA16 = 0;
   unsigned short* dB16 = nullptr; size_t capB16 = 0;
   int* dcolexp = nullptr; size_t capCe = 0;

@@ -86,22 +86,25 @@ cudaError_t ipiv_shift(const int* src, int* dst, int n, int delta, cudaStream_t 
 // are compared, never used as addresses, so any IPIV is safe. The walk is the
 // same for every thread of a warp (broadcast reads of one pivot at a time),
 // from shared memory when n*4 bytes fit in 192 KB.
-__global__ void __launch_bounds__(256)
-perm_compose_kernel(const int* __restrict__ ipiv, int n, int* perm, int use_smem) {
-  extern __shared__ int sp[];
+__device__ __forceinline__ void perm_compose_rows(int i, const int* __restrict__ ipiv, int n, int* perm,
+                                                  int* sp) {
   const int* pv = ipiv;
-  if (use_smem) {
+  if (sp) {
     for (int j = threadIdx.x; j < n; j += blockDim.x) sp[j] = ipiv[j];
     __syncthreads();
     pv = sp;
   }
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
   int q = i;
   for (int j = n - 1; j >= 0; --j) {
     const int p = pv[j];
     q = (q == j) ? p : ((q == p) ? j : q);
   }
   if (i < n) perm[i] = q;
+}
+__global__ void __launch_bounds__(256)
+perm_compose_kernel(const int* __restrict__ ipiv, int n, int* perm, int use_smem) {
+  extern __shared__ int sp[];
+  perm_compose_rows(blockIdx.x * blockDim.x + threadIdx.x, ipiv, n, perm, use_smem ? sp : nullptr);
 }
 
 cudaError_t perm_compose(const int* dipiv, int n, int* perm, cudaStream_t s) {
@@ -636,13 +639,12 @@ cudaError_t gemm_update<double>(bool transa, int m, int n, int k, double alpha, 
 // D + b*4096, column-major with leading dimension 64 (D[c*64 + r] =
 // inv(T_bb)(r, c)); a partial last block is padded with the identity.
 template <bool LOWER>
-__global__ void __launch_bounds__(256)
-tri_inv64_kernel(int n, const double* __restrict__ A, long long lda, double* D) {
-  extern __shared__ double inv_smem[];  // Ts[64][65], X[64][65], rdiag[64]
+__device__ __forceinline__ void tri_inv64_of(int b, int n, const double* __restrict__ A, long long lda,
+                                             double* D, double* inv_smem) {
+  // inv_smem: Ts[64][65], X[64][65], rdiag[64]
   double(*Ts)[65] = reinterpret_cast<double(*)[65]>(inv_smem);
   double(*X)[65] = reinterpret_cast<double(*)[65]>(inv_smem + 64 * 65);
   double* rd = inv_smem + 2 * 64 * 65;
-  const int b = blockIdx.x;
   const int r0 = b * 64, rb = min(64, n - r0);
   for (int idx = threadIdx.x; idx < 64 * 64; idx += 256) {
     const int r = idx & 63, c = idx >> 6;
@@ -660,6 +662,26 @@ tri_inv64_kernel(int n, const double* __restrict__ A, long long lda, double* D) 
     const int r = idx & 63, c = idx >> 6;
     Db[c * 64 + r] = X[r][c];
   }
+}
+
+// Everything a solve needs before its first step, in one launch: blocks
+// [0, nb64) invert L's diagonal blocks into D, [nb64, 2 nb64) U's behind them;
+// the rest compose the pivots into the row permutation (perm_compose_rows);
+// the status word and the tickets of the chained solve are reset.
+constexpr int kInvSmem = (2 * 64 * 65 + 64) * (int)sizeof(double);
+__global__ void __launch_bounds__(256)
+solve_prep_kernel(int n, const double* __restrict__ A, long long lda, double* D,
+                  const int* __restrict__ ipiv, int* perm, int* status, int* tickets) {
+  extern __shared__ double inv_smem[];
+  const int nb64 = (n + 63) / 64, b = blockIdx.x;
+  if (b == 0 && threadIdx.x == 0) {
+    *status = 0;
+    if (tickets) tickets[0] = tickets[1] = 0;
+  }
+  if (b < nb64) tri_inv64_of<true>(b, n, A, lda, D, inv_smem);
+  else if (b < 2 * nb64) tri_inv64_of<false>(b - nb64, n, A, lda, D + (size_t)nb64 * 4096, inv_smem);
+  else perm_compose_rows((b - 2 * nb64) * 256 + threadIdx.x, ipiv, n, perm,
+                         (size_t)n * sizeof(int) <= (size_t)kInvSmem ? reinterpret_cast<int*>(inv_smem) : nullptr);
 }
 
 // Balancing keys of the blocked NOTRAN solve's sliced products, once per
@@ -843,32 +865,58 @@ cudaError_t dgetrs_device(char trans, int n, int nrhs, const double* dA, long lo
   if (n <= 0 || nrhs <= 0) return cudaSuccess;
   const bool notran = (trans == 'N' || trans == 'n');
   phase_begin(kPhSolve, s);
-  SL_TRY(perm_compose(dipiv, n, ws.perm, s));
   double* X = ws.bswap;  // n x nrhs, ld = n
   // any NRHS whose products fit the scratch (PDGETRI solves with NRHS = N)
   const bool inv_path = g_f64_update == 1 && ws.dinv_solve && ws.dinv_solve_len >= kSolveInvDoubles(n) &&
                         oz_fits(ws.oz, n, nrhs, 128);
+  // up to 16 right-hand sides go through the chained solves, both TRANS: at
+  // n = 16384, 16 columns they take 9 ms (the blocked solve 13.6), below that
+  // 2 to 6 times less; beyond 16 the FP64 pipe's n^2 nrhs bound passes the
+  // blocked NOTRAN solve, whose products run on the tensor cores
+  const bool chain_path = g_f64_update == 1 && nrhs <= kChainRhs && ws.dinv_solve &&
+                          ws.dinv_solve_len >= kSolveInvDoubles(n) && ws.chain && ws.chain_epoch &&
+                          ws.chain_values >= (size_t)n * nrhs;
+  if (notran ? (inv_path || chain_path) : chain_path) {
+    static const cudaError_t a0 = cudaFuncSetAttribute(
+        solve_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kInvSmem);
+    SL_TRY(a0);
+    solve_prep_kernel<<<2 * ((n + 63) / 64) + (n + 255) / 256, 256, kInvSmem, s>>>(
+        n, dA, ldda, ws.dinv_solve, dipiv, ws.perm, ws.status, chain_path ? ws.chain : nullptr);
+    count_launches(1);
+    SL_TRY(cudaGetLastError());
+  } else {
+    SL_TRY(cudaMemsetAsync(ws.status, 0, sizeof(int), s));
+    SL_TRY(perm_compose(dipiv, n, ws.perm, s));
+  }
+  if (chain_path) {
+    // L then U (N), or U^T then L^T (T): the pivots' permutation is applied as
+    // the first triangle reads B, or as the second one writes it
+    unsigned long long* words = reinterpret_cast<unsigned long long*>(ws.chain + 16);
+    if (*ws.chain_epoch == 0 || *ws.chain_epoch > UINT_MAX - 2) {
+      SL_TRY(cudaMemsetAsync(words, 0, ws.chain_values * 16, s));
+      *ws.chain_epoch = 0;
+    }
+    const size_t ub = (size_t)((n + 63) / 64) * 4096;
+    const unsigned e1 = ++*ws.chain_epoch, e2 = ++*ws.chain_epoch;
+    SL_TRY(trsv64_chain(notran, !notran, dA, ldda, n, ws.dinv_solve + (notran ? 0 : ub), dB, lddb,
+                        notran ? ws.perm : nullptr, X, n, nullptr, nrhs, ws.chain, words, e1, ws.status, s));
+    SL_TRY(trsv64_chain(!notran, !notran, dA, ldda, n, ws.dinv_solve + (notran ? ub : 0), X, n, nullptr, dB,
+                        lddb, notran ? nullptr : ws.perm, nrhs, ws.chain + 1, words, e2, ws.status, s));
+    phase_end(kPhSolve, s, 2.0 * (double)n * n * nrhs, 8.0 * ((double)n * n + 4.0 * (double)n * nrhs));
+    return cudaSuccess;
+  }
   if (notran && inv_path) {
     SL_TRY((permute_rows<double, double>(dB, lddb, X, n, ws.perm, n, nrhs, 0, s)));
     const int nb64 = (n + 63) / 64;
-    constexpr int kInvSmem = (2 * 64 * 65 + 64) * (int)sizeof(double);
-    static const cudaError_t a0 = cudaFuncSetAttribute(
-        tri_inv64_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kInvSmem);
-    static const cudaError_t a1 = cudaFuncSetAttribute(
-        tri_inv64_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kInvSmem);
     static const cudaError_t a2 = cudaFuncSetAttribute(
         solve_block128_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBlkSmem);
     static const cudaError_t a3 = cudaFuncSetAttribute(
         solve_block128_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBlkSmem);
-    SL_TRY(a0);
-    SL_TRY(a1);
     SL_TRY(a2);
     SL_TRY(a3);
-    tri_inv64_kernel<true><<<nb64, 256, kInvSmem, s>>>(n, dA, ldda, ws.dinv_solve);
-    tri_inv64_kernel<false><<<nb64, 256, kInvSmem, s>>>(n, dA, ldda, ws.dinv_solve + (size_t)nb64 * 4096);
     solve_ckeys_kernel<<<(n + 7) / 8, 256, 0, s>>>(
         n, dA, ldda, reinterpret_cast<unsigned*>(ws.dinv_solve + (size_t)2 * nb64 * 4096), nb64 * 64);
-    count_launches(3);
+    count_launches(1);
     SL_TRY(cudaGetLastError());
     SL_TRY(tri_solve_inv(true, n, nrhs, dA, ldda, X, n, ws, s));
     SL_TRY(tri_solve_inv(false, n, nrhs, dA, ldda, X, n, ws, s));

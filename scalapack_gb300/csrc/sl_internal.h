@@ -4,6 +4,7 @@
 
 #include <functional>
 #include <stddef.h>
+#include <stdint.h>
 
 #ifndef SL_TRY
 #define SL_TRY(x)                     \
@@ -134,6 +135,12 @@ struct LuWork {
   // (kSolveInvDoubles(n) doubles), or null for the substitution solves.
   double* dinv_solve = nullptr;
   size_t dinv_solve_len = 0;
+  // Solve with few right-hand sides: published solution words (two per value,
+  // after 16 ints of tickets) and their epoch (host counter; the words start
+  // zeroed), or null for the blocked solves.
+  int* chain = nullptr;
+  size_t chain_values = 0;  // values the words hold
+  unsigned* chain_epoch = nullptr;
   // Columns still arriving (ncol_chunks = 0: all of A is in place). Chunk c
   // holds columns [c ? col_end[c-1] : 0, col_end[c]) and is in place once
   // ev_cols[c] has completed; step 0 of the factorization follows the chunks
@@ -221,6 +228,18 @@ cudaError_t dgetrf_device(int m, int n, double* dA, long long ldda, int* dipiv, 
 cudaError_t dgetrs_device(char trans, int n, int nrhs, const double* dA, long long ldda,
                           const int* dipiv, double* dB, long long lddb, const LuWork& ws,
                           cudaStream_t s);
+
+// Most right-hand sides of a chained solve.
+constexpr int kChainRhs = 16;
+// op(T) X = S with the lower (unit) or upper triangle of n x n LU factors in
+// one launch (trsv_f64.cu): D holds the inverses of that triangle's 64x64
+// diagonal blocks; S(i, c) = src[gather[i] + c lds], X(i, c) goes to
+// dst[scatter[i] + c ldd] (null: i). ticket is zero on entry; words holds two
+// per value and no word of this epoch.
+cudaError_t trsv64_chain(bool lower, bool trans, const double* A, long long lda, int n, const double* D,
+                         const double* src, long long lds, const int* gather, double* dst,
+                         long long ldd, const int* scatter, int nrhs, int* ticket,
+                         unsigned long long* words, uint32_t epoch, int* status, cudaStream_t s);
 
 // ---- low-precision trailing update (mixed_gemm.cu) ----
 // Pack L21 (m x k FP32 col-major) and U12 (k x n FP32 col-major, per-column

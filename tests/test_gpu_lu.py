@@ -333,3 +333,31 @@ def test_scratch_on_reused_dirty_memory(sl, orc, ctx, n, nb):
     assert sl.dgetrf_dev(n, n, dA.data_ptr(), n, dpiv.data_ptr(), nb) == 0
     LU = np.asfortranarray(dA.cpu().numpy().T)
     assert orc.fresid(LU, dpiv.cpu().numpy(), A0) < RESID_THRESH
+
+
+@pytest.mark.parametrize("trans", ["N", "T"])
+@pytest.mark.parametrize("n,nrhs", [(1, 1), (63, 2), (64, 1), (65, 16), (129, 3), (200, 17), (1300, 16), (2500, 5)])
+def test_chained_solve_edges(sl, gpu_required, n, nrhs, trans):
+    """PDGETRS over the edges of the chained solve: blocks of 64 rows, one or two
+    right-hand sides per CTA (1300 x 16, 2500 x 5), the blocked solves beyond
+    16; padded leading dimensions, untouched padding."""
+    import torch
+
+    rng = np.random.default_rng(n + nrhs)
+    A = rng.uniform(-0.5, 0.5, (n, n))
+    B = rng.uniform(-0.5, 0.5, (n, nrhs))
+    lda, ldb = n + 3, n + 1
+    dA = torch.full((n, lda), -9923.0, dtype=torch.float64, device="cuda")
+    dB = torch.full((nrhs, ldb), -9923.0, dtype=torch.float64, device="cuda")
+    dA[:, :n] = torch.from_numpy(A.T.copy())
+    dB[:, :n] = torch.from_numpy(B.T.copy())
+    ip = torch.zeros(n, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    assert sl.dgetrf_dev(n, n, dA.data_ptr(), lda, ip.data_ptr(), 64) == 0
+    assert sl.dgetrs_dev(trans, n, nrhs, dA.data_ptr(), lda, ip.data_ptr(), dB.data_ptr(), ldb) == 0
+    X = dB[:, :n].T.cpu().numpy()
+    assert (dB[:, n:] == -9923.0).all()
+    op = A if trans == "N" else A.T
+    res = np.abs(B - op @ X).max(axis=0)
+    scale = np.abs(op).sum(axis=1).max() * np.abs(X).max(axis=0) * n * 2.0**-53
+    assert (res / scale < 16.0).all()  # the tester's bound
