@@ -259,7 +259,7 @@ sl::LuWork make_work() {
 }
 
 cudaError_t ensure_solve_ws(int n, int nrhs) {
-  cudaError_t e = grow(&g_dev.dperm, &g_dev.capPerm, (size_t)n);
+  cudaError_t e = grow(&g_dev.dperm, &g_dev.capPerm, sl::perm_ints(n));
   if (e != cudaSuccess) return e;
   e = grow(&g_dev.dbswap, &g_dev.capBs, (size_t)n * (size_t)nrhs);
   if (e != cudaSuccess) return e;
@@ -761,7 +761,7 @@ int sl1x1_dgesv_ir_dev(int n, int nrhs, double* dA, long long ldda, int* dipiv, 
   GROW(dA16, capA16, (size_t)n * kpad);
   GROW(dB16, capB16, (size_t)n * kpad);
   GROW(dcolexp, capCe, n);
-  GROW(dpermx, capPermx, n);
+  GROW(dpermx, capPermx, sl::perm_ints(n));
   GROW(dR, capR, (size_t)n * nrhs);
   GROW(dD, capD, n);
   GROW(dXf, capXf, (size_t)n * nrhs);
@@ -771,7 +771,7 @@ int sl1x1_dgesv_ir_dev(int n, int nrhs, double* dA, long long ldda, int* dipiv, 
   GROW(dw, capW, n);
   GROW(dAx, capAx, n);
   GROW(dh, capH, m1 + 8);
-  GROW(dperm, capPerm, n);
+  GROW(dperm, capPerm, sl::perm_ints(n));
   GROW(dbswap, capBs, (size_t)n * nrhs);
   if (keep_a) GROW(dAcopy, capAcopy, (size_t)ldf * n);
   GROW(dsplitk, capSplitk, (size_t)32 * 4 * n);  // split-K partials of the FP64 products

@@ -80,42 +80,56 @@ cudaError_t ipiv_shift(const int* src, int* dst, int n, int delta, cudaStream_t 
 }
 
 // Composed row permutation of the n sequential interchanges j <-> ipiv[j]:
-// perm[i] = original row that ends in row i. Thread i walks the interchanges
-// backwards from the last, following the row whose content ends in row i
-// (interchange j moves it from ipiv[j] to j or from j to ipiv[j]); the pivots
-// are compared, never used as addresses, so any IPIV is safe. The walk is the
-// same for every thread of a warp (broadcast reads of one pivot at a time),
-// from shared memory when n*4 bytes fit in 192 KB.
-__device__ __forceinline__ void perm_compose_rows(int i, const int* __restrict__ ipiv, int n, int* perm,
-                                                  int* sp) {
-  const int* pv = ipiv;
-  if (sp) {
-    for (int j = threadIdx.x; j < n; j += blockDim.x) sp[j] = ipiv[j];
+// perm[i] = original row that ends in row i. The interchanges are cut into at
+// most kPermSegs segments; per segment, thread i walks its interchanges backwards
+// from the last, following the row whose content ends in row i (interchange j
+// moves it from ipiv[j] to j or from j to ipiv[j]), and rows then pass through
+// the segments' maps from the last to the first (follow_perm). One walk of all n
+// interchanges per row is a chain of two compares and selects each, 150 us at n =
+// 8192; in 16 segments, on all SMs, the launch that also inverts the diagonal
+// blocks takes 62. The pivots are
+// compared, never used as addresses: a row label outside the matrix (from an
+// invalid IPIV) is followed by walking the segment itself. A block does 256 rows
+// of one segment, from shared memory (sp, kPermSmem ints) when it fits.
+constexpr int kPermSmem = 8192;
+__device__ __forceinline__ int walk_pivots(const int* pv, int lo, int hi, int q) {
+#pragma unroll 4
+  for (int j = hi - 1; j >= lo; --j) {
+    const int p = pv[j - lo];
+    q = (q == j) ? p : ((q == p) ? j : q);
+  }
+  return q;
+}
+__device__ __forceinline__ void perm_segment(int block, const int* __restrict__ ipiv, int n, int* maps,
+                                             int* sp) {
+  const int len = perm_seg_len(n), nrb = (n + 255) / 256;
+  const int sgm = block / nrb, i = (block % nrb) * 256 + threadIdx.x;
+  const int lo = sgm * len, hi = min(n, lo + len);
+  const int* pv = ipiv + lo;
+  if (len <= kPermSmem) {
+    for (int j = threadIdx.x; j < hi - lo; j += 256) sp[j] = pv[j];
     __syncthreads();
     pv = sp;
   }
-  int q = i;
-  for (int j = n - 1; j >= 0; --j) {
-    const int p = pv[j];
-    q = (q == j) ? p : ((q == p) ? j : q);
-  }
-  if (i < n) perm[i] = q;
+  const int q = walk_pivots(pv, lo, hi, i);
+  if (i < n) maps[(size_t)sgm * n + i] = q;
+}
+__global__ void __launch_bounds__(256) perm_segments_kernel(const int* __restrict__ ipiv, int n, int* maps) {
+  __shared__ int sp[kPermSmem];
+  perm_segment(blockIdx.x, ipiv, n, maps, sp);
 }
 __global__ void __launch_bounds__(256)
-perm_compose_kernel(const int* __restrict__ ipiv, int n, int* perm, int use_smem) {
-  extern __shared__ int sp[];
-  perm_compose_rows(blockIdx.x * blockDim.x + threadIdx.x, ipiv, n, perm, use_smem ? sp : nullptr);
+perm_finish_kernel(const int* __restrict__ ipiv, int n, const int* __restrict__ maps, int* perm) {
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i < n) perm[i] = follow_perm(i, ipiv, n, maps);
 }
 
 cudaError_t perm_compose(const int* dipiv, int n, int* perm, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  const size_t smem = sizeof(int) * (size_t)n;
-  const int use_smem = smem <= 192 * 1024 ? 1 : 0;
-  static const cudaError_t attr = cudaFuncSetAttribute(
-      perm_compose_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 192 * 1024);
-  SL_TRY(attr);
-  perm_compose_kernel<<<(n + 255) / 256, 256, use_smem ? smem : 0, s>>>(dipiv, n, perm, use_smem);
-  count_launches(1);
+  const int nrb = (n + 255) / 256;
+  perm_segments_kernel<<<nrb * perm_segs(n), 256, 0, s>>>(dipiv, n, perm + n);
+  perm_finish_kernel<<<nrb, 256, 0, s>>>(dipiv, n, perm + n, perm);
+  count_launches(2);
   return cudaGetLastError();
 }
 
@@ -163,31 +177,18 @@ static cudaError_t lu_update(const OzScratch& sc, int m, int n, int k, double al
   return dgemm(false, m, n, k, alpha, A, lda, B, ldb, 1.0, C, ldc, s);
 }
 
-// Inverse of a 64x64 triangular block by column-oriented substitution, all
-// columns at once: X = I, then for each pivot row q in solve order, row q of
-// X is final (divided by T(q,q) for a non-unit upper T) and every later row
-// i loses T(i,q) X(q,:). 256 threads own 16 entries of X each, one shared
-// barrier per step: 64 steps instead of a 2000-long dependent chain.
+// Inverse of a 64x64 unit-lower block by column-oriented substitution, all
+// columns at once: X = I, then for each pivot row q, row q of X is final and
+// every later row i loses T(i,q) X(q,:). 256 threads own 16 entries of X each,
+// one shared barrier per step: 64 steps instead of a 2000-long dependent chain.
 // Ts and X are 64 x 65 shared arrays; returns with X = inv(T).
-template <bool LOWER>
-__device__ __forceinline__ void tri_inv64_block(double (*Ts)[65], double (*X)[65], double* rd) {
+__device__ __forceinline__ void unit_lower_inv64_block(double (*Ts)[65], double (*X)[65]) {
   const int t = threadIdx.x & 63, ib = threadIdx.x >> 6;  // column t, rows ib, ib+4, ...
-  if (LOWER) {
-    for (int q = 0; q < 63; ++q) {
-      const double xq = X[q][t];
-      if (t <= q)
-        for (int i = q + 1 + ((ib - (q + 1)) & 3); i < 64; i += 4) X[i][t] = fma(-Ts[i][q], xq, X[i][t]);
-      __syncthreads();
-    }
-  } else {
-    for (int q = 63; q >= 0; --q) {
-      if (threadIdx.x < 64 && t >= q) X[q][t] *= rd[q];
-      __syncthreads();
-      const double xq = X[q][t];
-      if (t >= q)
-        for (int i = ib; i < q; i += 4) X[i][t] = fma(-Ts[i][q], xq, X[i][t]);
-      __syncthreads();
-    }
+  for (int q = 0; q < 63; ++q) {
+    const double xq = X[q][t];
+    if (t <= q)
+      for (int i = q + 1 + ((ib - (q + 1)) & 3); i < 64; i += 4) X[i][t] = fma(-Ts[i][q], xq, X[i][t]);
+    __syncthreads();
   }
 }
 
@@ -208,7 +209,7 @@ unit_lower_inv64_kernel(int jb, const double* __restrict__ L, long long ldl, dou
     X[r][c] = (r == c) ? 1.0 : 0.0;
   }
   __syncthreads();
-  tri_inv64_block<true>(Ls, X, nullptr);
+  unit_lower_inv64_block(Ls, X);
   double* Nb = Ninv + (size_t)b * 4096;
   for (int idx = threadIdx.x; idx < 64 * 64; idx += 256) {
     const int i = idx & 63, c = idx >> 6;
@@ -634,54 +635,91 @@ cudaError_t gemm_update<double>(bool transa, int m, int n, int k, double alpha, 
   return dgemm(transa, m, n, k, alpha, A, lda, B, ldb, 1.0, C, ldc, s);
 }
 
-// Inverses of the 64x64 diagonal blocks of the unit-lower L (LOWER) or the
-// non-unit upper U of an n x n LU factor, for the blocked solves: block b at
-// D + b*4096, column-major with leading dimension 64 (D[c*64 + r] =
-// inv(T_bb)(r, c)); a partial last block is padded with the identity.
+// Columns part, part + 4, ... of the inverse of a 64x64 diagonal block of the
+// unit-lower L (LOWER) or the non-unit upper U of an n x n LU factor, for the
+// blocked solves: block b at D + b*4096, column-major with leading dimension 64
+// (D[c*64 + r] = inv(T_bb)(r, c)); a partial last block is padded with the
+// identity. A warp per column: lane l owns rows l and l + 32, x_q is passed by a
+// shuffle, in the order of a substitution. U's rows are divided by their
+// diagonal beforehand, so that both triangles are unit ones. The four parts of a
+// block are four CTAs: the FP64 unit of an SM takes 20 cycles per warp
+// instruction whatever lanes are active, and a column of the inverse costs 32
+// to 96 of them (one CTA per block and a barrier per row: 54 us for one block, 11
+// with four).
+constexpr int kInvSmem = (64 * 64 + 64) * (int)sizeof(double);
+constexpr int kInvParts = 4;
 template <bool LOWER>
-__device__ __forceinline__ void tri_inv64_of(int b, int n, const double* __restrict__ A, long long lda,
-                                             double* D, double* inv_smem) {
-  // inv_smem: Ts[64][65], X[64][65], rdiag[64]
-  double(*Ts)[65] = reinterpret_cast<double(*)[65]>(inv_smem);
-  double(*X)[65] = reinterpret_cast<double(*)[65]>(inv_smem + 64 * 65);
-  double* rd = inv_smem + 2 * 64 * 65;
+__device__ __forceinline__ void tri_inv64_of(int b, int part, int n, const double* __restrict__ A,
+                                             long long lda, double* D, double* inv_smem) {
+  double* Ts = inv_smem;  // Ts[q*64 + i] = T(i, q), zero outside the strict triangle
+  double* rd = inv_smem + 64 * 64;
   const int r0 = b * 64, rb = min(64, n - r0);
-  for (int idx = threadIdx.x; idx < 64 * 64; idx += 256) {
-    const int r = idx & 63, c = idx >> 6;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (!LOWER) {
+    if (tid < 64) rd[tid] = tid < rb ? 1.0 / A[(r0 + tid) + (long long)(r0 + tid) * lda] : 1.0;
+    __syncthreads();
+  }
+#pragma unroll 8
+  for (int idx = tid; idx < 64 * 64; idx += 256) {
+    const int i = idx & 63, q = idx >> 6;
     double v = 0.0;
-    if (r < rb && c < rb && (LOWER ? c < r : c >= r)) v = A[(r0 + r) + (long long)(r0 + c) * lda];
-    Ts[r][c] = v;
-    X[r][c] = (r == c) ? 1.0 : 0.0;
+    if (i < rb && q < rb && (LOWER ? q < i : q > i)) {
+      v = A[(r0 + i) + (long long)(r0 + q) * lda];
+      if (!LOWER) v *= rd[i];
+    }
+    Ts[idx] = v;
   }
   __syncthreads();
-  if (!LOWER && threadIdx.x < 64) rd[threadIdx.x] = (threadIdx.x < rb) ? 1.0 / Ts[threadIdx.x][threadIdx.x] : 1.0;
-  __syncthreads();
-  tri_inv64_block<LOWER>(Ts, X, rd);
   double* Db = D + (size_t)b * 4096;
-  for (int idx = threadIdx.x; idx < 64 * 64; idx += 256) {
-    const int r = idx & 63, c = idx >> 6;
-    Db[c * 64 + r] = X[r][c];
+  for (int h = 0; h < 2; ++h) {
+    const int c = part + kInvParts * (h ? 15 - warp : warp);  // a long column and a short one
+    const double d = LOWER ? 1.0 : rd[c];
+    double x0 = lane == c ? d : 0.0, x1 = lane + 32 == c ? d : 0.0;
+    if (LOWER) {
+      for (int q = c; q < 32; ++q) {
+        const double xq = __shfl_sync(0xffffffffu, x0, q);
+        if (lane > q) x0 = fma(-Ts[q * 64 + lane], xq, x0);
+        x1 = fma(-Ts[q * 64 + lane + 32], xq, x1);
+      }
+      for (int q = c > 32 ? c : 32; q < 63; ++q) {
+        const double xq = __shfl_sync(0xffffffffu, x1, q - 32);
+        if (lane + 32 > q) x1 = fma(-Ts[q * 64 + lane + 32], xq, x1);
+      }
+    } else {
+      for (int q = c; q >= 32; --q) {
+        const double xq = __shfl_sync(0xffffffffu, x1, q - 32);
+        if (lane + 32 < q) x1 = fma(-Ts[q * 64 + lane + 32], xq, x1);
+        x0 = fma(-Ts[q * 64 + lane], xq, x0);
+      }
+      for (int q = c < 31 ? c : 31; q > 0; --q) {
+        const double xq = __shfl_sync(0xffffffffu, x0, q);
+        if (lane < q) x0 = fma(-Ts[q * 64 + lane], xq, x0);
+      }
+    }
+    Db[c * 64 + lane] = x0;
+    Db[c * 64 + lane + 32] = x1;
   }
 }
 
-// Everything a solve needs before its first step, in one launch: blocks
-// [0, nb64) invert L's diagonal blocks into D, [nb64, 2 nb64) U's behind them;
-// the rest compose the pivots into the row permutation (perm_compose_rows);
-// the status word and the tickets of the chained solve are reset.
-constexpr int kInvSmem = (2 * 64 * 65 + 64) * (int)sizeof(double);
+// Everything a solve needs before its first step, in one launch: the first
+// blocks make the segment maps of the pivots' row permutation (perm_segment), the
+// next kInvParts * nb64 invert L's diagonal blocks into D, as many more U's
+// behind them; the status word and the tickets of the chained solve are reset.
 __global__ void __launch_bounds__(256)
 solve_prep_kernel(int n, const double* __restrict__ A, long long lda, double* D,
-                  const int* __restrict__ ipiv, int* perm, int* status, int* tickets) {
+                  const int* __restrict__ ipiv, int* maps, int* status, int* tickets) {
   extern __shared__ double inv_smem[];
-  const int nb64 = (n + 63) / 64, b = blockIdx.x;
-  if (b == 0 && threadIdx.x == 0) {
+  static_assert(kPermSmem * sizeof(int) <= (size_t)kInvSmem, "pivots of a segment");
+  const int nb64 = (n + 63) / 64, nperm = (n + 255) / 256 * perm_segs(n);
+  const int b = (int)blockIdx.x - nperm, part = b % kInvParts, blk = b / kInvParts;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
     *status = 0;
     if (tickets) tickets[0] = tickets[1] = 0;
   }
-  if (b < nb64) tri_inv64_of<true>(b, n, A, lda, D, inv_smem);
-  else if (b < 2 * nb64) tri_inv64_of<false>(b - nb64, n, A, lda, D + (size_t)nb64 * 4096, inv_smem);
-  else perm_compose_rows((b - 2 * nb64) * 256 + threadIdx.x, ipiv, n, perm,
-                         (size_t)n * sizeof(int) <= (size_t)kInvSmem ? reinterpret_cast<int*>(inv_smem) : nullptr);
+  if (b < 0)
+    perm_segment(blockIdx.x, ipiv, n, maps, reinterpret_cast<int*>(inv_smem));
+  else if (blk < nb64) tri_inv64_of<true>(blk, part, n, A, lda, D, inv_smem);
+  else tri_inv64_of<false>(blk - nb64, part, n, A, lda, D + (size_t)nb64 * 4096, inv_smem);
 }
 
 // Balancing keys of the blocked NOTRAN solve's sliced products, once per
@@ -870,7 +908,7 @@ cudaError_t dgetrs_device(char trans, int n, int nrhs, const double* dA, long lo
   const bool inv_path = g_f64_update == 1 && ws.dinv_solve && ws.dinv_solve_len >= kSolveInvDoubles(n) &&
                         oz_fits(ws.oz, n, nrhs, 128);
   // up to 16 right-hand sides go through the chained solves, both TRANS: at
-  // n = 16384, 16 columns they take 9 ms (the blocked solve 13.6), below that
+  // n = 16384, 16 columns they take 9.8 ms (the blocked solve 13.6), below that
   // 2 to 6 times less; beyond 16 the FP64 pipe's n^2 nrhs bound passes the
   // blocked NOTRAN solve, whose products run on the tensor cores
   const bool chain_path = g_f64_update == 1 && nrhs <= kChainRhs && ws.dinv_solve &&
@@ -880,10 +918,16 @@ cudaError_t dgetrs_device(char trans, int n, int nrhs, const double* dA, long lo
     static const cudaError_t a0 = cudaFuncSetAttribute(
         solve_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kInvSmem);
     SL_TRY(a0);
-    solve_prep_kernel<<<2 * ((n + 63) / 64) + (n + 255) / 256, 256, kInvSmem, s>>>(
-        n, dA, ldda, ws.dinv_solve, dipiv, ws.perm, ws.status, chain_path ? ws.chain : nullptr);
+    const int nrb = (n + 255) / 256;
+    solve_prep_kernel<<<2 * kInvParts * ((n + 63) / 64) + nrb * perm_segs(n), 256, kInvSmem, s>>>(
+        n, dA, ldda, ws.dinv_solve, dipiv, ws.perm + n, ws.status, chain_path ? ws.chain : nullptr);
     count_launches(1);
     SL_TRY(cudaGetLastError());
+    if (!chain_path) {
+      perm_finish_kernel<<<nrb, 256, 0, s>>>(dipiv, n, ws.perm + n, ws.perm);
+      count_launches(1);
+      SL_TRY(cudaGetLastError());
+    }
   } else {
     SL_TRY(cudaMemsetAsync(ws.status, 0, sizeof(int), s));
     SL_TRY(perm_compose(dipiv, n, ws.perm, s));
@@ -899,9 +943,9 @@ cudaError_t dgetrs_device(char trans, int n, int nrhs, const double* dA, long lo
     const size_t ub = (size_t)((n + 63) / 64) * 4096;
     const unsigned e1 = ++*ws.chain_epoch, e2 = ++*ws.chain_epoch;
     SL_TRY(trsv64_chain(notran, !notran, dA, ldda, n, ws.dinv_solve + (notran ? 0 : ub), dB, lddb,
-                        notran ? ws.perm : nullptr, X, n, nullptr, nrhs, ws.chain, words, e1, ws.status, s));
+                        notran ? dipiv : nullptr, X, n, nullptr, ws.perm + n, nrhs, ws.chain, words, e1, ws.status, s));
     SL_TRY(trsv64_chain(!notran, !notran, dA, ldda, n, ws.dinv_solve + (notran ? ub : 0), X, n, nullptr, dB,
-                        lddb, notran ? nullptr : ws.perm, nrhs, ws.chain + 1, words, e2, ws.status, s));
+                        lddb, notran ? nullptr : dipiv, ws.perm + n, nrhs, ws.chain + 1, words, e2, ws.status, s));
     phase_end(kPhSolve, s, 2.0 * (double)n * n * nrhs, 8.0 * ((double)n * n + 4.0 * (double)n * nrhs));
     return cudaSuccess;
   }

@@ -118,7 +118,7 @@ struct LuWork {
   // cleared before every launch.
   unsigned* cand_launches = nullptr;
   int* swap_plan = nullptr;  // kSwapPlanInts: composite form of a panel's interchanges
-  int* perm;         // n ints: composed row permutation (solve)
+  int* perm;         // perm_ints(n) ints: composed row permutation (solve)
   double* bswap;     // n * nrhs doubles: gathered right-hand sides (solve)
   size_t perm_len;
   size_t bswap_len;
@@ -233,12 +233,13 @@ cudaError_t dgetrs_device(char trans, int n, int nrhs, const double* dA, long lo
 constexpr int kChainRhs = 16;
 // op(T) X = S with the lower (unit) or upper triangle of n x n LU factors in
 // one launch (trsv_f64.cu): D holds the inverses of that triangle's 64x64
-// diagonal blocks; S(i, c) = src[gather[i] + c lds], X(i, c) goes to
-// dst[scatter[i] + c ldd] (null: i). ticket is zero on entry; words holds two
+// diagonal blocks; S is src with its rows permuted by the pivots `gather`, X goes
+// to dst through those of `scatter` (null: in place; maps: the pivots' segment
+// maps). ticket is zero on entry; words holds two
 // per value and no word of this epoch.
 cudaError_t trsv64_chain(bool lower, bool trans, const double* A, long long lda, int n, const double* D,
                          const double* src, long long lds, const int* gather, double* dst,
-                         long long ldd, const int* scatter, int nrhs, int* ticket,
+                         long long ldd, const int* scatter, const int* maps, int nrhs, int* ticket,
                          unsigned long long* words, uint32_t epoch, int* status, cudaStream_t s);
 
 // ---- low-precision trailing update (mixed_gemm.cu) ----
@@ -265,7 +266,7 @@ struct MixedWork {
   unsigned short* A16 = nullptr;  // 16-bit GEMM operands (rows x kpad)
   unsigned short* B16 = nullptr;
   int* col_exp = nullptr;      // per-column exponents of U12
-  int* perm = nullptr;         // composed pivot permutation (n)
+  int* perm = nullptr;         // composed pivot permutation (perm_ints(n))
   double* R = nullptr;         // residuals n x nrhs
   double* D = nullptr;         // GMRES correction (n)
   float* Xf = nullptr;         // FP32 right-hand sides n x nrhs
@@ -357,7 +358,15 @@ cudaError_t scale_rows_device(int n, int ncols, double* X, long long ldx, const 
 cudaError_t dgetri_device(int n, double* dA, long long lda, const int* dipiv, double* X,
                           const LuWork& ws, int* dflag, int* info, cudaStream_t s);
 
-// perm[i] = original row ending in row i after the n interchanges i <-> ipiv[i].
+// perm[i] = original row ending in row i after the n interchanges i <-> ipiv[i];
+// perm holds perm_ints(n) ints (the segments' maps follow the result).
+constexpr int kPermSegs = 16;
+__host__ __device__ inline int perm_seg_len(int n) {
+  const int len = (n + kPermSegs - 1) / kPermSegs;
+  return len < 512 ? 512 : len;
+}
+__host__ __device__ inline int perm_segs(int n) { return (n + perm_seg_len(n) - 1) / perm_seg_len(n); }
+inline size_t perm_ints(int n) { return (size_t)n * (1 + kPermSegs); }
 cudaError_t perm_compose(const int* dipiv, int n, int* perm, cudaStream_t s);
 
 // dst[i] = src[i] + delta, n entries (device arrays).

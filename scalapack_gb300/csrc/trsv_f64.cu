@@ -62,16 +62,18 @@ __device__ __forceinline__ bool get_x(const unsigned long long* p, uint32_t epoc
 }
 
 // op(T) X = S for one triangle of the LU factors A; TRANS: op(T) = T^T.
-// forward: block rows from the top (lower, or upper transposed). Element (i, c)
-// of S is src[(gather ? gather[i] : i) + c lds]; X goes to
-// dst[(scatter ? scatter[i] : i) + c ldd]. D: inverses of T's diagonal blocks,
+// forward: block rows from the top (lower, or upper transposed). Row i of S is
+// row i of src, of X row i of dst, or in either place the row that the pivots
+// `gather` / `scatter` permute there (null: i; maps: their segments' maps,
+// follow_perm). D: inverses of T's diagonal blocks,
 // 4096 doubles each, column-major.
 template <int NR, bool TRANS>
 __global__ void __launch_bounds__(256)
 trsv64_chain_kernel(const double* __restrict__ A, long long lda, int n, int forward,
                     const double* __restrict__ D, const double* __restrict__ src, long long lds,
                     const int* __restrict__ gather, double* dst, long long ldd,
-                    const int* __restrict__ scatter, int nrhs, int ngroups, int* ticket,
+                    const int* __restrict__ scatter, const int* __restrict__ maps, int nrhs,
+                    int ngroups, int* ticket,
                     unsigned long long* words, uint32_t epoch, int* status) {
   extern __shared__ double trsv_ring[];     // TRING tiles
   __shared__ double xs[2][TB * NR];         // solutions of the block being applied
@@ -121,7 +123,12 @@ trsv64_chain_kernel(const double* __restrict__ A, long long lda, int n, int forw
   const int pi = tid & (TB - 1), pc = tid >> 6;
   const bool mine = pc < NR && pi < rb && c0 + pc < nrhs;
   double bv = 0.0;
-  if (mine) bv = src[(gather ? gather[r0 + pi] : r0 + pi) + (long long)(c0 + pc) * lds];
+  int drow = r0 + pi;
+  if (mine) {
+    const int srow = gather ? follow_perm(drow, gather, n, maps) : drow;
+    if ((unsigned)srow < (unsigned)n) bv = src[srow + (long long)(c0 + pc) * lds];
+    if (scatter) drow = follow_perm(drow, scatter, n, maps);
+  }
 
   double acc[NR];
 #pragma unroll
@@ -195,14 +202,14 @@ trsv64_chain_kernel(const double* __restrict__ A, long long lda, int n, int forw
     const int e = pi * NR + pc;
     const double x = (part[0][e] + part[1][e]) + (part[2][e] + part[3][e]);
     put_x(words + ((size_t)(c0 + pc) * n + r0 + pi) * 2, x, epoch);
-    dst[(scatter ? scatter[r0 + pi] : r0 + pi) + (long long)(c0 + pc) * ldd] = x;
+    if ((unsigned)drow < (unsigned)n) dst[drow + (long long)(c0 + pc) * ldd] = x;  // (an invalid IPIV writes nothing)
   }
 }
 
 template <int NR, bool TRANS>
 cudaError_t launch_chain(const double* A, long long lda, int n, bool forward, const double* D,
                          const double* src, long long lds, const int* gather, double* dst,
-                         long long ldd, const int* scatter, int nrhs, int* ticket,
+                         long long ldd, const int* scatter, const int* maps, int nrhs, int* ticket,
                          unsigned long long* words, uint32_t epoch, int* status, cudaStream_t s) {
   constexpr int smem = TRING * TSLOT * (int)sizeof(double);
   auto kern = trsv64_chain_kernel<NR, TRANS>;
@@ -210,7 +217,7 @@ cudaError_t launch_chain(const double* A, long long lda, int n, bool forward, co
   SL_TRY(attr);
   const int ngroups = (nrhs + NR - 1) / NR;
   kern<<<(n + TB - 1) / TB * ngroups, 256, smem, s>>>(A, lda, n, forward ? 1 : 0, D, src, lds, gather, dst,
-                                                      ldd, scatter, nrhs, ngroups, ticket, words, epoch, status);
+                                                      ldd, scatter, maps, nrhs, ngroups, ticket, words, epoch, status);
   count_launches(1);
   return cudaGetLastError();
 }
@@ -219,13 +226,13 @@ cudaError_t launch_chain(const double* A, long long lda, int n, bool forward, co
 
 cudaError_t trsv64_chain(bool lower, bool trans, const double* A, long long lda, int n, const double* D,
                          const double* src, long long lds, const int* gather, double* dst,
-                         long long ldd, const int* scatter, int nrhs, int* ticket,
+                         long long ldd, const int* scatter, const int* maps, int nrhs, int* ticket,
                          unsigned long long* words, uint32_t epoch, int* status, cudaStream_t s) {
   const bool forward = lower != trans;
   // two right-hand sides a CTA once one each would queue several CTAs per SM
   const bool two = nrhs > 1 && (long long)((n + TB - 1) / TB) * nrhs > 2LL * num_sms();
 #define SL_CH(NR, TR)                                                                                 \
-  return launch_chain<NR, TR>(A, lda, n, forward, D, src, lds, gather, dst, ldd, scatter, nrhs, ticket, \
+  return launch_chain<NR, TR>(A, lda, n, forward, D, src, lds, gather, dst, ldd, scatter, maps, nrhs, ticket, \
                               words, epoch, status, s)
   if (two) {
     if (trans) SL_CH(2, true);
