@@ -354,9 +354,9 @@ void sl1x1_set_panel_ib(int subpanels);
 void sl1x1_set_lowp_stages(int stages);
 /* Arithmetic of the FP64 factorization's trailing update (PDGEMM step of
  * SRC/pdgetrf.f:288-290): 1 (default) = the product formed exactly on the
- * BF16 tensor cores (tcgen05) from 7-bit integer slices of the operands (8
- * slices, row and column power-of-two scales, diagonals d <= 6 of the slice
- * products summed exactly as integers), accurate to a few units of 2^-53 of
+ * BF16 tensor cores (tcgen05) from 8-bit integer slices of the operands (7
+ * balanced base-256 digits, row and column power-of-two scales, the leading
+ * diagonals of the slice products summed exactly as integers), accurate to a few units of 2^-53 of
  * max|L21(i,:)| max|U12(:,j)| and independent of the summation order; 0 =
  * FP64 DMMA (mma.sync m16n8k4). The sliced form needs device scratch of about
  * 4 KB per row plus 4 KB per column of the matrix; where it cannot be had

@@ -854,7 +854,7 @@ solve_block128_kernel(int kb, const double* __restrict__ A, long long lda, int k
     x[t] = ys[t];
     if (hkeys) {
       const unsigned long long w = oz_key_word(ys[t], epoch);
-      if (w) atomicMax(hkeys + t, w);
+      if (w) oz_raise_key(hkeys + t, w);
     }
   }
 }

@@ -728,10 +728,16 @@ trsm_strip_kernel(int w, int ncols, int eb, const T* __restrict__ Tm, long long 
     // w+8, ...; one coalesced load per column)
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
     const int i = ((int)blockIdx.x - nsolve) * 32 + lane;
-    for (int c = wp; c < kj.lcols; c += 8) {
-      const unsigned long long v = (i < kj.lrows) ? oz_key_word(kj.L[i + (long long)c * kj.ldl], kj.epoch) : 0ULL;
-      const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(v >> 12 == kj.epoch ? (v & 4095ULL) : 0ULL));
-      if (lane == 0 && hi) atomicMax(kj.ckeys + c, (kj.epoch << 12) | hi);
+    const double* row = kj.L + min(i, kj.lrows - 1);  // (a repeated row changes no maximum)
+    for (int c0 = wp; c0 < kj.lcols; c0 += 64) {
+      double v[8];  // eight columns' loads in flight
+#pragma unroll
+      for (int q = 0; q < 8; ++q) v[q] = row[(long long)min(c0 + 8 * q, kj.lcols - 1) * kj.ldl];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(oz_key_word(v[q], 0ULL) & 4095ULL));
+        if (lane == 0 && hi && c0 + 8 * q < kj.lcols) oz_raise_key(kj.ckeys + c0 + 8 * q, (kj.epoch << 12) | hi);
+      }
     }
     return;
   }
@@ -790,7 +796,7 @@ trsm_strip_kernel(int w, int ncols, int eb, const T* __restrict__ Tm, long long 
           const unsigned long long v = oz_key_word(Bs[r * LD + cc], kj.epoch);
           km = v > km ? v : km;
         }
-        if (km) atomicMax(kj.hkeys + r, km);
+        if (km) oz_raise_key(kj.hkeys + r, km);
       }
   }
 }

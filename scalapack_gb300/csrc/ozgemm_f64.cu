@@ -6,35 +6,40 @@
 // of matrix multiplication and its applications", Numer. Algorithms 59, 2012).
 //
 // Splitting. Row i of A is scaled by 2^-e_i (e_i the exponent of its largest
-// magnitude, so |A(i,k)| 2^-e_i < 1) and cut into S = 8 slices of 7 bits:
-//   A(i,k) 2^-e_i = sum_{s=1..8} a_s(i,k) 2^-7s,  a_s integer, |a_s| <= 127,
-// by exact FP64 truncation; column j of B likewise with 2^-f_j and b_t. The
-// slices are stored in BF16 as a_s 2^-7(s-1) (8 significant bits hold any
-// |a_s| <= 127 and the power of two is exact), K-major, so that the product of
-// slices s and t carries its weight 2^-7(s+t-2) by itself.
+// magnitude, so |A(i,k)| 2^-e_i < 1), rounded to a multiple of 2^-55 and cut into
+// S = 7 balanced base-256 digits:
+//   A(i,k) 2^-e_i = sum_{s=1..7} a_s(i,k) 2^(1-8s),  a_s integer, |a_s| <= 128;
+// column j of B likewise with 2^-f_j and b_t. BF16 holds every such digit exactly
+// (8 significant bits). Balanced digits carry 8 bits a slice where truncated ones
+// of the same exactness carry 7: 7 slices and 28 products instead of 8 and 36,
+// with the same 2^-56 of the scale kept and no bias.
 //
 // Exact products. For K <= 256, sum_k a_s b_t is an integer of magnitude at
-// most 256 * 127^2 < 2^22: up to four such products sum exactly in FP32, in
+// most 256 * 128^2 = 2^22: up to four such products sum exactly in FP32, in
 // any order and with any alignment the tensor core uses, because every partial
-// sum is an integer multiple of the diagonal's unit below 2^24. With
-// d = s + t, the update is
-//   (A B)(i,j) = 2^(e_i + f_j) sum_d 2^-7d P_d,   P_d = sum_{s+t=d} sum_k a_s b_t.
-// Each diagonal d = 2..9 has its own TMEM accumulator (8 x 64 columns, all of
-// TMEM). d <= 5 holds at most 4 products: exact; d = 6 holds 5, exact unless
-// their sum passes 2^24, which takes nearly all 1280 terms at full magnitude
-// with one sign; d = 7..9 are summed in plain FP32 (their rounding, 2^-24
-// relative to terms already 2^-49 below the row and column scales, is far
-// below FP64 rounding); d >= 10 is dropped. 36 slice products, issued as 12
-// instructions per 16-wide k step: A slice s against B slices t = 0..7-s
-// (consecutive in shared memory) into accumulators s..7 (consecutive in TMEM)
-// in groups of up to 4 (N up to 256).
+// sum is an integer of magnitude at most 2^24. With d = s + t, the update is
+//   (A B)(i,j) = 2^(e_i + f_j) sum_d 2^(2-8d) P_d,   P_d = sum_{s+t=d} sum_k a_s b_t.
+// Each diagonal d = 2..8 has its own TMEM accumulator (7 x 64 columns). d <= 5
+// holds at most 4 products: exact; d = 6..8 hold 5 to 7, exact unless their sum
+// passes 2^24, which takes most of the 1280 to 1792 terms at full magnitude with
+// one sign; d >= 9 is dropped: 6 products of weight 2^-70, whose balanced digits
+// have no common sign. 28 slice products, issued as 10 instructions per 16-wide
+// k step: A slice s against B slices t = 0..6-s (consecutive in shared memory)
+// into accumulators s..6 (consecutive in TMEM) in groups of up to 4 (N up to
+// 256).
 //
-// Epilogue. P_2..P_6 are read back as exact integers, combined with the FP32
-// sum of the tail diagonals into one 64-bit integer I = sum_d P_d 2^(52-7d) (|I| < 2^61), converted to
-// FP64 once, and C(i,j) = fma(alpha 2^(e_i+f_j-52), I, C(i,j)). The result is
-// within a few units of 2^-53 of 2^(e_i + f_j) of the exact product, and
-// independent of the accumulation order (run to run identical). Rows or
-// columns holding Inf or NaN give NaN in their row or column of C.
+// Epilogue. P_2..P_6 are read back as exact integers and combined with the
+// rounded P_7 + P_8/256 into one 64-bit integer I = sum_d P_d 2^(56-8d) (|I| <
+// 2^63), rounded to 53 bits once and scaled by 2^(e_i+f_j-54) with integer
+// arithmetic; C(i,j) then takes it by one FP64 addition (alpha = +-1; otherwise
+// by an fma with alpha). This GPU converts 64-bit integers and adds or
+// multiplies doubles at 2 lanes per cycle and SM, so a conversion, a
+// multiplication and an fma per element would take as long as the tile's
+// products, and a 64-bit conversion before the accumulators are released would
+// hold the products up. The result is within a few units of 2^-53 of
+// 2^(e_i + f_j) of the exact product, and independent of the accumulation order
+// (run to run identical). Rows or columns holding Inf or NaN give NaN in their
+// row or column of C.
 //
 // Balancing along k. A B = (A 2^-d)(2^d B) for any integers d_k, so the
 // scales are taken after an exact power-of-two balancing (ex x: |x| < 2^ex x,
@@ -68,20 +73,27 @@
 // normwise bound but not a componentwise one.
 //
 // Structure (one CTA per SM, a few 128 x 64 tiles of C per CTA, 10 warps):
-//   * warp 0 allocates all 512 TMEM columns (8 accumulators x 64 columns);
-//   * one thread issues TMA loads: for each 64-wide k block, the eight 128x64
-//     A slices one at a time through a 6-deep ring and the eight 64x64 B
+//   * warp 0 allocates all 512 TMEM columns (7 accumulators x 64 columns);
+//   * one thread issues TMA loads: for each 64-wide k block, the seven 128x64
+//     A slices one at a time through a 7-deep ring and the seven 64x64 B
 //     slices into one half of a double buffer, half a block ahead (128-byte
 //     swizzle);
 //   * one thread issues tcgen05.mma.kind::f16 (M=128, N=64..256, K=16): A
-//     slice s against B slices t <= 9 - s into accumulators s+t-2;
-//   * 8 epilogue warps read the accumulators with tcgen05.ld (warp w owns
-//     lanes 32(w%4).. = tile rows, and half of the columns), combine them
-//     into integers, hand the TMEM
+//     slice s against B slices t <= 8 - s into accumulators s+t-2;
+//   * 16 epilogue warps load their part of C while the tile's products run, read
+//     the accumulators with tcgen05.ld (warp w owns lanes 32(w%4).. = tile rows,
+//     and a quarter of the columns), combine them into integers, hand the TMEM
 //     back to the MMA thread, and update C in place (coalesced per column)
 //     while the next tile's products run.
 // Every mbarrier wait is bounded; on timeout the CTA records kFlagTimeout,
 // drains what it issued, frees its TMEM and returns.
+//
+// Bound: a tile's products take 14300 cycles of the tensor pipe; it takes 23500
+// (m = n = 16384, k = 256): its 672 KB of slices come from L2 at 8.3 TB/s, and
+// the read-out of the accumulators (3000) is not overlapped. Measured there:
+// 3.28 ms, 42 TFLOP/s FP64-equivalent; with 36 products of 7-bit slices, three
+// FP64-rate operations per element and descriptors computed per instruction,
+// 5.0 ms. 128 x 64 tiles of 8192 x 256 x 256: 47 us (72 before).
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -99,15 +111,13 @@ namespace sl {
 namespace {
 using namespace tc;
 
-constexpr int OZ_S = 8;          // slices per operand
-constexpr int OZ_BITS = 7;       // bits per slice
-constexpr int OZ_NACC = 8;       // accumulators, one per diagonal d = 2..9
+constexpr int OZ_S = 7;          // slices per operand: balanced base-256 digits
 constexpr int OZ_KMAX = 256;     // exactness bound on K per pass
 constexpr int OBM = 128, OBN = 64, OBK = 64;
 constexpr int A_SLICE_BYTES = OBM * OBK * 2;          // 16 KB
 constexpr int B_SLICE_BYTES = OBN * OBK * 2;          // 8 KB
-constexpr int B_CHUNK_BYTES = OZ_S * B_SLICE_BYTES;   // 64 KB per k block
-constexpr int A_RING = 6;
+constexpr int B_CHUNK_BYTES = OZ_S * B_SLICE_BYTES;   // 56 KB per k block
+constexpr int A_RING = 7;
 constexpr int OZ_TMEM_COLS = 512;
 constexpr int GROUP_M = 8;       // tile raster: 8 row tiles sweep the columns together
 
@@ -130,8 +140,9 @@ struct __align__(8) OzBars {
   uint32_t tmem_base;
 };
 
-constexpr int OZ_THREADS = 320;  // warp 0 TMA, warp 1 MMA, warps 2..9 epilogue
-constexpr int OZ_EPI_WARPS = 8;  // two per TMEM lane quadrant, 32 columns each
+constexpr int OZ_EPI_WARPS = 16;  // four per TMEM lane quadrant
+constexpr int OZ_EC = OBN / (OZ_EPI_WARPS / 4);  // columns of an epilogue warp: 16
+constexpr int OZ_THREADS = 64 + 32 * OZ_EPI_WARPS;  // warp 0 TMA, warp 1 MMA, the rest epilogue
 
 size_t oz_smem_bytes() {
   return 1024 + (size_t)A_RING * A_SLICE_BYTES + 2 * (size_t)B_CHUNK_BYTES + sizeof(OzBars) + 64;
@@ -166,7 +177,7 @@ __device__ __forceinline__ void oz_tile(int t, int tiles_m, int tiles_n, int& m0
   n0 = (in_group / gsize) * OBN;
 }
 
-// The eight B slices of chunk c (tile first + c / nkc, k block c % nkc) into
+// The B slices of chunk c (tile first + c / nkc, k block c % nkc) into
 // half c & 1 of the B double buffer, once chunk c-2 has released it.
 __device__ __forceinline__ bool oz_issue_b(int c, int first, int nkc, int tiles_m, int tiles_n,
                                            int n_pad, unsigned char* sB, const CUtensorMap* tmB,
@@ -190,7 +201,7 @@ __device__ __forceinline__ bool oz_issue_b(int c, int first, int nkc, int tiles_
 // them is written. When B aliases C (whole_cols) a CTA takes whole column
 // blocks instead -- tile t of the CTA is column block t with every row tile --
 // so no other CTA writes the columns it reads. Threads 64.. own one row and
-// 32 columns each; products accumulate in k order with one FMA each, then
+// OZ_EC columns each; products accumulate in k order with one FMA each, then
 // C = fma(alpha, acc, C).
 __device__ __noinline__ void oz_fp64_tiles(unsigned char* smem, int m, int n, int kb,
                                            const double* __restrict__ A, long long lda,
@@ -221,19 +232,19 @@ __device__ __noinline__ void oz_fp64_tiles(unsigned char* smem, int m, int n, in
     if (tid >= 64) {
       const int t = tid - 64, row = m0 + (t & (OBM - 1)), h = t >> 7;
       if (row < m) {
-        double acc[32];
+        double acc[OZ_EC];
 #pragma unroll
-        for (int j = 0; j < 32; ++j) acc[j] = 0.0;
+        for (int j = 0; j < OZ_EC; ++j) acc[j] = 0.0;
         const double* arow = A + row;
         for (int k = 0; k < kb; ++k) {
           const double a = arow[(long long)k * lda];
-          const double* bk = sB + k * OBN + h * 32;
+          const double* bk = sB + k * OBN + h * OZ_EC;
 #pragma unroll
-          for (int j = 0; j < 32; ++j) acc[j] = fma(a, bk[j], acc[j]);
+          for (int j = 0; j < OZ_EC; ++j) acc[j] = fma(a, bk[j], acc[j]);
         }
 #pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          const int col = n0 + h * 32 + j;
+        for (int j = 0; j < OZ_EC; ++j) {
+          const int col = n0 + h * OZ_EC + j;
           if (col < n) {
             double* cp = C + row + (long long)col * ldc;
             *cp = fma(alpha, acc[j], *cp);
@@ -244,15 +255,32 @@ __device__ __noinline__ void oz_fp64_tiles(unsigned char* smem, int m, int n, in
   }
 }
 
+// Exponent of a power of two (-1023 for zero, beyond any sum's range for NaN).
+__device__ __forceinline__ int oz_exp_field(double x) {
+  const int f = (__double2hiint(x) >> 20) & 0x7ff;
+  return f == 0x7ff ? 1 << 14 : f - 1023;
+}
+// v 2^E rounded to nearest once, E in [-1022, 960], on the integer pipe.
+__device__ __forceinline__ double oz_ldexp(long long v, int E) {
+  const unsigned long long u = (unsigned long long)(v < 0 ? -v : v);
+  const int lz = __clzll((long long)u);
+  const unsigned long long w = u << (lz & 63);
+  unsigned long long m = w >> 11;
+  m += ((unsigned)(w & 2047) + (unsigned)(m & 1)) > 1024u ? 1 : 0;
+  // the significand's leading bit adds one to the exponent below it
+  const unsigned long long bits = ((unsigned long long)(unsigned)(E + 63 - lz + 1022) << 52) + m;
+  return u == 0 ? 0.0 : __longlong_as_double((long long)(bits | ((unsigned long long)v & (1ULL << 63))));
+}
+
 // CTA b takes tiles b tpc .. b tpc + tpc - 1 of the raster (a few, so that
 // SMs turn over and the panel's kernels on the high-priority stream find
 // room between them). The TMA thread runs
 // ahead through a flat sequence of k blocks ("chunks", nkc per tile): for
-// chunk c it loads the eight A slices through the ring, and after the fourth
-// of them the eight B slices of chunk c+1 into the other half of the B double
+// chunk c it loads the A slices through the ring, and after the fourth of
+// them the B slices of chunk c+1 into the other half of the B double
 // buffer. The MMA thread starts a tile once the epilogue has drained the
 // previous tile's accumulators (tempty); the epilogue warps drain them into
-// 32 combined integers per thread (tmem -> registers), release the TMEM, and
+// 16 combined integers per thread (tmem -> registers), release the TMEM, and
 // update C from registers while the next tile's products run.
 __global__ void __launch_bounds__(OZ_THREADS, 1)
 ozgemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
@@ -263,7 +291,7 @@ ozgemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   unsigned char* sA = base;                                   // A_RING x 16 KB
-  unsigned char* sB = base + A_RING * A_SLICE_BYTES;          // 2 x 64 KB
+  unsigned char* sB = base + A_RING * A_SLICE_BYTES;          // 2 x 56 KB
   OzBars* bars = (OzBars*)(sB + 2 * B_CHUNK_BYTES);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -344,10 +372,11 @@ ozgemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
   } else if (warp == 1) {
     if (lane == 0) {
       // ---- MMA issuer ----
-      // A slice s against B slices t = 0 .. 7-s lands in accumulators s .. 7:
+      // A slice s against B slices t = 0 .. 6-s lands in accumulators s .. 6:
       // consecutive TMEM columns and, in the B buffer, consecutive slices, so
       // one instruction covers up to 4 of them (N up to 256).
       bool ok = true;
+      const uint64_t adesc = smem_desc_sw128(sA), bdesc = smem_desc_sw128(sB);
       for (int it = 0; ok && it < my_tiles; ++it) {
         if (it >= 1 && !mbar_wait(&bars->tempty, (it - 1) & 1)) { ok = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;");
@@ -355,27 +384,31 @@ ozgemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
           const int c = it * nkc + kc, hb = c & 1;
           if (!mbar_wait(&bars->bfull[hb], (c >> 1) & 1)) { ok = false; break; }
           s_bcons = c + 1;
-          const unsigned char* bchunk = sB + hb * B_CHUNK_BYTES;
+          // A slice sl of a chunk always stands in ring slot sl, so that every
+          // operand's place is a constant added to two descriptors: computed
+          // anew per instruction they took the one issuing thread 170 cycles an
+          // instruction, where the products take 90.
+          static_assert(A_RING == OZ_S, "slot of a slice");
+          const uint64_t b0 = bdesc + (uint64_t)((hb * B_CHUNK_BYTES) >> 4);
+#pragma unroll
           for (int sl = 0; sl < OZ_S; ++sl) {
-            const int g = c * OZ_S + sl, st = g % A_RING;
-            if (!mbar_wait(&bars->afull[st], (g / A_RING) & 1)) { ok = false; break; }
+            if (!mbar_wait(&bars->afull[sl], c & 1)) { ok = false; break; }
             asm volatile("tcgen05.fence::after_thread_sync;");
-            const unsigned char* aslice = sA + st * A_SLICE_BYTES;
 #pragma unroll
             for (int kk = 0; kk < OBK / 16; ++kk) {
-              const uint64_t ad = smem_desc_sw128(aslice + kk * 32);
               // the very first products write every accumulator (s = 0 covers
-              // all eight); every later one adds
-              const uint32_t accum = (kc > 0 || sl > 0 || kk > 0) ? 1u : 0u;
+              // them all); every later one adds
+              const uint32_t accum = (sl > 0 || kk > 0) ? 1u : (kc > 0 ? 1u : 0u);
+#pragma unroll
               for (int t0 = 0; t0 + sl < OZ_S; t0 += 4) {
-                const int cnt = min(4, OZ_S - sl - t0);
-                const uint32_t dst = tmem + (uint32_t)((sl + t0) * OBN);
-                const uint64_t bd = smem_desc_sw128(bchunk + t0 * B_SLICE_BYTES + kk * 32);
-                umma_f16(dst, ad, bd, oz_idesc(cnt * OBN), accum);
+                const int cnt = OZ_S - sl - t0 < 4 ? OZ_S - sl - t0 : 4;
+                umma_f16(tmem + (uint32_t)((sl + t0) * OBN),
+                         adesc + (uint64_t)((sl * A_SLICE_BYTES + kk * 32) >> 4),
+                         b0 + (uint64_t)((t0 * B_SLICE_BYTES + kk * 32) >> 4), oz_idesc(cnt * OBN), accum);
               }
             }
-            umma_commit(&bars->aempty[st]);
-            s_acons = g + 1;
+            umma_commit(&bars->aempty[sl]);
+            s_acons = c * OZ_S + sl + 1;
           }
           if (!ok) break;
           umma_commit(&bars->bempty[hb]);
@@ -390,11 +423,22 @@ ozgemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
     }
   } else {
     // ---- epilogue: warp w reads TMEM lanes 32 (w % 4) .. +31 = tile rows,
-    // columns 32 h .. 32 h + 31 with h = (w - 2) / 4 ----
-    constexpr int EC = OBN / 2;
-    const int quad = warp & 3, half = (warp - 2) >> 2;
-    const uint32_t trow = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(half * EC);
+    // columns EC g .. EC g + EC - 1 with g = (w - 2) / 4 ----
+    constexpr int EC = OZ_EC;
+    const int quad = warp & 3, cg = (warp - 2) >> 2;
+    const uint32_t trow = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(cg * EC);
+    const bool unit = alpha == 1.0 || alpha == -1.0, neg = alpha < 0.0;
     for (int it = 0; it < my_tiles; ++it) {
+      int m0, n0;
+      oz_tile(first_tile + it, tiles_m, tiles_n, m0, n0);
+      // this tile's part of C on its way while the products run
+      const int row = m0 + quad * 32 + lane, nb0 = n0 + cg * EC;
+      const int ncol = row < m ? min(EC, n - nb0) : 0;
+      double* crow = C + (long long)row + (long long)nb0 * ldc;
+      double cv[EC];
+#pragma unroll
+      for (int j = 0; j < EC; ++j) cv[j] = j < ncol ? crow[(long long)j * ldc] : 0.0;
+      const double rsc = ncol > 0 ? rs[row] : 0.0;
       if (!mbar_wait(&bars->tfull, it & 1)) {
         if (lane == 0) {
           atomicExch(status, (int)kFlagTimeout);
@@ -403,64 +447,64 @@ ozgemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;");
-      int m0, n0;
-      oz_tile(first_tile + it, tiles_m, tiles_n, m0, n0);
+      // two accumulators at a time keep the register count down; P_2 <= 2^22
+      // converts by an addition (1.5 * 2^23, whose bits are taken off again),
+      // the others at 16 lanes a cycle
       long long I[EC];
-#pragma unroll
-      for (int c0 = 0; c0 < EC; c0 += 16) {
-        // P_d = acc_d * 2^(7(d-2)) exactly for d <= 6; the tail d = 7..9
-        // is summed in FP32 and keeps 3 fraction bits of P_7's unit. Four
-        // accumulators at a time keep the register count down.
-        uint32_t r[4][16];
-#pragma unroll
-        for (int a = 0; a < 4; ++a) tmem_ld16_nowait(trow + (uint32_t)(a * OBN + c0), r[a]);
+      uint32_t r[2][16];
+      auto get2 = [&](int a, bool both) {
+        tmem_ld16_nowait(trow + (uint32_t)(a * OBN), r[0]);
+        if (both) tmem_ld16_nowait(trow + (uint32_t)((a + 1) * OBN), r[1]);
         tmem_ld_wait();
+        touch16(r[0]);
+        if (both) touch16(r[1]);
+      };
+      get2(0, true);
 #pragma unroll
-        for (int a = 0; a < 4; ++a) touch16(r[a]);
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const long long p2 = __float2int_rn(__uint_as_float(r[0][j]));
-          const long long p3 = __float2int_rn(__uint_as_float(r[1][j]) * 128.0f);
-          const long long p4 = __float2int_rn(__uint_as_float(r[2][j]) * 16384.0f);
-          const long long p5 = __float2int_rn(__uint_as_float(r[3][j]) * 2097152.0f);
-          I[c0 + j] = (p2 << 38) + (p3 << 31) + (p4 << 24) + (p5 << 17);
-        }
-#pragma unroll
-        for (int a = 0; a < 4; ++a) tmem_ld16_nowait(trow + (uint32_t)((a + 4) * OBN + c0), r[a]);
-        tmem_ld_wait();
-#pragma unroll
-        for (int a = 0; a < 4; ++a) touch16(r[a]);
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const long long p6 = __float2int_rn(__uint_as_float(r[0][j]) * 268435456.0f);
-          const float tail = (__uint_as_float(r[1][j]) + __uint_as_float(r[2][j])) + __uint_as_float(r[3][j]);
-          const long long t8 = __float2ll_rn(tail * 274877906944.0f);  // 2^38
-          I[c0 + j] += (p6 << 10) + t8;
-        }
+      for (int j = 0; j < EC; ++j) {
+        const unsigned p2 = __float_as_uint(__uint_as_float(r[0][j]) + 12582912.0f) - 0x4B400000u;
+        const unsigned p3 = (unsigned)__float2int_rn(__uint_as_float(r[1][j]));
+        const unsigned hi = (p2 << 8) + p3;  // (modulo 2^32, as the sum's high half)
+        I[j] = (long long)((unsigned long long)hi << 32);
       }
+      get2(2, true);
+#pragma unroll
+      for (int j = 0; j < EC; ++j) {
+        const long long p4 = __float2int_rn(__uint_as_float(r[0][j]));
+        const long long p5 = __float2int_rn(__uint_as_float(r[1][j]));
+        I[j] += (p4 << 24) + (p5 << 16);
+      }
+      get2(4, false);
+#pragma unroll
+      for (int j = 0; j < EC; ++j) I[j] += (long long)__float2int_rn(__uint_as_float(r[0][j])) << 8;
+      get2(5, true);
       // the accumulators are in registers: the next tile's products may start
       asm volatile("tcgen05.fence::before_thread_sync;");
       __syncwarp();
       if (lane == 0) mbar_arrive(&bars->tempty);
-      const int row = m0 + quad * 32 + lane;
-      if (row < m) {
-        const double rsc = alpha * rs[row];
-        const int nb0 = n0 + half * EC;
-        double* crow = C + (long long)row + (long long)nb0 * ldc;
 #pragma unroll
-        for (int c0 = 0; c0 < EC; c0 += 8) {
-          if (nb0 + c0 >= n) break;
-          const int ncol = min(8, n - (nb0 + c0));
-          double cv[8], sc[8];
+      for (int j = 0; j < EC; ++j)
+        I[j] += __float2int_rn(fmaf(__uint_as_float(r[1][j]), 0.00390625f, __uint_as_float(r[0][j])));
+      // one FP64 addition per element, unless some element of the warp needs
+      // the general form: general alpha, scales near the range's ends, zero and
+      // non-finite ones (a vote, so that the compiler does not compute both)
+      const int er = oz_exp_field(rsc);
+      double sc[EC];
+      bool plain = unit;
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            cv[j] = (j < ncol) ? crow[(long long)(c0 + j) * ldc] : 0.0;
-            sc[j] = (j < ncol) ? __ldg(cs + nb0 + c0 + j) : 0.0;
-          }
+      for (int j = 0; j < EC; ++j) {
+        sc[j] = __ldg(cs + min(nb0 + j, n - 1));
+        plain = plain && (j >= ncol || (unsigned)(er + oz_exp_field(sc[j]) + 1022) <= 1982u);
+      }
+      if (__all_sync(0xffffffffu, plain)) {
 #pragma unroll
-          for (int j = 0; j < 8; ++j)
-            if (j < ncol) crow[(long long)(c0 + j) * ldc] = fma(rsc * sc[j], __ll2double_rn(I[c0 + j]), cv[j]);
-        }
+        for (int j = 0; j < EC; ++j)
+          if (j < ncol)
+            crow[(long long)j * ldc] = cv[j] + oz_ldexp(neg ? -I[j] : I[j], er + oz_exp_field(sc[j]));
+      } else {
+#pragma unroll
+        for (int j = 0; j < EC; ++j)
+          if (j < ncol) crow[(long long)j * ldc] = fma(alpha * rsc * sc[j], __ll2double_rn(I[j]), cv[j]);
       }
       if (s_fail) break;
     }
@@ -482,16 +526,18 @@ ozgemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
 // ---- slicing (integer arithmetic on the FP64 bit patterns) ----------------
 //
 // With x = +-m 2^q (m the significand as an integer, 53 bits for normal x)
-// and a scale exponent e with |x| < 2^e, U = floor(|x| 2^(56-e)) is m shifted
-// left by at most 3 bits, or right (dropping the bits below 2^-56 of the
-// scale). Slice s (1-based) is bits [56-7s, 63-7s) of U with the sign of x:
-// exactly the integer parts of the FP64 truncation x 2^-e = sum a_s 2^-7s.
-// With the balancing, A(i,k) is cut against e_i + d_k and B(k,j) against
+// and a scale exponent e with |x| < 2^e, V = +-round(|x| 2^(55-e)) is m shifted
+// left by at most 2 bits, or right with rounding. Adding 128 to its six low
+// digits' places turns V's balanced base-256 digits into bytes: digit s (1-based)
+// is byte 7-s of the sum less 128, the first one what stands above them (-128 ..
+// 128). With the balancing, A(i,k) is cut against e_i + d_k and B(k,j) against
 // f_j - d_k.
 constexpr unsigned long long kMagMask = 0x7fffffffffffffffULL;
 constexpr unsigned long long kInfBits = 0x7ff0000000000000ULL;
 
-__device__ __forceinline__ unsigned long long oz_fixed(unsigned long long bits, int e) {
+// the sum V + 128 (1 + 256 + .. + 256^5) of x with the given bits
+constexpr unsigned long long kDigitBias = 0x0000808080808080ULL;
+__device__ __forceinline__ unsigned long long oz_digits(unsigned long long bits, int e) {
   const int bexp = (int)((bits >> 52) & 0x7ff);
   unsigned long long m = bits & 0xfffffffffffffULL;
   int q = -1074;
@@ -499,10 +545,11 @@ __device__ __forceinline__ unsigned long long oz_fixed(unsigned long long bits, 
     m |= 1ULL << 52;
     q = bexp - 1075;
   }
-  const int sh = q - e + 56;
-  if (sh >= 0) return m << sh;
-  if (sh <= -64) return 0ULL;
-  return m >> (-sh);
+  const int sh = q - e + 55;
+  unsigned long long U;
+  if (sh >= 0) U = m << sh;
+  else U = sh < -54 ? 0ULL : (m + (1ULL << (-sh - 1))) >> -sh;
+  return ((bits >> 63) ? 0ULL - U : U) + kDigitBias;
 }
 
 // frexp exponent of a magnitude given by its bit pattern (finite, nonzero):
@@ -513,22 +560,35 @@ __device__ __forceinline__ int oz_scale_exp(unsigned long long kmax) {
   return (63 - __clzll((long long)kmax)) - 1073;  // subnormal
 }
 
-// 2^(e - 26) as a double (the epilogue's scale factor half), NaN for a
+// 2^(e - 27) as a double (the epilogue's scale factor half), NaN for a
 // non-finite row or column, 0 for a zero one; the caller has checked that
-// e - 26 is a normal exponent
+// e - 27 is a normal exponent
 __device__ __forceinline__ double oz_scale_value(int e, bool bad) {
   if (bad) return __longlong_as_double(0x7ff8000000000000LL);
   if (e == OZ_NOEXP) return 0.0;
-  return __longlong_as_double((long long)((unsigned long long)(e - 26 + 1023) << 52));
+  return __longlong_as_double((long long)((unsigned long long)(e - 27 + 1023) << 52));
 }
 __device__ __forceinline__ bool oz_scale_in_range(int e) {
-  return e == OZ_NOEXP || (e - 26 >= -1022 && e - 26 <= 1023);
+  return e == OZ_NOEXP || (e - 27 >= -1022 && e - 27 <= 1023);
 }
 
-__device__ __forceinline__ __nv_bfloat16 oz_slice_bf16(unsigned long long U, int s, bool neg) {
-  // s is 0-based here: bits [49-7s, 56-7s), weight 2^-7s in the stored slice
-  const float a = (float)(unsigned)((U >> (49 - OZ_BITS * s)) & 127ULL);
-  return __float2bfloat16_rn((neg ? -a : a) * __int_as_float((127 - OZ_BITS * s) << 23));
+// Slice s (0-based) of two digit sums as a pair of BF16: each byte becomes the
+// low mantissa bits of 2^23, whose exact difference to 2^23 + 128 is the digit
+// (its upper 16 bits are its BF16); the first digit is the sum's signed top.
+__device__ __forceinline__ uint32_t oz_slice2(unsigned long long w0, unsigned long long w1, int s) {
+  const uint32_t hi0 = (uint32_t)(w0 >> 32), lo0 = (uint32_t)w0, hi1 = (uint32_t)(w1 >> 32), lo1 = (uint32_t)w1;
+  float f0, f1;
+  if (s == 0) {
+    f0 = (float)((int)hi0 >> 16);
+    f1 = (float)((int)hi1 >> 16);
+  } else {
+    const int byte = 6 - s;  // of the 64-bit sum
+    const uint32_t a0 = byte >= 4 ? hi0 : lo0, a1 = byte >= 4 ? hi1 : lo1;
+    const uint32_t sel = 0x7650u | (uint32_t)(byte & 3);
+    f0 = __uint_as_float(__byte_perm(a0, 0x4B000000u, sel)) - 8388736.0f;
+    f1 = __uint_as_float(__byte_perm(a1, 0x4B000000u, sel)) - 8388736.0f;
+  }
+  return __byte_perm(__float_as_uint(f0), __float_as_uint(f1), 0x7632);
 }
 
 __device__ __forceinline__ int oz_warp_imax(int v) {
@@ -548,9 +608,10 @@ __device__ __forceinline__ int oz_word_exp(unsigned long long w, unsigned long l
 
 // Balancing exponents of one pass, both operands in one launch. Blocks
 // [0, nab): 32 rows of A (m x kb) each; warp w takes columns k = w, w+8, ...
-// (one coalesced 256-byte load per column), reduces the lanes' exponent keys
-// with one __reduce_max_sync and keeps the column's maximum in shared memory:
-// c_k. Blocks after that: 64 columns of B (kb x n) each; warp w takes columns
+// (one coalesced 256-byte load per column, all of them issued before the first
+// is used: one by one, as a bound test before each load made them, the pass took
+// 32 memory latencies, 35 us at any size), reduces the lanes' exponent keys with
+// one __reduce_max_sync and keeps the column's maximum in shared memory: c_k. Blocks after that: 64 columns of B (kb x n) each; warp w takes columns
 // w, w+8, ..., lane l rows l, l+32, ...: h_k. Each block publishes its
 // maxima with atomicMax into the epoch-tagged words. Small blocks with many
 // independent loads, so the pass over both operands runs near copy speed.
@@ -562,33 +623,38 @@ oz_kscale_kernel(const double* __restrict__ A, long long lda, int m, const doubl
   __shared__ unsigned red[8][OZ_KMAX];
   if ((int)blockIdx.x < nab) {
     const int i = (int)blockIdx.x * 32 + lane;
-    const double* arow = A + i;
-#pragma unroll 8
-    for (int k = warp; k < kb; k += 8) {
-      const unsigned v = (i < m) ? oz_ekey(arow[(long long)k * lda]) : 0u;
-      const unsigned r = __reduce_max_sync(0xffffffffu, v);
-      if (lane == 0) red[0][k] = r;
+    const double* arow = A + (i < m ? i : m - 1);  // (a repeated row changes no maximum)
+    double v[OZ_KMAX / 8];  // every load of the warp's columns in flight at once
+#pragma unroll
+    for (int q = 0; q < OZ_KMAX / 8; ++q) v[q] = arow[(long long)min(warp + 8 * q, kb - 1) * lda];
+#pragma unroll
+    for (int q = 0; q < OZ_KMAX / 8; ++q) {
+      const unsigned r = __reduce_max_sync(0xffffffffu, oz_ekey(v[q]));
+      if (lane == 0) red[0][warp + 8 * q] = r;
     }
     __syncthreads();
     const int k = threadIdx.x;
-    if (k < kb && red[0][k]) atomicMax(kinfo + OZ_KI_C + k, (epoch << 12) | red[0][k]);
+    if (k < kb && red[0][k]) oz_raise_key(kinfo + OZ_KI_C + k, (epoch << 12) | red[0][k]);
     return;
   }
   const int c0 = ((int)blockIdx.x - nab) * 64;
   unsigned km[OZ_KMAX / 32];
 #pragma unroll
   for (int r = 0; r < OZ_KMAX / 32; ++r) km[r] = 0u;
-#pragma unroll 2
-  for (int q = 0; q < 8; ++q) {
-    const int j = c0 + warp + 8 * q;
-    if (j < n) {
-      const double* col = B + (long long)j * ldb;
 #pragma unroll
-      for (int r = 0; r < OZ_KMAX / 32; ++r) {
-        const int k = lane + 32 * r;
-        if (k < kb) km[r] = max(km[r], oz_ekey(col[k]));
-      }
+  for (int q0 = 0; q0 < 8; q0 += 4) {
+    double v[4][OZ_KMAX / 32];  // four columns' loads in flight
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const double* col = B + (long long)min(c0 + warp + 8 * (q0 + q), n - 1) * ldb;
+#pragma unroll
+      for (int r = 0; r < OZ_KMAX / 32; ++r) v[q][r] = col[min(lane + 32 * r, kb - 1)];
     }
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+      for (int r = 0; r < OZ_KMAX / 32; ++r)
+        if (lane + 32 * r < kb) km[r] = max(km[r], oz_ekey(v[q][r]));
   }
 #pragma unroll
   for (int r = 0; r < OZ_KMAX / 32; ++r) red[warp][lane + 32 * r] = km[r];
@@ -598,7 +664,7 @@ oz_kscale_kernel(const double* __restrict__ A, long long lda, int m, const doubl
     unsigned v = 0u;
 #pragma unroll
     for (int w = 0; w < 8; ++w) v = max(v, red[w][k]);
-    if (v) atomicMax(kinfo + OZ_KI_H + k, (epoch << 12) | v);
+    if (v) oz_raise_key(kinfo + OZ_KI_H + k, (epoch << 12) | v);
   }
 }
 
@@ -703,24 +769,23 @@ oz_split_kernel(const double* __restrict__ A, long long lda, int m, const double
     const int e = s_e[r];
     const bool zero = s_bad[r] != 0 || e == OZ_NOEXP;
     for (int k0 = 0; k0 < kpad; k0 += 64) {
-      unsigned long long U[8];
-      bool neg[8];
+      unsigned long long W[8];
 #pragma unroll
       for (int q = 0; q < 8; ++q) {
         const int kk = k0 + g * 8 + q;
         const unsigned long long bits = sA[kk * 33 + r];
-        neg[q] = (bits >> 63) != 0ULL;
         const int d = s_d[kk];
-        U[q] = (zero || d == OZ_NOEXP) ? 0ULL : oz_fixed(bits & kMagMask, e + d);
+        W[q] = (zero || d == OZ_NOEXP) ? kDigitBias : oz_digits(bits, e + d);
       }
       if (row < m_pad) {
 #pragma unroll
         for (int sl = 0; sl < OZ_S; ++sl) {
-          __align__(16) __nv_bfloat16 h[8];
-#pragma unroll
-          for (int q = 0; q < 8; ++q) h[q] = oz_slice_bf16(U[q], sl, neg[q]);
-          *reinterpret_cast<uint4*>(Sa + ((size_t)sl * m_pad + row) * kpad + k0 + g * 8) =
-              *reinterpret_cast<const uint4*>(h);
+          uint4 h;
+          h.x = oz_slice2(W[0], W[1], sl);
+          h.y = oz_slice2(W[2], W[3], sl);
+          h.z = oz_slice2(W[4], W[5], sl);
+          h.w = oz_slice2(W[6], W[7], sl);
+          *reinterpret_cast<uint4*>(Sa + ((size_t)sl * m_pad + row) * kpad + k0 + g * 8) = h;
         }
       }
     }
@@ -761,12 +826,13 @@ oz_split_kernel(const double* __restrict__ A, long long lda, int m, const double
   for (int q = 0; q < OZ_KMAX / 32; ++q) {
     const int kk = lane + 32 * q;
     if (kk >= kpad) break;
-    const bool neg = (bits[q] >> 63) != 0ULL;
     const int d = s_d[kk];
-    const unsigned long long U =
-        (bad || f == OZ_NOEXP || d == OZ_NOEXP) ? 0ULL : oz_fixed(bits[q] & kMagMask, f - d);
+    const unsigned long long W =
+        (bad || f == OZ_NOEXP || d == OZ_NOEXP) ? kDigitBias : oz_digits(bits[q], f - d);
 #pragma unroll
-    for (int sl = 0; sl < OZ_S; ++sl) Sb[((size_t)sl * n_pad + j) * kpad + kk] = oz_slice_bf16(U, sl, neg);
+    for (int sl = 0; sl < OZ_S; ++sl)
+      Sb[((size_t)sl * n_pad + j) * kpad + kk] =
+          __ushort_as_bfloat16((unsigned short)(oz_slice2(W, W, sl) & 0xffffu));
   }
 }
 

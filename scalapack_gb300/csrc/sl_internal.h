@@ -66,7 +66,7 @@ size_t oz_scratch_bytes(int m, int n, int k);
 void oz_set_tiles_per_cta(int t);
 bool oz_fits(const OzScratch& sc, int m, int n, int k);
 // C (m x n) += alpha * A (m x k) * B (k x n), FP64, column-major, on the BF16
-// tensor cores through exact 7-bit slices (needs oz_fits), balanced by the
+// tensor cores through exact 8-bit slices (needs oz_fits), balanced by the
 // column maxima of A; a pass whose slices would exceed the error budget is
 // computed in FP64 arithmetic by the same launches. B may alias C (same
 // pointer and leading dimension): the slices are cut before C is written, and
