@@ -14,15 +14,14 @@
 // so the tail of the launch is made of small systems); CTAs of one persistent
 // grid take the next system from an atomic ticket until the queue is empty.
 //
-// Per system, one CTA:
-//   factor   blocked right-looking LU with 32-column panels held in shared
-//            memory (IDAMAX by warp shuffles, swap, reciprocal scale, rank-1),
-//            row interchanges on the other columns, U12 by forward
-//            substitution from the shared L11, trailing update as a
-//            register-tiled GEMM (each thread owns rows, CH columns at a time)
-//   solve    composed permutation in shared memory, then 32-row blocked
-//            forward / backward substitution (one warp per right-hand side
-//            for the diagonal blocks, all threads for the off-diagonal update)
+// Per system, one CTA (two or three share an SM):
+//   factor   blocked right-looking LU with 16-column panels held in shared
+//            memory (factor_system), the right-hand sides among the columns it
+//            updates, so that their forward solve is part of it; the trailing
+//            update as a register-tiled GEMM (each thread owns rows)
+//   solve    32-row blocked backward (refinement steps: forward too)
+//            substitution, one warp per right-hand side for the diagonal blocks,
+//            all threads for the off-diagonal update
 //   refine   (mode 1) FP32 factors, FP64 residual and update, at most kMaxIr
 //            steps; a system that does not reach the tolerance is queued for
 //            the FP64 pass, which is a second persistent launch in the same
@@ -39,13 +38,14 @@
 #include <vector>
 
 #include "common.cuh"
+#include "lu_kernels.cuh"
 #include "sl_internal.h"
 
 namespace sl {
 
 constexpr int kBMaxN = 512;   // largest system order
 constexpr int kBMaxRhs = 8;   // largest number of right-hand sides
-constexpr int kBPB = 32;      // panel width
+constexpr int kBPB = 16;      // panel width
 constexpr int kMaxIr = 10;    // refinement steps in mode 1
 
 struct BatchArgs {
@@ -69,274 +69,312 @@ struct BatchArgs {
   int* iters;            // refinement steps; -1 = solved by the FP64 pass after refinement stalled
   double* sresid;
   double tol;
+  int nmax, rmax;        // largest order and number of right-hand sides in the batch
 };
 
-// ------------------------------------------------------------ helpers
-template <typename T>
-__device__ __forceinline__ void block_argmax(const T* P, int ldp, int k, int m, int& piv_out,
-                                             double* s_key, int* s_row) {
-  // IDAMAX over P[k..m-1][k]: first maximal |x|, NaN never wins except as the
-  // first element (reference BLAS).
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
-  double key = -2.0;
-  int row = 0x7fffffff;
-  for (int r = k + tid; r < m; r += blockDim.x) amax_combine(key, row, amax_key((double)P[r * ldp + k]), r);
-  warp_amax(key, row);
-  if (lane == 0) { s_key[warp] = key; s_row[warp] = row; }
-  __syncthreads();
-  if (warp == 0) {
-    key = lane < nw ? s_key[lane] : -2.0;
-    row = lane < nw ? s_row[lane] : 0x7fffffff;
-    warp_amax(key, row);
-    if (lane == 0) {
-      double d = (double)P[k * ldp + k];
-      if (d != d || key == 0.0) row = k;
-      s_row[0] = row;
-    }
-  }
-  __syncthreads();
-  piv_out = s_row[0];
-}
+// ------------------------------------------------------------ factorization
+constexpr int kPL = kBPB + 1;  // shared row stride of the panel: conflict-free row and column walks
 
-// Factor the n x n matrix W (column-major, ld n) in place. ipiv receives
-// 0-based rows; returns INFO (first zero pivot, 1-based) in *info.
-// stage / stage_len: shared scratch idle during the factorization, used to
-// apply each panel's row interchanges to the other columns.
-template <typename T, int CH>
-__device__ void factor_system(T* W, int n, int* ipiv, int* info, unsigned char* smem, T* stage,
-                              int stage_len) {
-  T* P = reinterpret_cast<T*>(smem);               // [kBMaxN][kBPB+1] panel, row-major
-  T* Us = P + kBMaxN * (kBPB + 1);                   // [kBPB][CH+1] U12 chunk (padded rows)
-  constexpr int UL = CH + 1;
-  __shared__ double s_key[32];
-  __shared__ int s_row[32];
+// Columns of a trailing update's chunk.
+template <typename T>
+__host__ __device__ constexpr int chunk_cols() { return sizeof(T) == 8 ? 16 : 32; }
+
+// Shared memory of one system of order <= nmax: while it is factored the panel
+// P [nmax][kPL], the rows' labels, and two chunks of U; afterwards, over the same
+// bytes, the right-hand sides (Xs, and Cx for FP32 factors), the residual, X in
+// FP64 and a diagonal block. The row order (org) lasts through both.
+template <typename T>
+struct BatchSmem {
+  T *P, *Us;
+  int* lab;
+  int* org;
+  T *Xs, *Ds;
+  double *Xsh, *Rs;
+  static size_t factor_bytes(int nmax) {
+    return sizeof(T) * ((size_t)nmax * kPL + 2 * kBPB * chunk_cols<T>()) + sizeof(int) * (size_t)nmax;
+  }
+  static size_t solve_bytes(int nmax, int rmax) {
+    // Xs and X in FP64 share their bytes; Rs (FP32 factors only) stands alone
+    return sizeof(double) * (size_t)nmax * rmax * (sizeof(T) == 8 ? 1 : 2) + sizeof(T) * 32 * 33;
+  }
+  static size_t bytes(int nmax, int rmax) {
+    const size_t f = factor_bytes(nmax), v = solve_bytes(nmax, rmax);
+    return sizeof(int) * (size_t)nmax + (f > v ? f : v) + 16;
+  }
+  __device__ BatchSmem(unsigned char* p, int nmax, int rmax) {
+    org = reinterpret_cast<int*>(p);
+    unsigned char* q = p + (sizeof(int) * (size_t)nmax + 15) / 16 * 16;
+    P = reinterpret_cast<T*>(q);
+    Us = P + (size_t)nmax * kPL;
+    lab = reinterpret_cast<int*>(Us + 2 * kBPB * chunk_cols<T>());
+    Xsh = reinterpret_cast<double*>(q);
+    Xs = reinterpret_cast<T*>(q);
+    Rs = Xsh + (size_t)nmax * rmax;
+    Ds = sizeof(T) == 8 ? reinterpret_cast<T*>(Xsh + (size_t)nmax * rmax)
+                        : reinterpret_cast<T*>(Rs + (size_t)nmax * rmax);
+  }
+};
+
+// Factor the leading n columns of the n x ncols matrix W (column-major, ld n)
+// in place and apply the interchanges and inv(L) to the columns beyond (the
+// right-hand sides: their forward solve). ipiv receives 0-based rows, org[i] the
+// original row that ends in row i; *info the first zero pivot (1-based) or 0.
+//
+// A panel's rows keep their place in shared memory and carry a label, the row
+// where their content stands after the interchanges so far (~k once it is pivot
+// row k), so a column takes one barrier: every warp reduces the warps' IDAMAX
+// candidates (integer keys, warp_best), each thread then scales and updates its
+// rows from the pivot row where it stands and forms their keys for the next
+// column. The labels are the panel's interchanges in composite form: one thread
+// per other column gathers its pivot rows, sends the displaced rows where they
+// go and solves with L11 in registers. Bound: the FP64 unit (FP64 factors) in the
+// trailing update; two or three systems share an SM so that the panels of one
+// run beside the updates of another. Measured, 4096 systems of order 16 .. 512:
+// FP64 119 ms (the unit's floor is 103; 188 with 32-column panels of four
+// barriers and FP64 compares per column and one system per SM), FP32 factors
+// with refinement 35 ms (87).
+template <typename T, int NT>
+__device__ __forceinline__ void factor_system(T* W, int n, int ncols, int* ipiv, int* info, const BatchSmem<T>& sm) {
+  constexpr int CH = chunk_cols<T>();
+  constexpr int NW = NT / 32;
+  T* P = sm.P;
+  int* lab = sm.lab;
+  __shared__ long long s_wk[2][NW];
+  __shared__ int s_wr[2][NW], s_wl[2][NW];
+  __shared__ int s_rowof[kBPB], s_dsp[kBPB];
+  __shared__ T s_L[kBPB][kPL];  // L11 by label
   __shared__ int s_info;
-  __shared__ int s_trow[2 * kBPB], s_tsrc[2 * kBPB], s_tcnt;
-  const int tid = threadIdx.x, NT = blockDim.x;
-  const int PL = kBPB + 1;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (tid == 0) s_info = 0;
+  for (int r = tid; r < n; r += NT) sm.org[r] = r;
+  auto row_key = [&](T v, int label, int k) -> long long {
+    const long long key = amax_ikey(v);
+    return (key < 0 && label == k) ? LLONG_MAX : key;  // IDAMAX keeps a leading NaN
+  };
+  auto put_candidate = [&](int buf, long long key, int label, int lrow) {
+    if (lane == warp_best(key, label)) {
+      s_wk[buf][warp] = key;
+      s_wr[buf][warp] = label;
+      s_wl[buf][warp] = lrow;
+    }
+  };
   for (int j = 0; j < n; j += kBPB) {
-    const int jb = min(kBPB, n - j);
-    const int m = n - j;  // panel rows
-    // load the panel rows j..n-1, columns j..j+jb-1
-    for (int idx = tid; idx < m * jb; idx += NT) {
-      int r = idx % m, c = idx / m;
-      P[r * PL + c] = W[(j + r) + (long long)(j + c) * n];
+    const int jb = min(kBPB, n - j), m = n - j;
+    {
+      long long key = -2;
+      int label = INT_MAX, lrow = 0;
+      for (int r = tid; r < m; r += NT) {
+        const T* src = W + (j + r) + (long long)j * n;
+        T v[kBPB];
+#pragma unroll
+        for (int c = 0; c < kBPB; ++c) v[c] = c < jb ? src[(long long)c * n] : (T)0;
+#pragma unroll
+        for (int c = 0; c < kBPB; ++c) P[r * kPL + c] = v[c];
+        lab[r] = r;
+        const long long k2 = row_key(v[0], r, 0);
+        if (k2 > key) { key = k2; label = r; lrow = r; }
+      }
+      put_candidate(0, key, label, lrow);
     }
-    __syncthreads();
     for (int k = 0; k < jb; ++k) {
-      int piv;
-      block_argmax<T>(P, PL, k, m, piv, s_key, s_row);
-      if (tid == 0) ipiv[j + k] = j + piv;
-      if (piv != k)
-        for (int c = tid; c < jb; c += NT) {
-          T t = P[k * PL + c];
-          P[k * PL + c] = P[piv * PL + c];
-          P[piv * PL + c] = t;
+      const int buf = k & 1;
+      __syncthreads();
+      long long key = lane < NW ? s_wk[buf][lane] : -3;
+      int label = lane < NW ? s_wr[buf][lane] : INT_MAX;
+      const int cw = warp_best(key, label);
+      const int lr = s_wl[buf][cw];
+      key = s_wk[buf][cw];
+      label = s_wr[buf][cw];
+      const T* U = P + lr * kPL;
+      const T g = U[k];
+      T rinv;  // ONE/GMAX, 1 for a zero pivot (its column is not scaled)
+      bool zero;
+      if constexpr (sizeof(T) == 8) {
+        const unsigned long long kb = (unsigned long long)key, gb = (unsigned long long)__double_as_longlong(g);
+        zero = (gb << 1) == 0;
+        if (kb - 1ULL < 0x7FEFFFFFFFFFFFFFULL)
+          rinv = __longlong_as_double(__double_as_longlong(recip_bits(kb)) | (long long)(gb & (1ULL << 63)));
+        else
+          rinv = zero ? 1.0 : 1.0 / g;
+      } else {
+        zero = g == (T)0;
+        rinv = zero ? (T)1 : (T)1 / g;
+      }
+      if (tid == 0) {
+        ipiv[j + k] = j + label;
+        if (zero && s_info == 0) s_info = j + k + 1;
+      }
+      long long nkey = -2;
+      int nlab = INT_MAX, nrow = 0;
+      const int kn = k + 1;
+      for (int r = tid; r < m; r += NT) {
+        int lb = lab[r];
+        if (r == lr) lab[r] = ~k;
+        if (lb < 0 || r == lr) continue;
+        if (lb == k) lab[r] = lb = label;
+        T* row = P + r * kPL;
+        const T l = row[k] * rinv;
+        row[k] = l;
+        if (kn < jb) {
+          const T v = fma(-l, U[kn], row[kn]);
+          row[kn] = v;
+          const long long k2 = row_key(v, lb, kn);
+          if (k2 > nkey || (k2 == nkey && lb < nlab)) { nkey = k2; nlab = lb; nrow = r; }
+#pragma unroll 4
+          for (int c = kn + 1; c < jb; ++c) row[c] = fma(-l, U[c], row[c]);
         }
-      __syncthreads();
-      const T g = P[k * PL + k];
-      if (g == (T)0) {
-        if (tid == 0 && s_info == 0) s_info = j + k + 1;
       }
-      const T rinv = (g != (T)0) ? (T)1 / g : (T)0;
-      for (int r = k + 1 + tid; r < m; r += NT) {
-        T l = P[r * PL + k];
-        if (g != (T)0) l *= rinv;
-        P[r * PL + k] = l;
-        for (int c = k + 1; c < jb; ++c) P[r * PL + c] = fma(-l, P[k * PL + c], P[r * PL + c]);
-      }
-      __syncthreads();
-    }
-    // write the panel back
-    for (int idx = tid; idx < m * jb; idx += NT) {
-      int r = idx % m, c = idx / m;
-      W[(j + r) + (long long)(j + c) * n] = P[r * PL + c];
+      if (kn < jb) put_candidate(buf ^ 1, nkey, nlab, nrow);
     }
     __syncthreads();
-    // Row interchanges on the other columns (PDLASWP) as one composite
-    // permutation: warp 0 replays the jb swaps on row labels (rows j..j+jb-1
-    // and the pivot rows below), then every moved value of a chunk of
-    // columns is read into `stage` before any is written back.
-    if (tid < 32) {
-      const int lane = tid;
-      int cnt = jb;
-      for (int e = lane; e < jb; e += 32) { s_trow[e] = j + e; s_tsrc[e] = j + e; }
-      __syncwarp();
-      for (int k = 0; k < jb; ++k) {
-        const int p = ipiv[j + k];
-        if (p == j + k) continue;
-        int e = -1;
-        if (p < j + jb) {
-          e = p - j;
-        } else {
-          for (int base = jb; base < cnt && e < 0; base += 32) {
-            const int q = base + lane;
-            const unsigned hit = __ballot_sync(0xffffffffu, q < cnt && s_trow[q] == p);
-            if (hit) e = base + __ffs(hit) - 1;
-          }
-          if (e < 0) {
-            e = cnt++;
-            if (lane == 0) { s_trow[e] = p; s_tsrc[e] = p; }
-          }
+    // rows to where their content stands; the interchanges for the other columns
+    int mv[kBMaxN / NT > 0 ? kBMaxN / NT : 1];
+    {
+      int q = 0;
+      for (int r = tid; r < m; r += NT, ++q) {
+        const int lb = lab[r], L = lb < 0 ? ~lb : lb;
+        mv[q] = sm.org[j + r];
+        T* dst = W + (j + L) + (long long)j * n;
+#pragma unroll
+        for (int c = 0; c < kBPB; ++c)
+          if (c < jb) dst[(long long)c * n] = P[r * kPL + c];
+        if (L < jb) {
+          s_rowof[L] = r;
+#pragma unroll
+          for (int c = 0; c < kBPB; ++c) s_L[L][c] = P[r * kPL + c];
         }
-        __syncwarp();
-        if (lane == 0) { const int t = s_tsrc[k]; s_tsrc[k] = s_tsrc[e]; s_tsrc[e] = t; }
-        __syncwarp();
+        if (r < jb) s_dsp[r] = L >= jb ? L : -1;
       }
-      if (lane == 0) s_tcnt = cnt;
     }
     __syncthreads();
     {
-      const int cnt = s_tcnt;
-      const int cw = stage_len / cnt;  // columns per chunk (cnt <= 64)
-      for (int c0 = 0; c0 < n; c0 += cw) {
-        const int nc = min(cw, n - c0);
-        for (int idx = tid; idx < nc * cnt; idx += NT) {
-          const int e = idx % cnt, c = c0 + idx / cnt;
-          if ((c < j || c >= j + jb) && s_tsrc[e] != s_trow[e])
-            stage[idx] = W[s_tsrc[e] + (long long)c * n];
-        }
-        __syncthreads();
-        for (int idx = tid; idx < nc * cnt; idx += NT) {
-          const int e = idx % cnt, c = c0 + idx / cnt;
-          if ((c < j || c >= j + jb) && s_tsrc[e] != s_trow[e])
-            W[s_trow[e] + (long long)c * n] = stage[idx];
-        }
-        __syncthreads();
+      int q = 0;
+      for (int r = tid; r < m; r += NT, ++q) {
+        const int lb = lab[r], L = lb < 0 ? ~lb : lb;
+        if (L != r) sm.org[j + L] = mv[q];
       }
     }
-    const int nr = n - j - jb;  // trailing columns
-    if (nr > 0) {
-      // U12 = L11^-1 A12, one thread per column, L11 from the shared panel
-      for (int c = j + jb + tid; c < n; c += NT) {
-        T* col = W + (long long)c * n + j;
-        T x[kBPB];
+    // one thread per other column: PDLASWP, and on the right U12 = inv(L11) A12
+    for (int ci = tid; ci < ncols - jb; ci += NT) {
+      const int c = ci < j ? ci : ci + jb;
+      T* col = W + (long long)c * n + j;
+      T x[kBPB], y[kBPB];
 #pragma unroll
-        for (int k = 0; k < kBPB; ++k) x[k] = k < jb ? col[k] : (T)0;
+      for (int k = 0; k < kBPB; ++k) {
+        x[k] = k < jb ? col[s_rowof[k]] : (T)0;
+        y[k] = (k < jb && s_dsp[k] >= 0) ? col[k] : (T)0;
+      }
+#pragma unroll
+      for (int k = 0; k < kBPB; ++k)
+        if (k < jb && s_dsp[k] >= 0) col[s_dsp[k]] = y[k];
+      if (c >= j + jb) {
 #pragma unroll
         for (int k = 0; k < kBPB; ++k)
 #pragma unroll
           for (int r = k + 1; r < kBPB; ++r)
-            if (r < jb) x[r] = fma(-P[r * PL + k], x[k], x[r]);
+            if (r < jb) x[r] = fma(-s_L[r][k], x[k], x[r]);
+      }
 #pragma unroll
-        for (int k = 0; k < kBPB; ++k)
-          if (k < jb) col[k] = x[k];
+      for (int k = 0; k < kBPB; ++k)
+        if (k < jb) col[k] = x[k];
+    }
+    __syncthreads();
+    if (m <= jb) break;
+    // A22 -= L21 U12 (jb = kBPB here): a chunk of U12 in shared memory, each
+    // thread owns rows and CH accumulators, C on its way meanwhile
+    for (int c0 = j + jb, it = 0; c0 < ncols; c0 += CH, ++it) {
+      T* Us = sm.Us + (it & 1) * kBPB * CH;
+      const int cw = min(CH, ncols - c0);
+      for (int idx = tid; idx < kBPB * CH; idx += NT) {
+        const int k = idx % kBPB, c = idx / kBPB;
+        Us[k * CH + c] = c < cw ? W[(j + k) + (long long)(c0 + c) * n] : (T)0;
       }
       __syncthreads();
-      const int mr = m - jb;  // trailing rows
-      if (mr > 0) {
-        // A22 -= L21 * U12 in CH-column chunks: U12 chunk staged in shared memory,
-        // each thread owns rows (coalesced column accesses) and CH accumulators.
-        for (int c0 = j + jb; c0 < n; c0 += CH) {
-          const int cw = min(CH, n - c0);
-          for (int idx = tid; idx < jb * CH; idx += NT) {
-            int k = idx % jb, c = idx / jb;
-            Us[k * UL + c] = c < cw ? W[(j + k) + (long long)(c0 + c) * n] : (T)0;
-          }
-          __syncthreads();
-          for (int r = tid; r < mr; r += NT) {
-            T acc[CH];
+      for (int r = tid; r < m; r += NT) {
+        const int L = lab[r];
+        if (L < 0) continue;
+        T* crow = W + (j + L) + (long long)c0 * n;
+        T cv[CH], acc[CH];
 #pragma unroll
-            for (int c = 0; c < CH; ++c) acc[c] = (T)0;
-            const T* lrow = P + (jb + r) * PL;
-            for (int k = 0; k < jb; ++k) {
-              const T a = lrow[k];
+        for (int c = 0; c < CH; ++c) cv[c] = c < cw ? crow[(long long)c * n] : (T)0;
+        const T* lrow = P + r * kPL;
 #pragma unroll
-              for (int c = 0; c < CH; ++c) acc[c] = fma(a, Us[k * UL + c], acc[c]);
-            }
-            T* crow = W + (j + jb + r) + (long long)c0 * n;
+        for (int k = 0; k < kBPB; ++k) {
+          const T a = lrow[k];
 #pragma unroll
-            for (int c = 0; c < CH; ++c)
-              if (c < cw) crow[(long long)c * n] -= acc[c];
-          }
-          __syncthreads();
+          for (int c = 0; c < CH; ++c) acc[c] = k == 0 ? a * Us[c] : fma(a, Us[k * CH + c], acc[c]);
         }
+#pragma unroll
+        for (int c = 0; c < CH; ++c)
+          if (c < cw) crow[(long long)c * n] = cv[c] - acc[c];
       }
     }
+    __syncthreads();
   }
   __syncthreads();
   if (tid == 0) *info = s_info;
   __syncthreads();
 }
 
-// The row permutation of the factorization (PDLAPIV's interchanges composed):
-// perm[i] = original row that ends up in row i. Computed once per system.
-__device__ void compose_perm(const int* ipiv, int n, int* perm) {
-  for (int i = threadIdx.x; i < n; i += blockDim.x) perm[i] = i;
-  __syncthreads();
-  if (threadIdx.x == 0)
-    for (int i = 0; i < n; ++i) {
-      const int q = ipiv[i];
-      if (q != i) { const int t = perm[i]; perm[i] = perm[q]; perm[q] = t; }
-    }
-  __syncthreads();
+// x / d from r = 1/d, rounded like the division (one correction step).
+__device__ __forceinline__ double div_by(double x, double d, double r) {
+  const double q = x * r;
+  const double f = fma(fma(-d, q, x), r, q);
+  return (f - f == 0.0) ? f : x / d;  // (infinities, zeros and NaN divide)
 }
+__device__ __forceinline__ float div_by(float x, float d, float) { return x / d; }
 
-// Solve with the factors of factor_system: X (n x nrhs, ldx) holds the
-// right-hand sides on entry and the solution on exit. Xs: shared scratch of
-// n*nrhs values; perm: the composed permutation (shared memory).
-template <typename T>
-__device__ void solve_system(const T* W, int n, const int* perm, T* X, int ldx, int nrhs, T* Xs) {
-  const int tid = threadIdx.x, NT = blockDim.x, lane = tid & 31, warp = tid >> 5;
-  const int nw = NT >> 5;
-  for (int idx = tid; idx < n * nrhs; idx += NT) {
-    int i = idx % n, c = idx / n;
-    Xs[i + c * n] = X[perm[i] + (long long)c * ldx];
-  }
-  __syncthreads();
-  // forward (unit lower), 32-row blocks
-  for (int k0 = 0; k0 < n; k0 += 32) {
-    const int kb = min(32, n - k0);
-    for (int c = warp; c < nrhs; c += nw) {
-      T x = lane < kb ? Xs[k0 + lane + c * n] : (T)0;
-      for (int i = 0; i < kb; ++i) {
-        T xi = __shfl_sync(0xffffffffu, x, i);
-        if (lane > i && lane < kb) x = fma(-W[(k0 + lane) + (long long)(k0 + i) * n], xi, x);
-      }
-      if (lane < kb) Xs[k0 + lane + c * n] = x;
-    }
-    __syncthreads();
-    for (int r = k0 + kb + tid; r < n; r += NT) {
-      T acc[kBMaxRhs];
-#pragma unroll
-      for (int c = 0; c < kBMaxRhs; ++c) acc[c] = (T)0;
-      for (int i = 0; i < kb; ++i) {
-        const T l = W[r + (long long)(k0 + i) * n];
-#pragma unroll
-        for (int c = 0; c < kBMaxRhs; ++c)
-          if (c < nrhs) acc[c] = fma(l, Xs[k0 + i + c * n], acc[c]);
-      }
-#pragma unroll
-      for (int c = 0; c < kBMaxRhs; ++c)
-        if (c < nrhs) Xs[r + c * n] -= acc[c];
-    }
-    __syncthreads();
-  }
-  // backward (non-unit upper), 32-row blocks from the bottom
+// Triangular solve with the unit-lower L (LOWER) or the upper U of the factors
+// in W on Xs (n x nrhs, shared), 32-row blocks: the diagonal block in shared
+// memory, a warp per right-hand side, then all threads subtract its columns
+// from the remaining rows, 16 loads in flight.
+template <typename T, int NT, bool LOWER>
+__device__ __forceinline__ void solve_tri(const T* W, int n, T* Xs, int nrhs, T* Ds) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nblk = (n + 31) / 32;
-  for (int b = nblk - 1; b >= 0; --b) {
-    const int k0 = b * 32;
-    const int kb = min(32, n - k0);
-    for (int c = warp; c < nrhs; c += nw) {
+  for (int bi = 0; bi < nblk; ++bi) {
+    const int k0 = (LOWER ? bi : nblk - 1 - bi) * 32, kb = min(32, n - k0);
+    for (int idx = tid; idx < 32 * 32; idx += NT) {
+      const int i = idx & 31, k = idx >> 5;
+      Ds[k * 33 + i] = (i < kb && k < kb) ? W[(k0 + i) + (long long)(k0 + k) * n] : (T)0;
+    }
+    __syncthreads();
+    for (int c = warp; c < nrhs; c += NT / 32) {
       T x = lane < kb ? Xs[k0 + lane + c * n] : (T)0;
-      for (int i = kb - 1; i >= 0; --i) {
-        if (lane == i) x = x / W[(k0 + i) + (long long)(k0 + i) * n];
-        T xi = __shfl_sync(0xffffffffu, x, i);
-        if (lane < i) x = fma(-W[(k0 + lane) + (long long)(k0 + i) * n], xi, x);
+      if (LOWER) {
+        for (int i = 0; i < kb; ++i) {
+          const T xi = __shfl_sync(0xffffffffu, x, i);
+          if (lane > i) x = fma(-Ds[i * 33 + lane], xi, x);
+        }
+      } else {
+        const T d = lane < kb ? Ds[lane * 33 + lane] : (T)1;
+        const T rd = (T)1 / d;
+        for (int i = kb - 1; i >= 0; --i) {
+          const T q = div_by(x, d, rd);
+          if (lane == i) x = q;
+          const T xi = __shfl_sync(0xffffffffu, x, i);
+          if (lane < i) x = fma(-Ds[i * 33 + lane], xi, x);
+        }
       }
       if (lane < kb) Xs[k0 + lane + c * n] = x;
     }
     __syncthreads();
-    for (int r = tid; r < k0; r += NT) {
+    const int lo = LOWER ? k0 + kb : 0, hi = LOWER ? n : k0;
+    for (int r = lo + tid; r < hi; r += NT) {
       T acc[kBMaxRhs];
 #pragma unroll
       for (int c = 0; c < kBMaxRhs; ++c) acc[c] = (T)0;
-      for (int i = 0; i < kb; ++i) {
-        const T u = W[r + (long long)(k0 + i) * n];
+      for (int i0 = 0; i0 < kb; i0 += 16) {
+        T l[16];
 #pragma unroll
-        for (int c = 0; c < kBMaxRhs; ++c)
-          if (c < nrhs) acc[c] = fma(u, Xs[k0 + i + c * n], acc[c]);
+        for (int i = 0; i < 16; ++i) l[i] = W[r + (long long)(k0 + min(i0 + i, kb - 1)) * n];
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+          if (i0 + i < kb) {
+#pragma unroll
+            for (int c = 0; c < kBMaxRhs; ++c)
+              if (c < nrhs) acc[c] = fma(l[i], Xs[k0 + i0 + i + c * n], acc[c]);
+          }
       }
 #pragma unroll
       for (int c = 0; c < kBMaxRhs; ++c)
@@ -344,145 +382,155 @@ __device__ void solve_system(const T* W, int n, const int* perm, T* X, int ldx, 
     }
     __syncthreads();
   }
-  for (int idx = tid; idx < n * nrhs; idx += NT) {
-    int i = idx % n, c = idx / n;
-    X[i + (long long)c * ldx] = Xs[i + c * n];
-  }
-  __syncthreads();
 }
 
-// NaN-propagating maximum (a NaN, once seen, stays): the tester's norm semantics.
-__device__ __forceinline__ double nanmax(double m, double v) { return (v > m || v != v) ? v : m; }
+// |v| as an integer: larger for larger magnitudes, largest for NaN, so that a
+// maximum keeps a NaN once seen (the tester's norm semantics) without FP64
+// compares.
+__device__ __forceinline__ unsigned long long mag_key(double v) {
+  return (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffULL;
+}
+__device__ __forceinline__ unsigned long long warp_max64(unsigned long long v) {
+  const unsigned h = (unsigned)(v >> 32), hm = __reduce_max_sync(0xffffffffu, h);
+  const unsigned l = __reduce_max_sync(0xffffffffu, h == hm ? (unsigned)v : 0u);
+  return ((unsigned long long)hm << 32) | l;
+}
 
-// R = B - A X (FP64) into shared Rs (n x nrhs); returns the scaled residual
-// max_c ||r_c|| / (||A|| ||x_c|| n eps) (tester semantics, LIN/pdlaschk.f).
-// X is staged in shared memory (Xsh, n*nrhs doubles) so the pass over A is the
-// only global stream, read with 8 loads in flight per thread; ||A||_inf is
-// passed in (*anorm >= 0, from the copy into the working matrix) or computed.
-__device__ double residual_system(const double* A, int lda, int n, const double* B, int ldb,
-                                  const double* X, int ldx, int nrhs, double* Rs, double* s_red,
-                                  double* Xsh, double* anorm) {
-  const int tid = threadIdx.x, NT = blockDim.x, lane = tid & 31, warp = tid >> 5;
-  const int nw = NT >> 5;
-  __shared__ double s_rm[32][kBMaxRhs], s_xm[32][kBMaxRhs];
-  for (int idx = tid; idx < n * nrhs; idx += NT) {
-    const int i = idx % n, c = idx / n;
-    Xsh[i + c * n] = X[i + (long long)c * ldx];
-  }
-  __syncthreads();
-  const bool need_norm = !(*anorm >= 0.0);
-  double rowmax = 0.0;
-  double rm[kBMaxRhs], xm[kBMaxRhs];
+// Scaled residual max_c ||b_c - A x_c|| / (||A|| ||x_c|| n eps) (tester
+// semantics, LIN/pdlaschk.f) of Xsh (n x nrhs, shared); with Rs set, the
+// residuals go there. rmax[c] receives the magnitude of ||r_c||_inf. The pass
+// over A is the only global stream, 8 loads in flight per thread.
+template <int NT>
+__device__ __forceinline__ double residual_system(const double* A, int lda, int n, const double* B, int ldb,
+                                  const double* Xsh, int nrhs, double* Rs, double anorm, double* rmax) {
+  constexpr int NW = NT / 32;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  __shared__ unsigned long long s_rm[NW][kBMaxRhs], s_xm[NW][kBMaxRhs];
+  __shared__ double s_worst;
+  unsigned long long rm[kBMaxRhs], xm[kBMaxRhs];
 #pragma unroll
-  for (int c = 0; c < kBMaxRhs; ++c) { rm[c] = 0.0; xm[c] = 0.0; }
+  for (int c = 0; c < kBMaxRhs; ++c) { rm[c] = 0ULL; xm[c] = 0ULL; }
   for (int r = tid; r < n; r += NT) {
     double acc[kBMaxRhs];
 #pragma unroll
     for (int c = 0; c < kBMaxRhs; ++c) acc[c] = (c < nrhs) ? B[r + (long long)c * ldb] : 0.0;
-    double rs = 0.0;
     const double* ar = A + r;
-#pragma unroll 8
-    for (int k = 0; k < n; ++k) {
-      const double a = ar[(long long)k * lda];
-      if (need_norm) rs += fabs(a);
+    for (int k0 = 0; k0 < n; k0 += 8) {
+      double a[8];
 #pragma unroll
-      for (int c = 0; c < kBMaxRhs; ++c)
-        if (c < nrhs) acc[c] = fma(-a, Xsh[k + c * n], acc[c]);
+      for (int k = 0; k < 8; ++k) a[k] = ar[(long long)min(k0 + k, n - 1) * lda];
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (k0 + k < n) {
+#pragma unroll
+          for (int c = 0; c < kBMaxRhs; ++c)
+            if (c < nrhs) acc[c] = fma(-a[k], Xsh[k0 + k + c * n], acc[c]);
+        }
     }
-    rowmax = fmax(rowmax, rs);
 #pragma unroll
     for (int c = 0; c < kBMaxRhs; ++c)
       if (c < nrhs) {
-        Rs[r + c * n] = acc[c];
-        rm[c] = nanmax(rm[c], fabs(acc[c]));
-        xm[c] = nanmax(xm[c], fabs(Xsh[r + c * n]));
+        if (Rs) Rs[r + c * n] = acc[c];
+        rm[c] = max(rm[c], mag_key(acc[c]));
+        xm[c] = max(xm[c], mag_key(Xsh[r + c * n]));
       }
   }
-  // block reductions: max row sum, and per column max |r| and max |x|
-  for (int off = 16; off > 0; off >>= 1) {
-    rowmax = fmax(rowmax, __shfl_xor_sync(0xffffffffu, rowmax, off));
 #pragma unroll
-    for (int c = 0; c < kBMaxRhs; ++c) {
-      rm[c] = nanmax(rm[c], __shfl_xor_sync(0xffffffffu, rm[c], off));
-      xm[c] = nanmax(xm[c], __shfl_xor_sync(0xffffffffu, xm[c], off));
+  for (int c = 0; c < kBMaxRhs; ++c)
+    if (c < nrhs) {
+      const unsigned long long r1 = warp_max64(rm[c]), x1 = warp_max64(xm[c]);
+      if (lane == 0) { s_rm[warp][c] = r1; s_xm[warp][c] = x1; }
     }
-  }
-  if (lane == 0) {
-    s_red[warp] = rowmax;
-#pragma unroll
-    for (int c = 0; c < kBMaxRhs; ++c) { s_rm[warp][c] = rm[c]; s_xm[warp][c] = xm[c]; }
+  __syncthreads();
+  if (warp == 0) {
+    double v = 0.0;
+    if (lane < nrhs) {
+      unsigned long long r1 = 0ULL, x1 = 0ULL;
+      for (int w = 0; w < NW; ++w) { r1 = max(r1, s_rm[w][lane]); x1 = max(x1, s_xm[w][lane]); }
+      const double rn = __longlong_as_double((long long)r1);
+      rmax[lane] = rn;
+      v = rn / (__longlong_as_double((long long)x1) * anorm * ldexp(1.0, -53) * n);
+    }
+    const unsigned long long w = warp_max64(mag_key(v));
+    if (lane == 0) s_worst = __longlong_as_double((long long)w);
   }
   __syncthreads();
-  if (tid == 0) {
-    double an = *anorm;
-    if (need_norm) {
-      an = 0.0;
-      for (int w = 0; w < nw; ++w) an = fmax(an, s_red[w]);
-      *anorm = an;
-    }
-    double worst = 0.0;
-    for (int c = 0; c < nrhs; ++c) {
-      double r1 = 0.0, x1 = 0.0;
-      for (int w = 0; w < nw; ++w) { r1 = nanmax(r1, s_rm[w][c]); x1 = nanmax(x1, s_xm[w][c]); }
-      const double v = r1 / (x1 * an * ldexp(1.0, -53) * n);
-      if (!(v <= worst)) worst = v;
-    }
-    s_red[32] = worst;
-  }
-  __syncthreads();
-  return s_red[32];
+  return s_worst;
 }
 
-template <typename TF, int CH>
-__device__ void run_system(const BatchArgs& a, int sys, bool fp64_pass, unsigned char* smem) {
+template <typename TF, int NT>
+__device__ __forceinline__ void run_system(const BatchArgs& a, int sys, bool fp64_pass, unsigned char* smem) {
   const int n = a.n[sys], nrhs = a.nrhs[sys];
-  const int tid = threadIdx.x, NT = blockDim.x;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const double* A = a.A[sys];
   const int lda = a.lda[sys];
-  TF* W = reinterpret_cast<TF*>(fp64_pass ? a.W64[sys] : a.W[sys]);
+  TF* W = reinterpret_cast<TF*>(fp64_pass ? a.W64[sys] : a.W[sys]);  // n x (n + nrhs)
   int* ipiv = a.ipiv[sys];
   double* X = a.X[sys];
   const int ldx = a.ldx[sys];
   const double* B = a.B[sys];
   const int ldb = a.ldb[sys];
-  // shared layout: factor scratch, then Xs (n*nrhs TF), Rs (n*nrhs double), perm (n ints)
-  unsigned char* after = smem + sizeof(TF) * (kBMaxN * (kBPB + 1) + kBPB * (CH + 1));
-  TF* Xs = reinterpret_cast<TF*>(after);
-  double* Rs = reinterpret_cast<double*>(after + sizeof(double) * kBMaxN * kBMaxRhs);
-  int* perm = reinterpret_cast<int*>(after + 2 * sizeof(double) * kBMaxN * kBMaxRhs);
-  double* Xsh = reinterpret_cast<double*>(after);  // X staged by residual_system (Xs is idle then)
-  __shared__ double s_red[40];
+  const BatchSmem<TF> sm(smem, a.nmax, a.rmax);
+  __shared__ unsigned long long s_red[NT / 32];
+  __shared__ double s_rmax[kBMaxRhs];
+  __shared__ int s_exp[kBMaxRhs];
   __shared__ double s_anorm;
   __shared__ int s_info;
-  __shared__ int s_ok;
-  // working copy in the factorization precision; one thread per row, so the
-  // same pass gives ||A||_inf (row sums of |a|)
+  // Working copy in the factorization precision; one thread per row, so the
+  // same pass gives ||A||_inf (row sums of |a|). The right-hand sides follow
+  // as columns n .. n+nrhs-1 (FP32 factors: each scaled by a power of two), so
+  // that the factorization does their forward solve.
   {
-    double rs_max = 0.0;
+    unsigned long long rs_max = 0ULL;
     for (int r = tid; r < n; r += NT) {
       double rs = 0.0;
       const double* ar = A + r;
-#pragma unroll 8
-      for (int c = 0; c < n; ++c) {
-        const double v = ar[(long long)c * lda];
-        rs += fabs(v);
-        W[r + (long long)c * n] = (TF)v;
+      for (int c0 = 0; c0 < n; c0 += 8) {
+        double v[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[q] = ar[(long long)min(c0 + q, n - 1) * lda];
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+          if (c0 + q < n) {
+            rs += fabs(v[q]);
+            W[r + (long long)(c0 + q) * n] = (TF)v[q];
+          }
       }
-      rs_max = fmax(rs_max, rs);
+      rs_max = max(rs_max, mag_key(rs));
     }
-    for (int off = 16; off > 0; off >>= 1) rs_max = fmax(rs_max, __shfl_xor_sync(0xffffffffu, rs_max, off));
-    if ((tid & 31) == 0) s_red[tid >> 5] = rs_max;
+    rs_max = warp_max64(rs_max);
+    if (lane == 0) s_red[warp] = rs_max;
+    if constexpr (sizeof(TF) == 4) {
+      for (int c = warp; c < nrhs; c += NT / 32) {
+        unsigned long long bm = 0ULL;
+        for (int i = lane; i < n; i += 32) bm = max(bm, mag_key(B[i + (long long)c * ldb]));
+        bm = warp_max64(bm);
+        if (lane == 0) s_rmax[c] = __longlong_as_double((long long)bm);
+      }
+    }
     __syncthreads();
     if (tid == 0) {
-      double an = 0.0;
-      for (int w = 0; w < (NT >> 5); ++w) an = fmax(an, s_red[w]);
-      s_anorm = an;
+      unsigned long long an = 0ULL;
+      for (int w = 0; w < NT / 32; ++w) an = max(an, s_red[w]);
+      s_anorm = __longlong_as_double((long long)an);
+    }
+    if (tid < nrhs) {
+      int e = 0;
+      if constexpr (sizeof(TF) == 4) {
+        const double mx = s_rmax[tid];
+        if (mx > 0.0 && isfinite(mx)) frexp(mx, &e);
+      }
+      s_exp[tid] = e;
     }
     __syncthreads();
+    for (int c = 0; c < nrhs; ++c)
+      for (int i = tid; i < n; i += NT) {
+        const double b = B[i + (long long)c * ldb];
+        W[i + (long long)(n + c) * n] = sizeof(TF) == 4 ? (TF)ldexp(b, -s_exp[c]) : (TF)b;
+      }
+    __syncthreads();
   }
-  // Xs and Rs are idle while factoring: they stage the row interchanges
-  factor_system<TF, CH>(W, n, ipiv, &s_info, smem, reinterpret_cast<TF*>(after),
-                        (int)(2 * sizeof(double) * kBMaxN * kBMaxRhs / sizeof(TF)));
+  factor_system<TF, NT>(W, n, n + nrhs, ipiv, &s_info, sm);
   const int info = s_info;
   if (info != 0) {
     // Exactly singular in the factorization precision: in mode 1 hand the
@@ -500,16 +548,15 @@ __device__ void run_system(const BatchArgs& a, int sys, bool fp64_pass, unsigned
     __syncthreads();
     return;
   }
-  compose_perm(ipiv, n, perm);
+  TF* Xs = sm.Xs;
+  for (int c = 0; c < nrhs; ++c)
+    for (int i = tid; i < n; i += NT) Xs[i + c * n] = W[i + (long long)(n + c) * n];
+  __syncthreads();
+  solve_tri<TF, NT, false>(W, n, Xs, nrhs, sm.Ds);
   if constexpr (sizeof(TF) == 8) {
-    // FP64: X = B, solve, residual
-    for (int idx = tid; idx < n * nrhs; idx += NT) {
-      int i = idx % n, c = idx / n;
-      X[i + (long long)c * ldx] = B[i + (long long)c * ldb];
-    }
-    __syncthreads();
-    solve_system<TF>(W, n, perm, reinterpret_cast<TF*>(X), ldx, nrhs, Xs);
-    double sr = residual_system(A, lda, n, B, ldb, X, ldx, nrhs, Rs, s_red, Xsh, &s_anorm);
+    for (int c = 0; c < nrhs; ++c)
+      for (int i = tid; i < n; i += NT) X[i + (long long)c * ldx] = Xs[i + c * n];
+    const double sr = residual_system<NT>(A, lda, n, B, ldb, sm.Xsh, nrhs, nullptr, s_anorm, s_rmax);
     if (tid == 0) {
       a.info[sys] = 0;
       a.iters[sys] = fp64_pass ? -1 : 0;
@@ -518,67 +565,56 @@ __device__ void run_system(const BatchArgs& a, int sys, bool fp64_pass, unsigned
     __syncthreads();
     return;
   } else {
-    // FP32 factors + FP64 refinement.
-    for (int idx = tid; idx < n * nrhs; idx += NT) {
-      int i = idx % n, c = idx / n;
-      X[i + (long long)c * ldx] = 0.0;
-    }
-    __syncthreads();
-    // initial residual r = b (x = 0): no pass over A
-    for (int idx = tid; idx < n * nrhs; idx += NT) {
-      const int i = idx % n, c = idx / n;
-      Rs[i + c * n] = B[i + (long long)c * ldb];
-    }
-    __syncthreads();
-    double sr = 1.0 / 0.0;  // scaled residual of x = 0 (the loop always refines at least once)
-    int steps = 0;
-    if (tid == 0) s_ok = 0;
-    __syncthreads();
-    for (int it = 0; it <= kMaxIr; ++it) {
-      if (it > 0 && sr <= a.tol) { if (tid == 0) s_ok = 1; break; }
-      if (it == kMaxIr) break;
+    // FP32 factors + FP64 refinement: the first correction (from x = 0) stands
+    // in Xs; X accumulates in global memory, Xsh holds it during the residual
+    int steps = 1;
+    double sr = 0.0;
+    bool ok = false;
+    for (;;) {
+      for (int c = 0; c < nrhs; ++c)
+        for (int i = tid; i < n; i += NT) {
+          const double d = ldexp((double)Xs[i + c * n], s_exp[c]);
+          double* xp = X + i + (long long)c * ldx;
+          *xp = steps == 1 ? d : *xp + d;
+        }
+      __syncthreads();
+      for (int c = 0; c < nrhs; ++c)
+        for (int i = tid; i < n; i += NT) sm.Xsh[i + c * n] = X[i + (long long)c * ldx];
+      __syncthreads();
+      sr = residual_system<NT>(A, lda, n, B, ldb, sm.Xsh, nrhs, sm.Rs, s_anorm, s_rmax);
+      if (sr <= a.tol) { ok = true; break; }
+      if (steps == kMaxIr) break;
       // correction: scale each residual column by a power of two into FP32, solve
-      __shared__ int s_exp[kBMaxRhs];
       if (tid < nrhs) {
-        double mx = 0.0;
-        for (int i = 0; i < n; ++i) mx = fmax(mx, fabs(Rs[i + tid * n]));
+        const double mx = s_rmax[tid];
         int e = 0;
         if (mx > 0.0 && isfinite(mx)) frexp(mx, &e);
         s_exp[tid] = e;
       }
       __syncthreads();
-      // copy the scaled residual into an FP32 buffer laid out like X (ld = n)
-      TF* Cx = Xs + n * nrhs;  // second half of the Xs region (n*nrhs <= 4096 floats)
-      for (int idx = tid; idx < n * nrhs; idx += NT) {
-        int i = idx % n, c = idx / n;
-        Cx[i + c * n] = (TF)ldexp(Rs[i + c * n], -s_exp[c]);
-      }
+      for (int c = 0; c < nrhs; ++c)
+        for (int i = tid; i < n; i += NT) Xs[i + c * n] = (TF)ldexp(sm.Rs[sm.org[i] + c * n], -s_exp[c]);
       __syncthreads();
-      solve_system<TF>(W, n, perm, Cx, n, nrhs, Xs);
-      for (int idx = tid; idx < n * nrhs; idx += NT) {
-        int i = idx % n, c = idx / n;
-        X[i + (long long)c * ldx] += ldexp((double)Cx[i + c * n], s_exp[c]);
-      }
-      __syncthreads();
+      solve_tri<TF, NT, true>(W, n, Xs, nrhs, sm.Ds);
+      solve_tri<TF, NT, false>(W, n, Xs, nrhs, sm.Ds);
       ++steps;
-      sr = residual_system(A, lda, n, B, ldb, X, ldx, nrhs, Rs, s_red, Xsh, &s_anorm);
     }
-    if (s_ok) {
-      if (tid == 0) {
+    if (tid == 0) {
+      if (ok) {
         a.info[sys] = 0;
         a.iters[sys] = steps;
         a.sresid[sys] = sr;
+      } else {
+        int slot = atomicAdd(&a.queue[2], 1);
+        a.fallback_list[slot] = sys;
       }
-    } else if (tid == 0) {
-      int slot = atomicAdd(&a.queue[2], 1);
-      a.fallback_list[slot] = sys;
     }
     __syncthreads();
   }
 }
 
-template <typename TF, int CH>
-__global__ void batched_kernel(BatchArgs a, int fp64_pass) {
+template <typename TF, int NT, int MINB>
+__global__ void __launch_bounds__(NT, MINB) batched_kernel(BatchArgs a, int fp64_pass) {
   extern __shared__ __align__(16) unsigned char bsmem[];
   __shared__ int s_item;
   const int ticket = fp64_pass ? 1 : 0;
@@ -590,31 +626,32 @@ __global__ void batched_kernel(BatchArgs a, int fp64_pass) {
     const int item = s_item;
     if (item >= count) break;
     const int sys = fp64_pass ? a.fallback_list[item] : a.order[item];
-    run_system<TF, CH>(a, sys, fp64_pass != 0, bsmem);
+    run_system<TF, NT>(a, sys, fp64_pass != 0, bsmem);
   }
 }
 
-template <typename TF, int CH>
-size_t batched_smem() {
-  return sizeof(TF) * (kBMaxN * (kBPB + 1) + kBPB * (CH + 1)) + 2 * sizeof(double) * kBMaxN * kBMaxRhs +
-         sizeof(int) * kBMaxN + 64;
-}
-
-template <typename TF, int CH>
-cudaError_t launch_batched(const BatchArgs& a, int fp64_pass, int threads, int ctas_per_sm,
-                           cudaStream_t s) {
-  const size_t smem = batched_smem<TF, CH>();
-  auto kern = batched_kernel<TF, CH>;
+template <typename TF, int NT, int MINB>
+cudaError_t launch_batched(const BatchArgs& a, int fp64_pass, int ctas_per_sm, cudaStream_t s) {
+  const size_t smem = BatchSmem<TF>::bytes(a.nmax, a.rmax);
+  auto kern = batched_kernel<TF, NT, MINB>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   int occ = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, threads, smem);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, NT, smem);
   if (e != cudaSuccess) return e;
   if (occ < 1) return cudaErrorInvalidConfiguration;
   const int per_sm = std::min(occ, std::max(1, ctas_per_sm));
-  kern<<<num_sms() * per_sm, threads, smem, s>>>(a, fp64_pass);
+  kern<<<num_sms() * per_sm, NT, smem, s>>>(a, fp64_pass);
   count_launches(1);
   return cudaGetLastError();
+}
+
+// threads in {128, 256, 512}; as many CTAs per SM as fit, up to ctas
+template <typename TF>
+cudaError_t launch_batched(const BatchArgs& a, int fp64_pass, int threads, int ctas, cudaStream_t s) {
+  if (threads == 128) return launch_batched<TF, 128, 4>(a, fp64_pass, ctas, s);
+  if (threads == 512) return launch_batched<TF, 512, 1>(a, fp64_pass, ctas, s);
+  return launch_batched<TF, 256, sizeof(TF) == 8 ? 2 : 3>(a, fp64_pass, ctas, s);
 }
 
 // ------------------------------------------------------------ plan
@@ -637,7 +674,8 @@ struct BatchPlan {
   int* ipiv_pool = nullptr;    // pivots (one block)
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
-  int threads = 256, chunk = 32, ctas_per_sm = 1;
+  int threads = 256, chunk = 16, ctas_per_sm = 1;
+  int nmax = 1, rmax = 1;
   double flops = 0.0;
 };
 
@@ -647,21 +685,17 @@ static BatchArgs plan_args(const BatchPlan& p) {
   a.B = p.d_B; a.ldb = p.d_ldb; a.X = p.d_X; a.ldx = p.d_ldx; a.ipiv = p.d_ipiv; a.W = p.d_W;
   a.W64 = p.mode == 0 ? p.d_W : p.d_W64;
   a.order = p.d_order; a.queue = p.d_queue; a.fallback_list = p.d_fb; a.info = p.d_info;
-  a.iters = p.d_iters; a.sresid = p.d_sresid; a.tol = p.tol;
+  a.iters = p.d_iters; a.sresid = p.d_sresid; a.tol = p.tol; a.nmax = p.nmax; a.rmax = p.rmax;
   return a;
 }
 
-static cudaError_t record_plan(const BatchPlan& p, int threads, int chunk, int ctas, cudaStream_t s) {
+static cudaError_t record_plan(const BatchPlan& p, int threads, int ctas, cudaStream_t s) {
   BatchArgs a = plan_args(p);
   SL_TRY(cudaMemsetAsync(p.d_queue, 0, 4 * sizeof(int), s));
-  if (p.mode == 0) {
-    if (chunk == 64) return launch_batched<double, 64>(a, 0, threads, ctas, s);
-    return launch_batched<double, 32>(a, 0, threads, ctas, s);
-  }
-  if (chunk == 64) SL_TRY((launch_batched<float, 64>(a, 0, threads, ctas, s)));
-  else SL_TRY((launch_batched<float, 32>(a, 0, threads, ctas, s)));
+  if (p.mode == 0) return launch_batched<double>(a, 0, threads, ctas, s);
+  SL_TRY(launch_batched<float>(a, 0, threads, ctas, s));
   // FP64 pass over the systems the refinement could not finish (may be empty)
-  return launch_batched<double, 32>(a, 1, 256, 1, s);
+  return launch_batched<double>(a, 1, 256, 2, s);
 }
 
 cudaError_t batch_plan_create(BatchPlan** out, int batch, const int* n, const int* nrhs,
@@ -681,7 +715,9 @@ cudaError_t batch_plan_create(BatchPlan** out, int batch, const int* n, const in
   size_t wtot = 0, ptot = 0;
   for (int i = 0; i < batch; ++i) {
     woff[i] = wtot;
-    wtot += ((size_t)n[i] * n[i] * esz + 255) / 256 * 256;
+    wtot += ((size_t)n[i] * (n[i] + nrhs[i]) * esz + 255) / 256 * 256;
+    p->nmax = std::max(p->nmax, n[i]);
+    p->rmax = std::max(p->rmax, nrhs[i]);
     poff[i] = ptot;
     ptot += (size_t)n[i];
     p->flops += 2.0 * n[i] * (double)n[i] * n[i] / 3.0;
@@ -713,7 +749,7 @@ cudaError_t batch_plan_create(BatchPlan** out, int batch, const int* n, const in
   if (mode == 1) {
     for (int i = 0; i < batch; ++i) {
       w64off[i] = w64;
-      w64 += ((size_t)n[i] * n[i] * sizeof(double) + 255) / 256 * 256;
+      w64 += ((size_t)n[i] * (n[i] + nrhs[i]) * sizeof(double) + 255) / 256 * 256;
     }
     alloc(&p->work64, w64);
     alloc(&p->d_W64, sizeof(void*) * batch);
@@ -744,9 +780,9 @@ cudaError_t batch_plan_create(BatchPlan** out, int batch, const int* n, const in
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) { batch_plan_destroy(p); return e; }
   // autotune: time the candidate shapes on this batch and keep the fastest
-  struct Cand { int threads, chunk, ctas; };
-  std::vector<Cand> cands = {{256, 32, 1}, {256, 64, 1}, {512, 32, 1}, {128, 32, 2}};
-  Cand best = cands[0];
+  struct Cand { int threads, ctas; };
+  std::vector<Cand> cands = {{256, 8}, {512, 8}, {128, 16}};
+  Cand best = p->nmax <= 128 ? cands[2] : cands[0];
   if (autotune) {
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
@@ -754,7 +790,7 @@ cudaError_t batch_plan_create(BatchPlan** out, int batch, const int* n, const in
     float best_ms = 1e30f;
     for (const Cand& c : cands) {
       cudaEventRecord(e0, s);
-      cudaError_t r = record_plan(*p, c.threads, c.chunk, c.ctas, s);
+      cudaError_t r = record_plan(*p, c.threads, c.ctas, s);
       cudaEventRecord(e1, s);
       if (r != cudaSuccess) { cudaGetLastError(); continue; }
       if (cudaEventSynchronize(e1) != cudaSuccess) break;
@@ -766,14 +802,14 @@ cudaError_t batch_plan_create(BatchPlan** out, int batch, const int* n, const in
     cudaEventDestroy(e1);
   }
   p->threads = best.threads;
-  p->chunk = best.chunk;
+  p->chunk = mode == 0 ? chunk_cols<double>() : chunk_cols<float>();
   p->ctas_per_sm = best.ctas;
   // capture the execution in a CUDA graph
   cudaStream_t cs;
   e = cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
   if (e == cudaSuccess) {
-    cudaError_t r = record_plan(*p, p->threads, p->chunk, p->ctas_per_sm, cs);
+    cudaError_t r = record_plan(*p, p->threads, p->ctas_per_sm, cs);
     cudaGraph_t g = nullptr;
     e = cudaStreamEndCapture(cs, &g);
     if (r != cudaSuccess) e = r;

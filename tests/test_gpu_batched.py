@@ -139,3 +139,26 @@ def test_batched_plan_rejects_bad_sizes(sl):
                                          0, None) == -3
     finally:
         L.sl1x1_batch_plan_create.argtypes = saved
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("orders", [(1, 2, 15, 16, 17), (31, 32, 33, 127, 128, 129), (255, 257, 496, 511, 512)])
+def test_batched_panel_edges(sl, orc, gpu_required, mode, orders):
+    """Orders around the panel width (16), the chunk widths, the threads per CTA
+    and the largest order, with 1 and 8 right-hand sides and a permuted matrix
+    whose columns interchange rows of every part of the panel."""
+    import torch
+
+    rng = np.random.default_rng(sum(orders) + mode)
+    systems = []
+    for n in orders:
+        for r in (1, 8):
+            A = rng.uniform(-0.5, 0.5, (n, n))
+            A[rng.permutation(n), np.arange(n)] += 0.5 * np.sqrt(n)
+            systems.append((np.asfortranarray(A), np.asfortranarray(rng.uniform(-0.5, 0.5, (n, r)))))
+    plan = Plan(sl, torch, systems, mode, autotune=0)
+    info, its, sr, X = plan.run()
+    for i, (A, B) in enumerate(systems):
+        assert info[i] == 0
+        assert orc.sresid(A, B, X[i]) < 16.0  # the tester's bound
+    plan.close()
