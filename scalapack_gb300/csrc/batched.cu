@@ -14,7 +14,7 @@
 // so the tail of the launch is made of small systems); CTAs of one persistent
 // grid take the next system from an atomic ticket until the queue is empty.
 //
-// Per system, one CTA (two or three share an SM):
+// Per system, one CTA (two share an SM):
 //   factor   blocked right-looking LU with 16-column panels held in shared
 //            memory (factor_system), the right-hand sides among the columns it
 //            updates, so that their forward solve is part of it; the trailing
@@ -77,7 +77,15 @@ constexpr int kPL = kBPB + 1;  // shared row stride of the panel: conflict-free 
 
 // Columns of a trailing update's chunk.
 template <typename T>
-__host__ __device__ constexpr int chunk_cols() { return sizeof(T) == 8 ? 16 : 32; }
+__host__ __device__ constexpr int chunk_cols() { return 16; }
+
+// The next column's offset: an addition the compiler keeps where it stands (as
+// products c * n it hoists a dozen of them out of every loop, and spills).
+__device__ __forceinline__ int next_col(int off, int ld) {
+  off += ld;
+  asm volatile("" : "+r"(off));
+  return off;
+}
 
 // Shared memory of one system of order <= nmax: while it is factored the panel
 // P [nmax][kPL], the rows' labels, and two chunks of U; afterwards, over the same
@@ -128,11 +136,12 @@ struct BatchSmem {
 // column. The labels are the panel's interchanges in composite form: one thread
 // per other column gathers its pivot rows, sends the displaced rows where they
 // go and solves with L11 in registers. Bound: the FP64 unit (FP64 factors) in the
-// trailing update; two or three systems share an SM so that the panels of one
-// run beside the updates of another. Measured, 4096 systems of order 16 .. 512:
+// trailing update; two systems share an SM so that the panels of one run beside
+// the updates of another (a third one's 80 registers a thread cost more in spills
+// than it gave). Measured, 4096 systems of order 16 .. 512:
 // FP64 119 ms (the unit's floor is 103; 188 with 32-column panels of four
 // barriers and FP64 compares per column and one system per SM), FP32 factors
-// with refinement 35 ms (87).
+// with refinement 31.5 ms (87), a third of it FP64 residuals.
 template <typename T, int NT>
 __device__ __forceinline__ void factor_system(T* W, int n, int ncols, int* ipiv, int* info, const BatchSmem<T>& sm) {
   constexpr int CH = chunk_cols<T>();
@@ -167,7 +176,7 @@ __device__ __forceinline__ void factor_system(T* W, int n, int ncols, int* ipiv,
         const T* src = W + (j + r) + (long long)j * n;
         T v[kBPB];
 #pragma unroll
-        for (int c = 0; c < kBPB; ++c) v[c] = c < jb ? src[(long long)c * n] : (T)0;
+        for (int c = 0, o = 0; c < kBPB; ++c, o = next_col(o, n)) v[c] = c < jb ? src[o] : (T)0;
 #pragma unroll
         for (int c = 0; c < kBPB; ++c) P[r * kPL + c] = v[c];
         lab[r] = r;
@@ -236,8 +245,8 @@ __device__ __forceinline__ void factor_system(T* W, int n, int ncols, int* ipiv,
         mv[q] = sm.org[j + r];
         T* dst = W + (j + L) + (long long)j * n;
 #pragma unroll
-        for (int c = 0; c < kBPB; ++c)
-          if (c < jb) dst[(long long)c * n] = P[r * kPL + c];
+        for (int c = 0, o = 0; c < kBPB; ++c, o = next_col(o, n))
+          if (c < jb) dst[o] = P[r * kPL + c];
         if (L < jb) {
           s_rowof[L] = r;
 #pragma unroll
@@ -296,7 +305,7 @@ __device__ __forceinline__ void factor_system(T* W, int n, int ncols, int* ipiv,
         T* crow = W + (j + L) + (long long)c0 * n;
         T cv[CH], acc[CH];
 #pragma unroll
-        for (int c = 0; c < CH; ++c) cv[c] = c < cw ? crow[(long long)c * n] : (T)0;
+        for (int c = 0, o = 0; c < CH; ++c, o = next_col(o, n)) cv[c] = c < cw ? crow[o] : (T)0;
         const T* lrow = P + r * kPL;
 #pragma unroll
         for (int k = 0; k < kBPB; ++k) {
@@ -305,8 +314,8 @@ __device__ __forceinline__ void factor_system(T* W, int n, int ncols, int* ipiv,
           for (int c = 0; c < CH; ++c) acc[c] = k == 0 ? a * Us[c] : fma(a, Us[k * CH + c], acc[c]);
         }
 #pragma unroll
-        for (int c = 0; c < CH; ++c)
-          if (c < cw) crow[(long long)c * n] = cv[c] - acc[c];
+        for (int c = 0, o = 0; c < CH; ++c, o = next_col(o, n))
+          if (c < cw) crow[o] = cv[c] - acc[c];
       }
     }
     __syncthreads();
@@ -366,8 +375,9 @@ __device__ __forceinline__ void solve_tri(const T* W, int n, T* Xs, int nrhs, T*
       for (int c = 0; c < kBMaxRhs; ++c) acc[c] = (T)0;
       for (int i0 = 0; i0 < kb; i0 += 16) {
         T l[16];
+        const T* wr = W + r + (long long)(k0 + i0) * n;
 #pragma unroll
-        for (int i = 0; i < 16; ++i) l[i] = W[r + (long long)(k0 + min(i0 + i, kb - 1)) * n];
+        for (int i = 0, o = 0; i < 16; ++i, o = next_col(o, n)) l[i] = i0 + i < kb ? wr[o] : (T)0;
 #pragma unroll
         for (int i = 0; i < 16; ++i)
           if (i0 + i < kb) {
@@ -403,53 +413,51 @@ __device__ __forceinline__ unsigned long long warp_max64(unsigned long long v) {
 template <int NT>
 __device__ __forceinline__ double residual_system(const double* A, int lda, int n, const double* B, int ldb,
                                   const double* Xsh, int nrhs, double* Rs, double anorm, double* rmax) {
-  constexpr int NW = NT / 32;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  __shared__ unsigned long long s_rm[NW][kBMaxRhs], s_xm[NW][kBMaxRhs];
+  __shared__ unsigned long long s_rm[kBMaxRhs], s_xm[kBMaxRhs];
   __shared__ double s_worst;
-  unsigned long long rm[kBMaxRhs], xm[kBMaxRhs];
-#pragma unroll
-  for (int c = 0; c < kBMaxRhs; ++c) { rm[c] = 0ULL; xm[c] = 0ULL; }
-  for (int r = tid; r < n; r += NT) {
+  if (tid < kBMaxRhs) s_rm[tid] = s_xm[tid] = 0ULL;
+  __syncthreads();
+  for (int r0 = 0; r0 < n; r0 += NT) {
+    const int r = r0 + tid;
+    const bool in = r < n;
     double acc[kBMaxRhs];
 #pragma unroll
-    for (int c = 0; c < kBMaxRhs; ++c) acc[c] = (c < nrhs) ? B[r + (long long)c * ldb] : 0.0;
-    const double* ar = A + r;
-    for (int k0 = 0; k0 < n; k0 += 8) {
-      double a[8];
+    for (int c = 0; c < kBMaxRhs; ++c) acc[c] = (in && c < nrhs) ? B[r + (long long)c * ldb] : 0.0;
+    if (__any_sync(0xffffffffu, in)) {
+      const double* ar = A + (in ? r : n - 1);
+      for (int k0 = 0; k0 < n; k0 += 8) {
+        double a[8];
 #pragma unroll
-      for (int k = 0; k < 8; ++k) a[k] = ar[(long long)min(k0 + k, n - 1) * lda];
+        for (int k = 0; k < 8; ++k) a[k] = ar[(long long)min(k0 + k, n - 1) * lda];
 #pragma unroll
-      for (int k = 0; k < 8; ++k)
-        if (k0 + k < n) {
+        for (int k = 0; k < 8; ++k)
+          if (k0 + k < n) {
 #pragma unroll
-          for (int c = 0; c < kBMaxRhs; ++c)
-            if (c < nrhs) acc[c] = fma(-a[k], Xsh[k0 + k + c * n], acc[c]);
+            for (int c = 0; c < kBMaxRhs; ++c)
+              if (c < nrhs) acc[c] = fma(-a[k], Xsh[k0 + k + c * n], acc[c]);
+          }
+      }
+#pragma unroll
+      for (int c = 0; c < kBMaxRhs; ++c)
+        if (c < nrhs) {
+          if (in && Rs) Rs[r + c * n] = acc[c];
+          const unsigned long long r1 = warp_max64(in ? mag_key(acc[c]) : 0ULL);
+          const unsigned long long x1 = warp_max64(in ? mag_key(Xsh[r + c * n]) : 0ULL);
+          if (lane == 0) {
+            atomicMax(&s_rm[c], r1);
+            atomicMax(&s_xm[c], x1);
+          }
         }
     }
-#pragma unroll
-    for (int c = 0; c < kBMaxRhs; ++c)
-      if (c < nrhs) {
-        if (Rs) Rs[r + c * n] = acc[c];
-        rm[c] = max(rm[c], mag_key(acc[c]));
-        xm[c] = max(xm[c], mag_key(Xsh[r + c * n]));
-      }
   }
-#pragma unroll
-  for (int c = 0; c < kBMaxRhs; ++c)
-    if (c < nrhs) {
-      const unsigned long long r1 = warp_max64(rm[c]), x1 = warp_max64(xm[c]);
-      if (lane == 0) { s_rm[warp][c] = r1; s_xm[warp][c] = x1; }
-    }
   __syncthreads();
   if (warp == 0) {
     double v = 0.0;
     if (lane < nrhs) {
-      unsigned long long r1 = 0ULL, x1 = 0ULL;
-      for (int w = 0; w < NW; ++w) { r1 = max(r1, s_rm[w][lane]); x1 = max(x1, s_xm[w][lane]); }
-      const double rn = __longlong_as_double((long long)r1);
+      const double rn = __longlong_as_double((long long)s_rm[lane]);
       rmax[lane] = rn;
-      v = rn / (__longlong_as_double((long long)x1) * anorm * ldexp(1.0, -53) * n);
+      v = rn / (__longlong_as_double((long long)s_xm[lane]) * anorm * ldexp(1.0, -53) * n);
     }
     const unsigned long long w = warp_max64(mag_key(v));
     if (lane == 0) s_worst = __longlong_as_double((long long)w);
@@ -651,7 +659,7 @@ template <typename TF>
 cudaError_t launch_batched(const BatchArgs& a, int fp64_pass, int threads, int ctas, cudaStream_t s) {
   if (threads == 128) return launch_batched<TF, 128, 4>(a, fp64_pass, ctas, s);
   if (threads == 512) return launch_batched<TF, 512, 1>(a, fp64_pass, ctas, s);
-  return launch_batched<TF, 256, sizeof(TF) == 8 ? 2 : 3>(a, fp64_pass, ctas, s);
+  return launch_batched<TF, 256, 2>(a, fp64_pass, ctas, s);
 }
 
 // ------------------------------------------------------------ plan
