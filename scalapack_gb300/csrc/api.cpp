@@ -269,9 +269,11 @@ cudaError_t ensure_solve_ws(int n, int nrhs) {
     ensure_oz(n, nrhs, 128);
     if (grow(&g_dev.ddinvs, &g_dev.capDinvs, sl::kSolveInvDoubles(n)) != cudaSuccess) cudaGetLastError();
     if (nrhs <= sl::kChainRhs) {
-      const int* old = g_dev.dchain64;
+      // a new buffer's words are cleared before their first use (told by its
+      // size: it may come back at the old one's address)
+      const size_t old = g_dev.capChain64;
       if (grow(&g_dev.dchain64, &g_dev.capChain64, 16 + 4 * (size_t)n * nrhs) != cudaSuccess) cudaGetLastError();
-      else if (g_dev.dchain64 != old) g_dev.chain64_epoch = 0;  // new words: cleared before their first use
+      if (g_dev.capChain64 != old) g_dev.chain64_epoch = 0;
     }
   }
   return cudaSuccess;

@@ -361,3 +361,31 @@ def test_chained_solve_edges(sl, gpu_required, n, nrhs, trans):
     res = np.abs(B - op @ X).max(axis=0)
     scale = np.abs(op).sum(axis=1).max() * np.abs(X).max(axis=0) * n * 2.0**-53
     assert (res / scale < 16.0).all()  # the tester's bound
+
+
+def test_chained_solve_on_reused_dirty_memory(sl, gpu_required):
+    """The chained solve's words start cleared in every buffer they grow into, also
+    when it stands at the old one's address among memory that holds the epochs
+    of the calls to come."""
+    import torch
+
+    L = sl.lib()
+    L.sl1x1_finalize()
+    rng = np.random.default_rng(2)
+    epoch = 0
+    for n in (40, 64, 90, 200, 333, 700, 1000, 1500):
+        dirty = [torch.full((1 << 24,), epoch + e, dtype=torch.int64, device="cuda") for e in (1, 2, 1, 2)]
+        dirty += [torch.full((4096,), epoch + 1 + i % 2, dtype=torch.int64, device="cuda") for i in range(64)]
+        torch.cuda.synchronize()
+        del dirty
+        torch.cuda.empty_cache()
+        A = rng.uniform(-0.5, 0.5, (n, n))
+        B = rng.uniform(-0.5, 0.5, (n, 3))
+        dA, dB = torch.from_numpy(A.T.copy()).cuda(), torch.from_numpy(B.T.copy()).cuda()
+        ip = torch.zeros(n, dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        assert sl.dgesv_dev(n, 3, dA.data_ptr(), n, ip.data_ptr(), dB.data_ptr(), n) == 0
+        epoch += 2
+        X = dB.T.cpu().numpy()
+        res = np.abs(B - A @ X).max(axis=0) / (np.abs(A).sum(axis=1).max() * np.abs(X).max(axis=0) * n * 2.0**-53)
+        assert (res < 16.0).all(), n
