@@ -25,6 +25,7 @@
 // exact arithmetic.
 #include <algorithm>
 #include <climits>
+
 #include <cmath>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -58,6 +59,7 @@ static int g_panel_ctas = 64;  // CTAs a panel's rows are spread over (before th
 static int g_panel_ib = 2;     // sub-panels per in-panel block (factor_panel)
 void set_panel_ib(int ib) { g_panel_ib = ib < 1 ? 1 : (ib > 8 ? 8 : ib); }
 int panel_ctas() { return g_panel_ctas; }
+int panel_cluster_rows() { return 128; }
 void set_panel_ctas(int g) { g_panel_ctas = g < 8 ? 8 : (g > 224 ? 224 : g); }
 void set_panel_min_rows(int rows) { g_panel_min_rows = rows <= 0 ? 0 : (rows < 8 ? 8 : (rows > 768 ? 768 : rows)); }
 

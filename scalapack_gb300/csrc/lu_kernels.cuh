@@ -511,6 +511,280 @@ panel_kernel(T* A, long long lda, int m, int r0, int c0, int w, int rpc, int* ip
   }
 }
 
+// The same factorization by one thread-block cluster of up to CMAXG CTAs, for
+// panels short enough that the cluster's FP64 units keep up (launch_panel): a
+// CTA's candidate row, key and label go straight into every CTA's shared memory
+// (st.async, counted by an mbarrier there), so that a column costs one
+// shared-memory hop between SMs instead of two round trips through L2, and every
+// warp then picks the winner by itself: one block barrier per column. Measured,
+// per column, FP64: 1.4 us at R = 600 (2.3 through L2), 1.8 at R = 2048 (2.4; with
+// 256 rows per CTA the FP64 units take as long, so launch_panel stops at 128);
+// FP32, R = 4096: 1.4 (2.1). Three
+// inboxes: column k's pivot row is read until column k+1 has been sent for, so a
+// CTA may be sent column k+2's while it still reads column k's, but not k+3's.
+// Waits are bounded (spin_limit polls); a CTA that gives up goes on to the
+// cluster barrier at the end, which keeps its shared memory in place until all
+// have stopped sending.
+constexpr int CMAXG = 16;
+template <typename T>
+struct PanelInbox {
+  long long key;
+  long long label;
+  double rmag;  // 1/|pivot| (FP64)
+  double pad;
+  T row[PW];
+};
+template <typename T>
+__host__ __device__ constexpr size_t panel_inbox_bytes() {
+  return 3 * CMAXG * sizeof(PanelInbox<T>);
+}
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t local, uint32_t rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// NTR row threads and the reciprocal's warp; a row thread has at most one row (rpc *
+// tpr <= NTR), whose label stays in a register.
+template <typename T, int NTR>
+__global__ void __launch_bounds__(NTR + 32, 512 / NTR)
+panel_cluster_kernel(T* A, long long lda, int m, int r0, int c0, int w, int rpc, int* ipiv, int* info_col,
+                     int* status, long long spin_limit, int tpr) {
+  extern __shared__ __align__(16) unsigned char panel_smem[];
+  PanelInbox<T>* inbox = reinterpret_cast<PanelInbox<T>*>(panel_smem);  // [3][CMAXG]
+  T* tile = reinterpret_cast<T*>(panel_smem + panel_inbox_bytes<T>());
+  int* lab = reinterpret_cast<int*>(tile + (size_t)rpc * PLD);
+  constexpr int NW = NTR / 32;
+  __shared__ __align__(8) unsigned long long s_bar[3];
+  __shared__ long long s_wk[2][NW];
+  __shared__ int s_wr[2][NW], s_wl[2][NW];
+  __shared__ int s_fail;
+
+  const int CS = gridDim.x, b = blockIdx.x, tid = threadIdx.x;
+  const int lane = tid & 31, warp = tid >> 5;
+  const bool exch = warp == NW;  // the warp that forms the reciprocal
+  const int R = m - r0;
+  const int kw = min(w, R);
+  const int lo = b * rpc;
+  const int nr = max(0, min(rpc, R - lo));
+  const uint32_t bar0 = (uint32_t)__cvta_generic_to_shared(s_bar);
+  const uint32_t in0 = (uint32_t)__cvta_generic_to_shared(inbox);
+  if (tid == 0) {
+    s_fail = 0;
+    for (int i = 0; i < 3; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0 + 8 * i));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  auto row_key = [&](T v, int label, int k) -> long long {
+    const long long key = amax_ikey(v);
+    return (key < 0 && label == k) ? LLONG_MAX : key;
+  };
+  auto put_candidate = [&](int buf, long long key, int label, int lrow) {
+    if (lane == warp_best(key, label)) {
+      s_wk[buf][warp] = key;
+      s_wr[buf][warp] = label;
+      s_wl[buf][warp] = lrow;
+    }
+  };
+  const int part = tid & (tpr - 1), row0 = exch ? nr : tid / tpr;
+  int mylab = row0 < nr ? lo + row0 : -1;  // the label of row row0
+  if (!exch) {
+    long long key = -2;
+    int label = INT_MAX, lrow = 0;
+    for (int r = tid; r < nr; r += NTR) {
+      const T* src = A + (long long)(r0 + lo + r) + (long long)c0 * lda;
+#pragma unroll
+      for (int cb = 0; cb < PW; cb += PCH) {
+        T v[PCH];
+#pragma unroll
+        for (int c = 0; c < PCH; ++c) v[c] = (cb + c < w) ? src[(long long)(cb + c) * lda] : (T)0;
+#pragma unroll
+        for (int c = 0; c < PCH; ++c) tile[r * PLD + cb + c] = v[c];
+      }
+    }
+    asm volatile("bar.sync 1, %0;" ::"n"(NTR) : "memory");
+    if (part == 0 && row0 < nr) {
+      key = row_key(tile[row0 * PLD], lo + row0, 0);
+      label = lo + row0;
+      lrow = row0;
+    }
+    put_candidate(0, key, label, lrow);
+  }
+  cluster_sync();  // every CTA's barriers are there
+
+  // columns kp+2 .. w-1 of the active rows, U = the pivot row of column kp
+  auto finish_update = [&](int kp, const T* U) {
+    if (row0 >= nr || mylab < 0) return;
+    T* row = tile + row0 * PLD;
+    const T l = row[kp];
+    int j = kp + 2 + part;
+    if (j >= w) return;
+    T v = row[j], u = U[j];
+#pragma unroll 2
+    for (; j + tpr < w; j += tpr) {
+      const T vn = row[j + tpr], un = U[j + tpr];
+      row[j] = fma(-l, u, v);
+      v = vn;
+      u = un;
+    }
+    row[j] = fma(-l, u, v);
+  };
+
+  const T* Uprev = nullptr;  // pivot row of column k-1
+  int k = 0;
+  for (; k < kw; ++k) {
+    const int buf = k % 3, par = k & 1;
+    __syncthreads();
+    if (s_fail) break;
+    // --- this CTA's candidate, into every CTA's inbox ---
+    long long key = lane < NW ? s_wk[par][lane] : -3;
+    int label = lane < NW ? s_wr[par][lane] : INT_MAX;
+    const int cw = warp_best(key, label);
+    const int lrow = s_wl[par][cw];
+    if (tid == 0)
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar0 + 8 * buf),
+                   "r"((uint32_t)(CS * (16 + (sizeof(T) == 8 ? 8 : 0) + PW * sizeof(T))))
+                   : "memory");
+    if (warp == cw) {
+      // the candidate row with column k-1's update of its columns beyond k
+      T v = (T)0;
+      if (nr > 0 && lane < w) {
+        v = tile[lrow * PLD + lane];
+        if (k > 0 && lane > k) v = fma(-tile[lrow * PLD + k - 1], Uprev[lane], v);
+      }
+      const uint32_t slot = in0 + (uint32_t)((buf * CMAXG + b) * sizeof(PanelInbox<T>));
+      const long long ck = s_wk[par][cw];
+      const long long cl = s_wr[par][cw];
+      if (lane < CS)
+        asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];" ::"r"(
+                         cluster_addr(slot, lane)),
+                     "l"(ck), "l"(cl), "r"(cluster_addr(bar0 + 8 * buf, lane))
+                     : "memory");
+      const uint32_t mine = slot + 32 + (uint32_t)(lane * sizeof(T));
+      for (int q = 0; q < CS; ++q) {
+        const uint32_t dst = cluster_addr(mine, q), bar = cluster_addr(bar0 + 8 * buf, q);
+        if constexpr (sizeof(T) == 8)
+          asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(dst),
+                       "l"(__double_as_longlong(v)), "r"(bar)
+                       : "memory");
+        else
+          asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(dst),
+                       "r"(__float_as_uint(v)), "r"(bar)
+                       : "memory");
+      }
+      __syncwarp();  // (the row is read before its owner goes on)
+    }
+    if (exch) {
+      if constexpr (sizeof(T) == 8) {
+        // 1/|candidate| on the integer pipe while the rows are updated: 450
+        // cycles that every thread would otherwise wait for after the exchange
+        const unsigned long long kb = (unsigned long long)s_wk[par][cw];
+        const double ra = kb - 1ULL < 0x7FEFFFFFFFFFFFFFULL ? recip_bits(kb) : 0.0;
+        const uint32_t slot = in0 + (uint32_t)((buf * CMAXG + b) * sizeof(PanelInbox<T>));
+        if (lane < CS)
+          asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(
+                           cluster_addr(slot + 16, lane)),
+                       "l"(__double_as_longlong(ra)), "r"(cluster_addr(bar0 + 8 * buf, lane))
+                       : "memory");
+      }
+    } else if (k > 0) {
+      finish_update(k - 1, Uprev);
+    }
+    // --- every CTA's candidate is here: the winner, U(k, :) and 1/pivot ---
+    bool ok = false;
+    for (long long spins = 0; spins < 8 * spin_limit; ++spins) {  // (a poll here takes an eighth of one in L2)
+      uint32_t done;
+      asm volatile(
+          "{\n .reg .pred p;\n mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+          " selp.u32 %0, 1, 0, p;\n}\n"
+          : "=r"(done)
+          : "r"(bar0 + 8 * buf), "r"((uint32_t)((k / 3) & 1))
+          : "memory");
+      if (done) { ok = true; break; }
+    }
+    ok = __all_sync(0xffffffffu, ok);
+    if (!ok) {
+      if (lane == 0) {
+        atomicExch(status, (int)kFlagTimeout);
+        s_fail = 1;
+      }
+      continue;
+    }
+    const PanelInbox<T>* in = inbox + buf * CMAXG;
+    key = lane < CS ? in[lane].key : -3;
+    label = lane < CS ? (int)in[lane].label : INT_MAX;
+    const int own = warp_best(key, label);
+    key = in[own].key;
+    label = (int)in[own].label;
+    const T* U = in[own].row;
+    const T g = U[k];
+    T rinv;  // ONE/GMAX (pdgetf2.f:224), 1 for a zero pivot: its column is not scaled
+    bool zero;
+    if constexpr (sizeof(T) == 8) {
+      const unsigned long long kb = (unsigned long long)key, gb = (unsigned long long)__double_as_longlong(g);
+      zero = (gb << 1) == 0;
+      if (kb - 1ULL < 0x7FEFFFFFFFFFFFFFULL)
+        rinv = __longlong_as_double(__double_as_longlong(in[own].rmag) | (long long)(gb & (1ULL << 63)));
+      else
+        rinv = zero ? (T)1 : (T)1 / g;
+    } else {
+      zero = g == (T)0;
+      rinv = zero ? (T)1 : (T)1 / g;
+    }
+    if (b == 0 && tid == 0) {
+      ipiv[c0 + k] = r0 + label;
+      if (zero) atomicMin(info_col, c0 + k);
+    }
+    const int piv = label, mine = own == b ? lrow : -1;
+    const int kn = k + 1;
+    const T un = U[kn < w ? kn : k];
+    {
+      T* row = tile + min(row0, rpc - 1) * PLD;
+      T l = row[k];
+      const T a = row[kn < w ? kn : k];
+      l *= rinv;
+      const T v = fma(-l, un, a);
+      const bool act = mylab >= 0 && row0 != mine && part == 0;
+      if (mylab == k) mylab = piv;   // the diagonal row goes where the pivot row stood
+      if (row0 == mine) mylab = ~k;  // pivot row k
+      if (act) {
+        row[k] = l;
+        if (kn < w) row[kn] = v;
+      }
+      if (kn < kw && !exch)
+        put_candidate(par ^ 1, act ? row_key(v, mylab, kn) : -2LL, act ? mylab : INT_MAX, row0);
+    }
+    Uprev = U;
+  }
+  __syncthreads();
+  if (s_fail) {
+    // pivots from the first one that was not chosen become the diagonal rows
+    if (b == 0)
+      for (int q = max(k - 1, 0) + tid; q < kw; q += NTR + 32) ipiv[c0 + q] = r0 + q;
+  } else {
+    if (kw > 0) finish_update(kw - 1, Uprev);
+    if (part == 0 && row0 < nr) lab[row0] = mylab;
+    __syncthreads();
+    for (int r = exch ? nr : tid; r < nr; r += NTR) {
+      const int lb = lab[r];
+      T* dst = A + (long long)(r0 + (lb < 0 ? ~lb : lb)) + (long long)c0 * lda;
+#pragma unroll
+      for (int cb = 0; cb < PW; cb += PCH) {
+        T v[PCH];
+#pragma unroll
+        for (int c = 0; c < PCH; ++c) v[c] = (cb + c < w) ? tile[r * PLD + cb + c] : (T)0;
+#pragma unroll
+        for (int c = 0; c < PCH; ++c)
+          if (cb + c < w) dst[(long long)(cb + c) * lda] = v[c];
+      }
+    }
+  }
+  if (s_fail) __nanosleep(20000);  // what was sent before the others stopped has landed
+  cluster_sync();
+}
+
 // Sequential row interchanges k1..k2-1 (rows i <-> ipiv[i]) on the columns
 // [cb1,ce1) and [cb2,ce2); one thread per column (PDLASWP 'Forward','Rows').
 // Used when the interchanges outnumber the composite form's table.
@@ -1184,6 +1458,42 @@ template <typename T>
 inline cudaError_t launch_panel(T* A, long long lda, int m, int r0, int c0, int w, int* ipiv,
                                 const LuWork& ws, cudaStream_t s) {
   const int R = m - r0;
+  // One cluster (16 CTAs at most, of 32 rows at least) while its rows stay
+  // within what its SMs' FP64 units do in a column's time. (The tuning knobs of
+  // the row slices and CTAs ask for the other form.)
+  const int cl_rows = sizeof(T) == 4 ? 512 : panel_cluster_rows();
+  if (panel_min_rows() == 0 && panel_ctas() == 64 && R <= CMAXG * cl_rows && w > 0) {
+    int cs = 1;
+    while (cs < CMAXG && R > 32 * cs) cs *= 2;
+    int crpc = ((R + cs - 1) / cs + 7) & ~7;
+    const size_t csmem = panel_inbox_bytes<T>() + (sizeof(T) * PLD + sizeof(int)) * (size_t)crpc;
+    static const cudaError_t at = [] {
+      for (const void* f : {(const void*)panel_cluster_kernel<T, PTR>, (const void*)panel_cluster_kernel<T, 2 * PTR>}) {
+        cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        if (e != cudaSuccess) return e;
+      }
+      return cudaSuccess;
+    }();
+    SL_TRY(at);
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute la[1];
+    la[0].id = cudaLaunchAttributeClusterDimension;
+    la[0].val.clusterDim.x = cs;
+    la[0].val.clusterDim.y = la[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(cs);
+    const int ntr = crpc > PTR ? 2 * PTR : PTR;
+    cfg.blockDim = dim3(ntr + 32);
+    cfg.dynamicSmemBytes = csmem;
+    cfg.stream = s;
+    cfg.attrs = la;
+    cfg.numAttrs = 1;
+    int ctpr = crpc > PTR / 4 ? 1 : (crpc > PTR / 8 ? 2 : 4);
+    count_launches(1);
+    auto kern = ntr == PTR ? panel_cluster_kernel<T, PTR> : panel_cluster_kernel<T, 2 * PTR>;
+    return cudaLaunchKernelEx(&cfg, kern, A, lda, m, r0, c0, w, crpc, ipiv, ws.info_col, ws.status,
+                              spin_limit(), ctpr);
+  }
   // Rows per CTA: about 64 CTAs per panel, and at least the type's minimum
   // (FP32 256, FP64 128, or the tuning knob). Fewer CTAs make the per-column
   // exchange cheaper (fewer keys to poll, less cross-die skew); more rows per

@@ -194,6 +194,8 @@ size_t panel_tile_doubles(int m);
 // default, means 256 rows for FP32 and 128 for FP64).
 int panel_min_rows();
 int panel_ctas();
+// Most FP64 rows per CTA of the one-cluster panel (launch_panel).
+int panel_cluster_rows();
 void set_panel_ib(int ib);
 void set_panel_ctas(int g);
 void set_panel_min_rows(int rows);

@@ -389,3 +389,39 @@ def test_chained_solve_on_reused_dirty_memory(sl, gpu_required):
         X = dB.T.cpu().numpy()
         res = np.abs(B - A @ X).max(axis=0) / (np.abs(A).sum(axis=1).max() * np.abs(X).max(axis=0) * n * 2.0**-53)
         assert (res < 16.0).all(), n
+
+
+@pytest.mark.parametrize("kind", ["random", "ties", "zero column", "nan"])
+@pytest.mark.parametrize("m", [1, 5, 31, 33, 64, 65, 128, 129, 513, 1024, 1025, 2047, 2048, 2049])
+def test_cluster_panel_equals_grid_panel(sl, gpu_required, m, kind):
+    """The one-cluster panel (up to 2048 rows) and the one that exchanges through L2
+    (asked for by a row-slice setting) give the same factors and pivots, bit for
+    bit: cluster sizes 1 to 16, partial rows and widths, ties, zero pivots, NaN in
+    and off the diagonal."""
+    import torch
+
+    n = 70
+    rng = np.random.default_rng(m)
+    A = rng.uniform(-0.5, 0.5, (m, n))
+    if kind == "ties":
+        A = rng.integers(-2, 3, (m, n)).astype(float)
+    elif kind == "zero column":
+        A[:, min(m, n) // 2] = 0.0
+    elif kind == "nan":
+        A[rng.integers(0, m), min(3, m - 1)] = np.nan
+        A[min(40, m - 1), min(40, m - 1)] = np.nan
+    L = sl.lib()
+    got = []
+    try:
+        for rows in (0, 256):
+            L.sl1x1_set_panel_rows(rows)
+            dA = torch.from_numpy(A.T.copy()).cuda()
+            ip = torch.zeros(min(m, n), dtype=torch.int32, device="cuda")
+            torch.cuda.synchronize()
+            info = sl.dgetrf_dev(m, n, dA.data_ptr(), m, ip.data_ptr(), 64)
+            got.append((info, ip.cpu().numpy(), dA.cpu().numpy()))
+    finally:
+        L.sl1x1_set_panel_rows(0)
+    assert got[0][0] == got[1][0]
+    np.testing.assert_array_equal(got[0][1], got[1][1])
+    np.testing.assert_array_equal(got[0][2], got[1][2])
