@@ -193,6 +193,14 @@ void release_all() {
   g_dev = DevState();
 }
 
+// Block size of the factorization of a matrix with mn = min(M, N) whose caller
+// gives NB, the distribution's block: on one process it decides nothing but the
+// order of the work (the pivots do not depend on it), and 256 columns suit the
+// sliced products best at every order measured: N = 600 2.27 ms (64 columns: 2.45,
+// 512: 2.75), N = 2000 7.98 (9.09, 10.3), N = 8192 39.9 (67.9, 55.0). Matrices of a
+// few panels, where it matters little, and the DMMA form keep the caller's.
+int factor_nb(int mn, int nb) { return mn > 512 && sl::f64_update_get() == 1 ? 256 : nb; }
+
 // Grows a sliced-product scratch buffer; a new one starts with its balancing
 // words zeroed (the memory may hold anything, including words that look like
 // a later epoch's).
@@ -309,11 +317,12 @@ int factor_host(int m, int n, double* A, int ia, int ja, const int* desca, int* 
   if (e == cudaSuccess) e = grow(&g_dev.dipiv, &g_dev.capP, (size_t)(mn > 0 ? mn : 1));
   if (e != cudaSuccess) return cuda_info(e);
   const double* src = A + (ia - 1) + (long long)(ja - 1) * lld;
-  ensure_oz(m, n, desca[NB_]);
+  const int nb = factor_nb(mn, desca[NB_]);
+  ensure_oz(m, n, nb);
   // With the look-ahead on and more than two panels, A goes over in column
   // chunks of about n/g_copy_chunks (whole panels, the first holding panels 0
   // and 1) on the copy stream, and step 0 of the factorization follows them.
-  const int nbk = desca[NB_] < 1024 ? desca[NB_] : 1024;
+  const int nbk = nb < 1024 ? nb : 1024;
   int col_end[sl::kMaxColChunks];
   int nck = 0;
   if (g_copy_chunks > 1 && g_lookahead && nbk > 0 && mn > 2 * nbk) {
@@ -344,7 +353,7 @@ int factor_host(int m, int n, double* A, int ia, int ja, const int* desca, int* 
   w.ncol_chunks = nck;
   w.col_end = col_end;
   w.ev_cols = g_dev.ev_cols;
-  e = sl::dgetrf_device(m, n, g_dev.dA, ldda, g_dev.dipiv, desca[NB_], w, s);
+  e = sl::dgetrf_device(m, n, g_dev.dA, ldda, g_dev.dipiv, nb, w, s);
   // (every chunk has been waited for on s unless the factorization stopped early)
   if (nck > 0) {
     const cudaError_t e2 = cudaStreamSynchronize(g_dev.h2d);
@@ -655,6 +664,7 @@ int sl1x1_dgetrf_dev(int m, int n, double* dA, long long ldda, int* dipiv, int n
   if (!ensure_device()) return cuda_info(cudaErrorNoDevice);
   cudaStream_t s = (cudaStream_t)stream;
   if (nb <= 0) nb = g_default_nb;
+  nb = factor_nb(m < n ? m : n, nb);
   ensure_oz(m, n, nb);
   sl::LuWork w = make_work();
   cudaError_t e = sl::dgetrf_device(m, n, dA, ldda, dipiv, nb, w, s);
