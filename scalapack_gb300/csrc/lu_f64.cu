@@ -56,8 +56,13 @@ void set_spin_limit(long long polls) { g_spin_limit = polls < 0 ? kSpinLimit : p
 static int g_panel_min_rows = 0;  // 0: automatic (FP32 256, FP64 128)
 int panel_min_rows() { return g_panel_min_rows; }
 static int g_panel_ctas = 64;  // CTAs a panel's rows are spread over (before the minimum rows)
-static int g_panel_ib = 2;     // sub-panels per in-panel block (factor_panel)
-void set_panel_ib(int ib) { g_panel_ib = ib < 1 ? 1 : (ib > 8 ? 8 : ib); }
+// Sub-panels per in-panel block (factor_panel); 0: one up to 5000 rows, where a
+// block's second step costs a launch more than its deeper products save (PDGESV N
+// = 600 2.00 ms with one, 2.11 with two; N = 4096 16.0, 16.6), two above (N = 8192
+// 36.8, 37.5, but a rounding less per element; N = 16384 127.4, 125.8: the update
+// beside the panel leaves it few SMs).
+static int g_panel_ib = 0;
+void set_panel_ib(int ib) { g_panel_ib = ib < 1 ? 0 : (ib > 8 ? 8 : ib); }
 int panel_ctas() { return g_panel_ctas; }
 int panel_cluster_rows() { return 128; }
 void set_panel_ctas(int g) { g_panel_ctas = g < 8 ? 8 : (g > 224 ? 224 : g); }
@@ -324,12 +329,13 @@ static cudaError_t factor_panel(int m, double* dA, long long ldda, int* dipiv, i
   const OzScratch& sc = (ws.aux && s == ws.aux) ? ws.oz_aux : ws.oz;
   phase_begin(kPhPanel, s);
   double pflops = 0.0;
-  // Sub-panels are grouped in blocks of g_panel_ib: inside a block only the
+  // Sub-panels are grouped in blocks of ib: inside a block only the
   // next sub-panel's columns are brought up to date after each sub-panel
   // (left-looking, with every pivot row of the block so far), and the
   // columns beyond the block once at its end, with the block's rows -- fewer,
   // deeper in-panel products than one per sub-panel over all the remaining
   // columns.
+  const int ib = g_panel_ib > 0 ? g_panel_ib : (m - j <= 5000 ? 1 : 2);
   int blk_r0 = j;  // first row (= column) of the current block
   for (int c = 0, q = 0; c < jb; c += PW, ++q) {
     const int w = (jb - c) < PW ? (jb - c) : PW;
@@ -342,16 +348,21 @@ static cudaError_t factor_panel(int m, double* dA, long long ldda, int* dipiv, i
     SL_TRY(launch_panel<double>(dA, ldda, m, r0, r0, w, dipiv, ws, s));
     phase_end(kPhPanelKernel, s, kflops, 16.0 * (double)(m - r0) * w);
     phase_begin(kPhPanelUpdate, s);
-    SL_TRY(laswp<double>(dA, ldda, r0, r0 + kw, dipiv, j, r0, r0 + w, j + jb, s));
-    if (c + w < jb) {
-      const bool block_end = (q + 1) % g_panel_ib == 0 || kw < w;
+    if (c + w >= jb) {
+      SL_TRY(inpanel_step<double>(dA, ldda, r0, r0 + kw, dipiv, j, r0, r0 + w, j + jb, 0, kw, s));
+    } else {
+      const bool block_end = (q + 1) % ib == 0 || kw < w;
       // columns brought up to date now: the next sub-panel's, or at the end
       // of a block every remaining one; rows: the block's pivot rows (U, by
       // the strip solve) and every row below them (the product)
       const int ncols = block_end ? jb - c - w : ((jb - c - w) < PW ? (jb - c - w) : PW);
       const int kb = r0 + kw - blk_r0;
       const int rl = r0 + kw;  // first row below the block's pivot rows
-      // The strip solve also publishes the balancing keys of the product that
+      const bool fused = kb <= 64 && (kb - kw) % 32 == 0;  // (two sub-panels per block at most)
+      if (!fused) SL_TRY(laswp<double>(dA, ldda, r0, r0 + kw, dipiv, j, r0, r0 + w, j + jb, s));
+      // (the block's earlier columns are read by the fused step: theirs first)
+      else if (blk_r0 < r0) SL_TRY(laswp<double>(dA, ldda, r0, r0 + kw, dipiv, blk_r0, r0, r0, r0, s));
+      // The solve also publishes the balancing keys of the product that
       // follows it: the row maxima of its own output (U) and, in extra blocks
       // of the same launch, the column maxima of the block's L.
       const bool keyed = rl < m && g_f64_update == 1 && oz_fits(sc, m - rl, ncols, kb);
@@ -365,8 +376,11 @@ static cudaError_t factor_panel(int m, double* dA, long long ldda, int* dipiv, i
         kj.lrows = m - rl;
         kj.lcols = kb;
       }
-      SL_TRY((trsm_strip<double, false, false, true>(kb, ncols, Ap(blk_r0, blk_r0), ldda,
-                                                      Ap(blk_r0, r0 + w), ldda, s, kj)));
+      if (fused)
+        SL_TRY(inpanel_step<double>(dA, ldda, r0, r0 + kw, dipiv, j, blk_r0, r0 + w, j + jb, ncols, kb, s, kj));
+      else
+        SL_TRY((trsm_strip<double, false, false, true>(kb, ncols, Ap(blk_r0, blk_r0), ldda,
+                                                        Ap(blk_r0, r0 + w), ldda, s, kj)));
       pflops += (double)kb * kb * ncols;
       if (keyed) {
         SL_TRY(oz_dgemm_keyed(sc, kj.epoch, m - rl, ncols, kb, -1.0, Ap(rl, blk_r0), ldda,

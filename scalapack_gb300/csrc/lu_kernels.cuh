@@ -984,6 +984,121 @@ laswp_apply_kernel(T* A, long long lda, const int* __restrict__ plan, int cb1, i
   }
 }
 
+// A sub-panel's in-panel step in one launch: its interchanges k1..k2-1 (at most
+// 32) on the panel's other columns [cb1, ce1) and [cb2, ce2), then, on the first
+// `nsolve` columns from cb2, the solve with the unit-lower kb x kb triangle T (kb
+// = k2 - k1, or 32 more: the rows of the sub-panel before it in the same block
+// come first, and the interchanges of T's and kj.L's columns are done beforehand) of
+// rows k2-kb .. k2-1, and the balancing keys of the product that
+// follows (kj: row maxima of the solution, and in extra CTAs column maxima of
+// kj.L). A warp per column: the composed interchanges bring the pivot rows into
+// the lane that solves for them (lane l owns rows l and l + 32 of the triangle),
+// and x_q is passed by a shuffle. The interchanges are composed by walking them
+// backwards for every touched row at once. Bound: the dependent steps (a shuffle
+// and an FP64 instruction each, about 110 cycles); four columns per CTA, since
+// four warps are what an SM's FP64 unit serves without queueing. One launch of
+// about 11 us instead of two of 12 and 13.
+constexpr int IPC = 4;  // columns (warps) per CTA
+template <typename T>
+__global__ void __launch_bounds__(32 * IPC)
+inpanel_step_kernel(T* A, long long lda, int k1, int k2, const int* __restrict__ ipiv, int cb1, int ce1,
+                    int cb2, int ce2, int nsolve, int kb, OzKeyJob kj) {
+  __shared__ T Ls[64 * 64];  // T(i, q) at q*64 + i, rows below the diagonal
+  __shared__ int s_piv[32], s_row[64], s_src[64];
+  __shared__ unsigned s_h[64];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int n1 = ce1 - cb1, ncols = n1 + (ce2 - cb2), ncta = (ncols + IPC - 1) / IPC;
+  if ((int)blockIdx.x >= ncta) {
+    if constexpr (sizeof(T) == 8) {
+      // column maxima of kj.L, 32 rows per CTA
+      const double* row = kj.L + min(((int)blockIdx.x - ncta) * 32 + lane, kj.lrows - 1);
+      double v[64 / IPC];
+#pragma unroll
+      for (int q = 0; q < 64 / IPC; ++q) v[q] = row[(long long)min(warp + IPC * q, kj.lcols - 1) * kj.ldl];
+#pragma unroll
+      for (int q = 0; q < 64 / IPC; ++q) {
+        const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(oz_key_word(v[q], 0ULL) & 4095ULL));
+        if (lane == 0 && hi && warp + IPC * q < kj.lcols)
+          oz_raise_key(kj.ckeys + warp + IPC * q, (kj.epoch << 12) | hi);
+      }
+    }
+    return;
+  }
+  const int npiv = k2 - k1, base = k2 - kb;  // base: first row of the triangle
+  const int ci = blockIdx.x * IPC + warp;
+  const bool in = ci < ncols;
+  const int col = ci < n1 ? cb1 + ci : cb2 + (ci - n1);
+  const bool solve = in && ci >= n1 && ci - n1 < nsolve;
+  T* a = A + (long long)(in ? col : cb2) * lda;
+  T x0 = (T)0, x1 = (T)0;
+  if (solve && kb > npiv && lane < kb - npiv) x0 = a[base + lane];
+  if (blockIdx.x * IPC + IPC > n1 && nsolve > 0) {  // some column of the CTA is solved
+    const T* Tm = A + base + (long long)base * lda;
+#pragma unroll 8
+    for (int idx = tid; idx < kb * 64; idx += 32 * IPC) {
+      const int i = idx & 63, q = idx >> 6;
+      Ls[idx] = (i > q && i < kb) ? Tm[i + (long long)q * lda] : (T)0;
+    }
+  }
+  if (tid < npiv) s_piv[tid] = ipiv[k1 + tid];
+  if (tid < 64) s_h[tid] = 0u;
+  __syncthreads();
+  if (tid < 64) {
+    // touched rows: k1.., then each pivot row outside them, once
+    int row = -1;
+    if (tid < 32) {
+      if (tid < npiv) row = k1 + tid;
+    } else if (tid - 32 < npiv) {
+      const int p = s_piv[tid - 32];
+      bool first = p < k1 || p >= k2;
+      for (int i = 0; i < tid - 32; ++i) first = first && s_piv[i] != p;
+      if (first) row = p;
+    }
+    int q = row;
+    for (int i = npiv - 1; i >= 0; --i) {
+      const int p = s_piv[i];
+      q = (q == k1 + i) ? p : ((q == p) ? k1 + i : q);
+    }
+    s_row[tid] = row;
+    s_src[tid] = q;
+  }
+  __syncthreads();
+  if (in) {
+    const int ra = s_row[lane], rb = s_row[lane + 32];
+    const T va = ra >= 0 ? a[s_src[lane]] : (T)0, vb = rb >= 0 ? a[s_src[lane + 32]] : (T)0;
+    __syncwarp();
+    if (rb >= 0) a[rb] = vb;
+    if (!solve) {
+      if (ra >= 0) a[ra] = va;
+    } else {
+      if (kb > npiv) x1 = va;
+      else x0 = va;
+      for (int q = 0; q < min(kb, 32); ++q) {
+        const T xq = __shfl_sync(0xffffffffu, x0, q);
+        if (lane > q) x0 = fma(-Ls[q * 64 + lane], xq, x0);
+        if (kb > 32) x1 = fma(-Ls[q * 64 + lane + 32], xq, x1);
+      }
+      for (int q = 32; q < kb; ++q) {
+        const T xq = __shfl_sync(0xffffffffu, x1, q - 32);
+        if (lane + 32 > q) x1 = fma(-Ls[q * 64 + lane + 32], xq, x1);
+      }
+      if (lane < kb) a[base + lane] = x0;
+      if (lane + 32 < kb) a[base + lane + 32] = x1;
+      if constexpr (sizeof(T) == 8) {
+        if (kj.hkeys) {
+          const unsigned h0 = (unsigned)(oz_key_word(x0, 0ULL) & 4095ULL), h1 = (unsigned)(oz_key_word(x1, 0ULL) & 4095ULL);
+          if (lane < kb && h0) atomicMax(&s_h[lane], h0);
+          if (lane + 32 < kb && h1) atomicMax(&s_h[lane + 32], h1);
+        }
+      }
+    }
+  }
+  if (kj.hkeys) {
+    __syncthreads();
+    if (tid < kb && s_h[tid]) oz_raise_key(kj.hkeys + tid, (kj.epoch << 12) | s_h[tid]);
+  }
+}
+
 // op(T) X = B for a w x w triangle (w <= 256) and a strip of NC columns of B
 // per CTA, held in shared memory. FORWARD solves top-down (lower, or upper^T),
 // otherwise bottom-up. The triangle is staged in shared memory eb (<= 32)
@@ -1563,6 +1678,20 @@ inline cudaError_t laswp(T* A, long long lda, int k1, int k2, const int* ipiv, i
     laswp_kernel<T><<<(unsigned)(want < cap ? want : cap), 256, 0, s>>>(A, lda, k1, k2, ipiv, cb1,
                                                                          ce1, cb2, ce2);
   }
+  count_launches(1);
+  return cudaGetLastError();
+}
+
+// The in-panel step of a sub-panel (kb <= 64, a multiple of 32 above k2 - k1), see
+// inpanel_step_kernel.
+template <typename T>
+inline cudaError_t inpanel_step(T* A, long long lda, int k1, int k2, const int* ipiv, int cb1, int ce1,
+                                int cb2, int ce2, int nsolve, int kb, cudaStream_t s,
+                                const OzKeyJob& kj = OzKeyJob()) {
+  const int ncols = (ce1 - cb1) + (ce2 - cb2);
+  if (ncols <= 0 || k2 <= k1) return cudaSuccess;
+  const int grid = (ncols + IPC - 1) / IPC + (kj.ckeys ? (kj.lrows + 31) / 32 : 0);
+  inpanel_step_kernel<T><<<grid, 32 * IPC, 0, s>>>(A, lda, k1, k2, ipiv, cb1, ce1, cb2, ce2, nsolve, kb, kj);
   count_launches(1);
   return cudaGetLastError();
 }

@@ -243,10 +243,8 @@ static cudaError_t factor_panel_f32(int n, float* F, long long ldf, int* dipiv, 
     const int r0 = j + c;
     SL_TRY(launch_panel<float>(F, ldf, m, r0, r0, w, dipiv, ws, s));
     const int kw = (m - r0) < w ? (m - r0) : w;
-    SL_TRY(laswp<float>(F, ldf, r0, r0 + kw, dipiv, j, r0, r0 + w, j + jb, s));
+    SL_TRY(inpanel_step<float>(F, ldf, r0, r0 + kw, dipiv, j, r0, r0 + w, j + jb, jb - c - w, kw, s));
     if (c + w < jb) {
-      SL_TRY((trsm_strip<float, false, false, true>(kw, jb - c - w, Fp(r0, r0), ldf,
-                                                     Fp(r0, r0 + w), ldf, s)));
       if (r0 + kw < m)
         SL_TRY(sgemm_simt(false, m - r0 - kw, jb - c - w, kw, -1.f, Fp(r0 + kw, r0), ldf,
                           Fp(r0, r0 + w), ldf, Fp(r0 + kw, r0 + w), ldf, s));

@@ -425,3 +425,32 @@ def test_cluster_panel_equals_grid_panel(sl, gpu_required, m, kind):
     assert got[0][0] == got[1][0]
     np.testing.assert_array_equal(got[0][1], got[1][1])
     np.testing.assert_array_equal(got[0][2], got[1][2])
+
+
+@pytest.mark.parametrize("ib", [1, 2, 3])
+@pytest.mark.parametrize("m,n", [(33, 33), (64, 70), (95, 97), (130, 40), (40, 130), (300, 257), (700, 321)])
+def test_in_panel_steps(sl, orc, gpu_required, m, n, ib):
+    """The in-panel step (interchanges, solve and product keys in one launch) for one
+    and two sub-panels per block, the unfused one beyond; partial sub-panels, wide
+    and tall matrices: pivots of the oracle's, and P A = L U to the tester's bound."""
+    import torch
+
+    rng = np.random.default_rng(m * n)
+    A = np.asfortranarray(rng.uniform(-0.5, 0.5, (m, n)))
+    dA = torch.from_numpy(A.T.copy()).cuda()
+    ip = torch.zeros(min(m, n), dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    L = sl.lib()
+    try:
+        L.sl1x1_set_panel_ib(ib)
+        assert sl.dgetrf_dev(m, n, dA.data_ptr(), m, ip.data_ptr(), 256) == 0
+    finally:
+        L.sl1x1_set_panel_ib(0)
+    F, piv = dA.T.cpu().numpy(), ip.cpu().numpy() - 1
+    PA = A.copy()
+    for k, p in enumerate(piv):
+        PA[[k, p]] = PA[[p, k]]
+    k = min(m, n)
+    low, up = np.tril(F[:, :k], -1) + np.eye(m, k), np.triu(F[:k])
+    assert np.abs(low).max() <= 1.0 + 1e-15  # partial pivoting
+    assert np.abs(PA - low @ up).max() < 16.0 * max(m, n) * 2.0**-53 * np.abs(A).sum(axis=1).max()
