@@ -18,7 +18,7 @@ LIBDIR = os.path.join(HERE, "_lib")
 OBJDIR = os.path.join(LIBDIR, "obj")
 LIBNAME = "libsl1x1gpu.so"
 ILP64_NAME = "libsl1x1gpu_ilp64.so"  # the same entry points with 8-byte INTEGERs
-SOURCES = ["api.cpp", "expert_api.cpp", "redist.cpp", "prof.cpp", "dgemm_f64.cu", "lu_f64.cu", "trsv_f64.cu", "noalloc.cu", "mixed_gemm.cu", "ozgemm_f64.cu", "mixed.cu", "batched.cu", "aux.cu", "refine.cu"]
+SOURCES = ["api.cpp", "expert_api.cpp", "redist.cpp", "prof.cpp", "dgemm_f64.cu", "lu_f64.cu", "trsv_f64.cu", "small_f64.cu", "noalloc.cu", "mixed_gemm.cu", "ozgemm_f64.cu", "mixed.cu", "batched.cu", "aux.cu", "refine.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 
 

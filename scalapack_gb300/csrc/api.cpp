@@ -709,6 +709,19 @@ int sl1x1_dgetrs_dev(char trans, int n, int nrhs, const double* dA, long long ld
 
 int sl1x1_dgesv_dev(int n, int nrhs, double* dA, long long ldda, int* dipiv, double* dB,
                     long long lddb, int nb, void* stream) {
+  // small systems in one launch (the DMMA form keeps its own path, and so does
+  // every call with an argument to refuse)
+  if (n > 0 && n <= sl::kSmallGesvMax && nrhs > 0 && nrhs <= sl::kSmallGesvRhs && ldda >= n && lddb >= n) {
+    std::lock_guard<std::mutex> lk(g_mu);
+    if (sl::f64_update_get() == 1) {
+      if (!ensure_device()) return cuda_info(cudaErrorNoDevice);
+      cudaStream_t s = (cudaStream_t)stream;
+      cudaError_t e = sl::small_gesv(n, nrhs, dA, ldda, dB, lddb, dipiv, g_dev.dsmall + 2, g_dev.dsmall + 3, s);
+      if (e != cudaSuccess) return cuda_info(e);
+      int info = 0;
+      return read_factor_info(s, n, &info);
+    }
+  }
   int info = sl1x1_dgetrf_dev(n, n, dA, ldda, dipiv, nb, stream);
   if (info != 0) return info;
   return sl1x1_dgetrs_dev('N', n, nrhs, dA, ldda, dipiv, dB, lddb, stream);

@@ -324,6 +324,15 @@ cudaError_t batch_plan_results(BatchPlan* p, int* info, int* iters, double* sres
 void batch_plan_shape(const BatchPlan* p, int* threads, int* chunk, int* ctas);
 void batch_plan_destroy(BatchPlan* p);
 
+// ---- one small system (small_f64.cu) ----
+// PDGESV of order n <= kSmallGesvMax with at most kSmallGesvRhs right-hand sides
+// in one launch: factors into A, 1-based pivots, the solution into B (left alone
+// when a pivot is zero); *status = 0, *info_col the first zero pivot's column or
+// INT_MAX.
+constexpr int kSmallGesvMax = 32, kSmallGesvRhs = 16;
+cudaError_t small_gesv(int n, int nrhs, double* A, long long lda, double* B, long long ldb, int* ipiv,
+                       int* status, int* info_col, cudaStream_t s);
+
 // ---- norms, condition estimate, inverse (aux.cu) ----
 cudaError_t dlange_device(char norm, int m, int n, const double* A, long long lda, double* work,
                           double* result, cudaStream_t s);

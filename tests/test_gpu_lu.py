@@ -454,3 +454,42 @@ def test_in_panel_steps(sl, orc, gpu_required, m, n, ib):
     low, up = np.tril(F[:, :k], -1) + np.eye(m, k), np.triu(F[:k])
     assert np.abs(low).max() <= 1.0 + 1e-15  # partial pivoting
     assert np.abs(PA - low @ up).max() < 16.0 * max(m, n) * 2.0**-53 * np.abs(A).sum(axis=1).max()
+
+
+@pytest.mark.parametrize("kind", ["random", "ties", "singular", "nan"])
+@pytest.mark.parametrize("n,nrhs", [(1, 1), (2, 3), (4, 4), (5, 1), (16, 16), (17, 15), (17, 16), (31, 1), (32, 1), (32, 16), (32, 17)])
+def test_small_gesv_equals_two_calls(sl, gpu_required, n, nrhs, kind):
+    """PDGESV of up to 32 rows and 16 right-hand sides is one launch: pivots, INFO and
+    factors bit for bit those of PDGETRF, X within the tester's bound, B untouched
+    when singular; NaN and ties as IDAMAX takes them; padded arrays."""
+    import torch
+
+    rng = np.random.default_rng(n * 40 + nrhs)
+    A = rng.uniform(-0.5, 0.5, (n, n))
+    if kind == "ties":
+        A = rng.integers(-2, 3, (n, n)).astype(float)
+    elif kind == "singular":
+        A[:, n // 2] = 0.0
+    elif kind == "nan":
+        A[n // 3, n // 2] = np.nan
+    B = rng.uniform(-0.5, 0.5, (n, nrhs))
+    lda, ldb = n + 2, n + 1
+    dA = torch.full((n, lda), -9923.0, dtype=torch.float64, device="cuda")
+    dA[:, :n] = torch.from_numpy(A.T.copy())
+    dB = torch.full((nrhs, ldb), -9923.0, dtype=torch.float64, device="cuda")
+    dB[:, :n] = torch.from_numpy(B.T.copy())
+    dF = dA.clone()
+    ip, ip2 = (torch.zeros(n, dtype=torch.int32, device="cuda") for _ in range(2))
+    torch.cuda.synchronize()
+    info = sl.dgesv_dev(n, nrhs, dA.data_ptr(), lda, ip.data_ptr(), dB.data_ptr(), ldb)
+    info2 = sl.dgetrf_dev(n, n, dF.data_ptr(), lda, ip2.data_ptr())
+    assert info == info2 and (kind != "singular" or info > 0)
+    np.testing.assert_array_equal(ip.cpu().numpy(), ip2.cpu().numpy())
+    np.testing.assert_array_equal(dA.cpu().numpy(), dF.cpu().numpy())
+    assert (dB[:, n:] == -9923.0).all()
+    X = dB[:, :n].T.cpu().numpy()
+    if info > 0:
+        np.testing.assert_array_equal(X, B)
+    elif kind in ("random", "ties"):
+        res = np.abs(B - A @ X).max(axis=0) / (np.abs(A).sum(axis=1).max() * np.abs(X).max(axis=0) * n * 2.0**-53)
+        assert (res < 16.0).all()
