@@ -875,6 +875,103 @@ solve_block128_kernel(int kb, const double* __restrict__ A, long long lda, int k
   }
 }
 
+// The same block step for many right-hand sides: a CTA stages the two inverses and
+// the coupling block once and takes eight right-hand sides at a time, two columns
+// per thread, so that all its warps feed the FP64 unit (the kernel above reloads 96
+// KB per right-hand side and leaves six of eight warps idle in each product); the
+// sums run in the same order. The triangles' zero quarters are skipped. Bound: the
+// FP64 pipe, 10240 FMAs per right-hand side and block. n = 3000, 3000 right-hand
+// sides: the whole solve 9.7 -> 7.4 ms.
+constexpr int kWideCols = 8;
+constexpr int kWideSmem = (3 * 64 * 64 + 2 * 128 * kWideCols) * (int)sizeof(double) + 128 * (int)sizeof(unsigned);
+template <bool LOWER>
+__global__ void __launch_bounds__(256)
+solve_block128_wide_kernel(int kb, const double* __restrict__ A, long long lda, int k0,
+                           const double* __restrict__ D, double* X, long long ldx, int nrhs,
+                           const unsigned* __restrict__ ck, unsigned long long* ckeys,
+                           unsigned long long* hkeys, unsigned long long epoch) {
+  extern __shared__ double blk_smem[];  // D0, D1 and the coupling block O, each [i*64 + r]
+  double* D0s = blk_smem;
+  double* D1s = blk_smem + 4096;
+  double* Os = blk_smem + 2 * 4096;
+  double* xs = blk_smem + 3 * 4096;           // [col][128]
+  double* ys = xs + 128 * kWideCols;
+  unsigned* s_h = reinterpret_cast<unsigned*>(ys + 128 * kWideCols);
+  const int t = threadIdx.x, r = t & 63, c = t >> 6;  // row, columns c and c + 4
+  const int w0 = kb < 64 ? kb : 64, w1 = kb - w0;
+  if (blockIdx.x == 0 && hkeys && t < kb && ck[k0 + t]) atomicMax(ckeys + t, (epoch << 12) | ck[k0 + t]);
+  const double* Dg = D + (size_t)(k0 / 64) * 4096;
+#pragma unroll 8
+  for (int idx = t; idx < 4096; idx += 256) {
+    const int rr = idx & 63, i = idx >> 6;
+    const bool in = LOWER ? (rr < w1 && i < w0) : (rr < w0 && i < w1);
+    const long long off = LOWER ? (k0 + 64 + rr) + (long long)(k0 + i) * lda
+                                : (k0 + rr) + (long long)(k0 + 64 + i) * lda;
+    D0s[idx] = Dg[idx];
+    D1s[idx] = w1 > 0 ? Dg[4096 + idx] : 0.0;
+    Os[idx] = in ? A[off] : 0.0;
+  }
+  if (t < 128) s_h[t] = 0u;
+  // y = M v for 64 rows: v, y at offset h of a column; i runs over the warp's part
+  // of the triangle (i0 .. i1)
+  auto tri = [&](const double* M, int h, int i0, int i1) {
+    double a0 = 0.0, a1 = 0.0;
+    for (int i = i0; i < i1; ++i) {
+      const double m = M[i * 64 + r];
+      a0 = fma(m, xs[c * 128 + h + i], a0);
+      a1 = fma(m, xs[(c + 4) * 128 + h + i], a1);
+    }
+    ys[c * 128 + h + r] = a0;
+    ys[(c + 4) * 128 + h + r] = a1;
+  };
+  // x -= O y, x at offset hx, y at offset hy, w columns of O
+  auto couple = [&](int hx, int hy, int w) {
+    double a0 = xs[c * 128 + hx + r], a1 = xs[(c + 4) * 128 + hx + r];
+    for (int i = 0; i < w; ++i) {
+      const double m = Os[i * 64 + r];
+      a0 = fma(-m, ys[c * 128 + hy + i], a0);
+      a1 = fma(-m, ys[(c + 4) * 128 + hy + i], a1);
+    }
+    xs[c * 128 + hx + r] = a0;
+    xs[(c + 4) * 128 + hx + r] = a1;
+  };
+  const int lo_i0 = LOWER ? 0 : (r & 32), lo_i1 = LOWER ? (r & 32) + 32 : 64;
+  for (int g = blockIdx.x * kWideCols; g < nrhs; g += gridDim.x * kWideCols) {
+    __syncthreads();  // the staging, or the previous group's last reads
+#pragma unroll
+    for (int q = 0; q < kWideCols / 2; ++q) {
+      const int row = t & 127, col = (t >> 7) + 2 * q;
+      xs[col * 128 + row] = (row < kb && g + col < nrhs) ? X[k0 + row + (long long)(g + col) * ldx] : 0.0;
+    }
+    __syncthreads();
+    if (LOWER) {  // y0 = inv(L00) x0; x1 -= L10 y0; y1 = inv(L11) x1
+      tri(D0s, 0, lo_i0, lo_i1);
+      __syncthreads();
+      couple(64, 0, w0);
+      __syncthreads();
+      tri(D1s, 64, lo_i0, lo_i1);
+    } else {      // y1 = inv(U11) x1; x0 -= U01 y1; y0 = inv(U00) x0
+      tri(D1s, 64, lo_i0, lo_i1);
+      __syncthreads();
+      couple(0, 64, max(w1, 0));
+      __syncthreads();
+      tri(D0s, 0, lo_i0, lo_i1);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < kWideCols / 2; ++q) {
+      const int row = t & 127, col = (t >> 7) + 2 * q;
+      if (row < kb && g + col < nrhs) {
+        const double y = ys[col * 128 + row];
+        X[k0 + row + (long long)(g + col) * ldx] = y;
+        if (hkeys) atomicMax(&s_h[row], (unsigned)(oz_key_word(y, 0ULL) & 4095ULL));
+      }
+    }
+  }
+  __syncthreads();
+  if (hkeys && t < kb && s_h[t]) oz_raise_key(hkeys + t, (epoch << 12) | s_h[t]);
+}
+
 // Blocked NOTRAN solve with the diagonal-block inverses (ws.dinv_solve: L
 // blocks, then U blocks, then the column keys) and the off-diagonal updates
 // as sliced products on the tensor cores: 128-row blocks, each applied by
@@ -895,7 +992,15 @@ static cudaError_t tri_solve_inv(bool lower, int n, int nrhs, const double* A, l
     const int k0 = b * KB, kb = (n - k0) < KB ? (n - k0) : KB;
     const int rest = lower ? n - k0 - kb : k0;
     const unsigned long long ep = rest > 0 ? oz_new_epoch() : 0ULL;
-    if (lower)
+    if (nrhs >= kWideRhs) {
+      const int grid = std::min(2 * num_sms(), (nrhs + kWideCols - 1) / kWideCols);
+      if (lower)
+        solve_block128_wide_kernel<true><<<grid, 256, kWideSmem, s>>>(
+            kb, A, lda, k0, D, X, ldx, nrhs, ck, ckeys, rest > 0 ? hkeys : nullptr, ep);
+      else
+        solve_block128_wide_kernel<false><<<grid, 256, kWideSmem, s>>>(
+            kb, A, lda, k0, D, X, ldx, nrhs, ck, ckeys, rest > 0 ? hkeys : nullptr, ep);
+    } else if (lower)
       solve_block128_kernel<true><<<nrhs + (rest > 0 ? 1 : 0), 256, kBlkSmem, s>>>(
           kb, A, lda, k0, D, X, ldx, nrhs, ck, ckeys, rest > 0 ? hkeys : nullptr, ep);
     else
@@ -923,11 +1028,14 @@ cudaError_t dgetrs_device(char trans, int n, int nrhs, const double* dA, long lo
   // any NRHS whose products fit the scratch (PDGETRI solves with NRHS = N)
   const bool inv_path = g_f64_update == 1 && ws.dinv_solve && ws.dinv_solve_len >= kSolveInvDoubles(n) &&
                         oz_fits(ws.oz, n, nrhs, 128);
-  // up to 16 right-hand sides go through the chained solves, both TRANS: at
-  // n = 16384, 16 columns they take 9.8 ms (the blocked solve 13.6), below that
-  // 2 to 6 times less; beyond 16 the FP64 pipe's n^2 nrhs bound passes the
-  // blocked NOTRAN solve, whose products run on the tensor cores
-  const bool chain_path = g_f64_update == 1 && nrhs <= kChainRhs && ws.dinv_solve &&
+  // Few right-hand sides go through the chained solves: NOTRAN up to 16 (n =
+  // 16384, 16 columns: 9.8 ms, the blocked solve 13.6; below that 2 to 6 times
+  // less) and up to 32 while n <= 4096 (n = 1000: 0.38 of 0.69 ms), where the FP64
+  // pipe's n^2 nrhs bound passes the blocked solve, whose products run on the
+  // tensor cores; transposed up to 128 (n = 8192, 64 columns: 11.6 of 31 ms: the
+  // blocked form there substitutes and multiplies on the FP64 pipe)
+  const int chain_rhs = notran ? (n <= 4096 ? 32 : 16) : kChainRhs;
+  const bool chain_path = g_f64_update == 1 && nrhs <= chain_rhs && ws.dinv_solve &&
                           ws.dinv_solve_len >= kSolveInvDoubles(n) && ws.chain && ws.chain_epoch &&
                           ws.chain_values >= (size_t)n * nrhs;
   if (notran ? (inv_path || chain_path) : chain_path) {
@@ -972,8 +1080,14 @@ cudaError_t dgetrs_device(char trans, int n, int nrhs, const double* dA, long lo
         solve_block128_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBlkSmem);
     static const cudaError_t a3 = cudaFuncSetAttribute(
         solve_block128_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBlkSmem);
+    static const cudaError_t a4 = cudaFuncSetAttribute(
+        solve_block128_wide_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWideSmem);
+    static const cudaError_t a5 = cudaFuncSetAttribute(
+        solve_block128_wide_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWideSmem);
     SL_TRY(a2);
     SL_TRY(a3);
+    SL_TRY(a4);
+    SL_TRY(a5);
     solve_ckeys_kernel<<<(n + 7) / 8, 256, 0, s>>>(
         n, dA, ldda, reinterpret_cast<unsigned*>(ws.dinv_solve + (size_t)2 * nb64 * 4096), nb64 * 64);
     count_launches(1);

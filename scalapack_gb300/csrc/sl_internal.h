@@ -177,6 +177,9 @@ constexpr int kOzKinfoBytes = 8192;
 inline size_t kSolveInvDoubles(int n) {
   return (size_t)2 * (size_t)((n + 63) / 64) * 64 * 64 + (size_t)((n + 63) / 64) * 64;
 }
+// Right-hand sides from which a blocked NOTRAN solve shares a CTA's staged blocks
+// among several of them.
+constexpr int kWideRhs = 256;
 // Doubles of the U12 solve's diagonal-block inverses: NB <= 1024 in 64-row blocks.
 constexpr size_t kDinv64Doubles = (size_t)16 * 64 * 64;
 
@@ -231,8 +234,8 @@ cudaError_t dgetrs_device(char trans, int n, int nrhs, const double* dA, long lo
                           const int* dipiv, double* dB, long long lddb, const LuWork& ws,
                           cudaStream_t s);
 
-// Most right-hand sides of a chained solve.
-constexpr int kChainRhs = 16;
+// Most right-hand sides of a chained solve (dgetrs_device has the rule).
+constexpr int kChainRhs = 128;
 // op(T) X = S with the lower (unit) or upper triangle of n x n LU factors in
 // one launch (trsv_f64.cu): D holds the inverses of that triangle's 64x64
 // diagonal blocks; S is src with its rows permuted by the pivots `gather`, X goes
