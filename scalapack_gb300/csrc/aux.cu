@@ -319,6 +319,7 @@ cudaError_t dgetri_device(int n, double* dA, long long lda, const int* dipiv, do
   const long long tot = (long long)n * n;
   identity_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(X, n, n);
   count_launches(1);
+  if (inverse_fits(n, ws)) return inverse_from_factors(n, dA, lda, dipiv, X, ws, s);
   SL_TRY(dgetrs_device('N', n, n, dA, lda, dipiv, X, n, ws, s));
   return cudaMemcpy2DAsync(dA, lda * sizeof(double), X, n * sizeof(double), n * sizeof(double), n,
                            cudaMemcpyDeviceToDevice, s);

@@ -977,8 +977,11 @@ solve_block128_wide_kernel(int kb, const double* __restrict__ A, long long lda, 
 // as sliced products on the tensor cores: 128-row blocks, each applied by
 // inverse and then subtracted from the rest. The products take their
 // balancing keys from the block step (no key pass over the factor per step).
-static cudaError_t tri_solve_inv(bool lower, int n, int nrhs, const double* A, long long lda,
-                                 double* X, long long ldx, const LuWork& ws, cudaStream_t s) {
+// With triangular set (LOWER), X is lower triangular on entry (an identity) and
+// stays so: a block step concerns only the columns up to its own.
+static cudaError_t tri_solve_inv(bool lower, int n, int ncols, const double* A, long long lda,
+                                 double* X, long long ldx, const LuWork& ws, cudaStream_t s,
+                                 bool triangular = false) {
   constexpr int KB = 128;
   const int nblk = (n + KB - 1) / KB;
   const int nb64 = (n + 63) / 64;
@@ -991,6 +994,7 @@ static cudaError_t tri_solve_inv(bool lower, int n, int nrhs, const double* A, l
     const int b = lower ? bi : nblk - 1 - bi;
     const int k0 = b * KB, kb = (n - k0) < KB ? (n - k0) : KB;
     const int rest = lower ? n - k0 - kb : k0;
+    const int nrhs = triangular ? std::min(ncols, k0 + kb) : ncols;
     const unsigned long long ep = rest > 0 ? oz_new_epoch() : 0ULL;
     if (nrhs >= kWideRhs) {
       const int grid = std::min(2 * num_sms(), (nrhs + kWideCols - 1) / kWideCols);
@@ -1018,6 +1022,64 @@ static cudaError_t tri_solve_inv(bool lower, int n, int nrhs, const double* A, l
   return cudaSuccess;
 }
 
+// Shared-memory opt-in of the blocked solve's kernels, once.
+static cudaError_t blocked_solve_attrs() {
+  static const cudaError_t a[] = {
+      cudaFuncSetAttribute(solve_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kInvSmem),
+      cudaFuncSetAttribute(solve_block128_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBlkSmem),
+      cudaFuncSetAttribute(solve_block128_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBlkSmem),
+      cudaFuncSetAttribute(solve_block128_wide_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWideSmem),
+      cudaFuncSetAttribute(solve_block128_wide_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWideSmem)};
+  for (cudaError_t e : a) SL_TRY(e);
+  return cudaSuccess;
+}
+
+// Diagonal-block inverses, the pivots' permutation (ws.perm) and, for the blocked
+// solve, the column keys.
+static cudaError_t prepare_solve(int n, const double* dA, long long ldda, const int* dipiv, const LuWork& ws,
+                                 int* tickets, bool blocked, cudaStream_t s) {
+  SL_TRY(blocked_solve_attrs());
+  const int nrb = (n + 255) / 256, nb64 = (n + 63) / 64;
+  solve_prep_kernel<<<2 * kInvParts * nb64 + nrb * perm_segs(n), 256, kInvSmem, s>>>(
+      n, dA, ldda, ws.dinv_solve, dipiv, ws.perm + n, ws.status, tickets);
+  count_launches(1);
+  if (blocked) {
+    perm_finish_kernel<<<nrb, 256, 0, s>>>(dipiv, n, ws.perm + n, ws.perm);
+    solve_ckeys_kernel<<<(n + 7) / 8, 256, 0, s>>>(
+        n, dA, ldda, reinterpret_cast<unsigned*>(ws.dinv_solve + (size_t)2 * nb64 * 4096), nb64 * 64);
+    count_launches(2);
+  }
+  return cudaGetLastError();
+}
+
+// dst(:, perm[i]) = X(:, i), n x n.
+__global__ void scatter_columns_kernel(int n, const double* __restrict__ X, double* dst, long long ldd,
+                                       const int* __restrict__ perm) {
+  const int c = blockIdx.y, p = perm[c];
+  const int r = blockIdx.x * 256 + threadIdx.x;
+  if (r < n && (unsigned)p < (unsigned)n) dst[r + (long long)p * ldd] = X[r + (long long)c * n];
+}
+
+// inv(A) = inv(U) inv(L) P: L's inverse is formed as a lower triangle (a third of
+// a full solve's work), U's solve runs over all columns, and the interchanges are
+// a permutation of the result's columns. n = 3000: 5.75 ms, 7.5 with the identity
+// permuted first and both solves full.
+bool inverse_fits(int n, const LuWork& ws) {
+  return n >= kWideRhs && n <= 65535 && g_f64_update == 1 && ws.dinv_solve &&
+         ws.dinv_solve_len >= kSolveInvDoubles(n) && oz_fits(ws.oz, n, n, 128);
+}
+cudaError_t inverse_from_factors(int n, double* dA, long long ldda, const int* dipiv, double* X,
+                                 const LuWork& ws, cudaStream_t s) {
+  phase_begin(kPhSolve, s);
+  SL_TRY(prepare_solve(n, dA, ldda, dipiv, ws, nullptr, true, s));
+  SL_TRY(tri_solve_inv(true, n, n, dA, ldda, X, n, ws, s, true));
+  SL_TRY(tri_solve_inv(false, n, n, dA, ldda, X, n, ws, s));
+  scatter_columns_kernel<<<dim3((n + 255) / 256, n), 256, 0, s>>>(n, X, dA, ldda, ws.perm);
+  count_launches(1);
+  phase_end(kPhSolve, s, 4.0 * (double)n * n * n / 3.0, 24.0 * (double)n * n);
+  return cudaGetLastError();
+}
+
 cudaError_t dgetrs_device(char trans, int n, int nrhs, const double* dA, long long ldda,
                           const int* dipiv, double* dB, long long lddb, const LuWork& ws,
                           cudaStream_t s) {
@@ -1039,19 +1101,7 @@ cudaError_t dgetrs_device(char trans, int n, int nrhs, const double* dA, long lo
                           ws.dinv_solve_len >= kSolveInvDoubles(n) && ws.chain && ws.chain_epoch &&
                           ws.chain_values >= (size_t)n * nrhs;
   if (notran ? (inv_path || chain_path) : chain_path) {
-    static const cudaError_t a0 = cudaFuncSetAttribute(
-        solve_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kInvSmem);
-    SL_TRY(a0);
-    const int nrb = (n + 255) / 256;
-    solve_prep_kernel<<<2 * kInvParts * ((n + 63) / 64) + nrb * perm_segs(n), 256, kInvSmem, s>>>(
-        n, dA, ldda, ws.dinv_solve, dipiv, ws.perm + n, ws.status, chain_path ? ws.chain : nullptr);
-    count_launches(1);
-    SL_TRY(cudaGetLastError());
-    if (!chain_path) {
-      perm_finish_kernel<<<nrb, 256, 0, s>>>(dipiv, n, ws.perm + n, ws.perm);
-      count_launches(1);
-      SL_TRY(cudaGetLastError());
-    }
+    SL_TRY(prepare_solve(n, dA, ldda, dipiv, ws, chain_path ? ws.chain : nullptr, !chain_path, s));
   } else {
     SL_TRY(cudaMemsetAsync(ws.status, 0, sizeof(int), s));
     SL_TRY(perm_compose(dipiv, n, ws.perm, s));
@@ -1075,23 +1125,6 @@ cudaError_t dgetrs_device(char trans, int n, int nrhs, const double* dA, long lo
   }
   if (notran && inv_path) {
     SL_TRY((permute_rows<double, double>(dB, lddb, X, n, ws.perm, n, nrhs, 0, s)));
-    const int nb64 = (n + 63) / 64;
-    static const cudaError_t a2 = cudaFuncSetAttribute(
-        solve_block128_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBlkSmem);
-    static const cudaError_t a3 = cudaFuncSetAttribute(
-        solve_block128_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBlkSmem);
-    static const cudaError_t a4 = cudaFuncSetAttribute(
-        solve_block128_wide_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWideSmem);
-    static const cudaError_t a5 = cudaFuncSetAttribute(
-        solve_block128_wide_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWideSmem);
-    SL_TRY(a2);
-    SL_TRY(a3);
-    SL_TRY(a4);
-    SL_TRY(a5);
-    solve_ckeys_kernel<<<(n + 7) / 8, 256, 0, s>>>(
-        n, dA, ldda, reinterpret_cast<unsigned*>(ws.dinv_solve + (size_t)2 * nb64 * 4096), nb64 * 64);
-    count_launches(1);
-    SL_TRY(cudaGetLastError());
     SL_TRY(tri_solve_inv(true, n, nrhs, dA, ldda, X, n, ws, s));
     SL_TRY(tri_solve_inv(false, n, nrhs, dA, ldda, X, n, ws, s));
     SL_TRY(cudaMemcpy2DAsync(dB, lddb * sizeof(double), X, n * sizeof(double),

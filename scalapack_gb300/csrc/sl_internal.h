@@ -247,6 +247,12 @@ cudaError_t trsv64_chain(bool lower, bool trans, const double* A, long long lda,
                          long long ldd, const int* scatter, const int* maps, int nrhs, int* ticket,
                          unsigned long long* words, uint32_t epoch, int* status, cudaStream_t s);
 
+// inv(A) from its factors over dA, X = the identity (n x n workspace, ld n), by the
+// blocked solves (inverse_fits: order and scratch allow it).
+bool inverse_fits(int n, const LuWork& ws);
+cudaError_t inverse_from_factors(int n, double* dA, long long ldda, const int* dipiv, double* X,
+                                 const LuWork& ws, cudaStream_t s);
+
 // ---- low-precision trailing update (mixed_gemm.cu) ----
 // Pack L21 (m x k FP32 col-major) and U12 (k x n FP32 col-major, per-column
 // power-of-two scaled) into 16-bit K-major operands of k rounded up to 64.

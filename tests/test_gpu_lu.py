@@ -493,3 +493,23 @@ def test_small_gesv_equals_two_calls(sl, gpu_required, n, nrhs, kind):
     elif kind in ("random", "ties"):
         res = np.abs(B - A @ X).max(axis=0) / (np.abs(A).sum(axis=1).max() * np.abs(X).max(axis=0) * n * 2.0**-53)
         assert (res < 16.0).all()
+
+
+@pytest.mark.parametrize("n", [255, 256, 257, 383, 640, 1000])
+def test_inverse_by_triangles(sl, gpu_required, n):
+    """PDGETRI on both sides of the order from which inv(L) is formed as a triangle
+    and the interchanges become a column permutation; partial last blocks."""
+    import torch
+
+    rng = np.random.default_rng(n)
+    A = rng.uniform(-0.5, 0.5, (n, n))
+    dA = torch.full((n, n + 3), -9923.0, dtype=torch.float64, device="cuda")
+    dA[:, :n] = torch.from_numpy(A.T.copy())
+    ip = torch.zeros(n, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    assert sl.dgetrf_dev(n, n, dA.data_ptr(), n + 3, ip.data_ptr()) == 0
+    assert sl.lib().sl1x1_dgetri_dev(n, dA.data_ptr(), n + 3, ip.data_ptr(), None) == 0
+    assert (dA[:, n:] == -9923.0).all()
+    V = dA[:, :n].T.cpu().numpy()
+    res = np.abs(A @ V - np.eye(n)).sum(axis=1).max()
+    assert res / (np.abs(A).sum(axis=1).max() * np.abs(V).sum(axis=1).max() * n * 2.0**-53) < 16.0  # the tester's bound
