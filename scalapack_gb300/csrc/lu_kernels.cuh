@@ -247,7 +247,10 @@ __device__ __forceinline__ double recip_bits(unsigned long long bits) {
 // instead (gtile, column-major per CTA: rpc rows x PW columns, so a warp's
 // row walk is one coalesced access; the labels follow all rows); the algorithm
 // is unchanged.
-template <typename T, bool GTILE = false>
+//
+// ONE: a row thread has at most one row (rpc * tpr <= PTR), whose label stays in a
+// register (its loops cost 400 cycles of a column's 4600).
+template <typename T, bool GTILE = false, bool ONE = false>
 __global__ void __launch_bounds__(PT, GTILE ? 1 : 3)
 panel_kernel(T* A, long long lda, int m, int r0, int c0, int w, int rpc, int* ipiv,
              int* info_col, double* cand, int* status, long long spin_limit, T* gtile,
@@ -297,7 +300,8 @@ panel_kernel(T* A, long long lda, int m, int r0, int c0, int w, int rpc, int* ip
     }
   };
   // row thread tid: part `part` of rows row0, row0 + rstep, ...
-  const int part = tid & (tpr - 1), row0 = tid / tpr, rstep = PTR / tpr;
+  const int part = tid & (tpr - 1), row0 = exch ? nr : tid / tpr, rstep = PTR / tpr;
+  int mylab = row0 < nr ? lo + row0 : -1;  // ONE: the label of row row0
 
   if (!exch) {
     // Sub-panel rows into shared memory, PCH columns' loads in flight at
@@ -332,8 +336,8 @@ panel_kernel(T* A, long long lda, int m, int r0, int c0, int w, int rpc, int* ip
   // row's threads; the next column's operands are read while one is updated
   auto finish_update = [&](int kp) {
     const T* U = s_U[kp & 1];
-    for (int r = row0; r < nr; r += rstep) {
-      if (lab[r] < 0) continue;
+    for (int r = row0; r < nr; r += ONE ? nr : rstep) {
+      if ((ONE ? mylab : lab[r]) < 0) continue;
       const T l = tile[tix(r, kp)];
       int j = kp + 2 + part;
       if (j >= w) continue;
@@ -470,6 +474,23 @@ panel_kernel(T* A, long long lda, int m, int r0, int c0, int w, int rpc, int* ip
       const int piv = s_piv, mine = s_own == b ? lrow : -1;
       const int kn = k + 1;
       const T un = s_U[par][kn < w ? kn : k];
+      if constexpr (ONE) {
+        const int r = min(row0, rpc - 1);
+        T l = tile[tix(r, k)];
+        const T a = tile[tix(r, kn < w ? kn : k)];
+        l *= rinv;
+        const T v = fma(-l, un, a);
+        const bool act = mylab >= 0 && row0 != mine && part == 0;
+        if (mylab == k) mylab = piv;   // the diagonal row goes where the pivot row stood
+        if (row0 == mine) mylab = ~k;  // pivot row k
+        if (act) {
+          tile[tix(r, k)] = l;
+          if (kn < w) tile[tix(r, kn)] = v;
+        }
+        if (kn < kw)
+          put_candidate(act ? row_key(v, mylab, kn) : -2LL, act ? mylab : INT_MAX, row0);
+        continue;
+      }
       long long nkey = -2;
       int nlab = INT_MAX, nrow = 0;
       for (int r = part == 0 ? row0 : nr; r < nr; r += rstep) {
@@ -495,6 +516,7 @@ panel_kernel(T* A, long long lda, int m, int r0, int c0, int w, int rpc, int* ip
   // fewer rows than columns), then every row to where its content stands
   if (exch) return;
   if (kw > 0) finish_update(kw - 1);
+  if (ONE && part == 0 && row0 < nr) lab[row0] = mylab;
   asm volatile("bar.sync 1, %0;" ::"n"(PTR) : "memory");
   for (int r = tid; r < nr; r += PTR) {
     const int lb = lab[r];
@@ -1641,7 +1663,10 @@ inline cudaError_t launch_panel(T* A, long long lda, int m, int r0, int c0, int 
       smem = 0;
     }
   }
-  if (!global_tile) SL_TRY(smem_attr_once((const void*)panel_kernel<T, false>, 212 * 1024));
+  if (!global_tile) {
+    SL_TRY(smem_attr_once((const void*)panel_kernel<T, false, false>, 212 * 1024));
+    SL_TRY(smem_attr_once((const void*)panel_kernel<T, false, true>, 212 * 1024));
+  }
   // Tags of this launch's words: 64 per launch, never used before in this
   // area since it was cleared (when new and when the launch count wraps).
   // Without a launch count the words are cleared for every launch.
@@ -1660,7 +1685,8 @@ inline cudaError_t launch_panel(T* A, long long lda, int m, int r0, int c0, int 
   count_launches(1);
   if (global_tile)
     return cudaLaunchCooperativeKernel((void*)panel_kernel<T, true>, dim3(G), dim3(PT), args, 0, s);
-  return cudaLaunchCooperativeKernel((void*)panel_kernel<T, false>, dim3(G), dim3(PT), args, smem, s);
+  void* kern = rpc * tpr <= PTR ? (void*)panel_kernel<T, false, true> : (void*)panel_kernel<T, false, false>;
+  return cudaLaunchCooperativeKernel(kern, dim3(G), dim3(PT), args, smem, s);
 }
 
 template <typename T>
