@@ -918,54 +918,57 @@ laswp_kernel(T* A, long long lda, int k1, int k2, const int* __restrict__ ipiv, 
 // panel, on the panel's stream; laswp_apply_kernel then only moves data.
 static __device__ __noinline__ void laswp_plan_block(int k1, int k2, const int* __restrict__ ipiv,
                                                     int* plan) {
-  __shared__ int s_piv[LSW_MAXP], s_first[LSW_MAXP], s_rank[LSW_MAXP];
-  __shared__ int s_row[2 * LSW_MAXP], s_src[2 * LSW_MAXP];
-  __shared__ int s_cnt;
+  __shared__ int s_piv[LSW_MAXP], s_row[2 * LSW_MAXP];
   const int npiv = k2 - k1, tid = threadIdx.x, nt = blockDim.x;
   for (int i = tid; i < npiv; i += nt) s_piv[i] = ipiv[k1 + i];
+  // exclusive rank of this thread's flag among the block's (in thread order), and
+  // the total: ballots and the warps' counts
+  __shared__ int s_wc[32];
+  auto rank = [&](bool f, int& total) {
+    const unsigned m = __ballot_sync(0xffffffffu, f);
+    __syncthreads();
+    if ((tid & 31) == 0) s_wc[tid >> 5] = __popc(m);
+    __syncthreads();
+    int before = 0;
+    total = 0;
+    for (int w = 0; w < nt / 32; ++w) {
+      if (w < tid / 32) before += s_wc[w];
+      total += s_wc[w];
+    }
+    return before + __popc(m & ((1u << (tid & 31)) - 1u));
+  };
   __syncthreads();
-  // interchange i reaches an outside row for the first time
-  for (int i = tid; i < npiv; i += nt) {
-    const int p = s_piv[i];
+  // each outside row where an interchange reaches it for the first time
+  int cnt = npiv, tot = 0;
+  for (int i0 = 0; i0 < npiv; i0 += nt) {
+    const int i = i0 + tid, p = i < npiv ? s_piv[i] : k1;
     bool first = p < k1 || p >= k2;
-    for (int i2 = 0; first && i2 < i; ++i2) first = s_piv[i2] != p;
-    s_first[i] = first ? 1 : 0;
+    for (int i2 = 0; i2 < min(i, npiv); ++i2)
+      if (s_piv[i2] == p) first = false;
+    const int q = rank(first, tot);
+    if (i < npiv) s_row[i] = k1 + i;
+    if (first) s_row[cnt + q] = p;
+    cnt += tot;
   }
   __syncthreads();
-  if (tid == 0) {
-    int c = 0;
-    for (int i = 0; i < npiv; ++i) {
-      s_rank[i] = c;
-      c += s_first[i];
-    }
-    s_cnt = npiv + c;
-  }
-  __syncthreads();
-  for (int i = tid; i < npiv; i += nt) {
-    s_row[i] = k1 + i;
-    if (s_first[i]) s_row[npiv + s_rank[i]] = s_piv[i];
-  }
-  __syncthreads();
-  const int cnt = s_cnt;
-  for (int e = tid; e < cnt; e += nt) {
-    int q = s_row[e];
-    for (int i = npiv - 1; i >= 0; --i) {
-      const int p = s_piv[i];
-      q = (q == k1 + i) ? p : ((q == p) ? k1 + i : q);
-    }
-    s_src[e] = q;
-  }
-  __syncthreads();
-  if (tid == 0) {
-    int np = 0;
-    for (int e = 0; e < cnt; ++e)
-      if (s_src[e] != s_row[e]) {
-        plan[1 + 2 * np] = s_row[e];
-        plan[2 + 2 * np] = s_src[e];
-        ++np;
+  int np = 0;
+  for (int e0 = 0; e0 < cnt; e0 += nt) {
+    const int e = e0 + tid, row = e < cnt ? s_row[e] : -1;
+    int q = row;
+    if (e < cnt)
+      for (int i = npiv - 1; i >= 0; --i) {
+        const int p = s_piv[i];
+        q = (q == k1 + i) ? p : ((q == p) ? k1 + i : q);
       }
-    plan[0] = np;
+    const bool moved = e < cnt && q != row;
+    const int at = np + rank(moved, tot);
+    if (moved) {
+      plan[1 + 2 * at] = row;
+      plan[2 + 2 * at] = q;
+    }
+    np += tot;
   }
+  if (tid == 0) plan[0] = np;
 }
 
 static __global__ void laswp_plan_kernel(int k1, int k2, const int* __restrict__ ipiv, int* plan) {
@@ -1210,6 +1213,69 @@ trsm_strip_kernel(int w, int ncols, int eb, const T* __restrict__ Tm, long long 
         if (km) oz_raise_key(kj.hkeys + r, km);
       }
   }
+}
+
+// L X = B in place for a unit-lower w x w triangle (w <= 256) and many columns: a
+// warp takes TCC columns, lane l owning rows l, l + 32, .. of each in registers, and
+// x_q passes by a shuffle; the triangle comes through shared memory 32 columns at a
+// time, with a barrier per 32 steps instead of one per step. Elements take their
+// updates in the order of the substitution, one fma each. Bound: the triangle's
+// reads from shared memory. FP32, w = 256, 8192 columns: 30 us (trsm_strip_kernel,
+// 145).
+constexpr int TCC = 2;
+template <typename T>
+__global__ void __launch_bounds__(256)
+trsm_cols_kernel(int w, int ncols, const T* __restrict__ L, long long ldl, T* B, long long ldb) {
+  __shared__ T Es[32 * 256];  // L(r, s0 + i) at i*256 + r
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int col0 = ((int)blockIdx.x * 8 + warp) * TCC;
+  T x[TCC][8];
+#pragma unroll
+  for (int c = 0; c < TCC; ++c)
+#pragma unroll
+    for (int t = 0; t < 8; ++t) {
+      const int r = lane + 32 * t;
+      x[c][t] = (r < w && col0 + c < ncols) ? B[r + (long long)(col0 + c) * ldb] : (T)0;
+    }
+  // thread tid stages row tid: the next 32 columns are on their way (addresses
+  // clamped into the triangle's square, no test before a load) while these are used
+  const T* lrow = L + min(tid, w - 1);
+  T e[32];
+#pragma unroll
+  for (int i = 0; i < 32; ++i) e[i] = lrow[(long long)min(i, w - 1) * ldl];
+#pragma unroll
+  for (int tq = 0; tq < 8; ++tq) {
+    const int s0 = 32 * tq;
+    if (s0 >= w) break;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 32; ++i) Es[i * 256 + tid] = (tid < w && s0 + i < tid) ? e[i] : (T)0;
+    __syncthreads();
+    if (s0 + 32 < w) {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) e[i] = lrow[(long long)min(s0 + 32 + i, w - 1) * ldl];
+    }
+#pragma unroll 4
+    for (int i = 0; i < 32; ++i) {
+      T xq[TCC];
+#pragma unroll
+      for (int c = 0; c < TCC; ++c) xq[c] = __shfl_sync(0xffffffffu, x[c][tq], i);
+#pragma unroll
+      for (int t = tq; t < 8; ++t) {
+        const T l = Es[i * 256 + lane + 32 * t];
+#pragma unroll
+        for (int c = 0; c < TCC; ++c)
+          if (t > tq || lane > i) x[c][t] = fma(-l, xq[c], x[c][t]);
+      }
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < TCC; ++c)
+#pragma unroll
+    for (int t = 0; t < 8; ++t) {
+      const int r = lane + 32 * t;
+      if (r < w && col0 + c < ncols) B[r + (long long)(col0 + c) * ldb] = x[c][t];
+    }
 }
 
 // op(T) x = b for a w x w diagonal block (w <= 128) and few right-hand sides:
@@ -1747,9 +1813,22 @@ inline cudaError_t laswp_planned(T* A, long long lda, int k1, int k2, const int*
   return cudaGetLastError();
 }
 
+// Unit-lower solve of many columns: trsm_cols_kernel up to 256 rows, else strips.
 template <typename T, bool UPPER, bool TRANS, bool UNIT, int NC = 8>
 inline cudaError_t trsm_strip(int w, int ncols, const T* Tm, long long ldt, T* B, long long ldb,
-                              cudaStream_t s, const OzKeyJob& kj = OzKeyJob()) {
+                              cudaStream_t s, const OzKeyJob& kj = OzKeyJob());
+template <typename T>
+inline cudaError_t trsm_cols(int w, int ncols, const T* L, long long ldl, T* B, long long ldb, cudaStream_t s) {
+  if (w <= 0 || ncols <= 0) return cudaSuccess;
+  if (w > 256) return trsm_strip<T, false, false, true>(w, ncols, L, ldl, B, ldb, s);
+  trsm_cols_kernel<T><<<(ncols + 8 * TCC - 1) / (8 * TCC), 256, 0, s>>>(w, ncols, L, ldl, B, ldb);
+  count_launches(1);
+  return cudaGetLastError();
+}
+
+template <typename T, bool UPPER, bool TRANS, bool UNIT, int NC>
+inline cudaError_t trsm_strip(int w, int ncols, const T* Tm, long long ldt, T* B, long long ldb,
+                              cudaStream_t s, const OzKeyJob& kj) {
   if (w <= 0 || ncols <= 0) return cudaSuccess;
   // staged triangle columns per block: up to 32, within 200 KB of shared memory
   constexpr size_t kBudget = 200 * 1024;

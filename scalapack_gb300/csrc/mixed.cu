@@ -82,10 +82,54 @@ sgemm_simt_kernel(int m, int n, int k, float alpha, const float* __restrict__ A,
     }
 }
 
+// C += alpha A B for k <= 32 (the products of a 32-column sub-panel): a thread per
+// row of C, 16 columns at a time; the row's k values of A and its 16 of C are
+// loaded at once, coalesced along the rows, B's chunk is broadcast from shared
+// memory. Bound: latency of the one round of loads and C's traffic. m = 8192, n =
+// 224: 6 us (16 with 64 x 64 tiles, whose threads' C accesses were 4 bytes apart
+// in different columns).
+constexpr int K32_N = 16;
+__global__ void __launch_bounds__(256)
+sgemm_k32_kernel(int m, int n, int k, float alpha, const float* __restrict__ A, long long lda,
+                 const float* __restrict__ B, long long ldb, float* C, long long ldc) {
+  __shared__ __align__(16) float Bs[32][K32_N];
+  const int row = blockIdx.x * 256 + threadIdx.x, n0 = blockIdx.y * K32_N, nc = min(K32_N, n - n0);
+  const float* a = A + min(row, m - 1);
+  float av[32], cv[K32_N], acc[K32_N];
+#pragma unroll
+  for (int q = 0; q < 32; ++q) av[q] = a[(long long)min(q, k - 1) * lda];
+  float* c = C + row + (long long)n0 * ldc;
+#pragma unroll
+  for (int j = 0; j < K32_N; ++j) {
+    cv[j] = (row < m && j < nc) ? c[(long long)j * ldc] : 0.f;
+    acc[j] = 0.f;
+  }
+  for (int idx = threadIdx.x; idx < 32 * K32_N; idx += 256) {
+    const int q = idx % 32, j = idx / 32;
+    Bs[q][j] = (q < k && j < nc) ? B[q + (long long)(n0 + j) * ldb] : 0.f;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < 32; ++q)
+    if (q < k) {
+#pragma unroll
+      for (int j = 0; j < K32_N; ++j) acc[j] = fmaf(av[q], Bs[q][j], acc[j]);
+    }
+#pragma unroll
+  for (int j = 0; j < K32_N; ++j)
+    if (row < m && j < nc) c[(long long)j * ldc] = cv[j] + alpha * acc[j];
+}
+
 static cudaError_t sgemm_simt(bool transa, int m, int n, int k, float alpha, const float* A,
                               long long lda, const float* B, long long ldb, float* C,
                               long long ldc, cudaStream_t s) {
   if (m <= 0 || n <= 0 || k <= 0) return cudaSuccess;
+  if (!transa && k <= 32) {
+    sgemm_k32_kernel<<<dim3((m + 255) / 256, (n + K32_N - 1) / K32_N), 256, 0, s>>>(m, n, k, alpha, A, lda, B,
+                                                                                  ldb, C, ldc);
+    count_launches(1);
+    return cudaGetLastError();
+  }
   dim3 grid((m + 63) / 64, (n + 63) / 64);
   if (transa) sgemm_simt_kernel<true><<<grid, 256, 0, s>>>(m, n, k, alpha, A, lda, B, ldb, C, ldc);
   else sgemm_simt_kernel<false><<<grid, 256, 0, s>>>(m, n, k, alpha, A, lda, B, ldb, C, ldc);
@@ -102,17 +146,6 @@ cudaError_t gemm_update<float>(bool transa, int m, int n, int k, float alpha, co
 }
 
 // ------------------------------------------------------------ small kernels
-__global__ void d2s_kernel(const double* __restrict__ A, long long lda, int m, int n, float* F,
-                           long long ldf) {
-  long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  long long total = (long long)m * n;
-  for (; idx < total; idx += (long long)gridDim.x * blockDim.x) {
-    int i = (int)(idx % m);
-    long long j = idx / m;
-    F[i + j * ldf] = (float)A[i + j * lda];
-  }
-}
-
 // out[c] = max_i |X(i,c)| (NaN propagates), one CTA per column.
 __global__ void colmax_abs_kernel(const double* __restrict__ X, long long ldx, int n, double* out) {
   __shared__ double sm[32];
@@ -138,13 +171,33 @@ __global__ void colmax_abs_kernel(const double* __restrict__ X, long long ldx, i
   }
 }
 
-// ||A||_inf = max_i sum_j |A(i,j)|: row sums by threads over rows.
-__global__ void rowsum_abs_kernel(const double* __restrict__ A, long long lda, int n,
-                                  double* rows) {
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+// The FP32 working copy and, in the same pass over A, the absolute row sums of a
+// chunk of columns (part[chunk * n + i]); then the rows' totals in chunk order.
+// One thread per row for all of A took 1.03 ms at n = 8192 beside the copy's 0.29.
+constexpr int kRowChunks = 32;
+__global__ void __launch_bounds__(256)
+copy_rowsum_kernel(const double* __restrict__ A, long long lda, int n, float* F, long long ldf, double* part) {
+  const int i = blockIdx.x * 256 + threadIdx.x, per = (n + kRowChunks - 1) / kRowChunks;
+  const int j0 = blockIdx.y * per, j1 = min(n, j0 + per);
   if (i >= n) return;
   double s = 0.0;
-  for (int j = 0; j < n; ++j) s += fabs(A[i + (long long)j * lda]);
+  for (int j = j0; j < j1; j += 8) {
+    double v[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) v[q] = j + q < j1 ? A[i + (long long)(j + q) * lda] : 0.0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      s += fabs(v[q]);
+      if (j + q < j1) F[i + (long long)(j + q) * ldf] = (float)v[q];
+    }
+  }
+  part[(long long)blockIdx.y * n + i] = s;
+}
+__global__ void rowsum_total_kernel(const double* __restrict__ part, int n, double* rows) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  double s = 0.0;
+  for (int c = 0; c < kRowChunks; ++c) s += part[(long long)c * n + i];
   rows[i] = s;
 }
 
@@ -278,7 +331,7 @@ cudaError_t sgetrf_mixed_device(int n, float* F, long long ldf, int* dipiv, int 
     phase_begin(kPhMixedPanel, s);
     SL_TRY(laswp_planned<float>(F, ldf, j, j + jb, dipiv, ws.swap_plan, 0, j, j + jb, n, s));
     if (jn < n)
-      SL_TRY((trsm_strip<float, false, false, true>(jb, n - jn, Fp(j, j), ldf, Fp(j, jn), ldf, s)));
+      SL_TRY(trsm_cols<float>(jb, n - jn, Fp(j, j), ldf, Fp(j, jn), ldf, s));
     phase_end(kPhMixedPanel, s, 0.0, 0.0);
     if (jn < n && jn < m) {
       const int mr = m - jn, nr = n - jn;
@@ -321,21 +374,24 @@ cudaError_t sgetrf_mixed_device(int n, float* F, long long ldf, int* dipiv, int 
 // solved just before b (b-1 for L, b+1 for U; zero for the first one), stored
 // the same way at Mp: the chained solve then finishes block b with one 64x64
 // product once x_p arrives, x_b = inv(T_bb) v_b - M_b x_p.
+// Both triangles in one launch (blockIdx.y); all 256 threads form M_b.
 template <bool LOWER>
-__global__ void __launch_bounds__(64)
-diag_inv_kernel(int n, const float* __restrict__ F, long long ldf, float* Dinv, float* Mp) {
+__device__ __forceinline__ void diag_inv_block(int n, const float* __restrict__ F, long long ldf, float* Dinv,
+                                               float* Mp, float (*T)[64], double (*X)[64]) {
+  // T is read as broadcasts: no padding needed; X[i][t]: column t of the inverse
+  // (thread t's own column)
   constexpr int KB = 64;
-  __shared__ float T[KB][KB];   // read as broadcasts: no padding needed
-  __shared__ double X[KB][KB];  // X[i][t]: column t of the inverse (thread t's own column)
-  const int b = blockIdx.x, t = threadIdx.x;
+  const int b = blockIdx.x, t = threadIdx.x & (KB - 1), g = threadIdx.x >> 6;
   const int r0 = b * KB, rb = min(KB, n - r0);
-  for (int r = 0; r < KB; ++r) {
+  for (int r = g; r < KB; r += 4) {
     const int i = t;
     const bool in = r < rb && i < rb && (LOWER ? i < r : i >= r);
     T[r][i] = in ? F[(r0 + r) + (long long)(r0 + i) * ldf] : (r == i ? 1.0f : 0.0f);
   }
   __syncthreads();
-  if (LOWER) {
+  if (g > 0) {
+    // (the substitution is a chain per column: 64 threads)
+  } else if (LOWER) {
     for (int i = 0; i < KB; ++i) {
       double acc = (i == t) ? 1.0 : 0.0;
       for (int j = t; j < i; ++j) acc -= (double)T[i][j] * X[j][t];
@@ -350,30 +406,39 @@ diag_inv_kernel(int n, const float* __restrict__ F, long long ldf, float* Dinv, 
   }
   __syncthreads();
   float* D = Dinv + (size_t)b * KB * KB;
-  for (int r = 0; r < KB; ++r) D[r * KB + t] = (float)X[r][t];
+  for (int r = g; r < KB; r += 4) D[r * KB + t] = (float)X[r][t];
   // the predecessor block into T (its triangle is no longer needed)
   const int nblk = (n + KB - 1) / KB;
   const int p = LOWER ? b - 1 : b + 1;
   const bool has_p = p >= 0 && p < nblk;
   const int wp = has_p ? min(KB, n - p * KB) : 0;
-  for (int r = 0; r < KB; ++r)
+  for (int r = g; r < KB; r += 4)
     T[r][t] = (r < rb && t < wp) ? F[(r0 + r) + (long long)(p * KB + t) * ldf] : 0.0f;
   __syncthreads();
   float* M = Mp + (size_t)b * KB * KB;
-  for (int r = 0; r < KB; ++r) {
+  for (int r = g; r < KB; r += 4) {
     double acc = 0.0;
     for (int i = 0; i < KB; ++i) acc = fma(X[r][i], (double)T[i][t], acc);
     M[r * KB + t] = (float)acc;
   }
 }
 
+__global__ void __launch_bounds__(256)
+diag_inv_kernel(int n, const float* __restrict__ F, long long ldf, float* dinv, size_t half) {
+  __shared__ float T[64][64];
+  extern __shared__ double inv_x[];
+  double(*X)[64] = reinterpret_cast<double(*)[64]>(inv_x);
+  if (blockIdx.y == 0) diag_inv_block<true>(n, F, ldf, dinv, dinv + 2 * half, T, X);
+  else diag_inv_block<false>(n, F, ldf, dinv + half, dinv + 3 * half, T, X);
+}
+
 // dinv: [inv L blocks | inv U blocks | M of L | M of U], each ceil(n/64) x 4096.
 cudaError_t diag_inverses(int n, const float* F, long long ldf, float* dinv, cudaStream_t s) {
   const int nblk = (n + 63) / 64;
   const size_t half = (size_t)nblk * 64 * 64;
-  diag_inv_kernel<true><<<nblk, 64, 0, s>>>(n, F, ldf, dinv, dinv + 2 * half);
-  diag_inv_kernel<false><<<nblk, 64, 0, s>>>(n, F, ldf, dinv + half, dinv + 3 * half);
-  count_launches(2);
+  constexpr int smem = 64 * 64 * (int)sizeof(double);
+  diag_inv_kernel<<<dim3(nblk, 2), 256, smem, s>>>(n, F, ldf, dinv, half);
+  count_launches(1);
   return cudaGetLastError();
 }
 
@@ -581,14 +646,15 @@ cudaError_t dgesv_ir_device(int n, int nrhs, double* dA, long long lda, const do
   cudaEventCreate(&e2);
   cudaEventRecord(e0, s);
   // ||A||_inf of the FP64 matrix (for the scaled residual)
-  rowsum_abs_kernel<<<blocks_for(n), 256, 0, s>>>(dA, lda, n, mw.w);
+  // ||A||_inf with the FP32 working copy (the Krylov basis is idle: partial sums)
+  static_assert(kRowChunks <= 64, "columns of the Krylov basis");
+  copy_rowsum_kernel<<<dim3((n + 255) / 256, kRowChunks), 256, 0, s>>>(dA, lda, n, mw.F, mw.ldf, mw.V);
+  rowsum_total_kernel<<<blocks_for(n), 256, 0, s>>>(mw.V, n, mw.w);
   colmax_abs_kernel<<<1, 1024, 0, s>>>(mw.w, n, n, mw.colmax);
-  count_launches(2);
+  count_launches(3);
   double anorm = 0.0;
   SL_TRY(cudaMemcpyAsync(&anorm, mw.colmax, sizeof(double), cudaMemcpyDeviceToHost, s));
-  // FP32 working copy and low-precision factorization
-  d2s_kernel<<<4 * num_sms(), 256, 0, s>>>(dA, lda, n, n, mw.F, mw.ldf);
-  count_launches(1);
+  // low-precision factorization
   SL_TRY(sgetrf_mixed_device(n, mw.F, mw.ldf, dipiv, opt.nb, opt.fmt, ws, mw, s));
   SL_TRY(perm_compose(dipiv, n, mw.perm, s));
   if (mw.dinv) SL_TRY(diag_inverses(n, mw.F, mw.ldf, mw.dinv, s));

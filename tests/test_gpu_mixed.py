@@ -201,3 +201,26 @@ def test_cost_rule_falls_back_early_and_stays_correct(sl, orc, gpu_required):
     assert it == -3
     assert st["gmres_inner"] < 100, st
     assert orc.sresid(A0, B0, X) < 16.0
+
+
+@pytest.mark.parametrize("n,nb", [(33, 256), (257, 256), (300, 100), (545, 200), (801, 37), (1030, 300)])
+def test_ir_panel_and_solve_edges(sl, gpu_required, n, nb):
+    """Partial blocks of the mixed factorization's U12 solve (whole 32-row groups or
+    not, more than 256 rows), its 32-column products and interchange plans: the
+    refined solution meets the tester's bound without the FP64 fallback."""
+    import torch
+
+    rng = np.random.default_rng(n + nb)
+    A = rng.uniform(-0.5, 0.5, (n, n))
+    A[rng.permutation(n), np.arange(n)] += 0.5 * np.sqrt(n)
+    B = rng.uniform(-0.5, 0.5, (n, 3))
+    dA, dB = torch.from_numpy(A.T.copy()).cuda(), torch.from_numpy(B.T.copy()).cuda()
+    dX = torch.zeros_like(dB)
+    ip = torch.zeros(n, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    info, it, st = sl.dgesv_ir_dev(n, 3, dA.data_ptr(), n, ip.data_ptr(), dB.data_ptr(), n, dX.data_ptr(), n,
+                                   fmt="bf16x3", nb=nb)
+    assert info == 0 and it >= 1 and not st["fell_back"]
+    X = dX.T.cpu().numpy()
+    res = np.abs(B - A @ X).max(axis=0) / (np.abs(A).sum(axis=1).max() * np.abs(X).max(axis=0) * n * 2.0**-53)
+    assert (res < 16.0).all()
