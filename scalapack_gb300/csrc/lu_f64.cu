@@ -228,70 +228,74 @@ unit_lower_inv64_kernel(int jb, const double* __restrict__ L, long long ldl, dou
 // U12 solve is then one product); larger blocks use 64-row inverses.
 constexpr int kFullInvMax = 256;
 
-// X = inv(L) - I for a unit-lower jb x jb L (jb <= 256), one warp per column
-// c: x = e_c, then for q = c, c+1, ... x_q is final and every row i > q loses
-// L(i,q) x_q -- forward substitution in the order of a strip solve, with x_q
-// passed by a shuffle from the lane that owns row q (lane l owns rows l, l+32,
-// ..., in registers). Column c costs about (jb-c)^2/2 FMAs on the FP64 pipe,
-// so warp pairs take columns p and jb-1-p (equal work per pair) and a CTA of
-// kInvColsWarps warps holds kInvColsWarps/2 pairs: the work spreads evenly
-// over jb/kInvColsWarps CTAs. L is read from global memory (L2) two columns
-// ahead of its use, no shared memory and no block barrier. With a plan to
-// make (plan != null), one extra block computes the panel's interchange plan
+// X = inv(L) - I for a unit-lower jb x jb L (jb <= 256): forward substitution of
+// x = e_c per column c, in the order of a strip solve. A CTA takes the columns p
+// and jb-1-p (a long one and a short one); its warp b owns rows 32b .. 32b+31, a
+// lane per row. Block step s: warp s solves its 32 rows (x_q passed by a shuffle)
+// and leaves them in shared memory, then the warps below subtract their 32 columns,
+// L's next columns on their way meanwhile. Bound: the chain of 256 dependent FP64
+// instructions and the FP64 unit's 20 cycles for each of a column's 1152: one warp
+// per column (64 cycles for each of them) took 71 us, this 30. With a plan to make
+// (plan != null), one extra block computes the panel's interchange plan
 // (laswp_plan_block) in the same launch: both only read the finished panel.
-constexpr int kInvColsWarps = 4;
-__host__ __device__ inline int inv_cols_blocks(int jb) {
-  const int pairs = (jb + 1) / 2;
-  return (pairs + kInvColsWarps / 2 - 1) / (kInvColsWarps / 2);
-}
-__global__ void __launch_bounds__(32 * kInvColsWarps)
+__host__ __device__ inline int inv_cols_blocks(int jb) { return (jb + 1) / 2; }
+__global__ void __launch_bounds__(256)
 unit_lower_inv_cols_kernel(int jb, const double* __restrict__ L, long long ldl, double* X,
                            int ldx, int k1, int k2, const int* __restrict__ ipiv, int* plan) {
   if (plan != nullptr && (int)blockIdx.x == inv_cols_blocks(jb)) {
     laswp_plan_block(k1, k2, ipiv, plan);
     return;
   }
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int p = (int)blockIdx.x * (kInvColsWarps / 2) + (warp >> 1);
-  const int c = (warp & 1) ? jb - 1 - p : p;
-  // the middle column of an odd jb has no partner; pairs past the end none
-  if (p >= (jb + 1) / 2 || ((warp & 1) && c == p)) return;
-  double xr[8];
+  __shared__ double xs[2][2][32];  // [step parity][column][row]
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, row = 32 * warp + lane;
+  const int c0 = blockIdx.x, c1 = jb - 1 - c0;  // c0 <= c1; the same column when jb is odd
+  const double* lrow = L + min(row, jb - 1);
+  double x0 = row == c0 ? 1.0 : 0.0, x1 = row == c1 ? 1.0 : 0.0;
+  const int nsteps = (jb + 31) / 32, sb = c0 / 32;
+  // L(row, 32 s + q); outside the strict triangle's blocks the values are not used
+  double lv[32], ln[32];
+  auto load = [&](int s, double* v) {
+    if (s <= warp && s < nsteps) {
 #pragma unroll
-  for (int t = 0; t < 8; ++t) xr[t] = (lane + 32 * t == c) ? 1.0 : 0.0;
-  // L(lane + 32 t, q) for t >= q / 32, rows > q and < jb (0 elsewhere)
-  auto load_col = [&](int q, int tq, double* v) {
-#pragma unroll
-    for (int t = 0; t < 8; ++t) {
-      const int i = lane + 32 * t;
-      v[t] = (t >= tq && q < jb && i > q && i < jb) ? __ldg(L + i + (long long)q * ldl) : 0.0;
+      for (int q = 0; q < 32; ++q) v[q] = lrow[(long long)min(32 * s + q, jb - 1) * ldl];
     }
   };
-  double v0[8], v1[8];
-  load_col(c, c >> 5, v0);
-  load_col(c + 1, (c + 1) >> 5, v1);
+  load(sb, lv);
+  for (int s = sb; s < nsteps; ++s) {
+    load(s + 1, ln);
+    // column c begins at its own row: earlier columns of L do not enter
+    const int f0 = c0 - 32 * s, f1 = c1 - 32 * s;
+    const bool two = f1 <= 31;
+    if (warp == s) {
 #pragma unroll
-  for (int tq = 0; tq < 8; ++tq) {
-    if (32 * tq + 31 < c || 32 * tq >= jb) continue;
-    for (int l = (c > 32 * tq ? c - 32 * tq : 0); l < 32; ++l) {
-      const int q = 32 * tq + l;
-      if (q >= jb) break;
-      double v2[8];
-      load_col(q + 2, (q + 2) >> 5, v2);  // two columns ahead
-      const double xq = __shfl_sync(0xffffffffu, xr[tq], l);
+      for (int q = 0; q < 32; ++q) {
+        const double u0 = __shfl_sync(0xffffffffu, x0, q);
+        if (lane > q && q >= f0) x0 = fma(-lv[q], u0, x0);
+        if (two) {
+          const double u1 = __shfl_sync(0xffffffffu, x1, q);
+          if (lane > q && q >= f1) x1 = fma(-lv[q], u1, x1);
+        }
+      }
+      xs[s & 1][0][lane] = x0;
+      xs[s & 1][1][lane] = x1;
+    }
+    __syncthreads();
+    if (warp > s && warp < nsteps) {
 #pragma unroll
-      for (int t = tq; t < 8; ++t) xr[t] = fma(-v0[t], xq, xr[t]);
+      for (int q = 0; q < 32; ++q)
+        if (q >= f0) x0 = fma(-lv[q], xs[s & 1][0][q], x0);
+      if (two) {
 #pragma unroll
-      for (int t = 0; t < 8; ++t) {
-        v0[t] = v1[t];
-        v1[t] = v2[t];
+        for (int q = 0; q < 32; ++q)
+          if (q >= f1) x1 = fma(-lv[q], xs[s & 1][1][q], x1);
       }
     }
-  }
 #pragma unroll
-  for (int t = 0; t < 8; ++t) {
-    const int i = lane + 32 * t;
-    if (i < jb) X[i + (long long)c * ldx] = (i > c) ? xr[t] : 0.0;
+    for (int q = 0; q < 32; ++q) lv[q] = ln[q];
+  }
+  if (row < jb) {
+    X[row + (long long)c0 * ldx] = row > c0 ? x0 : 0.0;
+    X[row + (long long)c1 * ldx] = row > c1 ? x1 : 0.0;
   }
 }
 
@@ -407,7 +411,7 @@ static cudaError_t factor_panel(int m, double* dA, long long ldda, int* dipiv, i
     // plan in the same launch
     if (want_plan && npiv <= 0) SL_TRY(cudaMemsetAsync(ws.swap_plan, 0, sizeof(int), s));
     const bool fused = want_plan && npiv > 0;
-    unit_lower_inv_cols_kernel<<<inv_cols_blocks(jb) + (fused ? 1 : 0), 32 * kInvColsWarps, 0, s>>>(
+    unit_lower_inv_cols_kernel<<<inv_cols_blocks(jb) + (fused ? 1 : 0), 256, 0, s>>>(
         jb, Ap(j, j), ldda, ws.dinv64, jb, j, j + npiv, dipiv, fused ? ws.swap_plan : nullptr);
     count_launches(1);
     SL_TRY(cudaGetLastError());

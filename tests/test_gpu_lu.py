@@ -513,3 +513,25 @@ def test_inverse_by_triangles(sl, gpu_required, n):
     V = dA[:, :n].T.cpu().numpy()
     res = np.abs(A @ V - np.eye(n)).sum(axis=1).max()
     assert res / (np.abs(A).sum(axis=1).max() * np.abs(V).sum(axis=1).max() * n * 2.0**-53) < 16.0  # the tester's bound
+
+
+@pytest.mark.parametrize("m", [1, 2, 31, 32, 33, 64, 65, 127, 129, 224, 255, 256])
+def test_u12_through_inverse_edges(sl, gpu_required, m):
+    """One panel of m columns and a block row of 200: U12 = inv(L11) A12 with the
+    inverse's last block partial, its middle column alone (odd m) or everything one
+    block. P A = L U to the tester's bound."""
+    import torch
+
+    n = m + 200
+    rng = np.random.default_rng(m)
+    A = np.asfortranarray(rng.uniform(-0.5, 0.5, (m, n)))
+    dA = torch.from_numpy(A.T.copy()).cuda()
+    ip = torch.zeros(m, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    assert sl.dgetrf_dev(m, n, dA.data_ptr(), m, ip.data_ptr(), 256) == 0
+    F, piv = dA.T.cpu().numpy(), ip.cpu().numpy() - 1
+    PA = A.copy()
+    for k, p in enumerate(piv):
+        PA[[k, p]] = PA[[p, k]]
+    low, up = np.tril(F[:, :m], -1) + np.eye(m), np.triu(F)
+    assert np.abs(PA - low @ up).max() < 16.0 * n * 2.0**-53 * np.abs(A).sum(axis=1).max()
