@@ -255,6 +255,17 @@ __device__ __noinline__ void oz_fp64_tiles(unsigned char* smem, int m, int n, in
   }
 }
 
+// An integer |x| <= 2^24 held in FP32, plus 5 kMagicBits modulo 2^32: the addition
+// of 1.5 2^23 leaves an integer of up to 22 bits in the low bits, so x is taken in
+// two parts, x = 4 h + l. Four FP32 operations at 128 lanes a cycle, where the
+// conversion instruction takes 16.
+constexpr float kMagic = 12582912.0f;
+constexpr unsigned kMagicBits = 0x4B400000u;
+__device__ __forceinline__ unsigned oz_int24(float x) {
+  const float h = fmaf(x, 0.25f, kMagic);
+  const float l = fmaf(h - kMagic, -4.0f, x) + kMagic;
+  return 4u * __float_as_uint(h) + __float_as_uint(l);
+}
 // Exponent of a power of two (-1023 for zero, beyond any sum's range for NaN).
 __device__ __forceinline__ int oz_exp_field(double x) {
   const int f = (__double2hiint(x) >> 20) & 0x7ff;
@@ -448,8 +459,8 @@ ozgemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
       }
       asm volatile("tcgen05.fence::after_thread_sync;");
       // two accumulators at a time keep the register count down; P_2 <= 2^22
-      // converts by an addition (1.5 * 2^23, whose bits are taken off again),
-      // the others at 16 lanes a cycle
+      // converts by an addition (1.5 * 2^23, whose bits are taken off again), the
+      // next ones by two or by the conversion instruction, turn about
       long long I[EC];
       uint32_t r[2][16];
       auto get2 = [&](int a, bool both) {
@@ -462,16 +473,16 @@ ozgemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
       get2(0, true);
 #pragma unroll
       for (int j = 0; j < EC; ++j) {
-        const unsigned p2 = __float_as_uint(__uint_as_float(r[0][j]) + 12582912.0f) - 0x4B400000u;
-        const unsigned p3 = (unsigned)__float2int_rn(__uint_as_float(r[1][j]));
-        const unsigned hi = (p2 << 8) + p3;  // (modulo 2^32, as the sum's high half)
+        const unsigned p2 = __float_as_uint(__uint_as_float(r[0][j]) + kMagic);
+        const unsigned p3 = oz_int24(__uint_as_float(r[1][j]));
+        const unsigned hi = (p2 << 8) + p3 - 261u * kMagicBits;  // (modulo 2^32, as the sum's high half)
         I[j] = (long long)((unsigned long long)hi << 32);
       }
       get2(2, true);
 #pragma unroll
       for (int j = 0; j < EC; ++j) {
         const long long p4 = __float2int_rn(__uint_as_float(r[0][j]));
-        const long long p5 = __float2int_rn(__uint_as_float(r[1][j]));
+        const long long p5 = (int)(oz_int24(__uint_as_float(r[1][j])) - 5u * kMagicBits);
         I[j] += (p4 << 24) + (p5 << 16);
       }
       get2(4, false);
