@@ -283,6 +283,71 @@ __device__ __forceinline__ double oz_ldexp(long long v, int E) {
   return u == 0 ? 0.0 : __longlong_as_double((long long)(bits | ((unsigned long long)v & (1ULL << 63))));
 }
 
+// An epilogue warp's part of the accumulators as integers I = sum_d P_d 2^(56-8d),
+// trow its TMEM address; release() once everything is in registers.
+template <class F>
+__device__ __forceinline__ void oz_read_sums(uint32_t trow, long long* I, F release) {
+  // two accumulators at a time keep the register count down; P_2 <= 2^22
+  // converts by an addition (1.5 * 2^23, whose bits are taken off again), the
+  // next ones by two or by the conversion instruction, turn about
+  uint32_t r[2][16];
+  auto get2 = [&](int a, bool both) {
+    tmem_ld16_nowait(trow + (uint32_t)(a * OBN), r[0]);
+    if (both) tmem_ld16_nowait(trow + (uint32_t)((a + 1) * OBN), r[1]);
+    tmem_ld_wait();
+    touch16(r[0]);
+    if (both) touch16(r[1]);
+  };
+  get2(0, true);
+#pragma unroll
+  for (int j = 0; j < OZ_EC; ++j) {
+    const unsigned p2 = __float_as_uint(__uint_as_float(r[0][j]) + kMagic);
+    const unsigned p3 = oz_int24(__uint_as_float(r[1][j]));
+    const unsigned hi = (p2 << 8) + p3 - 261u * kMagicBits;  // (modulo 2^32, as the sum's high half)
+    I[j] = (long long)((unsigned long long)hi << 32);
+  }
+  get2(2, true);
+#pragma unroll
+  for (int j = 0; j < OZ_EC; ++j) {
+    const long long p4 = __float2int_rn(__uint_as_float(r[0][j]));
+    const long long p5 = (int)(oz_int24(__uint_as_float(r[1][j])) - 5u * kMagicBits);
+    I[j] += (p4 << 24) + (p5 << 16);
+  }
+  get2(4, false);
+#pragma unroll
+  for (int j = 0; j < OZ_EC; ++j) I[j] += (long long)__float2int_rn(__uint_as_float(r[0][j])) << 8;
+  get2(5, true);
+  release();
+#pragma unroll
+  for (int j = 0; j < OZ_EC; ++j)
+    I[j] += __float2int_rn(fmaf(__uint_as_float(r[1][j]), 0.00390625f, __uint_as_float(r[0][j])));
+}
+// C(row, 16 columns) = cv + alpha 2^(e_i + f_j - 54) I, rsc and sc the scales.
+__device__ __forceinline__ void oz_update_c(const long long* I, const double* cv, double* crow,
+                                            long long ldc, int ncol, double alpha, double rsc,
+                                            const double* sc) {
+  // one FP64 addition per element, unless some element of the warp needs
+  // the general form: general alpha, scales near the range's ends, zero and
+  // non-finite ones (a vote, so that the compiler does not compute both)
+  const int er = oz_exp_field(rsc);
+  const bool unit = alpha == 1.0 || alpha == -1.0, neg = alpha < 0.0;
+  bool plain = unit;
+#pragma unroll
+  for (int j = 0; j < OZ_EC; ++j) {
+    plain = plain && (j >= ncol || (unsigned)(er + oz_exp_field(sc[j]) + 1022) <= 1982u);
+  }
+  if (__all_sync(0xffffffffu, plain)) {
+#pragma unroll
+    for (int j = 0; j < OZ_EC; ++j)
+      if (j < ncol)
+        crow[(long long)j * ldc] = cv[j] + oz_ldexp(neg ? -I[j] : I[j], er + oz_exp_field(sc[j]));
+  } else {
+#pragma unroll
+    for (int j = 0; j < OZ_EC; ++j)
+      if (j < ncol) crow[(long long)j * ldc] = fma(alpha * rsc * sc[j], __ll2double_rn(I[j]), cv[j]);
+  }
+}
+
 // CTA b takes tiles b tpc .. b tpc + tpc - 1 of the raster (a few, so that
 // SMs turn over and the panel's kernels on the high-priority stream find
 // room between them). The TMA thread runs
@@ -438,7 +503,6 @@ ozgemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
     constexpr int EC = OZ_EC;
     const int quad = warp & 3, cg = (warp - 2) >> 2;
     const uint32_t trow = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(cg * EC);
-    const bool unit = alpha == 1.0 || alpha == -1.0, neg = alpha < 0.0;
     for (int it = 0; it < my_tiles; ++it) {
       int m0, n0;
       oz_tile(first_tile + it, tiles_m, tiles_n, m0, n0);
@@ -458,65 +522,17 @@ ozgemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;");
-      // two accumulators at a time keep the register count down; P_2 <= 2^22
-      // converts by an addition (1.5 * 2^23, whose bits are taken off again), the
-      // next ones by two or by the conversion instruction, turn about
       long long I[EC];
-      uint32_t r[2][16];
-      auto get2 = [&](int a, bool both) {
-        tmem_ld16_nowait(trow + (uint32_t)(a * OBN), r[0]);
-        if (both) tmem_ld16_nowait(trow + (uint32_t)((a + 1) * OBN), r[1]);
-        tmem_ld_wait();
-        touch16(r[0]);
-        if (both) touch16(r[1]);
-      };
-      get2(0, true);
-#pragma unroll
-      for (int j = 0; j < EC; ++j) {
-        const unsigned p2 = __float_as_uint(__uint_as_float(r[0][j]) + kMagic);
-        const unsigned p3 = oz_int24(__uint_as_float(r[1][j]));
-        const unsigned hi = (p2 << 8) + p3 - 261u * kMagicBits;  // (modulo 2^32, as the sum's high half)
-        I[j] = (long long)((unsigned long long)hi << 32);
-      }
-      get2(2, true);
-#pragma unroll
-      for (int j = 0; j < EC; ++j) {
-        const long long p4 = __float2int_rn(__uint_as_float(r[0][j]));
-        const long long p5 = (int)(oz_int24(__uint_as_float(r[1][j])) - 5u * kMagicBits);
-        I[j] += (p4 << 24) + (p5 << 16);
-      }
-      get2(4, false);
-#pragma unroll
-      for (int j = 0; j < EC; ++j) I[j] += (long long)__float2int_rn(__uint_as_float(r[0][j])) << 8;
-      get2(5, true);
-      // the accumulators are in registers: the next tile's products may start
-      asm volatile("tcgen05.fence::before_thread_sync;");
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bars->tempty);
-#pragma unroll
-      for (int j = 0; j < EC; ++j)
-        I[j] += __float2int_rn(fmaf(__uint_as_float(r[1][j]), 0.00390625f, __uint_as_float(r[0][j])));
-      // one FP64 addition per element, unless some element of the warp needs
-      // the general form: general alpha, scales near the range's ends, zero and
-      // non-finite ones (a vote, so that the compiler does not compute both)
-      const int er = oz_exp_field(rsc);
+      oz_read_sums(trow, I, [&]() {
+        // the accumulators are in registers: the next tile's products may start
+        asm volatile("tcgen05.fence::before_thread_sync;");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars->tempty);
+      });
       double sc[EC];
-      bool plain = unit;
 #pragma unroll
-      for (int j = 0; j < EC; ++j) {
-        sc[j] = __ldg(cs + min(nb0 + j, n - 1));
-        plain = plain && (j >= ncol || (unsigned)(er + oz_exp_field(sc[j]) + 1022) <= 1982u);
-      }
-      if (__all_sync(0xffffffffu, plain)) {
-#pragma unroll
-        for (int j = 0; j < EC; ++j)
-          if (j < ncol)
-            crow[(long long)j * ldc] = cv[j] + oz_ldexp(neg ? -I[j] : I[j], er + oz_exp_field(sc[j]));
-      } else {
-#pragma unroll
-        for (int j = 0; j < EC; ++j)
-          if (j < ncol) crow[(long long)j * ldc] = fma(alpha * rsc * sc[j], __ll2double_rn(I[j]), cv[j]);
-      }
+      for (int j = 0; j < EC; ++j) sc[j] = __ldg(cs + min(nb0 + j, n - 1));
+      oz_update_c(I, cv, crow, ldc, ncol, alpha, rsc, sc);
       if (s_fail) break;
     }
   }
@@ -847,6 +863,204 @@ oz_split_kernel(const double* __restrict__ A, long long lda, int m, const double
   }
 }
 
+// One tile of C (128 x 64) per CTA for K <= 64, balancing side A, keys already
+// published: the CTA slices its own 128 x KP of A and KP x 64 of B into shared
+// memory (where the tensor maps' swizzle puts them) instead of reading slices that
+// oz_split_kernel left in memory. The same scales, digits and products as there;
+// a row of A is sliced once per column tile, so this is for narrow C. A tile with a
+// row outside the error budget (or a scale out of range) is computed in FP64
+// arithmetic by itself.
+//
+// For the products inside a panel, one per 32 columns and on its critical path:
+// what they take is latency (two launches, two trips through memory). Every LU
+// factor is bit for bit the one of oz_split_kernel and ozgemm_kernel. Measured: a
+// step of an LU of N = 4096 (128 of them) 6 us shorter.
+template <int KP>
+__global__ void __launch_bounds__(OZ_THREADS, 1)
+oz_tile_kernel(const double* A, long long lda, int m, const double* B, long long ldb, int n, int kb,
+               double alpha, double* C, long long ldc, int* status, unsigned long long* kinfo,
+               unsigned long long epoch) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  unsigned char* sA = base;                        // 7 x 16 KB: rows of 128 bytes (64 k)
+  unsigned char* sB = base + OZ_S * A_SLICE_BYTES; // 7 x 8 KB
+  constexpr int VA = KP / 4, VB = KP / 8;          // values of A and of B per worker thread
+  __shared__ uint64_t s_full;
+  __shared__ uint32_t s_tmem;
+  __shared__ int s_d[KP], s_h[KP];
+  __shared__ int s_E[4][OBM], s_F[4][OBM];
+  __shared__ double s_rs[OBM], s_cs[OBN];
+  if (*(volatile int*)status != 0) return;  // an earlier wait gave up
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int tiles_m = (m + OBM - 1) / OBM, tiles_n = (n + OBN - 1) / OBN;
+  int m0, n0;
+  oz_tile(blockIdx.x, tiles_m, tiles_n, m0, n0);
+  // worker threads: 16 warps; thread t has row t % 128 and k range t / 128 of A,
+  // column t / 8 and k range t % 8 of B
+  const int t = (int)threadIdx.x - 64;
+  const int ar = t & (OBM - 1), ak = (t >> 7) * VA, bc = t >> 3, bk = (t & 7) * VB;
+  double av[VA], bv[VB];
+  if (warp >= 2) {
+    const double* arow = A + min(m0 + ar, m - 1);
+    const double* bcol = B + (long long)min(n0 + bc, n - 1) * ldb;
+#pragma unroll
+    for (int q = 0; q < VA; ++q) av[q] = arow[(long long)min(ak + q, kb - 1) * lda];
+#pragma unroll
+    for (int q = 0; q < VB; ++q) bv[q] = bcol[min(bk + q, kb - 1)];
+    if (t < KP) {
+      int h = OZ_NOEXP, c = OZ_NOEXP;
+      if (t < kb) {
+        h = oz_word_exp(kinfo[OZ_KI_H + t], epoch);
+        c = oz_word_exp(kinfo[OZ_KI_C + t], epoch);
+        if (h == OZ_NOEXP || c == OZ_NOEXP) h = c = OZ_NOEXP;  // k contributes nothing
+      }
+      s_h[t] = h;
+      s_d[t] = c;
+    }
+  } else if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)),
+                 "r"(OZ_TMEM_COLS));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  } else if (lane == 0) {
+    mbar_init(&s_full, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;");
+  const uint32_t tmem = s_tmem;
+
+  // scales: e_i over the row's four k ranges, f_j over the column's eight
+  int f = OZ_NOEXP, G = OZ_NOEXP;
+  if (warp >= 2) {
+    int em = OZ_NOEXP, fm = OZ_NOEXP;
+    bool bad = false;
+#pragma unroll
+    for (int q = 0; q < VA; ++q) {
+      if (m0 + ar >= m || ak + q >= kb) av[q] = 0.0;
+      const unsigned long long mag = (unsigned long long)__double_as_longlong(av[q]) & kMagMask;
+      const int d = s_d[ak + q];
+      if (mag >= kInfBits) {
+        bad = true;
+      } else if (mag != 0ULL && d != OZ_NOEXP) {
+        const int ex = oz_scale_exp(mag);
+        em = max(em, ex - d);
+        fm = max(fm, ex + s_h[ak + q]);
+      }
+    }
+    s_E[t >> 7][ar] = bad ? INT_MAX : em;
+    s_F[t >> 7][ar] = fm;
+#pragma unroll
+    for (int q = 0; q < VB; ++q) {
+      if (n0 + bc >= n || bk + q >= kb) bv[q] = 0.0;
+      const unsigned long long mag = (unsigned long long)__double_as_longlong(bv[q]) & kMagMask;
+      const int d = s_d[bk + q];
+      if (mag >= kInfBits) f = INT_MAX;
+      else if (mag != 0ULL && d != OZ_NOEXP) f = max(f, oz_scale_exp(mag) + d);
+    }
+#pragma unroll
+    for (int off = 4; off > 0; off >>= 1) f = max(f, __shfl_xor_sync(0xffffffffu, f, off));
+#pragma unroll
+    for (int k = lane; k < KP; k += 32)
+      if (s_d[k] != OZ_NOEXP) G = max(G, s_d[k] + s_h[k]);
+    G = oz_warp_imax(G);
+  }
+  __syncthreads();
+  int e = OZ_NOEXP;
+  bool out = false;
+  if (warp >= 2) {
+    e = max(max(s_E[0][ar], s_E[1][ar]), max(s_E[2][ar], s_E[3][ar]));
+    const int F = max(max(s_F[0][ar], s_F[1][ar]), max(s_F[2][ar], s_F[3][ar]));
+    // (as in oz_split_kernel: row i's bound 2^(e_i + G) against its largest term)
+    if (e != INT_MAX && e != OZ_NOEXP) out = !oz_scale_in_range(e) || e + G - F > OZ_BUDGET;
+    if (f != INT_MAX && f != OZ_NOEXP) out = out || !oz_scale_in_range(f);
+    if (ak == 0) s_rs[ar] = oz_scale_value(e, e == INT_MAX);
+    if (bk == 0) s_cs[bc] = oz_scale_value(f, f == INT_MAX);
+  }
+  if (__syncthreads_or(out)) {
+    if (threadIdx.x == 0 && atomicMax(kinfo + OZ_KI_FLAG, epoch) < epoch) atomicAdd(&g_oz_fp64_routes, 1ULL);
+    oz_fp64_tiles(base, m, n, kb, A, lda, B, ldb, alpha, C, ldc, blockIdx.x, 1, tiles_m, tiles_n, 0);
+  } else {
+    if (warp >= 2) {
+      // slices; 8 values are one 16-byte piece of a row, piece p of row r at p ^ (r % 8)
+#pragma unroll
+      for (int q0 = 0; q0 < VA; q0 += 8) {
+        unsigned long long W[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const int d = s_d[ak + q0 + q];
+          W[q] = (e == INT_MAX || e == OZ_NOEXP || d == OZ_NOEXP)
+                     ? kDigitBias
+                     : oz_digits((unsigned long long)__double_as_longlong(av[q0 + q]), e + d);
+        }
+        unsigned char* dst = sA + ar * 128 + ((((ak + q0) >> 3) ^ (ar & 7)) << 4);
+#pragma unroll
+        for (int sl = 0; sl < OZ_S; ++sl)
+          *reinterpret_cast<uint4*>(dst + sl * A_SLICE_BYTES) =
+              make_uint4(oz_slice2(W[0], W[1], sl), oz_slice2(W[2], W[3], sl), oz_slice2(W[4], W[5], sl),
+                         oz_slice2(W[6], W[7], sl));
+      }
+      unsigned long long W[VB];
+#pragma unroll
+      for (int q = 0; q < VB; ++q) {
+        const int d = s_d[bk + q];
+        W[q] = (f == INT_MAX || f == OZ_NOEXP || d == OZ_NOEXP)
+                   ? kDigitBias
+                   : oz_digits((unsigned long long)__double_as_longlong(bv[q]), f - d);
+      }
+      unsigned char* dst = sB + bc * 128 + (((bk >> 3) ^ (bc & 7)) << 4) + (bk & 7) * 2;
+#pragma unroll
+      for (int sl = 0; sl < OZ_S; ++sl)
+#pragma unroll
+        for (int q = 0; q < VB; q += 4)
+          *reinterpret_cast<uint2*>(dst + sl * B_SLICE_BYTES + q * 2) =
+              make_uint2(oz_slice2(W[q], W[q + 1], sl), oz_slice2(W[q + 2], W[q + 3], sl));
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // (the tensor core reads them)
+    }
+    __syncthreads();
+    if (warp == 1) {
+      if (lane == 0) {
+        const uint64_t adesc = smem_desc_sw128(sA), bdesc = smem_desc_sw128(sB);
+#pragma unroll
+        for (int sl = 0; sl < OZ_S; ++sl)
+#pragma unroll
+          for (int kk = 0; kk < KP / 16; ++kk)
+#pragma unroll
+            for (int t0 = 0; t0 + sl < OZ_S; t0 += 4) {
+              const int cnt = OZ_S - sl - t0 < 4 ? OZ_S - sl - t0 : 4;
+              umma_f16(tmem + (uint32_t)((sl + t0) * OBN), adesc + (uint64_t)((sl * A_SLICE_BYTES + kk * 32) >> 4),
+                       bdesc + (uint64_t)((t0 * B_SLICE_BYTES + kk * 32) >> 4), oz_idesc(cnt * OBN),
+                       sl > 0 || kk > 0 ? 1u : 0u);
+            }
+        umma_commit(&s_full);
+      }
+    } else if (warp >= 2) {
+      const int quad = warp & 3, cg = (warp - 2) >> 2;
+      const int lr = quad * 32 + lane, nb0 = n0 + cg * OZ_EC;
+      const int ncol = m0 + lr < m ? min(OZ_EC, n - nb0) : 0;
+      double* crow = C + (long long)(m0 + lr) + (long long)nb0 * ldc;
+      double cv[OZ_EC], sc[OZ_EC];
+#pragma unroll
+      for (int j = 0; j < OZ_EC; ++j) cv[j] = j < ncol ? crow[(long long)j * ldc] : 0.0;
+      if (mbar_wait(&s_full, 0)) {
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        long long I[OZ_EC];
+        oz_read_sums(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(cg * OZ_EC), I, [] {});
+#pragma unroll
+        for (int j = 0; j < OZ_EC; ++j) sc[j] = s_cs[cg * OZ_EC + j];
+        oz_update_c(I, cv, crow, ldc, ncol, alpha, s_rs[lr], sc);
+      } else if (lane == 0) {
+        atomicExch(status, (int)kFlagTimeout);
+      }
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;");
+  __syncthreads();
+  if (warp == 0)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(OZ_TMEM_COLS));
+}
+constexpr int kTileSmem = 1024 + OZ_S * (A_SLICE_BYTES + B_SLICE_BYTES);
+
 // 2D map over the slices: rows = S * rows_pad (slice-major), kpad columns of
 // BF16, box {64, box_rows}, 128-byte swizzle.
 bool make_slice_map(CUtensorMap* map, const void* ptr, int rows_total, int kpad, int box_rows) {
@@ -870,12 +1084,26 @@ cudaError_t oz_smem_once() {
       ozgemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)oz_smem_bytes());
   static const cudaError_t e2 = cudaFuncSetAttribute(
       oz_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)oz_split_smem(OZ_KMAX));
-  return e != cudaSuccess ? e : e2;
+  static const cudaError_t e3 =
+      cudaFuncSetAttribute(oz_tile_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileSmem);
+  static const cudaError_t e4 =
+      cudaFuncSetAttribute(oz_tile_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileSmem);
+  for (cudaError_t x : {e, e2, e3, e4})
+    if (x != cudaSuccess) return x;
+  return cudaSuccess;
 }
 
 inline int round_up(int x, int q) { return (x + q - 1) / q * q; }
 
 int g_oz_tiles_per_cta = 4;
+
+// A product of k <= 64 in one launch (oz_tile_kernel): up to two tiles per SM, each
+// tile slicing its operands itself. In us for a whole LU, with and without: N = 600
+// 1699 / 1794, 4096 14020 / 14750; without the limit N = 16384 takes 117.2 ms instead
+// of 115.8 (116.7 without), its products of 512 tiles then being the slower way.
+inline bool oz_one_launch(int m, int n) {
+  return (m + OBM - 1) / OBM * ((n + OBN - 1) / OBN) <= 2 * num_sms();
+}
 
 }  // namespace
 
@@ -924,6 +1152,14 @@ static cudaError_t oz_dgemm_impl(int side_b, unsigned long long keyed_epoch, con
   if (keyed_epoch && k > OZ_KMAX) return cudaErrorInvalidValue;
   SL_TRY(oz_smem_once());
   const int m_pad = round_up(m, OBM), n_pad = round_up(n, OBN);
+  if (keyed_epoch && !side_b && k <= 64 && oz_one_launch(m, n)) {
+    unsigned long long* kinfo = reinterpret_cast<unsigned long long*>(sc.ptr);
+    auto kern = k <= 32 ? oz_tile_kernel<32> : oz_tile_kernel<64>;
+    kern<<<m_pad / OBM * (n_pad / OBN), OZ_THREADS, kTileSmem, s>>>(A, lda, m, B, ldb, n, k, alpha, C, ldc, status,
+                                                                     kinfo, keyed_epoch);
+    count_launches(1);
+    return cudaGetLastError();
+  }
   for (int k0 = 0; k0 < k; k0 += OZ_KMAX) {
     const int kb = (k - k0) < OZ_KMAX ? (k - k0) : OZ_KMAX;
     const int kpad = round_up(kb, OBK);

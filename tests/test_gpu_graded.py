@@ -137,3 +137,46 @@ def test_graded_sliced_and_dmma_modes_agree(sl, orc, ctx, kind):
     LU0, LU1 = out[0][1], out[1][1]
     scale = np.maximum(np.max(np.abs(LU0), axis=1, keepdims=True), 1e-300)
     assert np.max(np.abs(LU0 - LU1) / scale) < 1e-8
+
+
+@pytest.mark.parametrize("ib", [1, 2])
+@pytest.mark.parametrize("m", [64, 129, 300])
+def test_in_panel_tile_beyond_budget(sl, gpu_required, m, ib):
+    """Rows whose only terms in a panel's product are tiny beside the other rows':
+    their tiles of it take FP64 arithmetic, so that P A = L U holds componentwise
+    there (tiles of 128 rows with and without such rows, partial tiles, one and two
+    sub-panels deep)."""
+    import torch
+
+    rng = np.random.default_rng(m + ib)
+    n, tiny = 96, np.arange(33, m, 2)
+    A = np.zeros((m, n))
+    A[:32, :32] = np.eye(32)  # the first sub-panel's pivots, in place
+    A[32:, :32] = rng.uniform(-0.5, 0.5, (m - 32, 32))
+    A[:32, 32:] = rng.uniform(0.5, 1.0, (32, 64)) * 2.0**20
+    A[0, 32:] *= 2.0**-60
+    A[32:, 32:] = rng.uniform(-0.5, 0.5, (m - 32, 64)) * 2.0**20
+    A[tiny, 1:] = 0.0
+    A[tiny, 32:] = rng.uniform(-0.5, 0.5, (len(tiny), 64)) * 2.0**-40
+    A = np.asfortranarray(A)
+    dA = torch.from_numpy(A.T.copy()).cuda()
+    ip = torch.zeros(min(m, n), dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    before = _routes(sl)
+    try:
+        sl.lib().sl1x1_set_panel_ib(ib)
+        assert sl.dgetrf_dev(m, n, dA.data_ptr(), m, ip.data_ptr(), 256) >= 0
+    finally:
+        sl.lib().sl1x1_set_panel_ib(0)
+    assert _routes(sl) > before
+    F, piv = dA.T.cpu().numpy(), ip.cpu().numpy() - 1
+    PA, row = A.copy(), np.arange(m)
+    for k, p in enumerate(piv):
+        PA[[k, p]] = PA[[p, k]]
+        row[[k, p]] = row[[p, k]]
+    k = min(m, n)
+    low, up = np.tril(F[:, :k], -1) + np.eye(m, k), np.triu(F[:k])
+    err, mag = np.abs(PA - low @ up), np.abs(low) @ np.abs(up)
+    t = np.isin(row, tiny)
+    assert (err[t] <= 16.0 * n * 2.0**-53 * mag[t]).all()
+    assert np.nanmax(err) < 16.0 * n * 2.0**-53 * np.abs(A).sum(axis=1).max()
