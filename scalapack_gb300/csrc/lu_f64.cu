@@ -349,7 +349,7 @@ static cudaError_t factor_panel(int m, double* dA, long long ldda, int* dipiv, i
     for (int k = 0; k < kw; ++k) kflops += 2.0 * (double)(m - r0 - k - 1) * (w - k - 1) + (m - r0 - k - 1);
     pflops += kflops;
     phase_begin(kPhPanelKernel, s);
-    SL_TRY(launch_panel<double>(dA, ldda, m, r0, r0, w, dipiv, ws, s));
+    SL_TRY(launch_panel<double>(dA, ldda, m, r0, r0, w, dipiv, ws, s, c > 0));
     phase_end(kPhPanelKernel, s, kflops, 16.0 * (double)(m - r0) * w);
     phase_begin(kPhPanelUpdate, s);
     if (c + w >= jb) {

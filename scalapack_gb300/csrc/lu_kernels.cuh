@@ -514,6 +514,7 @@ panel_kernel(T* A, long long lda, int m, int r0, int c0, int w, int rpc, int* ip
   }
   // the last column's remaining update (columns beyond kw when the panel has
   // fewer rows than columns), then every row to where its content stands
+  launch_dependents();
   if (exch) return;
   if (kw > 0) finish_update(kw - 1);
   if (ONE && part == 0 && row0 < nr) lab[row0] = mylab;
@@ -612,6 +613,7 @@ panel_cluster_kernel(T* A, long long lda, int m, int r0, int c0, int w, int rpc,
   };
   const int part = tid & (tpr - 1), row0 = exch ? nr : tid / tpr;
   int mylab = row0 < nr ? lo + row0 : -1;  // the label of row row0
+  wait_for_previous();
   if (!exch) {
     long long key = -2;
     int label = INT_MAX, lrow = 0;
@@ -780,6 +782,7 @@ panel_cluster_kernel(T* A, long long lda, int m, int r0, int c0, int w, int rpc,
     }
     Uprev = U;
   }
+  launch_dependents();
   __syncthreads();
   if (s_fail) {
     // pivots from the first one that was not chosen become the diagonal rows
@@ -1033,6 +1036,8 @@ inpanel_step_kernel(T* A, long long lda, int k1, int k2, const int* __restrict__
   __shared__ unsigned s_h[64];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int n1 = ce1 - cb1, ncols = n1 + (ce2 - cb2), ncta = (ncols + IPC - 1) / IPC;
+  wait_for_previous();
+  launch_dependents();
   if ((int)blockIdx.x >= ncta) {
     if constexpr (sizeof(T) == 8) {
       // column maxima of kj.L, 32 rows per CTA
@@ -1659,7 +1664,7 @@ gemm_skinny_kernel(int m, int n, int k, T alpha, const T* __restrict__ A, long l
 
 template <typename T>
 inline cudaError_t launch_panel(T* A, long long lda, int m, int r0, int c0, int w, int* ipiv,
-                                const LuWork& ws, cudaStream_t s) {
+                                const LuWork& ws, cudaStream_t s, bool after_kernel = false) {
   const int R = m - r0;
   // One cluster (16 CTAs at most, of 32 rows at least) while its rows stay
   // within what its SMs' FP64 units do in a column's time. (The tuning knobs of
@@ -1680,17 +1685,19 @@ inline cudaError_t launch_panel(T* A, long long lda, int m, int r0, int c0, int 
     }();
     SL_TRY(at);
     cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute la[1];
+    cudaLaunchAttribute la[2];
     la[0].id = cudaLaunchAttributeClusterDimension;
     la[0].val.clusterDim.x = cs;
     la[0].val.clusterDim.y = la[0].val.clusterDim.z = 1;
+    la[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // (see launch_after)
+    la[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.gridDim = dim3(cs);
     const int ntr = crpc > PTR ? 2 * PTR : PTR;
     cfg.blockDim = dim3(ntr + 32);
     cfg.dynamicSmemBytes = csmem;
     cfg.stream = s;
     cfg.attrs = la;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = after_kernel ? 2 : 1;
     int ctpr = crpc > PTR / 4 ? 1 : (crpc > PTR / 8 ? 2 : 4);
     count_launches(1);
     auto kern = ntr == PTR ? panel_cluster_kernel<T, PTR> : panel_cluster_kernel<T, 2 * PTR>;
@@ -1783,9 +1790,9 @@ inline cudaError_t inpanel_step(T* A, long long lda, int k1, int k2, const int* 
   const int ncols = (ce1 - cb1) + (ce2 - cb2);
   if (ncols <= 0 || k2 <= k1) return cudaSuccess;
   const int grid = (ncols + IPC - 1) / IPC + (kj.ckeys ? (kj.lrows + 31) / 32 : 0);
-  inpanel_step_kernel<T><<<grid, 32 * IPC, 0, s>>>(A, lda, k1, k2, ipiv, cb1, ce1, cb2, ce2, nsolve, kb, kj);
   count_launches(1);
-  return cudaGetLastError();
+  return launch_after(inpanel_step_kernel<T>, dim3(grid), 32 * IPC, 0, s, A, lda, k1, k2, ipiv, cb1, ce1, cb2, ce2,
+                      nsolve, kb, kj);
 }
 
 // Plan of a panel's interchanges (k2 - k1 <= LSW_MAXP), see laswp_plan_kernel.

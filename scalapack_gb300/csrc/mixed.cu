@@ -294,7 +294,7 @@ static cudaError_t factor_panel_f32(int n, float* F, long long ldf, int* dipiv, 
   for (int c = 0; c < jb; c += PW) {
     const int w = (jb - c) < PW ? (jb - c) : PW;
     const int r0 = j + c;
-    SL_TRY(launch_panel<float>(F, ldf, m, r0, r0, w, dipiv, ws, s));
+    SL_TRY(launch_panel<float>(F, ldf, m, r0, r0, w, dipiv, ws, s, c > 0));
     const int kw = (m - r0) < w ? (m - r0) : w;
     SL_TRY(inpanel_step<float>(F, ldf, r0, r0 + kw, dipiv, j, r0, r0 + w, j + jb, jb - c - w, kw, s));
     if (c + w < jb) {

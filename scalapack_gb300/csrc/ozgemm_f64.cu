@@ -890,8 +890,10 @@ oz_tile_kernel(const double* A, long long lda, int m, const double* B, long long
   __shared__ int s_d[KP], s_h[KP];
   __shared__ int s_E[4][OBM], s_F[4][OBM];
   __shared__ double s_rs[OBM], s_cs[OBN];
-  if (*(volatile int*)status != 0) return;  // an earlier wait gave up
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  wait_for_previous();
+  launch_dependents();
+  if (*(volatile int*)status != 0) return;  // an earlier wait gave up
   const int tiles_m = (m + OBM - 1) / OBM, tiles_n = (n + OBN - 1) / OBN;
   int m0, n0;
   oz_tile(blockIdx.x, tiles_m, tiles_n, m0, n0);
@@ -1155,10 +1157,9 @@ static cudaError_t oz_dgemm_impl(int side_b, unsigned long long keyed_epoch, con
   if (keyed_epoch && !side_b && k <= 64 && oz_one_launch(m, n)) {
     unsigned long long* kinfo = reinterpret_cast<unsigned long long*>(sc.ptr);
     auto kern = k <= 32 ? oz_tile_kernel<32> : oz_tile_kernel<64>;
-    kern<<<m_pad / OBM * (n_pad / OBN), OZ_THREADS, kTileSmem, s>>>(A, lda, m, B, ldb, n, k, alpha, C, ldc, status,
-                                                                     kinfo, keyed_epoch);
     count_launches(1);
-    return cudaGetLastError();
+    return launch_after(kern, dim3(m_pad / OBM * (n_pad / OBN)), OZ_THREADS, kTileSmem, s, A, lda, m, B, ldb, n, k,
+                        alpha, C, ldc, status, kinfo, keyed_epoch);
   }
   for (int k0 = 0; k0 < k; k0 += OZ_KMAX) {
     const int kb = (k - k0) < OZ_KMAX ? (k - k0) : OZ_KMAX;
