@@ -242,6 +242,7 @@ __host__ __device__ inline int inv_cols_blocks(int jb) { return (jb + 1) / 2; }
 __global__ void __launch_bounds__(256)
 unit_lower_inv_cols_kernel(int jb, const double* __restrict__ L, long long ldl, double* X,
                            int ldx, int k1, int k2, const int* __restrict__ ipiv, int* plan) {
+  wait_for_previous();
   if (plan != nullptr && (int)blockIdx.x == inv_cols_blocks(jb)) {
     laswp_plan_block(k1, k2, ipiv, plan);
     return;
@@ -411,10 +412,9 @@ static cudaError_t factor_panel(int m, double* dA, long long ldda, int* dipiv, i
     // plan in the same launch
     if (want_plan && npiv <= 0) SL_TRY(cudaMemsetAsync(ws.swap_plan, 0, sizeof(int), s));
     const bool fused = want_plan && npiv > 0;
-    unit_lower_inv_cols_kernel<<<inv_cols_blocks(jb) + (fused ? 1 : 0), 256, 0, s>>>(
-        jb, Ap(j, j), ldda, ws.dinv64, jb, j, j + npiv, dipiv, fused ? ws.swap_plan : nullptr);
+    SL_TRY(launch_after(unit_lower_inv_cols_kernel, dim3(inv_cols_blocks(jb) + (fused ? 1 : 0)), 256, 0, s, jb, Ap(j, j),
+                        ldda, ws.dinv64, jb, j, j + npiv, dipiv, fused ? ws.swap_plan : nullptr));
     count_launches(1);
-    SL_TRY(cudaGetLastError());
   } else if (want_plan) {
     SL_TRY(laswp_plan(j, j + npiv, dipiv, ws.swap_plan, s));
   }

@@ -96,6 +96,8 @@ sgemm_k32_kernel(int m, int n, int k, float alpha, const float* __restrict__ A, 
   const int row = blockIdx.x * 256 + threadIdx.x, n0 = blockIdx.y * K32_N, nc = min(K32_N, n - n0);
   const float* a = A + min(row, m - 1);
   float av[32], cv[K32_N], acc[K32_N];
+  wait_for_previous();
+  launch_dependents();
 #pragma unroll
   for (int q = 0; q < 32; ++q) av[q] = a[(long long)min(q, k - 1) * lda];
   float* c = C + row + (long long)n0 * ldc;
@@ -125,10 +127,9 @@ static cudaError_t sgemm_simt(bool transa, int m, int n, int k, float alpha, con
                               long long ldc, cudaStream_t s) {
   if (m <= 0 || n <= 0 || k <= 0) return cudaSuccess;
   if (!transa && k <= 32) {
-    sgemm_k32_kernel<<<dim3((m + 255) / 256, (n + K32_N - 1) / K32_N), 256, 0, s>>>(m, n, k, alpha, A, lda, B,
-                                                                                  ldb, C, ldc);
     count_launches(1);
-    return cudaGetLastError();
+    return launch_after(sgemm_k32_kernel, dim3((m + 255) / 256, (n + K32_N - 1) / K32_N), 256, 0, s, m, n, k, alpha, A,
+                        lda, B, ldb, C, ldc);
   }
   dim3 grid((m + 63) / 64, (n + 63) / 64);
   if (transa) sgemm_simt_kernel<true><<<grid, 256, 0, s>>>(m, n, k, alpha, A, lda, B, ldb, C, ldc);
