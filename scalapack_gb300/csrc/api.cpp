@@ -193,13 +193,21 @@ void release_all() {
   g_dev = DevState();
 }
 
-// Block size of the factorization of a matrix with mn = min(M, N) whose caller
-// gives NB, the distribution's block: on one process it decides nothing but the
-// order of the work (the pivots do not depend on it), and 256 columns suit the
-// sliced products best at every order measured: N = 600 2.27 ms (64 columns: 2.45,
-// 512: 2.75), N = 2000 7.98 (9.09, 10.3), N = 8192 39.9 (67.9, 55.0). Matrices of a
-// few panels, where it matters little, and the DMMA form keep the caller's.
-int factor_nb(int mn, int nb) { return mn > 512 && sl::f64_update_get() == 1 ? 256 : nb; }
+// Block size of the factorization of an m x n matrix whose caller gives NB, the
+// distribution's block: on one process it decides nothing but the order of the work
+// (the pivots do not depend on it). A matrix whose in-panel products (rank 32, one
+// launch) have at most two tiles per SM is one panel: what a block costs beside its
+// panel (inverse, U12, update, interchanges: about 90 us of launches) is more than
+// the wider products. PDGETRF in us, one panel / 256 / 64 columns: N = 100 244 / 244 /
+// 305, N = 600 1338 / 1558 / 1782, N = 1000 2324 / 2617 / 3073, N = 1536 4009 / 4228 /
+// 5019 (and at N = 2000 7904 in panels of 1024). Beyond that 256 columns suit the
+// sliced products best: N = 2000 5756 (64: 6972, 512: 8379), N = 8192 39.9 ms (67.9,
+// 55.0). The DMMA form keeps the caller's.
+int factor_nb(int m, int n, int nb) {
+  if (sl::f64_update_get() != 1) return nb;
+  const long long tiles = ((m + 127LL) / 128) * ((n + 63) / 64);
+  return n <= m && n <= sl::kOnePanelMax && tiles <= 2LL * sl::num_sms() ? n : 256;
+}
 
 // Grows a sliced-product scratch buffer; a new one starts with its balancing
 // words zeroed (the memory may hold anything, including words that look like
@@ -317,7 +325,7 @@ int factor_host(int m, int n, double* A, int ia, int ja, const int* desca, int* 
   if (e == cudaSuccess) e = grow(&g_dev.dipiv, &g_dev.capP, (size_t)(mn > 0 ? mn : 1));
   if (e != cudaSuccess) return cuda_info(e);
   const double* src = A + (ia - 1) + (long long)(ja - 1) * lld;
-  const int nb = factor_nb(mn, desca[NB_]);
+  const int nb = factor_nb(m, n, desca[NB_]);
   ensure_oz(m, n, nb);
   // With the look-ahead on and more than two panels, A goes over in column
   // chunks of about n/g_copy_chunks (whole panels, the first holding panels 0
@@ -664,7 +672,7 @@ int sl1x1_dgetrf_dev(int m, int n, double* dA, long long ldda, int* dipiv, int n
   if (!ensure_device()) return cuda_info(cudaErrorNoDevice);
   cudaStream_t s = (cudaStream_t)stream;
   if (nb <= 0) nb = g_default_nb;
-  nb = factor_nb(m < n ? m : n, nb);
+  nb = factor_nb(m, n, nb);
   ensure_oz(m, n, nb);
   sl::LuWork w = make_work();
   cudaError_t e = sl::dgetrf_device(m, n, dA, ldda, dipiv, nb, w, s);

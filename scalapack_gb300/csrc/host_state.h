@@ -96,8 +96,8 @@ int cuda_info(cudaError_t e);
 // Creates the streams and small buffers on first use; false without an sm_103 GPU.
 bool ensure_device();
 sl::LuWork make_work();
-// Block size the factorization uses for a caller's NB.
-int factor_nb(int mn, int nb);
+// Block size the factorization of an m x n matrix uses for a caller's NB.
+int factor_nb(int m, int n, int nb);
 cudaError_t ensure_solve_ws(int n, int nrhs);
 // INFO after a factorization (>0 singular, <= -20000 device status)
 int read_factor_info(cudaStream_t s, int mn, int* out_info);

@@ -328,7 +328,7 @@ static cudaError_t solve_u12(int jb, int nr, const double* L11, long long ldl, d
 // PDGETF2 on columns [j, j+jb), rows [j, m): 32-wide cooperative sub-panels,
 // each followed by its row interchanges on the rest of the panel, the U solve
 // and the GEMM update of the panel's remaining columns.
-static cudaError_t factor_panel(int m, double* dA, long long ldda, int* dipiv, int j, int jb,
+static cudaError_t factor_panel(int m, int n, double* dA, long long ldda, int* dipiv, int j, int jb,
                                 const LuWork& ws, cudaStream_t s) {
   auto Ap = [&](long long i, long long c) { return dA + i + c * ldda; };
   const OzScratch& sc = (ws.aux && s == ws.aux) ? ws.oz_aux : ws.oz;
@@ -405,9 +405,10 @@ static cudaError_t factor_panel(int m, double* dA, long long ldda, int* dipiv, i
   // the panel's interchanges in composite form, for the row interchanges of
   // the other columns (computed here, on the panel's stream)
   const int npiv = (m - j) < jb ? (m - j) : jb;
-  const bool want_plan = ws.swap_plan && npiv <= LSW_MAXP;
+  const bool more = j + jb < n;  // columns to the right: they want both of what follows
+  const bool want_plan = ws.swap_plan && npiv <= LSW_MAXP && (more || j > 0);
   // inverses of L11's diagonal blocks for the U12 solve of this step
-  if (g_f64_update == 1 && ws.dinv64 && npiv == jb && jb <= kFullInvMax) {
+  if (more && g_f64_update == 1 && ws.dinv64 && npiv == jb && jb <= kFullInvMax) {
     // inv(L11) - I whole (jb x jb, leading dimension jb), and the interchange
     // plan in the same launch
     if (want_plan && npiv <= 0) SL_TRY(cudaMemsetAsync(ws.swap_plan, 0, sizeof(int), s));
@@ -418,7 +419,7 @@ static cudaError_t factor_panel(int m, double* dA, long long ldda, int* dipiv, i
   } else if (want_plan) {
     SL_TRY(laswp_plan(j, j + npiv, dipiv, ws.swap_plan, s));
   }
-  if (g_f64_update == 1 && ws.dinv64 && npiv == jb && jb > kFullInvMax && jb <= 1024) {
+  if (more && g_f64_update == 1 && ws.dinv64 && npiv == jb && jb > kFullInvMax && jb <= 1024) {
     constexpr int kInvSmem = 2 * 64 * 65 * (int)sizeof(double);
     static const cudaError_t attr = cudaFuncSetAttribute(
         unit_lower_inv64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kInvSmem);
@@ -476,7 +477,7 @@ static cudaError_t step0_by_chunks(int m, int n, double* dA, long long ldda, int
   }
   SL_TRY(cudaEventRecord(ws.ev_next, s));
   SL_TRY(cudaStreamWaitEvent(ws.aux, ws.ev_next, 0));
-  SL_TRY(factor_panel(m, dA, ldda, dipiv, jn, jb2, ws, ws.aux));
+  SL_TRY(factor_panel(m, n, dA, ldda, dipiv, jn, jb2, ws, ws.aux));
   SL_TRY(cudaEventRecord(ws.ev_panel, ws.aux));
   const int nck = ws.ncol_chunks < kMaxColChunks ? ws.ncol_chunks : kMaxColChunks;
   for (int c = 0; c < nck; ++c) {
@@ -512,7 +513,7 @@ cudaError_t dgetrf_device(int m, int n, double* dA, long long ldda, int* dipiv, 
   SL_TRY(cudaMemsetAsync(ws.status, 0, sizeof(int), s));
   SL_TRY(cudaMemsetAsync(ws.info_col, 0x7f, sizeof(int), s));
   const int mn = m < n ? m : n;
-  if (nb > 1024) nb = 1024;
+  if (nb > 1024 && !(nb == n && n <= m && n <= kOnePanelMax && g_f64_update == 1)) nb = 1024;
   auto Ap = [&](long long i, long long j) { return dA + i + j * ldda; };
   const bool lookahead = ws.aux && ws.ev_next && ws.ev_panel && mn > 2 * nb;
   // column chunks: s waits for every chunk that starts below column `upto`
@@ -528,7 +529,7 @@ cudaError_t dgetrf_device(int m, int n, double* dA, long long ldda, int* dipiv, 
   };
   const bool stream_step0 = nck > 0 && lookahead && ws.dinv64_step0 && ws.col_end[nck - 1] >= n;
   SL_TRY(wait_cols(stream_step0 ? nb : INT_MAX));
-  if (mn > 0) SL_TRY(factor_panel(m, dA, ldda, dipiv, 0, (mn < nb ? mn : nb), ws, s));
+  if (mn > 0) SL_TRY(factor_panel(m, n, dA, ldda, dipiv, 0, (mn < nb ? mn : nb), ws, s));
   bool panel_on_aux = false;
   if (stream_step0) {
     SL_TRY(step0_by_chunks(m, n, dA, ldda, dipiv, nb, ws, s, wait_cols));
@@ -579,7 +580,7 @@ cudaError_t dgetrf_device(int m, int n, double* dA, long long ldda, int* dipiv, 
                        ldda, ws, ws.aux, (g_cap_mask & 2) ? free_sms : 0));
       phase_end(kPhGemm, ws.aux, 2.0 * mr * jb2 * jb, 8.0 * (mr * jb + (double)jb * jb2 + 2.0 * mr * jb2));
       nxt.inpanel_ctas = (g_cap_mask & 1) ? free_sms : 0;
-      SL_TRY(factor_panel(m, dA, ldda, dipiv, jn, jb2, nxt, ws.aux));
+      SL_TRY(factor_panel(m, n, dA, ldda, dipiv, jn, jb2, nxt, ws.aux));
       SL_TRY(cudaEventRecord(ws.ev_panel, ws.aux));
       panel_on_aux = true;
       // the other columns on the caller's stream
@@ -621,7 +622,7 @@ cudaError_t dgetrf_device(int m, int n, double* dA, long long ldda, int* dipiv, 
           phase_end(kPhGemm, s, 2.0 * mr * jb2 * jb, 8.0 * (mr * jb + (double)jb * jb2 + 2.0 * mr * jb2));
           SL_TRY(cudaEventRecord(ws.ev_next, s));
           SL_TRY(cudaStreamWaitEvent(ws.aux, ws.ev_next, 0));
-          SL_TRY(factor_panel(m, dA, ldda, dipiv, jn, jb2, ws, ws.aux));
+          SL_TRY(factor_panel(m, n, dA, ldda, dipiv, jn, jb2, ws, ws.aux));
           SL_TRY(cudaEventRecord(ws.ev_panel, ws.aux));
           panel_on_aux = true;
           const int rest = n - jn - jb2;
@@ -640,7 +641,7 @@ cudaError_t dgetrf_device(int m, int n, double* dA, long long ldda, int* dipiv, 
         }
       }
     }
-    if (jb2 > 0 && !panel_on_aux) SL_TRY(factor_panel(m, dA, ldda, dipiv, jn, jb2, ws, s));
+    if (jb2 > 0 && !panel_on_aux) SL_TRY(factor_panel(m, n, dA, ldda, dipiv, jn, jb2, ws, s));
   }
   if (panel_on_aux) SL_TRY(cudaStreamWaitEvent(s, ws.ev_panel, 0));
   return cudaGetLastError();

@@ -182,6 +182,8 @@ inline size_t kSolveInvDoubles(int n) {
 constexpr int kWideRhs = 256;
 // Doubles of the U12 solve's diagonal-block inverses: NB <= 1024 in 64-row blocks.
 constexpr size_t kDinv64Doubles = (size_t)16 * 64 * 64;
+// Columns up to which a matrix may be factored as one panel (factor_nb).
+constexpr int kOnePanelMax = 1536;
 
 size_t panel_cand_doubles();
 // 8-byte words of the panel kernel's exchange area (2 x 160 x 160 16-byte keys,

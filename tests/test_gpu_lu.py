@@ -535,3 +535,30 @@ def test_u12_through_inverse_edges(sl, gpu_required, m):
         PA[[k, p]] = PA[[p, k]]
     low, up = np.tril(F[:, :m], -1) + np.eye(m), np.triu(F)
     assert np.abs(PA - low @ up).max() < 16.0 * n * 2.0**-53 * np.abs(A).sum(axis=1).max()
+
+
+@pytest.mark.parametrize("m,n", [(1024, 1024), (1025, 1025), (1536, 1536), (1537, 1537), (2432, 1024), (2433, 1024), (257, 256), (40, 257), (600, 601)])
+def test_one_panel_rule_edges(sl, orc, gpu_required, m, n):
+    """Both sides of the sizes up to which a matrix is one panel (width, tiles of its
+    in-panel products, wide matrices never): P A = L U to the tester's bound, and the
+    caller's block size changes nothing."""
+    import torch
+
+    rng = np.random.default_rng(m + n)
+    A = np.asfortranarray(rng.uniform(-0.5, 0.5, (m, n)))
+    k, got = min(m, n), []
+    for nb in (64, 1024):
+        dA = torch.from_numpy(A.T.copy()).cuda()
+        ip = torch.zeros(k, dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        assert sl.dgetrf_dev(m, n, dA.data_ptr(), m, ip.data_ptr(), nb) == 0
+        got.append((dA.T.cpu().numpy(), ip.cpu().numpy() - 1))
+    F, piv = got[0]
+    np.testing.assert_array_equal(F, got[1][0])
+    np.testing.assert_array_equal(piv, got[1][1])
+    PA = A.copy()
+    for q, p in enumerate(piv):
+        PA[[q, p]] = PA[[p, q]]
+    low, up = np.tril(F[:, :k], -1) + np.eye(m, k), np.triu(F[:k])
+    assert np.abs(low).max() <= 1.0 + 1e-15  # partial pivoting
+    assert np.abs(PA - low @ up).max() < 16.0 * max(m, n) * 2.0**-53 * np.abs(A).sum(axis=1).max()
