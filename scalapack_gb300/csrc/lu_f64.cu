@@ -2,27 +2,28 @@
 //
 // Structure follows PDGETRF on a 1x1 grid (SRC/pdgetrf.f:219-295):
 //   for each NB-wide block column j:
-//     panel      PDGETF2 (SRC/pdgetf2.f:206-237)  -> panel_kernel<double>, blocked by 32
+//     panel      PDGETF2 (SRC/pdgetf2.f:206-237)  -> panel_cluster_kernel / panel_kernel
+//                                                    <double>, blocked by 32
 //     swaps      PDLASWP (SRC/pdlaswp.f:163-172)  -> laswp_apply_kernel (composite plan of
 //                                                    the panel's interchanges, both sides)
-//     U12        PDTRSM  (SRC/pdgetrf.f:280-282)  -> 64x64 block inverses of L11 and
-//                                                    sliced products (trsm_strip_kernel
-//                                                    in the DMMA mode)
+//     U12        PDTRSM  (SRC/pdgetrf.f:280-282)  -> inverse of L11 and a sliced product
+//                                                    (trsm_strip_kernel in the DMMA mode)
 //     update     PDGEMM  (SRC/pdgetrf.f:288-290)  -> oz_dgemm (FP64 from exact BF16 slice
 //                                                    products, ozgemm_f64.cu; dgemm DMMA,
 //                                                    dgemm_f64.cu, in the DMMA mode)
 // with the next panel factored on a second stream (look-ahead), and PDGETRS
 // (SRC/pdgetrs.f:250-284): pivots on B (PDLAPIV) as one composed permutation,
-// then unit-lower and non-unit-upper blocked solves (diagonal-block inverses
+// then unit-lower and non-unit-upper solves: chained over 64-row blocks for few
+// right-hand sides (trsv_f64.cu), else by 128-row blocks (diagonal-block inverses
 // and sliced products for NOTRAN, substitution strips otherwise).
 //
-// The NB-wide panel is factored as 32-column sub-panels; each sub-panel is one
-// cooperative kernel whose CTAs hold disjoint row slices of the sub-panel in
-// shared memory and exchange each column's pivot candidates through tagged
-// words in L2 (bounded polls, no grid barrier). The remaining columns of the NB panel are brought up to date
-// with the same swap / triangular-solve / GEMM kernels, so the final factors,
-// pivots and INFO are those of the reference's column-by-column PDGETF2 in
-// exact arithmetic.
+// The NB-wide panel is factored as 32-column sub-panels; each is one kernel whose
+// CTAs hold disjoint row slices of the sub-panel in shared memory and exchange
+// each column's pivot candidates, within a cluster through distributed shared
+// memory or between more CTAs through tagged words in L2 (bounded polls, no grid
+// barrier). The remaining columns of the panel are brought up to date by
+// inpanel_step_kernel and a sliced product, so the final factors, pivots and INFO
+// are those of the reference's column-by-column PDGETF2 in exact arithmetic.
 #include <algorithm>
 #include <climits>
 
@@ -1095,14 +1096,15 @@ cudaError_t dgetrs_device(char trans, int n, int nrhs, const double* dA, long lo
   // any NRHS whose products fit the scratch (PDGETRI solves with NRHS = N)
   const bool inv_path = g_f64_update == 1 && ws.dinv_solve && ws.dinv_solve_len >= kSolveInvDoubles(n) &&
                         oz_fits(ws.oz, n, nrhs, 128);
-  // Few right-hand sides go through the chained solves: NOTRAN up to 16 (n =
-  // 16384, 16 columns: 9.8 ms, the blocked solve 13.6; below that 2 to 6 times
-  // less) and up to 32 while n <= 4096 (n = 1000: 0.38 of 0.69 ms), where the FP64
-  // pipe's n^2 nrhs bound passes the blocked solve, whose products run on the
-  // tensor cores; transposed up to 128 (n = 8192, 64 columns: 11.6 of 31 ms: the
-  // blocked form there substitutes and multiplies on the FP64 pipe)
-  const int chain_rhs = notran ? (n <= 4096 ? 32 : 16) : kChainRhs;
-  const bool chain_path = g_f64_update == 1 && nrhs <= chain_rhs && ws.dinv_solve &&
+  // Few right-hand sides go through the chained solves, whose FP64 work grows with n^2
+  // nrhs: NOTRAN while n nrhs <= 2^18, beyond which the blocked solve, its products on
+  // the tensor cores, takes less. In ms, chained / blocked: n = 2048, 128 columns
+  // 1.24 / 1.39; n = 4096, 64: 2.36 / 2.99, 96: 3.41 / 2.99; n = 8192, 32: 4.54 /
+  // 5.81, 48: 6.57 / 6.03; n = 16384, 16: 9.08 / 12.33, 24: 13.14 / 12.36.
+  // Transposed always (n = 8192, 64 columns: 8.6 / 31 ms: the blocked form there
+  // substitutes and multiplies on the FP64 pipe).
+  const bool few = nrhs <= kChainRhs && (!notran || (long long)n * nrhs <= 1LL << 18);
+  const bool chain_path = g_f64_update == 1 && few && ws.dinv_solve &&
                           ws.dinv_solve_len >= kSolveInvDoubles(n) && ws.chain && ws.chain_epoch &&
                           ws.chain_values >= (size_t)n * nrhs;
   if (notran ? (inv_path || chain_path) : chain_path) {

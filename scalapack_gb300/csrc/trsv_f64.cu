@@ -2,8 +2,8 @@
 // SRC/pdgetrs.f:250-284, both TRANS): two launches, one per triangle, instead
 // of two or three launches per 128 rows.
 //
-// Work is cut into 64-row blocks of op(T) times groups of NR right-hand sides;
-// each CTA takes the next (block, group) in solve order from an atomic ticket,
+// Work is cut into 64-row blocks of op(T) times right-hand sides; each CTA takes
+// the next (block, right-hand side) in solve order from an atomic ticket,
 // so every block it depends on belongs to a CTA that has already started and
 // the waits always end (no residency assumption). A CTA streams its 64x64
 // blocks of the factor through a ring in shared memory with cp.async, ahead of
@@ -15,12 +15,14 @@
 // Bound: n^2 nrhs FMAs on the FP64 pipe (a 64x64 block times one vector takes
 // 2560 cycles of an SM) when there are many right-hand sides; with one, the
 // chain of n/64 steps (one poll, one block product, one inverse product: about
-// 4 us each). One right-hand side per CTA keeps that chain short; two halve the
-// factor's reads through L2 once the pipe is the bound. Measured, GB300: n = 8192
-// with one right-hand side, 0.97 ms for the whole PDGETRS (two chains of 0.39,
-// the rest before them; 6.27 with three launches per 128 rows); n = 8192, TRANS
-// = 'T', 16 right-hand sides, 3.07 ms (16.96 by substitution and DMMA
-// products), of which the FP64 pipe needs 2.0.
+// 3.5 us each). Two right-hand sides per CTA would halve the factor's reads
+// through L2, which are not the bound, and lengthen a block's turn in the chain,
+// which is: n = 4096, 8 right-hand sides 0.93 ms (one per CTA: 0.59), n = 8192, 16
+// of them 2.98 (2.56), n = 16384 9.70 (9.12). Measured, GB300: n = 8192 with one
+// right-hand side, 0.90 ms for the whole PDGETRS (two chains of 0.39, the rest
+// before them; 6.27 with three launches per 128 rows); n = 8192, TRANS = 'T', 16
+// right-hand sides, 2.55 ms (16.96 by substitution and DMMA products), of which
+// the FP64 pipe needs 2.0.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -67,18 +69,17 @@ __device__ __forceinline__ bool get_x(const unsigned long long* p, uint32_t epoc
 // `gather` / `scatter` permute there (null: i; maps: their segments' maps,
 // follow_perm). D: inverses of T's diagonal blocks,
 // 4096 doubles each, column-major.
-template <int NR, bool TRANS>
+template <bool TRANS>
 __global__ void __launch_bounds__(256)
 trsv64_chain_kernel(const double* __restrict__ A, long long lda, int n, int forward,
                     const double* __restrict__ D, const double* __restrict__ src, long long lds,
                     const int* __restrict__ gather, double* dst, long long ldd,
                     const int* __restrict__ scatter, const int* __restrict__ maps, int nrhs,
-                    int ngroups, int* ticket,
-                    unsigned long long* words, uint32_t epoch, int* status) {
-  extern __shared__ double trsv_ring[];     // TRING tiles
-  __shared__ double xs[2][TB * NR];         // solutions of the block being applied
-  __shared__ double part[4][TB * NR];
-  __shared__ double vs[TB * NR];
+                    int* ticket, unsigned long long* words, uint32_t epoch, int* status) {
+  extern __shared__ double trsv_ring[];  // TRING tiles
+  __shared__ double xs[2][TB];           // solution of the block being applied
+  __shared__ double part[4][TB];
+  __shared__ double vs[TB];
   __shared__ int s_t, s_fail;
   const int tid = threadIdx.x;
   if (tid == 0) {
@@ -87,7 +88,7 @@ trsv64_chain_kernel(const double* __restrict__ A, long long lda, int n, int forw
   }
   __syncthreads();
   const int nblk = (n + TB - 1) / TB;
-  const int sidx = s_t / ngroups, c0 = (s_t % ngroups) * NR;
+  const int sidx = s_t / nrhs, col = s_t % nrhs;
   if (sidx >= nblk || s_fail) return;
   const int b = forward ? sidx : nblk - 1 - sidx;
   const int r0 = b * TB, rb = min(TB, n - r0);
@@ -119,33 +120,30 @@ trsv64_chain_kernel(const double* __restrict__ A, long long lda, int n, int forw
 #pragma unroll
   for (int t = 0; t < TRING - 1; ++t) fetch(t);
 
-  // thread (pi, pc) of the first TB*NR carries value pi of right-hand side pc
-  const int pi = tid & (TB - 1), pc = tid >> 6;
-  const bool mine = pc < NR && pi < rb && c0 + pc < nrhs;
+  // thread r of the first TB carries value r of the block
+  const bool mine = tid < rb;
   double bv = 0.0;
-  int drow = r0 + pi;
+  int drow = r0 + r;
   if (mine) {
     const int srow = gather ? follow_perm(drow, gather, n, maps) : drow;
-    if ((unsigned)srow < (unsigned)n) bv = src[srow + (long long)(c0 + pc) * lds];
+    if ((unsigned)srow < (unsigned)n) bv = src[srow + (long long)col * lds];
     if (scatter) drow = follow_perm(drow, scatter, n, maps);
   }
 
-  double acc[NR];
-#pragma unroll
-  for (int c = 0; c < NR; ++c) acc[c] = 0.0;
+  double acc = 0.0;
   for (int t = 0; t < sidx; ++t) {
     const int k0 = (forward ? t : nblk - 1 - t) * TB;
-    if (pc < NR) {
+    if (tid < TB) {
       double v = 0.0;
-      if (k0 + pi < n && c0 + pc < nrhs) {
-        const unsigned long long* p = words + ((size_t)(c0 + pc) * n + k0 + pi) * 2;
+      if (k0 + r < n) {
+        const unsigned long long* p = words + ((size_t)col * n + k0 + r) * 2;
         for (long long spins = 0; !get_x(p, epoch, v);) {
           if (++spins > kSpinLimit) { s_fail = 1; break; }
           // far from its turn a CTA leaves the L2 to the ones that are next
           if (sidx - t > 2) __nanosleep(200);
         }
       }
-      xs[t & 1][pi * NR + pc] = v;
+      xs[t & 1][r] = v;
     }
     cp_wait<TRING - 2>();
     __syncthreads();
@@ -159,65 +157,52 @@ trsv64_chain_kernel(const double* __restrict__ A, long long lda, int n, int forw
     // that a row of any length meets one rounding per tile at the sum's size
     const double* T = trsv_ring + (t % TRING) * TSLOT;
     const double* x = xs[t & 1];
-    double p[NR];
+    double p = 0.0;
 #pragma unroll
     for (int kk = 0; kk < 16; ++kk) {
       const int k = q * 16 + kk;
       const double a = TRANS ? T[r * CS + k] : T[k * CS + r];
-#pragma unroll
-      for (int c = 0; c < NR; ++c) p[c] = kk == 0 ? a * x[k * NR + c] : fma(a, x[k * NR + c], p[c]);
+      p = kk == 0 ? a * x[k] : fma(a, x[k], p);
     }
-#pragma unroll
-    for (int c = 0; c < NR; ++c) acc[c] += p[c];
+    acc += p;
   }
-#pragma unroll
-  for (int c = 0; c < NR; ++c) part[q][r * NR + c] = acc[c];
+  part[q][r] = acc;
   cp_wait<0>();
   __syncthreads();
-  if (pc < NR) {
-    const int e = pi * NR + pc;
-    vs[e] = bv - ((part[0][e] + part[1][e]) + (part[2][e] + part[3][e]));
-  }
+  if (tid < TB) vs[r] = bv - ((part[0][r] + part[1][r]) + (part[2][r] + part[3][r]));
   __syncthreads();
   {
     // x = inv(T_bb) v over the triangle only, so that an Inf or NaN in v
     // reaches no row that does not depend on it
     const double* T = trsv_ring + (sidx % TRING) * TSLOT;
-#pragma unroll
-    for (int c = 0; c < NR; ++c) acc[c] = 0.0;
+    acc = 0.0;
 #pragma unroll
     for (int kk = 0; kk < 16; ++kk) {
       const int k = q * 16 + kk;
       const double a = TRANS ? T[r * CS + k] : T[k * CS + r];
-      if (forward ? k <= r : k >= r) {
-#pragma unroll
-        for (int c = 0; c < NR; ++c) acc[c] = fma(a, vs[k * NR + c], acc[c]);
-      }
+      if (forward ? k <= r : k >= r) acc = fma(a, vs[k], acc);
     }
-#pragma unroll
-    for (int c = 0; c < NR; ++c) part[q][r * NR + c] = acc[c];
+    part[q][r] = acc;
   }
   __syncthreads();
   if (mine) {
-    const int e = pi * NR + pc;
-    const double x = (part[0][e] + part[1][e]) + (part[2][e] + part[3][e]);
-    put_x(words + ((size_t)(c0 + pc) * n + r0 + pi) * 2, x, epoch);
-    if ((unsigned)drow < (unsigned)n) dst[drow + (long long)(c0 + pc) * ldd] = x;  // (an invalid IPIV writes nothing)
+    const double x = (part[0][r] + part[1][r]) + (part[2][r] + part[3][r]);
+    put_x(words + ((size_t)col * n + r0 + r) * 2, x, epoch);
+    if ((unsigned)drow < (unsigned)n) dst[drow + (long long)col * ldd] = x;  // (an invalid IPIV writes nothing)
   }
 }
 
-template <int NR, bool TRANS>
+template <bool TRANS>
 cudaError_t launch_chain(const double* A, long long lda, int n, bool forward, const double* D,
                          const double* src, long long lds, const int* gather, double* dst,
                          long long ldd, const int* scatter, const int* maps, int nrhs, int* ticket,
                          unsigned long long* words, uint32_t epoch, int* status, cudaStream_t s) {
   constexpr int smem = TRING * TSLOT * (int)sizeof(double);
-  auto kern = trsv64_chain_kernel<NR, TRANS>;
+  auto kern = trsv64_chain_kernel<TRANS>;
   static const cudaError_t attr = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   SL_TRY(attr);
-  const int ngroups = (nrhs + NR - 1) / NR;
-  kern<<<(n + TB - 1) / TB * ngroups, 256, smem, s>>>(A, lda, n, forward ? 1 : 0, D, src, lds, gather, dst,
-                                                      ldd, scatter, maps, nrhs, ngroups, ticket, words, epoch, status);
+  kern<<<(n + TB - 1) / TB * nrhs, 256, smem, s>>>(A, lda, n, forward ? 1 : 0, D, src, lds, gather, dst, ldd,
+                                                   scatter, maps, nrhs, ticket, words, epoch, status);
   count_launches(1);
   return cudaGetLastError();
 }
@@ -229,18 +214,8 @@ cudaError_t trsv64_chain(bool lower, bool trans, const double* A, long long lda,
                          long long ldd, const int* scatter, const int* maps, int nrhs, int* ticket,
                          unsigned long long* words, uint32_t epoch, int* status, cudaStream_t s) {
   const bool forward = lower != trans;
-  // two right-hand sides a CTA once one each would queue several CTAs per SM
-  const bool two = nrhs > 1 && (long long)((n + TB - 1) / TB) * nrhs > 2LL * num_sms();
-#define SL_CH(NR, TR)                                                                                 \
-  return launch_chain<NR, TR>(A, lda, n, forward, D, src, lds, gather, dst, ldd, scatter, maps, nrhs, ticket, \
-                              words, epoch, status, s)
-  if (two) {
-    if (trans) SL_CH(2, true);
-    SL_CH(2, false);
-  }
-  if (trans) SL_CH(1, true);
-  SL_CH(1, false);
-#undef SL_CH
+  auto launch = trans ? launch_chain<true> : launch_chain<false>;
+  return launch(A, lda, n, forward, D, src, lds, gather, dst, ldd, scatter, maps, nrhs, ticket, words, epoch, status, s);
 }
 
 }  // namespace sl

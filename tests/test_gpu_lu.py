@@ -562,3 +562,22 @@ def test_one_panel_rule_edges(sl, orc, gpu_required, m, n):
     low, up = np.tril(F[:, :k], -1) + np.eye(m, k), np.triu(F[:k])
     assert np.abs(low).max() <= 1.0 + 1e-15  # partial pivoting
     assert np.abs(PA - low @ up).max() < 16.0 * max(m, n) * 2.0**-53 * np.abs(A).sum(axis=1).max()
+
+
+@pytest.mark.parametrize("trans", ["N", "T"])
+@pytest.mark.parametrize("n,nrhs", [(1000, 128), (1000, 129), (2048, 128), (2049, 128), (4097, 64)])
+def test_solve_dispatch_edges(sl, gpu_required, n, nrhs, trans):
+    """Both sides of the number of right-hand sides up to which the solves are chained:
+    the tester's scaled residual of every column below 16."""
+    import torch
+
+    rng = np.random.default_rng(n + nrhs)
+    A, B = rng.uniform(-0.5, 0.5, (n, n)), rng.uniform(-0.5, 0.5, (n, nrhs))
+    dA, dB = torch.from_numpy(A.T.copy()).cuda(), torch.from_numpy(B.T.copy()).cuda()
+    ip = torch.zeros(n, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    assert sl.dgetrf_dev(n, n, dA.data_ptr(), n, ip.data_ptr()) == 0
+    assert sl.dgetrs_dev(trans, n, nrhs, dA.data_ptr(), n, ip.data_ptr(), dB.data_ptr(), n) == 0
+    X, op = dB.T.cpu().numpy(), A if trans == "N" else A.T
+    res = np.abs(op @ X - B).max(axis=0) / (np.abs(op).sum(axis=1).max() * np.abs(X).max(axis=0) * n * 2.0**-53)
+    assert (res < 16.0).all()
