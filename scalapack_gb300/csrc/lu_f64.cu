@@ -330,7 +330,8 @@ static cudaError_t solve_u12(int jb, int nr, const double* L11, long long ldl, d
 // each followed by its row interchanges on the rest of the panel, the U solve
 // and the GEMM update of the panel's remaining columns.
 static cudaError_t factor_panel(int m, int n, double* dA, long long ldda, int* dipiv, int j, int jb,
-                                const LuWork& ws, cudaStream_t s) {
+                                const LuWork& ws, cudaStream_t s, int left = -1) {
+  const int cb = left < 0 ? j : left;  // first column whose rows are interchanged
   auto Ap = [&](long long i, long long c) { return dA + i + c * ldda; };
   const OzScratch& sc = (ws.aux && s == ws.aux) ? ws.oz_aux : ws.oz;
   phase_begin(kPhPanel, s);
@@ -355,7 +356,7 @@ static cudaError_t factor_panel(int m, int n, double* dA, long long ldda, int* d
     phase_end(kPhPanelKernel, s, kflops, 16.0 * (double)(m - r0) * w);
     phase_begin(kPhPanelUpdate, s);
     if (c + w >= jb) {
-      SL_TRY(inpanel_step<double>(dA, ldda, r0, r0 + kw, dipiv, j, r0, r0 + w, j + jb, 0, kw, s));
+      SL_TRY(inpanel_step<double>(dA, ldda, r0, r0 + kw, dipiv, cb, r0, r0 + w, j + jb, 0, kw, s));
     } else {
       const bool block_end = (q + 1) % ib == 0 || kw < w;
       // columns brought up to date now: the next sub-panel's, or at the end
@@ -365,7 +366,7 @@ static cudaError_t factor_panel(int m, int n, double* dA, long long ldda, int* d
       const int kb = r0 + kw - blk_r0;
       const int rl = r0 + kw;  // first row below the block's pivot rows
       const bool fused = kb <= 64 && (kb - kw) % 32 == 0;  // (two sub-panels per block at most)
-      if (!fused) SL_TRY(laswp<double>(dA, ldda, r0, r0 + kw, dipiv, j, r0, r0 + w, j + jb, s));
+      if (!fused) SL_TRY(laswp<double>(dA, ldda, r0, r0 + kw, dipiv, cb, r0, r0 + w, j + jb, s));
       // (the block's earlier columns are read by the fused step: theirs first)
       else if (blk_r0 < r0) SL_TRY(laswp<double>(dA, ldda, r0, r0 + kw, dipiv, blk_r0, r0, r0, r0, s));
       // The solve also publishes the balancing keys of the product that
@@ -383,7 +384,7 @@ static cudaError_t factor_panel(int m, int n, double* dA, long long ldda, int* d
         kj.lcols = kb;
       }
       if (fused)
-        SL_TRY(inpanel_step<double>(dA, ldda, r0, r0 + kw, dipiv, j, blk_r0, r0 + w, j + jb, ncols, kb, s, kj));
+        SL_TRY(inpanel_step<double>(dA, ldda, r0, r0 + kw, dipiv, cb, blk_r0, r0 + w, j + jb, ncols, kb, s, kj));
       else
         SL_TRY((trsm_strip<double, false, false, true>(kb, ncols, Ap(blk_r0, blk_r0), ldda,
                                                         Ap(blk_r0, r0 + w), ldda, s, kj)));
@@ -491,6 +492,15 @@ static cudaError_t step0_by_chunks(int m, int n, double* dA, long long ldda, int
   return wait_cols(INT_MAX);
 }
 
+// The last columns of a factorization as one panel, as small matrices are (the
+// launches of a block beside its panel cost more than the wider products), their
+// interchanges applied to the `left` columns before them by the in-panel steps. In us,
+// without / with: N = 1600 4519 / 4229, N = 2000 5746 / 5454 (up to 1536 columns: 5510),
+// N = 3000 9198 / 8923, N = 4096 13210 / 13148, N = 8192 no difference.
+static bool one_panel_tail(int m, int n, int left) {
+  return n <= 1024 && left <= 4096 && ((m + 127LL) / 128) * ((n + 63) / 64) <= 2LL * num_sms();
+}
+
 // Right-looking blocked LU. With look-ahead resources in `ws`, the panel of
 // step j+1 is factored on ws.aux while the trailing update of step j runs on
 // s: the columns of the next panel are updated first (event ev_next), the
@@ -558,7 +568,9 @@ cudaError_t dgetrf_device(int m, int n, double* dA, long long ldda, int* dipiv, 
     panel_on_aux = false;
     const int jn = j + jb;                                   // next panel's first column
     const int jb2 = jn < mn ? ((mn - jn) < nb ? (mn - jn) : nb) : 0;
-    if (split && jb2 > 0) {
+    const bool tail = nb < n && n <= m && jn < n && n - jn > jb2 && g_f64_update == 1 &&
+                      one_panel_tail(m - jn, n - jn, jn) && oz_fits(ws.oz, m - jn, n - jn, nb);
+    if (split && jb2 > 0 && !tail) {
       const double mr = (double)(m - jn);
       // panel j, and every update of the caller's stream before it
       SL_TRY(cudaEventRecord(ws.ev_next, s));
@@ -615,7 +627,7 @@ cudaError_t dgetrf_device(int m, int n, double* dA, long long ldda, int* dipiv, 
       // ---- PDGEMM: A22 -= L21 * U12 ----
       if (jn < m) {
         const double mr = (double)(m - jn);
-        if (lookahead && jb2 > 0) {
+        if (lookahead && jb2 > 0 && !tail) {
           // next panel's columns first, then the panel on the look-ahead stream
           phase_begin(kPhGemm, s);
           SL_TRY(lu_update(ws.oz, m - jn, jb2, jb, -1.0, Ap(jn, j), ldda, Ap(j, jn), ldda,
@@ -641,6 +653,10 @@ cudaError_t dgetrf_device(int m, int n, double* dA, long long ldda, int* dipiv, 
           phase_end(kPhGemm, s, 2.0 * mr * nr * jb, 8.0 * (mr * jb + jb * nr + 2.0 * mr * nr));
         }
       }
+    }
+    if (tail) {
+      SL_TRY(factor_panel(m, n, dA, ldda, dipiv, jn, n - jn, ws, s, 0));
+      break;
     }
     if (jb2 > 0 && !panel_on_aux) SL_TRY(factor_panel(m, n, dA, ldda, dipiv, jn, jb2, ws, s));
   }

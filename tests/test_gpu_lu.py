@@ -581,3 +581,25 @@ def test_solve_dispatch_edges(sl, gpu_required, n, nrhs, trans):
     X, op = dB.T.cpu().numpy(), A if trans == "N" else A.T
     res = np.abs(op @ X - B).max(axis=0) / (np.abs(op).sum(axis=1).max() * np.abs(X).max(axis=0) * n * 2.0**-53)
     assert (res < 16.0).all()
+
+
+@pytest.mark.parametrize("m,n", [(1792, 1792), (1793, 1793), (2000, 1700), (5120, 5120), (5121, 5121)])
+def test_tail_as_one_panel_edges(sl, gpu_required, m, n):
+    """The last columns as one panel that also interchanges the rows of the columns
+    before it: widths and left parts on both sides of its limits. P A = L U to the
+    tester's bound over every column."""
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    A = torch.rand((n, m), dtype=torch.float64, device="cuda", generator=g) - 0.5  # column-major m x n
+    dA, ip = A.clone(), torch.zeros(n, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    assert sl.dgetrf_dev(m, n, dA.data_ptr(), m, ip.data_ptr()) == 0
+    perm = np.arange(m)
+    for k, p in enumerate(ip.cpu().numpy() - 1):
+        perm[[k, p]] = perm[[p, k]]
+    low = torch.tril(dA.T, -1)
+    assert low.abs().max().item() <= 1.0 + 1e-15  # partial pivoting
+    low.diagonal().fill_(1.0)
+    res = A.T[torch.from_numpy(perm).cuda()] - low @ torch.triu(dA.T[:n])
+    assert res.abs().max().item() < 16.0 * m * 2.0**-53 * A.T.abs().sum(dim=1).max().item()
