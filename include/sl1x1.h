@@ -278,7 +278,9 @@ int sl1x1_dgerfs_dev(char trans, int n, int nrhs, const double* dA, long long ld
 /* ---- Library control ----------------------------------------------------- */
 /* Free every device buffer the library holds (also done by blacs_exit_). */
 void sl1x1_finalize(void);
-/* Block size NB used by the device entry points when nb <= 0 (default 256). */
+/* Block size NB used by the device entry points when nb <= 0 (default 256).
+ * With the sliced update the FP64 factorization chooses its own width whatever
+ * NB is: the whole matrix up to 1536 columns, 256 columns beyond. */
 void sl1x1_set_default_nb(int nb);
 /* Look-ahead in the factorizations (default on): the next panel is factored
  * on a second stream while the trailing update runs. Same pivots (except
@@ -342,8 +344,9 @@ void sl1x1_set_panel_rows(int rows);
  * applies. Changes only the speed, not the results. */
 void sl1x1_set_panel_ctas(int ctas);
 /* 32-column sub-panels per in-panel block of the FP64 panel factorization
- * (1..8; 0, the default: 1 for panels of up to 5000 rows, else 2): inside a block only the next sub-panel's columns are
- * updated after each sub-panel, the columns beyond the block once at its end.
+ * (1..8; 0, the default: 1 for panels of up to 5000 rows, else 2): inside a
+ * block only the next sub-panel's columns are updated after each sub-panel,
+ * the columns beyond the block once at its end.
  * Same pivots except where candidates tie to rounding; factors equal to
  * rounding. */
 void sl1x1_set_panel_ib(int subpanels);
@@ -356,8 +359,9 @@ void sl1x1_set_lowp_stages(int stages);
  * SRC/pdgetrf.f:288-290): 1 (default) = the product formed exactly on the
  * BF16 tensor cores (tcgen05) from 8-bit integer slices of the operands (7
  * balanced base-256 digits, row and column power-of-two scales, the leading
- * diagonals of the slice products summed exactly as integers), accurate to a few units of 2^-53 of
- * max|L21(i,:)| max|U12(:,j)| and independent of the summation order; 0 =
+ * diagonals of the slice products summed exactly as integers), accurate to a
+ * few units of 2^-53 of max|L21(i,:)| max|U12(:,j)| and independent of the
+ * summation order; 0 =
  * FP64 DMMA (mma.sync m16n8k4). The sliced form needs device scratch of about
  * 4 KB per row plus 4 KB per column of the matrix; where it cannot be had
  * (sl1x1_dgetrf_noalloc) the DMMA form runs. */

@@ -58,10 +58,10 @@ static int g_panel_min_rows = 0;  // 0: automatic (FP32 256, FP64 128)
 int panel_min_rows() { return g_panel_min_rows; }
 static int g_panel_ctas = 64;  // CTAs a panel's rows are spread over (before the minimum rows)
 // Sub-panels per in-panel block (factor_panel); 0: one up to 5000 rows, where a
-// block's second step costs a launch more than its deeper products save (PDGESV N
-// = 600 2.00 ms with one, 2.11 with two; N = 4096 16.0, 16.6), two above (N = 8192
-// 36.8, 37.5, but a rounding less per element; N = 16384 127.4, 125.8: the update
-// beside the panel leaves it few SMs).
+// block's second step costs a launch more than its deeper products save (PDGESV, ms,
+// one / two: N = 600 1.47 / 1.63, N = 4096 13.7 / 14.5), two above, where the time is
+// about the same (N = 8192 32.9 / 34.0, N = 16384 119.1 / 119.2: the update beside the
+// panel leaves it few SMs) and an element takes half as many roundings.
 static int g_panel_ib = 0;
 void set_panel_ib(int ib) { g_panel_ib = ib < 1 ? 0 : (ib > 8 ? 8 : ib); }
 int panel_ctas() { return g_panel_ctas; }

@@ -72,7 +72,7 @@
 // entries cross (row i large at k1 only, column j large at k2 only) keep the
 // normwise bound but not a componentwise one.
 //
-// Structure (one CTA per SM, a few 128 x 64 tiles of C per CTA, 10 warps):
+// Structure (one CTA per SM, a few 128 x 64 tiles of C per CTA, 18 warps):
 //   * warp 0 allocates all 512 TMEM columns (7 accumulators x 64 columns);
 //   * one thread issues TMA loads: for each 64-wide k block, the seven 128x64
 //     A slices one at a time through a 7-deep ring and the seven 64x64 B
@@ -88,11 +88,12 @@
 // Every mbarrier wait is bounded; on timeout the CTA records kFlagTimeout,
 // drains what it issued, frees its TMEM and returns.
 //
-// Bound: a tile's products take 14300 cycles of the tensor pipe; it takes 23500
-// (m = n = 16384, k = 256): its 672 KB of slices come from L2 at 8.3 TB/s, and
-// the read-out of the accumulators (3000) is not overlapped. Measured there:
-// 3.28 ms, 42 TFLOP/s FP64-equivalent; with 36 products of 7-bit slices, three
-// FP64-rate operations per element and descriptors computed per instruction,
+// Bound: a tile's products take 14300 cycles of the tensor pipe; it takes 30000 (m =
+// n = 6144 .. 16384, k = 256), 3000 of them the read-out of the accumulators, which
+// is not overlapped; the rest is no throughput (L2 at 9.9 TB/s, but a third less of
+// it by multicast to two CTAs takes as long; shared-memory banks 39 %). Measured, m =
+// n = 16384: 3.3 ms, 42 TFLOP/s FP64-equivalent; with 36 products of 7-bit slices,
+// three FP64-rate operations per element and descriptors computed per instruction,
 // 5.0 ms. 128 x 64 tiles of 8192 x 256 x 256: 47 us (72 before).
 #include <cuda.h>
 #include <cuda_bf16.h>
