@@ -344,7 +344,7 @@ void sl1x1_set_panel_rows(int rows);
  * applies. Changes only the speed, not the results. */
 void sl1x1_set_panel_ctas(int ctas);
 /* 32-column sub-panels per in-panel block of the FP64 panel factorization
- * (1..8; 0, the default: 1 for panels of up to 5000 rows, else 2): inside a
+ * (1..8; 0, the default: 1 for panels of up to 12000 rows, else 2): inside a
  * block only the next sub-panel's columns are updated after each sub-panel,
  * the columns beyond the block once at its end.
  * Same pivots except where candidates tie to rounding; factors equal to

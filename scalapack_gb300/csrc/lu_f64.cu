@@ -57,11 +57,12 @@ void set_spin_limit(long long polls) { g_spin_limit = polls < 0 ? kSpinLimit : p
 static int g_panel_min_rows = 0;  // 0: automatic (FP32 256, FP64 128)
 int panel_min_rows() { return g_panel_min_rows; }
 static int g_panel_ctas = 64;  // CTAs a panel's rows are spread over (before the minimum rows)
-// Sub-panels per in-panel block (factor_panel); 0: one up to 5000 rows, where a
-// block's second step costs a launch more than its deeper products save (PDGESV, ms,
-// one / two: N = 600 1.47 / 1.63, N = 4096 13.7 / 14.5), two above, where the time is
-// about the same (N = 8192 32.9 / 34.0, N = 16384 119.1 / 119.2: the update beside the
-// panel leaves it few SMs) and an element takes half as many roundings.
+// Sub-panels per in-panel block (factor_panel); 0: one up to 12000 rows, where a
+// block's second step costs a launch more than its deeper products save, two above,
+// where the products are what takes the time. PDGETRF, ms, one / two: N = 4096 13.2 /
+// 14.0, 6001 x 3007 11.1 / 11.7, N = 8192 31.7 / 32.7, N = 12000 61.6 / 62.6; 20000 x
+// 4000 28.2 / 27.4, 30000 x 1000 8.2 / 7.6.
+constexpr int kDeepPanelRows = 12000;
 static int g_panel_ib = 0;
 void set_panel_ib(int ib) { g_panel_ib = ib < 1 ? 0 : (ib > 8 ? 8 : ib); }
 int panel_ctas() { return g_panel_ctas; }
@@ -342,7 +343,7 @@ static cudaError_t factor_panel(int m, int n, double* dA, long long ldda, int* d
   // columns beyond the block once at its end, with the block's rows -- fewer,
   // deeper in-panel products than one per sub-panel over all the remaining
   // columns.
-  const int ib = g_panel_ib > 0 ? g_panel_ib : (m - j <= 5000 ? 1 : 2);
+  const int ib = g_panel_ib > 0 ? g_panel_ib : (m - j <= kDeepPanelRows ? 1 : 2);
   int blk_r0 = j;  // first row (= column) of the current block
   for (int c = 0, q = 0; c < jb; c += PW, ++q) {
     const int w = (jb - c) < PW ? (jb - c) : PW;

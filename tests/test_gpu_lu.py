@@ -338,9 +338,9 @@ def test_scratch_on_reused_dirty_memory(sl, orc, ctx, n, nb):
 @pytest.mark.parametrize("trans", ["N", "T"])
 @pytest.mark.parametrize("n,nrhs", [(1, 1), (63, 2), (64, 1), (65, 16), (129, 3), (200, 17), (1300, 16), (2500, 5)])
 def test_chained_solve_edges(sl, gpu_required, n, nrhs, trans):
-    """PDGETRS over the edges of the chained solve: blocks of 64 rows, one or two
-    right-hand sides per CTA (1300 x 16, 2500 x 5), the blocked solves beyond
-    16; padded leading dimensions, untouched padding."""
+    """PDGETRS over the edges of the chained solve: blocks of 64 rows, one
+    to many CTAs per SM (1300 x 16, 2500 x 5); padded leading dimensions,
+    untouched padding."""
     import torch
 
     rng = np.random.default_rng(n + nrhs)
