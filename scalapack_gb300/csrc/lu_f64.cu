@@ -755,6 +755,7 @@ solve_prep_kernel(int n, const double* __restrict__ A, long long lda, double* D,
     *status = 0;
     if (tickets) tickets[0] = tickets[1] = 0;
   }
+  launch_dependents();
   if (b < 0)
     perm_segment(blockIdx.x, ipiv, n, maps, reinterpret_cast<int*>(inv_smem));
   else if (blk < nb64) tri_inv64_of<true>(blk, part, n, A, lda, D, inv_smem);
