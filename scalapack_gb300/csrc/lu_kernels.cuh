@@ -545,9 +545,13 @@ panel_kernel(T* A, long long lda, int m, int r0, int c0, int w, int rpc, int* ip
 // FP32, R = 4096: 1.4 (2.1). Three
 // inboxes: column k's pivot row is read until column k+1 has been sent for, so a
 // CTA may be sent column k+2's while it still reads column k's, but not k+3's.
-// Waits are bounded (spin_limit polls); a CTA that gives up goes on to the
-// cluster barrier at the end, which keeps its shared memory in place until all
-// have stopped sending.
+// Waits are bounded (spin_limit polls). A warp that gives up at column k raises the
+// column parity's flag, which is read only after the barrier of column k+1, when no
+// warp can still write it: all of a CTA's warps stop at the same column. The CTAs
+// may stop one column apart; each tells the others how many columns it has sent, and
+// after the cluster barrier the ones behind send the missing column (its content is
+// not used), so that every message has its count of bytes and can be waited for
+// before shared memory goes.
 constexpr int CMAXG = 16;
 template <typename T>
 struct PanelInbox {
@@ -584,7 +588,8 @@ panel_cluster_kernel(T* A, long long lda, int m, int r0, int c0, int w, int rpc,
   __shared__ __align__(8) unsigned long long s_bar[3];
   __shared__ long long s_wk[2][NW];
   __shared__ int s_wr[2][NW], s_wl[2][NW];
-  __shared__ int s_fail;
+  __shared__ int s_fail[2];       // a wait gave up, by column parity
+  __shared__ int s_sent[CMAXG];   // 2 x columns each CTA has sent, + 1 if it gave up
 
   const int CS = gridDim.x, b = blockIdx.x, tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
@@ -595,8 +600,9 @@ panel_cluster_kernel(T* A, long long lda, int m, int r0, int c0, int w, int rpc,
   const int nr = max(0, min(rpc, R - lo));
   const uint32_t bar0 = (uint32_t)__cvta_generic_to_shared(s_bar);
   const uint32_t in0 = (uint32_t)__cvta_generic_to_shared(inbox);
+  if (tid < CMAXG) s_sent[tid] = 2 * kw;
   if (tid == 0) {
-    s_fail = 0;
+    s_fail[0] = s_fail[1] = 0;
     for (int i = 0; i < 3; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0 + 8 * i));
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -656,21 +662,71 @@ panel_cluster_kernel(T* A, long long lda, int m, int r0, int c0, int w, int rpc,
     row[j] = fma(-l, u, v);
   };
 
+  // column c of a CTA: bytes that each CTA receives from all of them
+  const uint32_t col_bytes = (uint32_t)(CS * (16 + (sizeof(T) == 8 ? 8 : 0) + PW * sizeof(T)));
+  auto expect_column = [&](int c) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar0 + 8 * (c % 3)), "r"(col_bytes)
+                 : "memory");
+  };
+  // one warp sends this CTA's candidate of column c (its key, label and row) to every
+  // CTA's inbox, and for FP64 one warp the reciprocal of its magnitude
+  auto send_candidate = [&](int c, long long ckey, long long clabel, T v) {
+    const int buf = c % 3;
+    const uint32_t slot = in0 + (uint32_t)((buf * CMAXG + b) * sizeof(PanelInbox<T>));
+    if (lane < CS)
+      asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];" ::"r"(
+                       cluster_addr(slot, lane)),
+                   "l"(ckey), "l"(clabel), "r"(cluster_addr(bar0 + 8 * buf, lane))
+                   : "memory");
+    const uint32_t mine = slot + 32 + (uint32_t)(lane * sizeof(T));
+    for (int q = 0; q < CS; ++q) {
+      const uint32_t dst = cluster_addr(mine, q), bar = cluster_addr(bar0 + 8 * buf, q);
+      if constexpr (sizeof(T) == 8)
+        asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(dst),
+                     "l"(__double_as_longlong(v)), "r"(bar)
+                     : "memory");
+      else
+        asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(dst),
+                     "r"(__float_as_uint(v)), "r"(bar)
+                     : "memory");
+    }
+  };
+  auto send_reciprocal = [&](int c, double ra) {
+    const int buf = c % 3;
+    const uint32_t slot = in0 + (uint32_t)((buf * CMAXG + b) * sizeof(PanelInbox<T>));
+    if (lane < CS)
+      asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(
+                       cluster_addr(slot + 16, lane)),
+                   "l"(__double_as_longlong(ra)), "r"(cluster_addr(bar0 + 8 * buf, lane))
+                   : "memory");
+  };
+  // at most `polls` looks at whether column c of every CTA is here
+  auto column_here = [&](int c, long long polls) {
+    for (long long spins = 0; spins < polls; ++spins) {
+      uint32_t done;
+      asm volatile(
+          "{\n .reg .pred p;\n mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+          " selp.u32 %0, 1, 0, p;\n}\n"
+          : "=r"(done)
+          : "r"(bar0 + 8 * (c % 3)), "r"((uint32_t)((c / 3) & 1))
+          : "memory");
+      if (done) return true;
+    }
+    return false;
+  };
+
   const T* Uprev = nullptr;  // pivot row of column k-1
-  int k = 0;
+  int k = 0;                 // columns sent
   for (; k < kw; ++k) {
     const int buf = k % 3, par = k & 1;
     __syncthreads();
-    if (s_fail) break;
+    if (k > 0 && s_fail[par ^ 1]) break;
     // --- this CTA's candidate, into every CTA's inbox ---
     long long key = lane < NW ? s_wk[par][lane] : -3;
     int label = lane < NW ? s_wr[par][lane] : INT_MAX;
     const int cw = warp_best(key, label);
     const int lrow = s_wl[par][cw];
-    if (tid == 0)
-      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar0 + 8 * buf),
-                   "r"((uint32_t)(CS * (16 + (sizeof(T) == 8 ? 8 : 0) + PW * sizeof(T))))
-                   : "memory");
+    if (tid == 0) expect_column(k);
     if (warp == cw) {
       // the candidate row with column k-1's update of its columns beyond k
       T v = (T)0;
@@ -678,26 +734,7 @@ panel_cluster_kernel(T* A, long long lda, int m, int r0, int c0, int w, int rpc,
         v = tile[lrow * PLD + lane];
         if (k > 0 && lane > k) v = fma(-tile[lrow * PLD + k - 1], Uprev[lane], v);
       }
-      const uint32_t slot = in0 + (uint32_t)((buf * CMAXG + b) * sizeof(PanelInbox<T>));
-      const long long ck = s_wk[par][cw];
-      const long long cl = s_wr[par][cw];
-      if (lane < CS)
-        asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];" ::"r"(
-                         cluster_addr(slot, lane)),
-                     "l"(ck), "l"(cl), "r"(cluster_addr(bar0 + 8 * buf, lane))
-                     : "memory");
-      const uint32_t mine = slot + 32 + (uint32_t)(lane * sizeof(T));
-      for (int q = 0; q < CS; ++q) {
-        const uint32_t dst = cluster_addr(mine, q), bar = cluster_addr(bar0 + 8 * buf, q);
-        if constexpr (sizeof(T) == 8)
-          asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(dst),
-                       "l"(__double_as_longlong(v)), "r"(bar)
-                       : "memory");
-        else
-          asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(dst),
-                       "r"(__float_as_uint(v)), "r"(bar)
-                       : "memory");
-      }
+      send_candidate(k, s_wk[par][cw], s_wr[par][cw], v);
       __syncwarp();  // (the row is read before its owner goes on)
     }
     if (exch) {
@@ -705,34 +742,17 @@ panel_cluster_kernel(T* A, long long lda, int m, int r0, int c0, int w, int rpc,
         // 1/|candidate| on the integer pipe while the rows are updated: 450
         // cycles that every thread would otherwise wait for after the exchange
         const unsigned long long kb = (unsigned long long)s_wk[par][cw];
-        const double ra = kb - 1ULL < 0x7FEFFFFFFFFFFFFFULL ? recip_bits(kb) : 0.0;
-        const uint32_t slot = in0 + (uint32_t)((buf * CMAXG + b) * sizeof(PanelInbox<T>));
-        if (lane < CS)
-          asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(
-                           cluster_addr(slot + 16, lane)),
-                       "l"(__double_as_longlong(ra)), "r"(cluster_addr(bar0 + 8 * buf, lane))
-                       : "memory");
+        send_reciprocal(k, kb - 1ULL < 0x7FEFFFFFFFFFFFFFULL ? recip_bits(kb) : 0.0);
       }
     } else if (k > 0) {
       finish_update(k - 1, Uprev);
     }
     // --- every CTA's candidate is here: the winner, U(k, :) and 1/pivot ---
-    bool ok = false;
-    for (long long spins = 0; spins < 8 * spin_limit; ++spins) {  // (a poll here takes an eighth of one in L2)
-      uint32_t done;
-      asm volatile(
-          "{\n .reg .pred p;\n mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
-          " selp.u32 %0, 1, 0, p;\n}\n"
-          : "=r"(done)
-          : "r"(bar0 + 8 * buf), "r"((uint32_t)((k / 3) & 1))
-          : "memory");
-      if (done) { ok = true; break; }
-    }
-    ok = __all_sync(0xffffffffu, ok);
-    if (!ok) {
+    // (a poll here takes an eighth of one in L2)
+    if (!__all_sync(0xffffffffu, column_here(k, 8 * spin_limit))) {
       if (lane == 0) {
         atomicExch(status, (int)kFlagTimeout);
-        s_fail = 1;
+        s_fail[par] = 1;
       }
       continue;
     }
@@ -784,10 +804,15 @@ panel_cluster_kernel(T* A, long long lda, int m, int r0, int c0, int w, int rpc,
   }
   launch_dependents();
   __syncthreads();
-  if (s_fail) {
+  if (s_fail[0] | s_fail[1]) {
     // pivots from the first one that was not chosen become the diagonal rows
     if (b == 0)
       for (int q = max(k - 1, 0) + tid; q < kw; q += NTR + 32) ipiv[c0 + q] = r0 + q;
+    if (tid < CS)
+      asm volatile("st.relaxed.cluster.shared::cluster.b32 [%0], %1;" ::"r"(
+                       cluster_addr((uint32_t)__cvta_generic_to_shared(s_sent) + 4 * b, tid)),
+                   "r"(2 * k + 1)
+                   : "memory");
   } else {
     if (kw > 0) finish_update(kw - 1, Uprev);
     if (part == 0 && row0 < nr) lab[row0] = mylab;
@@ -806,7 +831,23 @@ panel_cluster_kernel(T* A, long long lda, int m, int r0, int c0, int w, int rpc,
       }
     }
   }
-  if (s_fail) __nanosleep(20000);  // what was sent before the others stopped has landed
+  cluster_sync();
+  int most = 0, gave_up = 0;
+  for (int q = 0; q < CS; ++q) {
+    most = max(most, s_sent[q] >> 1);
+    gave_up |= s_sent[q] & 1;
+  }
+  if (!gave_up) return;  // every CTA has received all columns
+  // (every CTA reads the same counts) complete what was begun, and wait for what this
+  // CTA was sent before its shared memory goes
+  if (warp == 0)
+    for (int c = s_sent[b] >> 1; c < most; ++c) {
+      if (lane == 0) expect_column(c);
+      send_candidate(c, 0, 0, (T)0);
+      if constexpr (sizeof(T) == 8) send_reciprocal(c, 0.0);
+    }
+  __syncthreads();
+  for (int c = max(0, most - 3); c < most; ++c) column_here(c, kSpinLimit);
   cluster_sync();
 }
 

@@ -136,3 +136,32 @@ def test_panel_wait_runs_out_and_library_recovers(sl, orc, ctx, polls):
     bad, _ = compare_ipiv(orc, A0, ipiv[:n], nb)
     assert bad == 0
     assert orc.sresid(A0, B0, X) < RESID_THRESH
+
+
+def _recovers(sl, orc, ctx, n, nrhs, nb, polls, repeats):
+    """Calls with a poll limit of `polls` return INFO 0 or -20002 (always the latter
+    with none allowed), and the next call with the default limit is right."""
+    from lu_helpers import compare_ipiv, run_pdgesv
+
+    A0, B0 = system(orc, n, nrhs)
+    L = sl.lib()
+    try:
+        L.sl1x1_debug_set_spin_limit(polls)
+        for _ in range(repeats):
+            info, _ = _pdgesv(sl, ctx, A0, B0, nb)
+            assert info == -20002 if polls == 0 else info in (-20002, 0)
+    finally:
+        L.sl1x1_debug_set_spin_limit(-1)
+    info, _, ipiv, X = run_pdgesv(sl, ctx, A0, B0, nb)
+    assert info == 0
+    bad, _ = compare_ipiv(orc, A0, ipiv, nb)
+    assert bad == 0
+    assert orc.sresid(A0, B0, X) < RESID_THRESH
+
+
+@pytest.mark.parametrize("polls", [0, 1, 2, 4, 16])
+@pytest.mark.parametrize("n", [33, 40, 520, 1500])
+def test_cluster_panel_gives_up_whole(sl, orc, ctx, n, polls):
+    """Panels of 2, 4 and 16 CTAs of one cluster whose waits run out, at different
+    warps and columns: every CTA stops as a whole and the cluster ends."""
+    _recovers(sl, orc, ctx, n, 1, 64, polls, 8)
