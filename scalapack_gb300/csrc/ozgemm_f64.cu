@@ -379,8 +379,9 @@ ozgemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
   const int nkc = kpad / OBK;
   const int total = my_tiles * nkc;  // chunks of this CTA
   __shared__ int s_fail, s_aiss, s_acons, s_biss, s_bcons;
-  // a CTA that timed out already marked the launch failed: skip the work
-  if (*(volatile int*)status != 0) return;
+  // a CTA that timed out already marked the launch failed: skip the work (the word may
+  // be written meanwhile, by the other stream too: the block decides as one)
+  if (__syncthreads_or(*(volatile int*)status != 0)) return;
   // the slicing found the pass outside the error budget: FP64 route
   if (*(volatile const unsigned long long*)(kinfo + OZ_KI_FLAG) == epoch) {
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&g_oz_fp64_routes, 1ULL);
@@ -894,7 +895,7 @@ oz_tile_kernel(const double* A, long long lda, int m, const double* B, long long
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   wait_for_previous();
   launch_dependents();
-  if (*(volatile int*)status != 0) return;  // an earlier wait gave up
+  const int failed = *(volatile int*)status != 0;  // an earlier wait gave up
   const int tiles_m = (m + OBM - 1) / OBM, tiles_n = (n + OBN - 1) / OBN;
   int m0, n0;
   oz_tile(blockIdx.x, tiles_m, tiles_n, m0, n0);
@@ -929,9 +930,14 @@ oz_tile_kernel(const double* A, long long lda, int m, const double* B, long long
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
-  __syncthreads();
+  const int skip = __syncthreads_or(failed);  // (threads may have read different words)
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = s_tmem;
+  if (skip) {
+    if (warp == 0)
+      asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(OZ_TMEM_COLS));
+    return;
+  }
 
   // scales: e_i over the row's four k ranges, f_j over the column's eight
   int f = OZ_NOEXP, G = OZ_NOEXP;

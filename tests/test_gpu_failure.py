@@ -165,3 +165,39 @@ def test_cluster_panel_gives_up_whole(sl, orc, ctx, n, polls):
     """Panels of 2, 4 and 16 CTAs of one cluster whose waits run out, at different
     warps and columns: every CTA stops as a whole and the cluster ends."""
     _recovers(sl, orc, ctx, n, 1, 64, polls, 8)
+
+
+@pytest.mark.parametrize("polls", [0, 1, 8, 64])
+def test_products_beside_a_panel_that_gives_up(sl, orc, ctx, polls):
+    """With the look-ahead the products on the other stream meet the status word while
+    it changes: blocks of both product kernels leave as a whole. At 2600 rows the first
+    panels exchange through L2 (panel_kernel), the later ones within a cluster."""
+    _recovers(sl, orc, ctx, 2600, 1, 256, polls, 4)
+
+
+@pytest.mark.parametrize("n,polls", [(700, 0), (700, 2), (3000, 0), (3000, 2), (9000, 0)])
+def test_mixed_panel_gives_up(sl, orc, ctx, n, polls):
+    """The FP32 panel's waits (a cluster up to 8192 rows, through L2 beyond), and
+    those of the FP64 factorization that it falls back to."""
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(n)
+    A = torch.rand((n, n), dtype=torch.float64, device="cuda", generator=g).sub_(0.5)
+    B = torch.rand((1, n), dtype=torch.float64, device="cuda", generator=g).sub_(0.5)
+    X = torch.zeros_like(B)
+    piv = torch.zeros(n, dtype=torch.int32, device="cuda")
+
+    def run():
+        torch.cuda.synchronize()
+        return sl.dgesv_ir_dev(n, 1, A.data_ptr(), n, piv.data_ptr(), B.data_ptr(), n, X.data_ptr(), n,
+                               fmt="bf16x3", nb=256, keep_a=True)[0]
+
+    try:
+        sl.lib().sl1x1_debug_set_spin_limit(polls)
+        info = run()
+        assert info == -20002 if polls == 0 else info in (-20002, 0)
+    finally:
+        sl.lib().sl1x1_debug_set_spin_limit(-1)
+    assert run() == 0
+    r = (B - X @ A).abs().max()
+    assert r / (A.abs().sum(0).max() * X.abs().max() * n * 2.0**-53) < RESID_THRESH
