@@ -331,7 +331,9 @@ void sl1x1_set_inpanel_cap(int mask);
  * first poll). A panel that gives up records a device timeout, writes the
  * identity for the pivots it has not chosen and returns; the call then
  * returns INFO = -20002 and the library stays usable. No counterpart in the
- * reference, whose panel has no device waits. */
+ * reference, whose panel has no device waits. The chained solves of PDGETRS
+ * take the same limit for their waits on the blocks before (INFO = -20002,
+ * B is then undefined). */
 void sl1x1_debug_set_spin_limit(long long polls);
 /* Smallest row slice per CTA of the cooperative panel kernel (8..768; 0, the
  * default, picks 256 rows for the FP32 panel and 128 for the FP64 one, with

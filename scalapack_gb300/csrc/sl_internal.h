@@ -204,7 +204,7 @@ int panel_cluster_rows();
 void set_panel_ib(int ib);
 void set_panel_ctas(int g);
 void set_panel_min_rows(int rows);
-// Polls a panel CTA makes for another CTA's published words before it gives
+// Polls a CTA of a panel or a chained solve makes for another CTA's words before it gives
 // up (kSpinLimit by default; a test lowers it to make the waits run out).
 long long spin_limit();
 void set_spin_limit(long long polls);

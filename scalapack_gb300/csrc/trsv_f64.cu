@@ -5,7 +5,9 @@
 // Work is cut into 64-row blocks of op(T) times right-hand sides; each CTA takes
 // the next (block, right-hand side) in solve order from an atomic ticket,
 // so every block it depends on belongs to a CTA that has already started and
-// the waits always end (no residency assumption). A CTA streams its 64x64
+// the waits always end (no residency assumption); each is bounded all the same
+// (spin_limit polls), and a CTA that gives up sets the status word, at which the
+// CTAs after it leave at once. A CTA streams its 64x64
 // blocks of the factor through a ring in shared memory with cp.async, ahead of
 // the solutions it needs; solved values are published as single-copy atomic
 // 16-byte words {x, epoch}, so a consumer polls the data itself (one L2 round
@@ -76,7 +78,7 @@ trsv64_chain_kernel(const double* __restrict__ A, long long lda, int n, int forw
                     const double* __restrict__ D, const double* __restrict__ src, long long lds,
                     const int* __restrict__ gather, double* dst, long long ldd,
                     const int* __restrict__ scatter, const int* __restrict__ maps, int nrhs,
-                    int* ticket, unsigned long long* words, uint32_t epoch, int* status) {
+                    int* ticket, unsigned long long* words, uint32_t epoch, int* status, long long spin_limit) {
   extern __shared__ double trsv_ring[];  // TRING tiles
   __shared__ double xs[2][TB];           // solution of the block being applied
   __shared__ double part[4][TB];
@@ -135,12 +137,14 @@ trsv64_chain_kernel(const double* __restrict__ A, long long lda, int n, int forw
   double acc = 0.0;
   for (int t = 0; t < sidx; ++t) {
     const int k0 = (forward ? t : nblk - 1 - t) * TB;
+    int fail = 0;
     if (tid < TB) {
       double v = 0.0;
       if (k0 + r < n) {
         const unsigned long long* p = words + ((size_t)col * n + k0 + r) * 2;
-        for (long long spins = 0; !get_x(p, epoch, v);) {
-          if (++spins > kSpinLimit) { s_fail = 1; break; }
+        for (long long spins = 0;; ++spins) {
+          if (spins >= spin_limit) { fail = 1; break; }
+          if (get_x(p, epoch, v)) break;
           // far from its turn a CTA leaves the L2 to the ones that are next
           if (sidx - t > 2) __nanosleep(200);
         }
@@ -148,8 +152,7 @@ trsv64_chain_kernel(const double* __restrict__ A, long long lda, int n, int forw
       xs[t & 1][r] = v;
     }
     cp_wait<TRING - 2>();
-    __syncthreads();
-    if (s_fail) {
+    if (__syncthreads_or(fail)) {  // (the CTA gives up as a whole)
       if (tid == 0) atomicExch(status, (int)kFlagTimeout);
       cp_wait<0>();
       return;
@@ -206,7 +209,7 @@ cudaError_t launch_chain(const double* A, long long lda, int n, bool forward, co
   SL_TRY(attr);
   count_launches(1);
   return launch_after(kern, dim3((n + TB - 1) / TB * nrhs), 256, smem, s, A, lda, n, forward ? 1 : 0, D, src, lds, gather,
-                      dst, ldd, scatter, maps, nrhs, ticket, words, epoch, status);
+                      dst, ldd, scatter, maps, nrhs, ticket, words, epoch, status, spin_limit());
 }
 
 }  // namespace

@@ -201,3 +201,38 @@ def test_mixed_panel_gives_up(sl, orc, ctx, n, polls):
     assert run() == 0
     r = (B - X @ A).abs().max()
     assert r / (A.abs().sum(0).max() * X.abs().max() * n * 2.0**-53) < RESID_THRESH
+
+
+@pytest.mark.parametrize("trans", ["N", "T"])
+@pytest.mark.parametrize("polls,nrhs", [(0, 1), (0, 7), (1, 1), (3, 16), (20, 3)])
+def test_chained_solve_gives_up(sl, orc, ctx, trans, polls, nrhs):
+    """The chained solve's waits for the blocks before (four blocks of 64 rows and a
+    partial one) run out: INFO = -20002, and the next solve is right."""
+    import torch
+
+    n = 300
+    g = torch.Generator(device="cuda").manual_seed(nrhs)
+    A0 = torch.rand((n, n), dtype=torch.float64, device="cuda", generator=g).sub_(0.5)
+    B0 = torch.rand((nrhs, n), dtype=torch.float64, device="cuda", generator=g).sub_(0.5)
+    A = A0.clone()
+    piv = torch.zeros(n, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    assert sl.dgetrf_dev(n, n, A.data_ptr(), n, piv.data_ptr()) == 0
+
+    def solve():
+        X = B0.clone()
+        torch.cuda.synchronize()
+        return sl.dgetrs_dev(trans, n, nrhs, A.data_ptr(), n, piv.data_ptr(), X.data_ptr(), n), X
+
+    try:
+        sl.lib().sl1x1_debug_set_spin_limit(polls)
+        for _ in range(4):
+            info, _ = solve()
+            assert info == -20002 if polls == 0 else info in (-20002, 0)
+    finally:
+        sl.lib().sl1x1_debug_set_spin_limit(-1)
+    info, X = solve()
+    assert info == 0
+    M = A0 if trans == "T" else A0.T  # (a torch tensor holds the transpose)
+    r = (B0.T - M @ X.T).abs().max()
+    assert r / (M.abs().sum(1).max() * X.abs().max() * n * 2.0**-53) < RESID_THRESH
