@@ -161,6 +161,7 @@ bool ensure_device() {
       if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) return false;
   }
   if (cudaMalloc(&g_dev.dsmall, 16 * sizeof(int)) != cudaSuccess) return false;
+  if (cudaMemset(g_dev.dsmall, 0, 16 * sizeof(int)) != cudaSuccess) return false;
   if (cudaMalloc(&g_dev.dcand, sl::panel_cand_doubles() * sizeof(double)) != cudaSuccess) return false;
   if (cudaMalloc(&g_dev.dplan, 2 * sl::kSwapPlanInts * sizeof(int)) != cudaSuccess) return false;
   g_dev.ok = true;
@@ -297,12 +298,28 @@ cudaError_t ensure_solve_ws(int n, int nrhs) {
 
 // Reads the device status word and the first zero-pivot column after a
 // factorization; returns INFO (>0 singular, <=-20000 device status).
+// A status word that is set is cleared once read: every call finds it zero, and the
+// solves, of which a call may make several, leave it alone unless a wait gives up.
+static int clear_status(cudaStream_t s, int st) {
+  cudaError_t e = cudaMemsetAsync(g_dev.dsmall + 2, 0, sizeof(int), s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  return e == cudaSuccess ? -20000 - st : cuda_info(e);
+}
+
+int take_status(cudaStream_t s) {
+  int st = 0;
+  cudaError_t e = cudaMemcpyAsync(&st, g_dev.dsmall + 2, sizeof(int), cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  if (e != cudaSuccess) return cuda_info(e);
+  return st ? clear_status(s, st) : 0;
+}
+
 int read_factor_info(cudaStream_t s, int mn, int* out_info) {
   int h[2] = {0, 0};
   cudaError_t e = cudaMemcpyAsync(h, g_dev.dsmall + 2, 2 * sizeof(int), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) { *out_info = cuda_info(e); return *out_info; }
-  if (h[0] != 0) { *out_info = -20000 - h[0]; return *out_info; }
+  if (h[0] != 0) { *out_info = clear_status(s, h[0]); return *out_info; }
   *out_info = (h[1] >= 0 && h[1] < mn) ? h[1] + 1 : 0;
   return *out_info;
 }
@@ -479,11 +496,7 @@ static int solve_host(char trans, int n, int nrhs, long long ldda, double* B, in
   if (e != cudaSuccess) return cuda_info(e);
   e = cudaMemcpy2DAsync(hb, lldb * sizeof(double), g_dev.dB, lddb * sizeof(double),
                         (size_t)n * sizeof(double), nrhs, cudaMemcpyDeviceToHost, s);
-  int st = 0;
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&st, g_dev.dsmall + 2, sizeof(int), cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  if (e != cudaSuccess) return cuda_info(e);
-  return st ? -20000 - st : 0;
+  return e == cudaSuccess ? take_status(s) : cuda_info(e);
 }
 
 void pdgetrs_(const char* TRANS, const int* N, const int* NRHS, const double* A, const int* IA,
@@ -708,11 +721,7 @@ int sl1x1_dgetrs_dev(char trans, int n, int nrhs, const double* dA, long long ld
   if (e != cudaSuccess) return cuda_info(e);
   sl::LuWork w = make_work();
   e = sl::dgetrs_device(trans, n, nrhs, dA, ldda, g_dev.dipiv, dB, lddb, w, s);
-  int st = 0;
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&st, g_dev.dsmall + 2, sizeof(int), cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  if (e != cudaSuccess) return cuda_info(e);
-  return st ? -20000 - st : 0;
+  return e == cudaSuccess ? take_status(s) : cuda_info(e);
 }
 
 int sl1x1_dgesv_dev(int n, int nrhs, double* dA, long long ldda, int* dipiv, double* dB,
@@ -756,12 +765,7 @@ int sl1x1_lowp_update_dev(int fmt, int m, int n, int k, const float* dL, long lo
   if (e == cudaSuccess)
     e = sl::lowp_gemm(fmt, m, n, k, g_dev.dA16, g_dev.dB16, g_dev.dcolexp, dC, ldc,
                       g_dev.dsmall + 2, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  if (e != cudaSuccess) return cuda_info(e);
-  int st = 0;
-  e = cudaMemcpy(&st, g_dev.dsmall + 2, sizeof(int), cudaMemcpyDeviceToHost);
-  if (e != cudaSuccess) return cuda_info(e);
-  return st ? -20000 - st : 0;
+  return e == cudaSuccess ? take_status(s) : cuda_info(e);
 }
 
 int sl1x1_dgesv_ir_dev(int n, int nrhs, double* dA, long long ldda, int* dipiv, const double* dB,
@@ -843,6 +847,10 @@ int sl1x1_dgesv_ir_dev(int n, int nrhs, double* dA, long long ldda, int* dipiv, 
                           opt, &st, w, mw, s);
   if (e == cudaErrorInvalidValue) return -30000;
   if (e != cudaSuccess) return cuda_info(e);
+  if (st.fell_back) {  // the FP64 factorization and solve
+    const int r = take_status(s);
+    if (r != 0) return r;
+  }
   if (stats) {
     stats[0] = st.classical; stats[1] = st.gmres_outer; stats[2] = st.gmres_inner;
     stats[3] = st.fell_back ? (st.gave_up ? 2 : 1) : 0; stats[4] = st.sresid; stats[5] = st.anorm;
@@ -1045,8 +1053,9 @@ int sl1x1_dgetri_dev(int n, double* dA, long long ldda, const int* dipiv, void* 
   sl::LuWork w = make_work();
   e = sl::dgetri_device(n, dA, ldda, g_dev.dipiv, g_dev.daux, w,
                         reinterpret_cast<int*>(g_dev.daux + (size_t)n * n), &info, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  return e == cudaSuccess ? info : cuda_info(e);
+  if (e != cudaSuccess) return cuda_info(e);
+  const int r = take_status(s);
+  return r != 0 ? r : info;
 }
 
 // PDGETRI (SRC/pdgetri.f): validation and workspace query as the reference,
@@ -1103,6 +1112,7 @@ void pdgetri_(const int* N, double* A, const int* IA, const int* JA, const int* 
   if (e == cudaSuccess)
     e = sl::dgetri_device(n, g_dev.dA, ldda, g_dev.dipiv, g_dev.daux, w,
                           reinterpret_cast<int*>(g_dev.daux + (size_t)n * n), &dinfo, s);
+  if (e == cudaSuccess && dinfo == 0) dinfo = take_status(s);
   if (e == cudaSuccess && dinfo == 0)
     e = cudaMemcpy2DAsync(hA, lld * sizeof(double), g_dev.dA, ldda * sizeof(double),
                           (size_t)n * sizeof(double), n, cudaMemcpyDeviceToHost, s);
@@ -1194,12 +1204,7 @@ int sl1x1_ozgemm_dev(int m, int n, int k, double alpha, const double* dA, long l
   sc.bytes = g_dev.capOz;
   cudaError_t e = cudaMemsetAsync(g_dev.dsmall + 2, 0, sizeof(int), s);
   if (e == cudaSuccess) e = sl::oz_dgemm(sc, m, n, k, alpha, dA, ldda, dB, lddb, dC, lddc, g_dev.dsmall + 2, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  if (e != cudaSuccess) return cuda_info(e);
-  int st = 0;
-  e = cudaMemcpy(&st, g_dev.dsmall + 2, sizeof(int), cudaMemcpyDeviceToHost);
-  if (e != cudaSuccess) return cuda_info(e);
-  return st ? -20000 - st : 0;
+  return e == cudaSuccess ? take_status(s) : cuda_info(e);
 }
 
 void sl1x1_set_update_reserve(int min_sms, int max_sms) {

@@ -142,7 +142,7 @@ int gerfs_staged(char trans, int n, int nrhs, const Staging& st, double* ferr, d
   cudaError_t e = sl::dgerfs_device(trans, n, nrhs, g_dev.dA2, st.ldd, g_dev.dA, st.ldd,
                                     g_dev.dipiv, g_dev.dB, st.ldd, g_dev.dX, st.ldd, ferr, berr, w,
                                     g_dev.drw, st.iw, s);
-  return e == cudaSuccess ? 0 : cuda_info(e);
+  return e == cudaSuccess ? take_status(s) : cuda_info(e);
 }
 
 }  // namespace
@@ -580,8 +580,7 @@ int sl1x1_dgerfs_dev(char trans, int n, int nrhs, const double* dA, long long ld
   sl::LuWork w = make_work();
   e = sl::dgerfs_device(t, n, nrhs, dA, ldda, dAF, lddaf, g_dev.dipiv2, dB, lddb, dX, lddx, ferr,
                         berr, w, g_dev.drw, g_dev.dipiv2 + n, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  return e == cudaSuccess ? 0 : cuda_info(e);
+  return e == cudaSuccess ? take_status(s) : cuda_info(e);
 }
 
 }  // extern "C"

@@ -101,6 +101,8 @@ int factor_nb(int m, int n, int nb);
 cudaError_t ensure_solve_ws(int n, int nrhs);
 // INFO after a factorization (>0 singular, <= -20000 device status)
 int read_factor_info(cudaStream_t s, int mn, int* out_info);
+// The same status after a call's other work: waits for the stream; 0 or INFO
+int take_status(cudaStream_t s);
 // Device leading dimension for m rows (multiple of 32)
 long long round_ld(long long m);
 // Stages sub(A) into g_dev.dA, factors it, copies L\U and IPIV back.

@@ -743,18 +743,15 @@ __device__ __forceinline__ void tri_inv64_of(int b, int part, int n, const doubl
 // Everything a solve needs before its first step, in one launch: the first
 // blocks make the segment maps of the pivots' row permutation (perm_segment), the
 // next kInvParts * nb64 invert L's diagonal blocks into D, as many more U's
-// behind them; the status word and the tickets of the chained solve are reset.
+// behind them; the tickets of the chained solve are reset.
 __global__ void __launch_bounds__(256)
 solve_prep_kernel(int n, const double* __restrict__ A, long long lda, double* D,
-                  const int* __restrict__ ipiv, int* maps, int* status, int* tickets) {
+                  const int* __restrict__ ipiv, int* maps, int* tickets) {
   extern __shared__ double inv_smem[];
   static_assert(kPermSmem * sizeof(int) <= (size_t)kInvSmem, "pivots of a segment");
   const int nb64 = (n + 63) / 64, nperm = (n + 255) / 256 * perm_segs(n);
   const int b = (int)blockIdx.x - nperm, part = b % kInvParts, blk = b / kInvParts;
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    *status = 0;
-    if (tickets) tickets[0] = tickets[1] = 0;
-  }
+  if (blockIdx.x == 0 && threadIdx.x == 0 && tickets) tickets[0] = tickets[1] = 0;
   launch_dependents();
   if (b < 0)
     perm_segment(blockIdx.x, ipiv, n, maps, reinterpret_cast<int*>(inv_smem));
@@ -1065,7 +1062,7 @@ static cudaError_t prepare_solve(int n, const double* dA, long long ldda, const 
   SL_TRY(blocked_solve_attrs());
   const int nrb = (n + 255) / 256, nb64 = (n + 63) / 64;
   solve_prep_kernel<<<2 * kInvParts * nb64 + nrb * perm_segs(n), 256, kInvSmem, s>>>(
-      n, dA, ldda, ws.dinv_solve, dipiv, ws.perm + n, ws.status, tickets);
+      n, dA, ldda, ws.dinv_solve, dipiv, ws.perm + n, tickets);
   count_launches(1);
   if (blocked) {
     perm_finish_kernel<<<nrb, 256, 0, s>>>(dipiv, n, ws.perm + n, ws.perm);
@@ -1128,7 +1125,6 @@ cudaError_t dgetrs_device(char trans, int n, int nrhs, const double* dA, long lo
   if (notran ? (inv_path || chain_path) : chain_path) {
     SL_TRY(prepare_solve(n, dA, ldda, dipiv, ws, chain_path ? ws.chain : nullptr, !chain_path, s));
   } else {
-    SL_TRY(cudaMemsetAsync(ws.status, 0, sizeof(int), s));
     SL_TRY(perm_compose(dipiv, n, ws.perm, s));
   }
   if (chain_path) {

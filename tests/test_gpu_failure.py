@@ -236,3 +236,54 @@ def test_chained_solve_gives_up(sl, orc, ctx, trans, polls, nrhs):
     M = A0 if trans == "T" else A0.T  # (a torch tensor holds the transpose)
     r = (B0.T - M @ X.T).abs().max()
     assert r / (M.abs().sum(1).max() * X.abs().max() * n * 2.0**-53) < RESID_THRESH
+
+
+def test_solve_that_gives_up_is_reported_by_every_caller(sl, orc, ctx):
+    """PDGETRI, PDGERFS and PDGESVX make several solves in one call: a wait that gives
+    up in any of them is INFO = -20002, and nothing of it is left for the next call."""
+    import torch
+
+    n, nrhs = 120, 2
+    A0, B0 = system(orc, n, nrhs)
+    d = np.array([1, ctx, n, n, 32, 32, 0, 0, n], np.int32)
+    db = np.array([1, ctx, n, nrhs, 32, 32, 0, 0, n], np.int32)
+    LU = np.asfortranarray(A0.copy())
+    ipiv = np.zeros(n + 32, np.int32)
+    assert sl.pdgetrf(n, n, LU, 1, 1, d, ipiv) == 0
+    dev = {k: torch.from_numpy(np.ascontiguousarray(v.T)).cuda() for k, v in (("A", A0), ("LU", LU), ("B", B0))}
+    piv = torch.from_numpy(ipiv[:n].copy()).cuda()
+    X = {t: np.linalg.solve(A0.T if t == "T" else A0, B0) for t in "NT"}
+
+    def getri():
+        inv = np.asfortranarray(LU.copy())
+        r = sl.pdgetri(n, inv, 1, 1, d, ipiv.copy())[0]
+        return r, abs(inv @ A0 - np.eye(n)).max()
+
+    def getri_dev():
+        inv = dev["LU"].clone()
+        torch.cuda.synchronize()
+        r = sl.lib().sl1x1_dgetri_dev(n, inv.data_ptr(), n, piv.data_ptr(), None)
+        return r, abs(inv.cpu().numpy().T @ A0 - np.eye(n)).max()
+
+    def gerfs(t):
+        x = torch.from_numpy(np.ascontiguousarray(X[t].T) * (1 + 1e-9)).cuda()
+        torch.cuda.synchronize()
+        r = sl.dgerfs_dev(t, n, nrhs, dev["A"].data_ptr(), n, dev["LU"].data_ptr(), n, piv.data_ptr(),
+                          dev["B"].data_ptr(), n, x.data_ptr(), n)
+        return r[0], abs(x.cpu().numpy().T - X[t]).max()
+
+    def gesvx(t):
+        a, af, b, x = (np.asfortranarray(v.copy()) for v in (A0, LU, B0, 0 * B0))
+        r = sl.pdgesvx("F", t, n, nrhs, a, 1, 1, d, af, 1, 1, d, ipiv.copy(), "N", np.ones(n), np.ones(n), b, 1, 1,
+                       db, x, 1, 1, db, np.zeros(nrhs), np.zeros(nrhs))
+        return r["info"], abs(x - X[t]).max()
+
+    calls = [getri, getri_dev] + [(lambda f=f, t=t: f(t)) for f in (gerfs, gesvx) for t in "NT"]
+    for call in calls:
+        try:
+            sl.lib().sl1x1_debug_set_spin_limit(0)
+            assert call()[0] == -20002
+        finally:
+            sl.lib().sl1x1_debug_set_spin_limit(-1)
+        info, err = call()
+        assert info == 0 and err < 1e-9
