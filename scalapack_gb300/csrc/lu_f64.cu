@@ -1122,6 +1122,12 @@ cudaError_t dgetrs_device(char trans, int n, int nrhs, const double* dA, long lo
   const bool chain_path = g_f64_update == 1 && few && ws.dinv_solve &&
                           ws.dinv_solve_len >= kSolveInvDoubles(n) && ws.chain && ws.chain_epoch &&
                           ws.chain_values >= (size_t)n * nrhs;
+  unsigned long long* words = chain_path ? reinterpret_cast<unsigned long long*>(ws.chain + 16) : nullptr;
+  if (chain_path && (*ws.chain_epoch == 0 || *ws.chain_epoch > UINT_MAX - 2)) {
+    // (before the preparation: the chained launches follow a kernel, launch_after)
+    SL_TRY(cudaMemsetAsync(words, 0, ws.chain_values * 16, s));
+    *ws.chain_epoch = 0;
+  }
   if (notran ? (inv_path || chain_path) : chain_path) {
     SL_TRY(prepare_solve(n, dA, ldda, dipiv, ws, chain_path ? ws.chain : nullptr, !chain_path, s));
   } else {
@@ -1130,11 +1136,6 @@ cudaError_t dgetrs_device(char trans, int n, int nrhs, const double* dA, long lo
   if (chain_path) {
     // L then U (N), or U^T then L^T (T): the pivots' permutation is applied as
     // the first triangle reads B, or as the second one writes it
-    unsigned long long* words = reinterpret_cast<unsigned long long*>(ws.chain + 16);
-    if (*ws.chain_epoch == 0 || *ws.chain_epoch > UINT_MAX - 2) {
-      SL_TRY(cudaMemsetAsync(words, 0, ws.chain_values * 16, s));
-      *ws.chain_epoch = 0;
-    }
     const size_t ub = (size_t)((n + 63) / 64) * 4096;
     const unsigned e1 = ++*ws.chain_epoch, e2 = ++*ws.chain_epoch;
     SL_TRY(trsv64_chain(notran, !notran, dA, ldda, n, ws.dinv_solve + (notran ? 0 : ub), dB, lddb,
