@@ -685,17 +685,36 @@ cudaError_t gemm_update<double>(bool transa, int m, int n, int k, double alpha, 
 // instruction whatever lanes are active, and a column of the inverse costs 32
 // to 96 of them (one CTA per block and a barrier per row: 54 us for one block, 11
 // with four).
-constexpr int kInvSmem = (64 * 64 + 64) * (int)sizeof(double);
+//
+// x = inv(T_bb) v has an error of eps |inv(T_bb)| |v|, a substitution one of eps |T_bb|
+// |x|: what the inverse costs grows with its size against that of T_bb with its rows over
+// their diagonal (the sizes of the rows do not matter). flag[part] = 1 where an entry of
+// inv(T_bb) times its column's diagonal is 16 or more (8 may be taken for it), or is not finite, or
+// a diagonal entry's reciprocal is not a normal number: such a block is solved by
+// substitution. Largest over the 64-row blocks of the factors of random matrices, N = 256 ..
+// 4096: 4.1 (uniform and normal entries; 1.0 with a heavy diagonal). Scaled residual of
+// a 64-row solve, worst of 1500 triangles per size: entries up to 8: 0.7 (substitution
+// 0.4), up to 64: 1.8, up to 2^11: 12, up to 2^16: 270; with 8 rows 1.5, 12 and 62 (bound
+// of the tester: 16). Exponents are compared, off the FP64 unit.
+constexpr int kInvSmem = (64 * 64 + 64 + 32) * (int)sizeof(double);
 constexpr int kInvParts = 4;
 template <bool LOWER>
 __device__ __forceinline__ void tri_inv64_of(int b, int part, int n, const double* __restrict__ A,
-                                             long long lda, double* D, double* inv_smem) {
+                                             long long lda, double* D, int* flag, double* inv_smem) {
   double* Ts = inv_smem;  // Ts[q*64 + i] = T(i, q), zero outside the strict triangle
   double* rd = inv_smem + 64 * 64;
+  int* de = reinterpret_cast<int*>(rd + 64);  // biased exponents of the diagonal
+  auto exp_of = [](double x) { return (__double2hiint(x) >> 20) & 0x7ff; };
+  bool bad = false;
   const int r0 = b * 64, rb = min(64, n - r0);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (!LOWER) {
-    if (tid < 64) rd[tid] = tid < rb ? 1.0 / A[(r0 + tid) + (long long)(r0 + tid) * lda] : 1.0;
+    if (tid < 64) {
+      const double d = tid < rb ? A[(r0 + tid) + (long long)(r0 + tid) * lda] : 1.0;
+      rd[tid] = 1.0 / d;
+      de[tid] = exp_of(d);
+      bad = de[tid] == 0 || de[tid] > 2044;
+    }
     __syncthreads();
   }
 #pragma unroll 8
@@ -737,15 +756,19 @@ __device__ __forceinline__ void tri_inv64_of(int b, int part, int n, const doubl
     }
     Db[c * 64 + lane] = x0;
     Db[c * 64 + lane + 32] = x1;
+    const int e = max(exp_of(x0), exp_of(x1));
+    bad = bad || e == 0x7ff || e + (LOWER ? 1023 : de[c]) > 2 * 1023 + 2;
   }
+  const int any = __syncthreads_or(bad);
+  if (tid == 0) flag[b * kInvParts + part] = any;
 }
 
 // Everything a solve needs before its first step, in one launch: the first
 // blocks make the segment maps of the pivots' row permutation (perm_segment), the
-// next kInvParts * nb64 invert L's diagonal blocks into D, as many more U's
-// behind them; the tickets of the chained solve are reset.
+// next kInvParts * nb64 invert L's diagonal blocks into D (flags: which of them not to
+// use), as many more U's behind them; the tickets of the chained solve are reset.
 __global__ void __launch_bounds__(256)
-solve_prep_kernel(int n, const double* __restrict__ A, long long lda, double* D,
+solve_prep_kernel(int n, const double* __restrict__ A, long long lda, double* D, int* flags,
                   const int* __restrict__ ipiv, int* maps, int* tickets) {
   extern __shared__ double inv_smem[];
   static_assert(kPermSmem * sizeof(int) <= (size_t)kInvSmem, "pivots of a segment");
@@ -755,8 +778,9 @@ solve_prep_kernel(int n, const double* __restrict__ A, long long lda, double* D,
   launch_dependents();
   if (b < 0)
     perm_segment(blockIdx.x, ipiv, n, maps, reinterpret_cast<int*>(inv_smem));
-  else if (blk < nb64) tri_inv64_of<true>(blk, part, n, A, lda, D, inv_smem);
-  else tri_inv64_of<false>(blk - nb64, part, n, A, lda, D + (size_t)nb64 * 4096, inv_smem);
+  else if (blk < nb64) tri_inv64_of<true>(blk, part, n, A, lda, D, flags, inv_smem);
+  else
+    tri_inv64_of<false>(blk - nb64, part, n, A, lda, D + (size_t)nb64 * 4096, flags + nb64 * kInvParts, inv_smem);
 }
 
 // Balancing keys of the blocked NOTRAN solve's sliced products, once per
@@ -786,17 +810,39 @@ solve_ckeys_kernel(int n, const double* __restrict__ A, long long lda, unsigned*
 // inv(T_bb) X(k0:k0+kb, c) for the 128-row block at k0 of the unit-lower L
 // (LOWER, forward) or the upper U (backward), from the inverses of its two
 // 64x64 diagonal blocks and its off-diagonal 64x64 block, staged in shared
-// memory. CTA c < nrhs takes right-hand side c (threads 0..127 one row each);
+// memory; a 64-row block whose four words of flags are not all zero is solved by
+// substitution with its own triangle. CTA c < nrhs takes right-hand side c (threads 0..127 one row each);
 // with ckeys set, the CTAs also publish the balancing keys of the sliced
 // product that follows (A: the factor's columns k0..k0+kb outside the block,
 // B: the solved rows): the h keys from each column's solved values and, in
 // the extra CTA nrhs, the c keys from ck.
 constexpr int kBlkSmem = 3 * 64 * 64 * (int)sizeof(double);
+__device__ __forceinline__ bool block_flagged(const int* flags, int b) {
+  static_assert(kInvParts == 4, "one int4 per block");
+  const int4 f = reinterpret_cast<const int4*>(flags)[b];
+  return (f.x | f.y | f.z | f.w) != 0;
+}
+// Ts[i*64 + r] = T(r, i) of the w x w triangle at T
+__device__ __noinline__ void stage_triangle(int w, const double* __restrict__ T, long long lda, double* Ts) {
+  for (int idx = threadIdx.x; idx < 4096; idx += 256) {
+    const int r = idx & 63, i = idx >> 6;
+    Ts[idx] = r < w && i < w ? T[r + (long long)i * lda] : 0.0;
+  }
+}
+// y = inv(T) x by the calling warp, T from stage_triangle
+template <bool LOWER>
+__device__ __noinline__ void warp_solve_triangle(int w, const double* Ts, const double* x, double* y) {
+  const int lane = threadIdx.x & 31;
+  double x0 = x[lane], x1 = x[lane + 32];
+  warp_substitute64(LOWER, LOWER, w, [&](int i, int k) { return Ts[k * 64 + i]; }, x0, x1);
+  y[lane] = x0;
+  y[lane + 32] = x1;
+}
 template <bool LOWER>
 __global__ void __launch_bounds__(256)
 solve_block128_kernel(int kb, const double* __restrict__ A, long long lda, int k0,
-                      const double* __restrict__ D, double* X, long long ldx, int nrhs,
-                      const unsigned* __restrict__ ck, unsigned long long* ckeys,
+                      const double* __restrict__ D, const int* __restrict__ flags, double* X, long long ldx,
+                      int nrhs, const unsigned* __restrict__ ck, unsigned long long* ckeys,
                       unsigned long long* hkeys, unsigned long long epoch) {
   extern __shared__ double blk_smem[];  // D0, D1 and the off-diagonal block O, each [c*64 + r]
   __shared__ double xs[128], ys[128];
@@ -842,10 +888,18 @@ solve_block128_kernel(int kb, const double* __restrict__ A, long long lda, int k
     for (int q = 0; q < 16; ++q) Os[t + 256 * q] = ro[q];
     if (t < 128) xs[t] = xv;
   }
+  const bool sub0 = block_flagged(flags, b0), sub1 = w1 > 0 && block_flagged(flags, b0 + 1);
   __syncthreads();
+  if (sub0 || sub1) {
+    if (sub0) stage_triangle(w0, A + k0 + (long long)k0 * lda, lda, D0s);
+    if (sub1) stage_triangle(w1, A + (k0 + 64) + (long long)(k0 + 64) * lda, lda, D1s);
+    __syncthreads();
+  }
   if (LOWER) {
     // y0 = inv(L00) x0; x1 -= L10 y0; y1 = inv(L11) x1
-    if (t < 64) {
+    if (sub0) {
+      if (t < 32) warp_solve_triangle<LOWER>(w0, D0s, xs, ys);
+    } else if (t < 64) {
       double acc = 0.0;
       for (int i = 0; i < 64; ++i) acc = fma(D0s[i * 64 + t], xs[i], acc);
       ys[t] = acc;
@@ -857,7 +911,9 @@ solve_block128_kernel(int kb, const double* __restrict__ A, long long lda, int k
       xs[t] = acc;
     }
     __syncthreads();
-    if (t >= 64 && t < 128 && w1 > 0) {  // (no second 64-block when kb <= 64)
+    if (sub1) {
+      if (t < 32) warp_solve_triangle<LOWER>(w1, D1s, xs + 64, ys + 64);
+    } else if (t >= 64 && t < 128 && w1 > 0) {  // (no second 64-block when kb <= 64)
       const int r = t - 64;
       double acc = 0.0;
       for (int i = 0; i < 64; ++i) acc = fma(D1s[i * 64 + r], xs[64 + i], acc);
@@ -865,7 +921,9 @@ solve_block128_kernel(int kb, const double* __restrict__ A, long long lda, int k
     }
   } else {
     // y1 = inv(U11) x1; x0 -= U01 y1; y0 = inv(U00) x0
-    if (t >= 64 && t < 128 && w1 > 0) {
+    if (sub1) {
+      if (t < 32) warp_solve_triangle<LOWER>(w1, D1s, xs + 64, ys + 64);
+    } else if (t >= 64 && t < 128 && w1 > 0) {
       const int r = t - 64;
       double acc = 0.0;
       for (int i = 0; i < 64; ++i) acc = fma(D1s[i * 64 + r], xs[64 + i], acc);
@@ -880,7 +938,9 @@ solve_block128_kernel(int kb, const double* __restrict__ A, long long lda, int k
       xs[t] = acc;
     }
     __syncthreads();
-    if (t < 64) {
+    if (sub0) {
+      if (t < 32) warp_solve_triangle<LOWER>(w0, D0s, xs, ys);
+    } else if (t < 64) {
       double acc = 0.0;
       for (int i = 0; i < 64; ++i) acc = fma(D0s[i * 64 + t], xs[i], acc);
       ys[t] = acc;
@@ -908,8 +968,8 @@ constexpr int kWideSmem = (3 * 64 * 64 + 2 * 128 * kWideCols) * (int)sizeof(doub
 template <bool LOWER>
 __global__ void __launch_bounds__(256)
 solve_block128_wide_kernel(int kb, const double* __restrict__ A, long long lda, int k0,
-                           const double* __restrict__ D, double* X, long long ldx, int nrhs,
-                           const unsigned* __restrict__ ck, unsigned long long* ckeys,
+                           const double* __restrict__ D, const int* __restrict__ flags, double* X,
+                           long long ldx, int nrhs, const unsigned* __restrict__ ck, unsigned long long* ckeys,
                            unsigned long long* hkeys, unsigned long long epoch) {
   extern __shared__ double blk_smem[];  // D0, D1 and the coupling block O, each [i*64 + r]
   double* D0s = blk_smem;
@@ -933,9 +993,20 @@ solve_block128_wide_kernel(int kb, const double* __restrict__ A, long long lda, 
     Os[idx] = in ? A[off] : 0.0;
   }
   if (t < 128) s_h[t] = 0u;
+  const bool sub0 = block_flagged(flags, k0 / 64), sub1 = w1 > 0 && block_flagged(flags, k0 / 64 + 1);
+  if (sub0 || sub1) {
+    __syncthreads();
+    if (sub0) stage_triangle(w0, A + k0 + (long long)k0 * lda, lda, D0s);
+    if (sub1) stage_triangle(w1, A + (k0 + 64) + (long long)(k0 + 64) * lda, lda, D1s);
+  }
   // y = M v for 64 rows: v, y at offset h of a column; i runs over the warp's part
   // of the triangle (i0 .. i1)
-  auto tri = [&](const double* M, int h, int i0, int i1) {
+  // (sub: M is the triangle itself, a warp per column)
+  auto tri = [&](const double* M, int h, int i0, int i1, bool sub) {
+    if (sub) {
+      warp_solve_triangle<LOWER>(h ? w1 : w0, M, xs + (t >> 5) * 128 + h, ys + (t >> 5) * 128 + h);
+      return;
+    }
     double a0 = 0.0, a1 = 0.0;
     for (int i = i0; i < i1; ++i) {
       const double m = M[i * 64 + r];
@@ -966,17 +1037,17 @@ solve_block128_wide_kernel(int kb, const double* __restrict__ A, long long lda, 
     }
     __syncthreads();
     if (LOWER) {  // y0 = inv(L00) x0; x1 -= L10 y0; y1 = inv(L11) x1
-      tri(D0s, 0, lo_i0, lo_i1);
+      tri(D0s, 0, lo_i0, lo_i1, sub0);
       __syncthreads();
       couple(64, 0, w0);
       __syncthreads();
-      tri(D1s, 64, lo_i0, lo_i1);
+      tri(D1s, 64, lo_i0, lo_i1, sub1);
     } else {      // y1 = inv(U11) x1; x0 -= U01 y1; y0 = inv(U00) x0
-      tri(D1s, 64, lo_i0, lo_i1);
+      tri(D1s, 64, lo_i0, lo_i1, sub1);
       __syncthreads();
       couple(0, 64, max(w1, 0));
       __syncthreads();
-      tri(D0s, 0, lo_i0, lo_i1);
+      tri(D0s, 0, lo_i0, lo_i1, sub0);
     }
     __syncthreads();
 #pragma unroll
@@ -1007,6 +1078,7 @@ static cudaError_t tri_solve_inv(bool lower, int n, int ncols, const double* A, 
   const int nblk = (n + KB - 1) / KB;
   const int nb64 = (n + 63) / 64;
   const double* D = ws.dinv_solve + (lower ? 0 : (size_t)nb64 * 4096);
+  const int* flags = solve_inv_flags(ws.dinv_solve, n) + (lower ? 0 : nb64 * kInvParts);
   const unsigned* ck = reinterpret_cast<const unsigned*>(ws.dinv_solve + (size_t)2 * nb64 * 4096) +
                        (lower ? 0 : nb64 * 64);
   unsigned long long* ckeys = oz_ckeys(ws.oz);
@@ -1021,16 +1093,16 @@ static cudaError_t tri_solve_inv(bool lower, int n, int ncols, const double* A, 
       const int grid = std::min(2 * num_sms(), (nrhs + kWideCols - 1) / kWideCols);
       if (lower)
         solve_block128_wide_kernel<true><<<grid, 256, kWideSmem, s>>>(
-            kb, A, lda, k0, D, X, ldx, nrhs, ck, ckeys, rest > 0 ? hkeys : nullptr, ep);
+            kb, A, lda, k0, D, flags, X, ldx, nrhs, ck, ckeys, rest > 0 ? hkeys : nullptr, ep);
       else
         solve_block128_wide_kernel<false><<<grid, 256, kWideSmem, s>>>(
-            kb, A, lda, k0, D, X, ldx, nrhs, ck, ckeys, rest > 0 ? hkeys : nullptr, ep);
+            kb, A, lda, k0, D, flags, X, ldx, nrhs, ck, ckeys, rest > 0 ? hkeys : nullptr, ep);
     } else if (lower)
       solve_block128_kernel<true><<<nrhs + (rest > 0 ? 1 : 0), 256, kBlkSmem, s>>>(
-          kb, A, lda, k0, D, X, ldx, nrhs, ck, ckeys, rest > 0 ? hkeys : nullptr, ep);
+          kb, A, lda, k0, D, flags, X, ldx, nrhs, ck, ckeys, rest > 0 ? hkeys : nullptr, ep);
     else
       solve_block128_kernel<false><<<nrhs + (rest > 0 ? 1 : 0), 256, kBlkSmem, s>>>(
-          kb, A, lda, k0, D, X, ldx, nrhs, ck, ckeys, rest > 0 ? hkeys : nullptr, ep);
+          kb, A, lda, k0, D, flags, X, ldx, nrhs, ck, ckeys, rest > 0 ? hkeys : nullptr, ep);
     count_launches(1);
     SL_TRY(cudaGetLastError());
     if (rest > 0 && lower)
@@ -1062,7 +1134,7 @@ static cudaError_t prepare_solve(int n, const double* dA, long long ldda, const 
   SL_TRY(blocked_solve_attrs());
   const int nrb = (n + 255) / 256, nb64 = (n + 63) / 64;
   solve_prep_kernel<<<2 * kInvParts * nb64 + nrb * perm_segs(n), 256, kInvSmem, s>>>(
-      n, dA, ldda, ws.dinv_solve, dipiv, ws.perm + n, tickets);
+      n, dA, ldda, ws.dinv_solve, solve_inv_flags(ws.dinv_solve, n), dipiv, ws.perm + n, tickets);
   count_launches(1);
   if (blocked) {
     perm_finish_kernel<<<nrb, 256, 0, s>>>(dipiv, n, ws.perm + n, ws.perm);
@@ -1136,11 +1208,12 @@ cudaError_t dgetrs_device(char trans, int n, int nrhs, const double* dA, long lo
   if (chain_path) {
     // L then U (N), or U^T then L^T (T): the pivots' permutation is applied as
     // the first triangle reads B, or as the second one writes it
-    const size_t ub = (size_t)((n + 63) / 64) * 4096;
+    const size_t ub = (size_t)((n + 63) / 64) * 4096, uf = (size_t)((n + 63) / 64) * kInvParts;
+    const int* flags = solve_inv_flags(ws.dinv_solve, n);
     const unsigned e1 = ++*ws.chain_epoch, e2 = ++*ws.chain_epoch;
-    SL_TRY(trsv64_chain(notran, !notran, dA, ldda, n, ws.dinv_solve + (notran ? 0 : ub), dB, lddb,
+    SL_TRY(trsv64_chain(notran, !notran, dA, ldda, n, ws.dinv_solve + (notran ? 0 : ub), flags + (notran ? 0 : uf), dB, lddb,
                         notran ? dipiv : nullptr, X, n, nullptr, ws.perm + n, nrhs, ws.chain, words, e1, ws.status, s));
-    SL_TRY(trsv64_chain(!notran, !notran, dA, ldda, n, ws.dinv_solve + (notran ? ub : 0), X, n, nullptr, dB,
+    SL_TRY(trsv64_chain(!notran, !notran, dA, ldda, n, ws.dinv_solve + (notran ? ub : 0), flags + (notran ? uf : 0), X, n, nullptr, dB,
                         lddb, notran ? nullptr : dipiv, ws.perm + n, nrhs, ws.chain + 1, words, e2, ws.status, s));
     phase_end(kPhSolve, s, 2.0 * (double)n * n * nrhs, 8.0 * ((double)n * n + 4.0 * (double)n * nrhs));
     return cudaSuccess;

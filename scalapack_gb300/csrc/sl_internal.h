@@ -175,7 +175,12 @@ constexpr int kMaxColChunks = 16;
 // zeroed (a stale word of a larger epoch would never be replaced).
 constexpr int kOzKinfoBytes = 8192;
 inline size_t kSolveInvDoubles(int n) {
-  return (size_t)2 * (size_t)((n + 63) / 64) * 64 * 64 + (size_t)((n + 63) / 64) * 64;
+  return (size_t)2 * (size_t)((n + 63) / 64) * 64 * 64 + (size_t)((n + 63) / 64) * (64 + 4);
+}
+// ... the last 8 ints per block: for each triangle (L's blocks first) four words of a
+// block, nonzero where its inverse is not to be used (tri_inv64_of).
+inline int* solve_inv_flags(double* dinv_solve, int n) {
+  return reinterpret_cast<int*>(dinv_solve + kSolveInvDoubles(n) - (size_t)((n + 63) / 64) * 4);
 }
 // Right-hand sides from which a blocked NOTRAN solve shares a CTA's staged blocks
 // among several of them.
@@ -240,12 +245,12 @@ cudaError_t dgetrs_device(char trans, int n, int nrhs, const double* dA, long lo
 constexpr int kChainRhs = 128;
 // op(T) X = S with the lower (unit) or upper triangle of n x n LU factors in
 // one launch (trsv_f64.cu): D holds the inverses of that triangle's 64x64
-// diagonal blocks; S is src with its rows permuted by the pivots `gather`, X goes
+// diagonal blocks, flags four words per block (solve_inv_flags); S is src with its rows permuted by the pivots `gather`, X goes
 // to dst through those of `scatter` (null: in place; maps: the pivots' segment
 // maps). ticket is zero on entry; words holds two
 // per value and no word of this epoch.
 cudaError_t trsv64_chain(bool lower, bool trans, const double* A, long long lda, int n, const double* D,
-                         const double* src, long long lds, const int* gather, double* dst,
+                         const int* flags, const double* src, long long lds, const int* gather, double* dst,
                          long long ldd, const int* scatter, const int* maps, int nrhs, int* ticket,
                          unsigned long long* words, uint32_t epoch, int* status, cudaStream_t s);
 

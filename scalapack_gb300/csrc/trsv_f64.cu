@@ -12,7 +12,9 @@
 // the solutions it needs; solved values are published as single-copy atomic
 // 16-byte words {x, epoch}, so a consumer polls the data itself (one L2 round
 // trip, no flag, no fence). With all of them applied, x_b = inv(T_bb) v_b from
-// the precomputed inverse of the diagonal block (the last tile of the ring).
+// the precomputed inverse of the diagonal block (the last tile of the ring); a block
+// whose inverse is large (tri_inv64_of) is solved by substitution instead, its own
+// triangle then being the last tile.
 //
 // Bound: n^2 nrhs FMAs on the FP64 pipe (a 64x64 block times one vector takes
 // 2560 cycles of an SM) when there are many right-hand sides; with one, the
@@ -21,7 +23,7 @@
 // through L2, which are not the bound, and lengthen a block's turn in the chain,
 // which is: n = 4096, 8 right-hand sides 0.93 ms (one per CTA: 0.59), n = 8192, 16
 // of them 2.98 (2.56), n = 16384 9.70 (9.12). Measured, GB300: n = 8192 with one
-// right-hand side, 0.90 ms for the whole PDGETRS (two chains of 0.39, the rest
+// right-hand side, 0.91 ms for the whole PDGETRS (two chains of 0.39, the rest
 // before them; 6.27 with three launches per 128 rows); n = 8192, TRANS = 'T', 16
 // right-hand sides, 2.55 ms (16.96 by substitution and DMMA products), of which
 // the FP64 pipe needs 2.0. The three launches of a PDGETRS overlap (launch_after):
@@ -66,17 +68,36 @@ __device__ __forceinline__ bool get_x(const unsigned long long* p, uint32_t epoc
   return (uint32_t)b == epoch;
 }
 
+// x = op(T) \ v over the tile T by the first warp, out: four partial sums of x (the
+// first is x). Not inlined: a CTA comes to the end of the kernel once, and what stands
+// between the loop and the product there is fetched on every step of the chain (n = 8192
+// with one right-hand side: 0.90 ms without this way, 0.91 with it, 1.00 inlined).
+template <bool TRANS>
+__device__ __noinline__ void substitute_tile(int forward, int w, const double* T, const double* v, double* out) {
+  constexpr int CS = TRANS ? TB + 1 : TB;
+  const int tid = threadIdx.x;
+  if (tid < 32) {
+    double x0 = v[tid], x1 = v[tid + 32];
+    // (the unit triangle is L: forward without TRANS, backward with it)
+    warp_substitute64(forward, (forward != 0) != TRANS, w,
+                      [&](int i, int k) { return TRANS ? T[i * CS + k] : T[k * CS + i]; }, x0, x1);
+    out[tid] = x0;
+    out[tid + 32] = x1;
+  }
+  if (tid >= TB) out[tid] = 0.0;
+}
+
 // op(T) X = S for one triangle of the LU factors A; TRANS: op(T) = T^T.
 // forward: block rows from the top (lower, or upper transposed). Row i of S is
 // row i of src, of X row i of dst, or in either place the row that the pivots
 // `gather` / `scatter` permute there (null: i; maps: their segments' maps,
-// follow_perm). D: inverses of T's diagonal blocks,
-// 4096 doubles each, column-major.
+// follow_perm). D: inverses of T's diagonal blocks, 4096 doubles each, column-major;
+// flags: four words per block, nonzero where it is solved by substitution.
 template <bool TRANS>
 __global__ void __launch_bounds__(256)
 trsv64_chain_kernel(const double* __restrict__ A, long long lda, int n, int forward,
-                    const double* __restrict__ D, const double* __restrict__ src, long long lds,
-                    const int* __restrict__ gather, double* dst, long long ldd,
+                    const double* __restrict__ D, const int* __restrict__ flags, const double* __restrict__ src,
+                    long long lds, const int* __restrict__ gather, double* dst, long long ldd,
                     const int* __restrict__ scatter, const int* __restrict__ maps, int nrhs,
                     int* ticket, unsigned long long* words, uint32_t epoch, int* status, long long spin_limit) {
   extern __shared__ double trsv_ring[];  // TRING tiles
@@ -97,8 +118,10 @@ trsv64_chain_kernel(const double* __restrict__ A, long long lda, int n, int forw
   const int b = forward ? sidx : nblk - 1 - sidx;
   const int r0 = b * TB, rb = min(TB, n - r0);
   const int r = tid & (TB - 1), q = tid >> 6;
+  const int4 fl = reinterpret_cast<const int4*>(flags)[b];
+  const bool subst = (fl.x | fl.y | fl.z | fl.w) != 0;
 
-  // tile t of the ring: block (b, k(t)) of op(T) for t < sidx, inv(T_bb) for
+  // tile t of the ring: block (b, k(t)) of op(T) for t < sidx, inv(T_bb) (or T_bb) for
   // t = sidx; columns of the stored block at stride 64, or 65 when transposed
   // (both ways the threads of a warp then read one column of op(T) without
   // bank conflicts)
@@ -107,11 +130,12 @@ trsv64_chain_kernel(const double* __restrict__ A, long long lda, int n, int forw
     if (t <= sidx) {
       double* slot = trsv_ring + (t % TRING) * TSLOT;
       const int k0 = (forward ? t : nblk - 1 - t) * TB;
-      const double* g = t == sidx ? D + (size_t)b * (TB * TB)
-                                  : (TRANS ? A + k0 + (long long)r0 * lda : A + r0 + (long long)k0 * lda);
-      const long long ld = t == sidx ? TB : lda;
-      const int kb = t == sidx ? TB : min(TB, n - k0);
-      const int rows = t == sidx ? TB : (TRANS ? kb : rb), cols = t == sidx ? TB : (TRANS ? rb : kb);
+      const bool inv = t == sidx && !subst;
+      const double* g = inv ? D + (size_t)b * (TB * TB)
+                            : (TRANS ? A + k0 + (long long)r0 * lda : A + r0 + (long long)k0 * lda);
+      const long long ld = inv ? TB : lda;
+      const int kb = inv ? TB : min(TB, n - k0);
+      const int rows = inv ? TB : (TRANS ? kb : rb), cols = inv ? TB : (TRANS ? rb : kb);
 #pragma unroll 4
       for (int idx = tid; idx < TB * TB; idx += 256) {
         const int i = idx & (TB - 1), j = idx >> 6;
@@ -177,10 +201,12 @@ trsv64_chain_kernel(const double* __restrict__ A, long long lda, int n, int forw
   __syncthreads();
   if (tid < TB) vs[r] = bv - ((part[0][r] + part[1][r]) + (part[2][r] + part[3][r]));
   __syncthreads();
-  {
+  const double* T = trsv_ring + (sidx % TRING) * TSLOT;
+  if (__builtin_expect(subst, false)) {
+    substitute_tile<TRANS>(forward, rb, T, vs, part[0]);
+  } else {
     // x = inv(T_bb) v over the triangle only, so that an Inf or NaN in v
     // reaches no row that does not depend on it
-    const double* T = trsv_ring + (sidx % TRING) * TSLOT;
     acc = 0.0;
 #pragma unroll
     for (int kk = 0; kk < 16; ++kk) {
@@ -200,7 +226,7 @@ trsv64_chain_kernel(const double* __restrict__ A, long long lda, int n, int forw
 
 template <bool TRANS>
 cudaError_t launch_chain(const double* A, long long lda, int n, bool forward, const double* D,
-                         const double* src, long long lds, const int* gather, double* dst,
+                         const int* flags, const double* src, long long lds, const int* gather, double* dst,
                          long long ldd, const int* scatter, const int* maps, int nrhs, int* ticket,
                          unsigned long long* words, uint32_t epoch, int* status, cudaStream_t s) {
   constexpr int smem = TRING * TSLOT * (int)sizeof(double);
@@ -208,19 +234,19 @@ cudaError_t launch_chain(const double* A, long long lda, int n, bool forward, co
   static const cudaError_t attr = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   SL_TRY(attr);
   count_launches(1);
-  return launch_after(kern, dim3((n + TB - 1) / TB * nrhs), 256, smem, s, A, lda, n, forward ? 1 : 0, D, src, lds, gather,
+  return launch_after(kern, dim3((n + TB - 1) / TB * nrhs), 256, smem, s, A, lda, n, forward ? 1 : 0, D, flags, src, lds, gather,
                       dst, ldd, scatter, maps, nrhs, ticket, words, epoch, status, spin_limit());
 }
 
 }  // namespace
 
 cudaError_t trsv64_chain(bool lower, bool trans, const double* A, long long lda, int n, const double* D,
-                         const double* src, long long lds, const int* gather, double* dst,
+                         const int* flags, const double* src, long long lds, const int* gather, double* dst,
                          long long ldd, const int* scatter, const int* maps, int nrhs, int* ticket,
                          unsigned long long* words, uint32_t epoch, int* status, cudaStream_t s) {
   const bool forward = lower != trans;
   auto launch = trans ? launch_chain<true> : launch_chain<false>;
-  return launch(A, lda, n, forward, D, src, lds, gather, dst, ldd, scatter, maps, nrhs, ticket, words, epoch, status, s);
+  return launch(A, lda, n, forward, D, flags, src, lds, gather, dst, ldd, scatter, maps, nrhs, ticket, words, epoch, status, s);
 }
 
 }  // namespace sl

@@ -363,6 +363,72 @@ def test_chained_solve_edges(sl, gpu_required, n, nrhs, trans):
     assert (res / scale < 16.0).all()  # the tester's bound
 
 
+def _triangle(kind, n, seed):
+    """Triangles with large inverses that are their own LU factors."""
+    r = np.random.default_rng(seed)
+    if kind == "uniform":
+        return np.triu(r.uniform(-0.5, 0.5, (n, n)))
+    if kind == "normal":
+        return np.triu(r.standard_normal((n, n)))
+    if kind == "lower":  # inv(L) doubles with every row
+        return np.tril(-np.ones((n, n)), -1) + np.eye(n)
+    # rows of very different size: 1/u_ii and u_ij/u_ii leave the range of a double
+    a = np.triu(r.uniform(-0.5, 0.5, (n, n))) + np.eye(n)
+    a[0, 0] *= 1e-200
+    a[0, 1:] *= 1e110
+    a[n // 2, n // 2] *= 2.0**-1030
+    a[n // 2, n // 2 + 1:] *= 2.0**-1030
+    a[:n // 2, n // 2] *= 2.0**-1030
+    return a
+
+
+@pytest.mark.parametrize("trans", ["N", "T"])
+@pytest.mark.parametrize("nrhs", [1, 16, 128, 129, 300])
+@pytest.mark.parametrize("kind,n,seed", [("uniform", 32, 0), ("uniform", 32, 1), ("normal", 32, 2), ("uniform", 64, 0),
+                                         ("uniform", 100, 3), ("uniform", 300, 4), ("lower", 60, 0), ("lower", 200, 0)])
+def test_solve_with_ill_conditioned_triangles(sl, gpu_required, kind, n, seed, nrhs, trans):
+    """Diagonal blocks whose inverses are large are solved as accurately as by substitution:
+    the tester's bound, which their inverses miss by up to 12 orders of magnitude."""
+    import torch
+
+    A = _triangle(kind, n, seed)
+    op = A if trans == "N" else A.T
+    B = op @ np.random.default_rng(seed).uniform(-1, 1, (n, nrhs))
+    dA, dB = torch.from_numpy(A.T.copy()).cuda(), torch.from_numpy(B.T.copy()).cuda()
+    ip = torch.zeros(n, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    assert sl.dgetrf_dev(n, n, dA.data_ptr(), n, ip.data_ptr()) == 0
+    assert torch.equal(dA.cpu(), torch.from_numpy(A.T.copy()))
+    assert sl.dgetrs_dev(trans, n, nrhs, dA.data_ptr(), n, ip.data_ptr(), dB.data_ptr(), n) == 0
+    X = dB.T.cpu().numpy()
+    res = np.abs(B - op @ X).max(axis=0) / (np.abs(op).sum(axis=1).max() * np.abs(X).max(axis=0) * n * 2.0**-53)
+    assert (res < RESID_THRESH).all(), res.max()
+
+
+@pytest.mark.parametrize("trans", ["N", "T"])
+@pytest.mark.parametrize("nrhs", [1, 129, 300])
+@pytest.mark.parametrize("n", [20, 90])
+def test_solve_with_rows_of_extreme_size(sl, gpu_required, n, nrhs, trans):
+    """A subnormal diagonal entry, and a row whose quotients by its own leave the range: no
+    overflow that a substitution does not have."""
+    import torch
+
+    A = _triangle("extreme", n, 5)
+    x0 = np.random.default_rng(n).uniform(0.5, 1, (n, nrhs))
+    x0[0] = 1e-120  # (T: u_0j x_0 far below the others)
+    B = (A if trans == "N" else A.T) @ x0
+    dA, dB = torch.from_numpy(A.T.copy()).cuda(), torch.from_numpy(B.T.copy()).cuda()
+    ip = torch.arange(1, n + 1, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    assert sl.dgetrs_dev(trans, n, nrhs, dA.data_ptr(), n, ip.data_ptr(), dB.data_ptr(), n) == 0
+    X = dB.T.cpu().numpy()
+    assert np.isfinite(X).all()
+    op = np.abs(A if trans == "N" else A.T)
+    # componentwise: |b - op x| <= n eps |op| |x| for either order of the sums (Higham, 8.5)
+    r = np.abs(B - (A if trans == "N" else A.T) @ X)
+    assert (r <= 4 * n * 2.0**-53 * (op @ np.abs(X)) + 2.0**-1040).all()
+
+
 def test_chained_solve_on_reused_dirty_memory(sl, gpu_required):
     """The chained solve's words start cleared in every buffer they grow into, also
     when it stands at the old one's address among memory that holds the epochs
