@@ -785,7 +785,7 @@ int sl1x1_dgesv_ir_dev(int n, int nrhs, double* dA, long long ldda, int* dipiv, 
   sl::IrOptions opt;
   opt.fmt = fmt;
   opt.nb = nb > 0 ? nb : 256;
-  opt.nb_fp64 = g_default_nb;
+  opt.nb_fp64 = factor_nb(n, n, g_default_nb);
   if (tol > 0) opt.tol = tol;
   opt.fp64_cost_ratio = g_ir_cost_ratio;
   ensure_oz(n, n, opt.nb_fp64);  // the FP64 fallback factorization

@@ -186,49 +186,10 @@ static cudaError_t lu_update(const OzScratch& sc, int m, int n, int k, double al
   return dgemm(false, m, n, k, alpha, A, lda, B, ldb, 1.0, C, ldc, s);
 }
 
-// Inverse of a 64x64 unit-lower block by column-oriented substitution, all
-// columns at once: X = I, then for each pivot row q, row q of X is final and
-// every later row i loses T(i,q) X(q,:). 256 threads own 16 entries of X each,
-// one shared barrier per step: 64 steps instead of a 2000-long dependent chain.
-// Ts and X are 64 x 65 shared arrays; returns with X = inv(T).
-__device__ __forceinline__ void unit_lower_inv64_block(double (*Ts)[65], double (*X)[65]) {
-  const int t = threadIdx.x & 63, ib = threadIdx.x >> 6;  // column t, rows ib, ib+4, ...
-  for (int q = 0; q < 63; ++q) {
-    const double xq = X[q][t];
-    if (t <= q)
-      for (int i = q + 1 + ((ib - (q + 1)) & 3); i < 64; i += 4) X[i][t] = fma(-Ts[i][q], xq, X[i][t]);
-    __syncthreads();
-  }
-}
-
-// N_b = inv(L_bb) - I for the 64x64 diagonal blocks of the unit-lower L11
-// (jb x jb, leading dimension ldl): block b at Ninv + b*4096, column-major
-// with leading dimension 64; a partial last block is padded with the
-// identity.
-__global__ void __launch_bounds__(256)
-unit_lower_inv64_kernel(int jb, const double* __restrict__ L, long long ldl, double* Ninv) {
-  extern __shared__ double inv_smem[];  // Ls[64][65] then X[64][65]
-  double(*Ls)[65] = reinterpret_cast<double(*)[65]>(inv_smem);
-  double(*X)[65] = reinterpret_cast<double(*)[65]>(inv_smem + 64 * 65);
-  const int b = blockIdx.x;
-  const int r0 = b * 64, rb = min(64, jb - r0);
-  for (int idx = threadIdx.x; idx < 64 * 64; idx += 256) {
-    const int r = idx & 63, c = idx >> 6;  // coalesced along rows
-    Ls[r][c] = (r < rb && c < r) ? L[(r0 + r) + (long long)(r0 + c) * ldl] : 0.0;
-    X[r][c] = (r == c) ? 1.0 : 0.0;
-  }
-  __syncthreads();
-  unit_lower_inv64_block(Ls, X);
-  double* Nb = Ninv + (size_t)b * 4096;
-  for (int idx = threadIdx.x; idx < 64 * 64; idx += 256) {
-    const int i = idx & 63, c = idx >> 6;
-    Nb[i + 64 * c] = (i > c) ? X[i][c] : 0.0;
-  }
-}
-
-// Largest NB whose whole inv(L11) - I is formed at the end of the panel (the
-// U12 solve is then one product); larger blocks use 64-row inverses.
+// Largest NB whose inv(L11) - I is formed at the end of the panel (the U12 solve is
+// then one product): the widest that factor_nb gives when blocks follow.
 constexpr int kFullInvMax = 256;
+static_assert(kDinv64Doubles >= (size_t)kFullInvMax * kFullInvMax, "inverse of L11");
 
 // X = inv(L) - I for a unit-lower jb x jb L (jb <= 256): forward substitution of
 // x = e_c per column c, in the order of a strip solve. A CTA takes the columns p
@@ -302,29 +263,16 @@ unit_lower_inv_cols_kernel(int jb, const double* __restrict__ L, long long ldl, 
   }
 }
 
-// U12 = L11^-1 A12 (jb x nr, in place). With the sliced product and inverses
-// of L11 at hand (formed at the end of its panel): for jb <= 256,
-// U12 = A12 + (inv(L11) - I) A12 as one product; otherwise per 64-row block
-// b, X_b = A12_b + (inv(L_bb) - I) A12_b, then the rows below lose
-// L(below, b) X_b -- every product on the tensor cores, the inverse products
-// balanced by the rows of A12, which carry the pivots' scales. Otherwise the
-// FP64 strip solve.
+// U12 = L11^-1 A12 (jb x nr, in place): with the sliced product and the inverse of L11
+// at hand (formed at the end of its panel), A12 + (inv(L11) - I) A12 as one product,
+// balanced by the rows of A12, which carry the pivots' scales. Otherwise the FP64
+// strip solve.
 static cudaError_t solve_u12(int jb, int nr, const double* L11, long long ldl, double* A12,
                              long long lda, const LuWork& ws, cudaStream_t s, int max_ctas = 0) {
   if (g_f64_update == 1 && ws.dinv64 && jb <= kFullInvMax && oz_fits(ws.oz, jb, nr, jb))
     return oz_dgemm_bside(ws.oz, jb, nr, jb, 1.0, ws.dinv64, jb, A12, lda, A12, lda, ws.status, s,
                           max_ctas);
-  if (!(g_f64_update == 1 && ws.dinv64 && jb <= 1024 && oz_fits(ws.oz, jb, nr, 64)))
-    return trsm_strip<double, false, false, true>(jb, nr, L11, ldl, A12, lda, s);
-  for (int r0 = 0; r0 < jb; r0 += 64) {
-    const int w = (jb - r0) < 64 ? (jb - r0) : 64;
-    SL_TRY(oz_dgemm_bside(ws.oz, w, nr, w, 1.0, ws.dinv64 + (size_t)(r0 / 64) * 4096, 64,
-                          A12 + r0, lda, A12 + r0, lda, ws.status, s));
-    if (r0 + w < jb)
-      SL_TRY(oz_dgemm(ws.oz, jb - r0 - w, nr, w, -1.0, L11 + (r0 + w) + (long long)r0 * ldl, ldl,
-                      A12 + r0, lda, A12 + r0 + w, lda, ws.status, s));
-  }
-  return cudaSuccess;
+  return trsm_strip<double, false, false, true>(jb, nr, L11, ldl, A12, lda, s);
 }
 
 // PDGETF2 on columns [j, j+jb), rows [j, m): 32-wide cooperative sub-panels,
@@ -422,14 +370,6 @@ static cudaError_t factor_panel(int m, int n, double* dA, long long ldda, int* d
   } else if (want_plan) {
     SL_TRY(laswp_plan(j, j + npiv, dipiv, ws.swap_plan, s));
   }
-  if (more && g_f64_update == 1 && ws.dinv64 && npiv == jb && jb > kFullInvMax && jb <= 1024) {
-    constexpr int kInvSmem = 2 * 64 * 65 * (int)sizeof(double);
-    static const cudaError_t attr = cudaFuncSetAttribute(
-        unit_lower_inv64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kInvSmem);
-    SL_TRY(attr);
-    unit_lower_inv64_kernel<<<(jb + 63) / 64, 256, kInvSmem, s>>>(jb, Ap(j, j), ldda, ws.dinv64);
-    count_launches(1);
-  }
   phase_end(kPhPanelInverse, s, (double)jb * jb * jb / 3.0, 16.0 * (double)jb * jb);
   phase_end(kPhPanel, s, pflops, 16.0 * (double)(m - j) * jb);
   return cudaSuccess;
@@ -473,9 +413,7 @@ static cudaError_t step0_by_chunks(int m, int n, double* dA, long long ldda, int
   LuWork w0 = ws;
   w0.swap_plan = nullptr;
   if (g_f64_update == 1 && ws.dinv64) {
-    SL_TRY(cudaMemcpyAsync(ws.dinv64_step0, ws.dinv64,
-                           (jb <= kFullInvMax ? (size_t)jb * jb : (size_t)((jb + 63) / 64) * 4096) * sizeof(double),
-                           cudaMemcpyDeviceToDevice, s));
+    SL_TRY(cudaMemcpyAsync(ws.dinv64_step0, ws.dinv64, kDinv64Doubles * sizeof(double), cudaMemcpyDeviceToDevice, s));
     w0.dinv64 = ws.dinv64_step0;
   }
   SL_TRY(cudaEventRecord(ws.ev_next, s));

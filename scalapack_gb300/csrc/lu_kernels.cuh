@@ -1716,8 +1716,9 @@ inline cudaError_t launch_panel(T* A, long long lda, int m, int r0, int c0, int 
     while (cs < CMAXG && R > 32 * cs) cs *= 2;
     int crpc = ((R + cs - 1) / cs + 7) & ~7;
     const size_t csmem = panel_inbox_bytes<T>() + (sizeof(T) * PLD + sizeof(int)) * (size_t)crpc;
+    constexpr int kWide = sizeof(T) == 4 ? 2 * PTR : PTR;  // (FP64 rows per CTA never pass PTR)
     static const cudaError_t at = [] {
-      for (const void* f : {(const void*)panel_cluster_kernel<T, PTR>, (const void*)panel_cluster_kernel<T, 2 * PTR>}) {
+      for (const void* f : {(const void*)panel_cluster_kernel<T, PTR>, (const void*)panel_cluster_kernel<T, kWide>}) {
         cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         if (e != cudaSuccess) return e;
@@ -1733,7 +1734,7 @@ inline cudaError_t launch_panel(T* A, long long lda, int m, int r0, int c0, int 
     la[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // (see launch_after)
     la[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.gridDim = dim3(cs);
-    const int ntr = crpc > PTR ? 2 * PTR : PTR;
+    const int ntr = crpc > PTR ? kWide : PTR;
     cfg.blockDim = dim3(ntr + 32);
     cfg.dynamicSmemBytes = csmem;
     cfg.stream = s;
@@ -1741,7 +1742,7 @@ inline cudaError_t launch_panel(T* A, long long lda, int m, int r0, int c0, int 
     cfg.numAttrs = after_kernel ? 2 : 1;
     int ctpr = crpc > PTR / 4 ? 1 : (crpc > PTR / 8 ? 2 : 4);
     count_launches(1);
-    auto kern = ntr == PTR ? panel_cluster_kernel<T, PTR> : panel_cluster_kernel<T, 2 * PTR>;
+    auto kern = ntr == PTR ? panel_cluster_kernel<T, PTR> : panel_cluster_kernel<T, kWide>;
     return cudaLaunchKernelEx(&cfg, kern, A, lda, m, r0, c0, w, crpc, ipiv, ws.info_col, ws.status,
                               spin_limit(), ctpr);
   }

@@ -128,7 +128,7 @@ struct LuWork {
   cudaEvent_t ev_next = nullptr;
   cudaEvent_t ev_panel = nullptr;
   // Sliced-product scratch for the caller's stream and for the panel's
-  // stream, and 64x64 FP64 blocks for the U12 solve (kDinv64Doubles).
+  // stream, and the inverse of L11 for the U12 solve (kDinv64Doubles).
   OzScratch oz, oz_aux;
   double* dinv64 = nullptr;
   // Solve: inverses of the 64x64 diagonal blocks of L then of U
@@ -185,8 +185,8 @@ inline int* solve_inv_flags(double* dinv_solve, int n) {
 // Right-hand sides from which a blocked NOTRAN solve shares a CTA's staged blocks
 // among several of them.
 constexpr int kWideRhs = 256;
-// Doubles of the U12 solve's diagonal-block inverses: NB <= 1024 in 64-row blocks.
-constexpr size_t kDinv64Doubles = (size_t)16 * 64 * 64;
+// Doubles of the U12 solve's inv(L11) - I, NB <= 256.
+constexpr size_t kDinv64Doubles = (size_t)256 * 256;
 // Columns up to which a matrix may be factored as one panel (factor_nb).
 constexpr int kOnePanelMax = 1536;
 
