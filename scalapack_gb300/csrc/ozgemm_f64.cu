@@ -64,8 +64,8 @@
 // ex B(k,j)). Where any row (column) is more than OZ_BUDGET bits above it (a
 // row of A small exactly where a row of B holds an entry far above the rest),
 // or a scale leaves the normal FP64 range, the whole pass is computed in FP64
-// arithmetic instead (fixed order, every product an FMA) by the same
-// launches. Accuracy model: each row's (column's) error is within about
+// arithmetic instead (fixed order, every product an FMA; side B: by substitution
+// with L_bb) by the same launches. Accuracy model: each row's (column's) error is within about
 // 2^OZ_BUDGET of the FP64 GEMM's error bound for its largest |A||B| term
 // (normwise per row or column); for inputs that are diagonal scalings of
 // well-scaled data that is the componentwise level. Operands whose large
@@ -194,6 +194,46 @@ __device__ __forceinline__ bool oz_issue_b(int c, int first, int nkc, int tiles_
                 t * n_pad + n0);
   *issued = c + 1;
   return true;
+}
+
+// The unit-lower factor of a side-B pass: the pass is B <- B + N B with N = inv(L) - I,
+// flags nonzero where N is not to be used.
+struct OzUnitLower {
+  const double* L = nullptr;
+  long long ldl = 0;
+  const int* flags = nullptr;
+  int nflags = 0;
+};
+
+// B <- inv(L) B by forward substitution: the FP64 route of a side-B pass. A CTA
+// takes 64 columns of B (kb <= 256 rows, 128 KB) into shared memory; thread t
+// has column t % 64 and every ninth row below the one that is final. Bound: the
+// FP64 unit: a 256-wide block that goes this way adds 0.65 ms (two such passes) to a
+// factorization of N = 4096 (13.1 ms).
+__device__ __noinline__ void oz_substitute(unsigned char* smem, int n, int kb, OzUnitLower ul, double* B,
+                                           long long ldb, int tiles_n) {
+  double* sB = reinterpret_cast<double*>(smem);  // [kb][64]
+  const int tid = threadIdx.x, c = tid & (OBN - 1), g = tid / OBN;
+  for (int t = blockIdx.x; t < tiles_n; t += gridDim.x) {
+    const int n0 = t * OBN;
+    __syncthreads();
+    for (int idx = tid; idx < kb * OBN; idx += OZ_THREADS) {
+      const int cc = idx / kb, k = idx - cc * kb;
+      sB[k * OBN + cc] = (n0 + cc < n) ? B[k + (long long)(n0 + cc) * ldb] : 0.0;
+    }
+    __syncthreads();
+    for (int q = 0; q < kb; ++q) {
+      const double x = sB[q * OBN + c];
+      const double* l = ul.L + (long long)q * ul.ldl;
+#pragma unroll 4
+      for (int r = q + 1 + g; r < kb; r += OZ_THREADS / OBN) sB[r * OBN + c] = fma(-l[r], x, sB[r * OBN + c]);
+      __syncthreads();
+    }
+    for (int idx = tid; idx < kb * OBN; idx += OZ_THREADS) {
+      const int cc = idx / kb, k = idx - cc * kb;
+      if (n0 + cc < n) B[k + (long long)(n0 + cc) * ldb] = sB[k * OBN + cc];
+    }
+  }
 }
 
 // The FP64 route of a pass whose slices would exceed the error budget: the
@@ -364,7 +404,7 @@ ozgemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
               int m, int n, int kpad, int m_pad, int n_pad, const double* __restrict__ rs,
               const double* __restrict__ cs, double alpha, double* C, long long ldc, int tpc,
               int* status, const double* __restrict__ A64, long long lda, const double* B64,
-              long long ldb, int kb, const unsigned long long* kinfo, unsigned long long epoch) {
+              long long ldb, int kb, const unsigned long long* kinfo, unsigned long long epoch, OzUnitLower ul) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   unsigned char* sA = base;                                   // A_RING x 16 KB
@@ -385,8 +425,11 @@ ozgemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
   // the slicing found the pass outside the error budget: FP64 route
   if (*(volatile const unsigned long long*)(kinfo + OZ_KI_FLAG) == epoch) {
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&g_oz_fp64_routes, 1ULL);
-    oz_fp64_tiles(base, m, n, kb, A64, lda, B64, ldb, alpha, C, ldc, first_tile, my_tiles,
-                  tiles_m, tiles_n, B64 == C ? 1 : 0);
+    if (ul.L)
+      oz_substitute(base, n, kb, ul, C, ldc, tiles_n);
+    else
+      oz_fp64_tiles(base, m, n, kb, A64, lda, B64, ldb, alpha, C, ldc, first_tile, my_tiles,
+                    tiles_m, tiles_n, B64 == C ? 1 : 0);
     return;
   }
 
@@ -704,13 +747,16 @@ oz_kscale_kernel(const double* __restrict__ A, long long lda, int m, const doubl
 // that: 8 columns of B (kb x n, column-major, a column contiguous in k) each,
 // one warp per column; slices Sb[t][j][kk] cut against f_j - d_k, and on side
 // B the column's test. Padding rows, columns and k are zero; so is every k
-// whose column of A or row of B is zero (its products vanish).
+// whose column of A or row of B is zero (its products vanish). ul.L set: side B, and
+// a flag sends the pass to the FP64 route.
 __global__ void __launch_bounds__(256)
 oz_split_kernel(const double* __restrict__ A, long long lda, int m, const double* __restrict__ B,
                 long long ldb, int n, int kb, int kpad, int m_pad, int n_pad,
                 __nv_bfloat16* Sa, __nv_bfloat16* Sb, double* rs, double* cs,
-                unsigned long long* kinfo, unsigned long long epoch, int side_b) {
+                unsigned long long* kinfo, unsigned long long epoch, OzUnitLower ul) {
   __shared__ int s_c[OZ_KMAX], s_h[OZ_KMAX], s_d[OZ_KMAX];
+  const bool side_b = ul.L != nullptr;
+  if (blockIdx.x == 0 && (int)threadIdx.x < ul.nflags && ul.flags[threadIdx.x]) atomicMax(kinfo + OZ_KI_FLAG, epoch);
   // A blocks: the CTA's 32 rows x kpad of A, as bits, sA[kk * 33 + row],
   // loaded once (before the balancing words, so both reads overlap) and read
   // by the budget test and the slicing
@@ -1152,7 +1198,7 @@ unsigned long long* oz_hkeys(const OzScratch& sc) {
 // C (m x n) += alpha * A (m x k) * B (k x n), all FP64 column-major, through
 // the sliced BF16 product; K is taken in passes of at most 256, each with its
 // own balancing, budget test and (when the test trips) FP64 route.
-static cudaError_t oz_dgemm_impl(int side_b, unsigned long long keyed_epoch, const OzScratch& sc,
+static cudaError_t oz_dgemm_impl(const OzUnitLower& ul, unsigned long long keyed_epoch, const OzScratch& sc,
                                  int m, int n, int k, double alpha, const double* A, long long lda,
                                  const double* B, long long ldb, double* C, long long ldc,
                                  int* status, cudaStream_t s, int max_ctas = 0) {
@@ -1161,7 +1207,7 @@ static cudaError_t oz_dgemm_impl(int side_b, unsigned long long keyed_epoch, con
   if (keyed_epoch && k > OZ_KMAX) return cudaErrorInvalidValue;
   SL_TRY(oz_smem_once());
   const int m_pad = round_up(m, OBM), n_pad = round_up(n, OBN);
-  if (keyed_epoch && !side_b && k <= 64 && oz_one_launch(m, n)) {
+  if (keyed_epoch && !ul.L && k <= 64 && oz_one_launch(m, n)) {
     unsigned long long* kinfo = reinterpret_cast<unsigned long long*>(sc.ptr);
     auto kern = k <= 32 ? oz_tile_kernel<32> : oz_tile_kernel<64>;
     count_launches(1);
@@ -1187,7 +1233,7 @@ static cudaError_t oz_dgemm_impl(int side_b, unsigned long long keyed_epoch, con
     }
     oz_split_kernel<<<m_pad / 32 + n_pad / 8, 256, oz_split_smem(kpad), s>>>(Ak, lda, m, Bk, ldb, n, kb, kpad, m_pad,
                                                           n_pad, sa, sb, rs, cs, kinfo, epoch,
-                                                          side_b);
+                                                          ul);
     CUtensorMap ta, tb;
     if (!make_slice_map(&ta, sa, OZ_S * m_pad, kpad, OBM) ||
         !make_slice_map(&tb, sb, OZ_S * n_pad, kpad, OBN))
@@ -1201,7 +1247,7 @@ static cudaError_t oz_dgemm_impl(int side_b, unsigned long long keyed_epoch, con
     const int grid = (tiles + tpc - 1) / tpc;
     ozgemm_kernel<<<grid, OZ_THREADS, oz_smem_bytes(), s>>>(ta, tb, m, n, kpad, m_pad, n_pad, rs,
                                                             cs, alpha, C, ldc, tpc, status, Ak,
-                                                            lda, Bk, ldb, kb, kinfo, epoch);
+                                                            lda, Bk, ldb, kb, kinfo, epoch, ul);
     count_launches(2);
     SL_TRY(cudaGetLastError());
   }
@@ -1211,20 +1257,26 @@ static cudaError_t oz_dgemm_impl(int side_b, unsigned long long keyed_epoch, con
 cudaError_t oz_dgemm(const OzScratch& sc, int m, int n, int k, double alpha, const double* A,
                      long long lda, const double* B, long long ldb, double* C, long long ldc,
                      int* status, cudaStream_t s, int max_ctas) {
-  return oz_dgemm_impl(0, 0ULL, sc, m, n, k, alpha, A, lda, B, ldb, C, ldc, status, s, max_ctas);
+  return oz_dgemm_impl(OzUnitLower(), 0ULL, sc, m, n, k, alpha, A, lda, B, ldb, C, ldc, status, s, max_ctas);
 }
 
 cudaError_t oz_dgemm_keyed(const OzScratch& sc, unsigned long long epoch, int m, int n, int k,
                            double alpha, const double* A, long long lda, const double* B,
                            long long ldb, double* C, long long ldc, int* status, cudaStream_t s,
                            int max_ctas) {
-  return oz_dgemm_impl(0, epoch, sc, m, n, k, alpha, A, lda, B, ldb, C, ldc, status, s, max_ctas);
+  return oz_dgemm_impl(OzUnitLower(), epoch, sc, m, n, k, alpha, A, lda, B, ldb, C, ldc, status, s, max_ctas);
 }
 
-cudaError_t oz_dgemm_bside(const OzScratch& sc, int m, int n, int k, double alpha,
-                           const double* A, long long lda, const double* B, long long ldb,
-                           double* C, long long ldc, int* status, cudaStream_t s, int max_ctas) {
-  return oz_dgemm_impl(1, 0ULL, sc, m, n, k, alpha, A, lda, B, ldb, C, ldc, status, s, max_ctas);
+cudaError_t oz_unit_lower_solve(const OzScratch& sc, int m, int n, const double* N, long long ldn,
+                                const double* L, long long ldl, const int* flags, int nflags, double* B,
+                                long long ldb, int* status, cudaStream_t s, int max_ctas) {
+  if (m > OZ_KMAX || nflags > OZ_KMAX) return cudaErrorInvalidValue;
+  OzUnitLower ul;
+  ul.L = L;
+  ul.ldl = ldl;
+  ul.flags = flags;
+  ul.nflags = nflags;
+  return oz_dgemm_impl(ul, 0ULL, sc, m, n, m, 1.0, N, ldn, B, ldb, B, ldb, status, s, max_ctas);
 }
 
 }  // namespace sl

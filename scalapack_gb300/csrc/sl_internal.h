@@ -76,12 +76,14 @@ bool oz_fits(const OzScratch& sc, int m, int n, int k);
 cudaError_t oz_dgemm(const OzScratch& sc, int m, int n, int k, double alpha, const double* A,
                      long long lda, const double* B, long long ldb, double* C, long long ldc,
                      int* status, cudaStream_t s, int max_ctas = 0);
-// The same balanced by the row maxima of B, with the budget tested per
-// column: for A = inv(T) - I of a unit-lower diagonal block T and B the rows
-// it updates (the U12 solve), whose rows carry the pivots' scales.
-cudaError_t oz_dgemm_bside(const OzScratch& sc, int m, int n, int k, double alpha,
-                           const double* A, long long lda, const double* B, long long ldb,
-                           double* C, long long ldc, int* status, cudaStream_t s, int max_ctas = 0);
+// B <- inv(L) B for a unit-lower L (m x m, m <= 256) as B + (inv(L) - I) B, inv(L) - I
+// at N (the U12 solve): the same product balanced by the row maxima of B, which
+// carry the pivots' scales, with the budget tested per column. Where a word of
+// flags (nflags <= 256 of them) is not zero, or a column is beyond the budget, the same
+// launches solve by substitution with L.
+cudaError_t oz_unit_lower_solve(const OzScratch& sc, int m, int n, const double* N, long long ldn,
+                                const double* L, long long ldl, const int* flags, int nflags, double* B,
+                                long long ldb, int* status, cudaStream_t s, int max_ctas = 0);
 // The same (side A) with the balancing keys of its single pass (k <= 256)
 // already published with `epoch` (from oz_new_epoch) into oz_ckeys(sc) and
 // oz_hkeys(sc) by the kernels that produced A and B: one launch fewer.
@@ -185,8 +187,10 @@ inline int* solve_inv_flags(double* dinv_solve, int n) {
 // Right-hand sides from which a blocked NOTRAN solve shares a CTA's staged blocks
 // among several of them.
 constexpr int kWideRhs = 256;
-// Doubles of the U12 solve's inv(L11) - I, NB <= 256.
-constexpr size_t kDinv64Doubles = (size_t)256 * 256;
+// Doubles of the U12 solve's inv(L11) - I, NB <= 256, and behind it an int per pair of
+// its columns, nonzero where the inverse is not to be used (unit_lower_inv_cols_kernel).
+constexpr size_t kDinvFlagsAt = (size_t)256 * 256;
+constexpr size_t kDinv64Doubles = kDinvFlagsAt + 64;
 // Columns up to which a matrix may be factored as one panel (factor_nb).
 constexpr int kOnePanelMax = 1536;
 

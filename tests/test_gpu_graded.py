@@ -180,3 +180,34 @@ def test_in_panel_tile_beyond_budget(sl, gpu_required, m, ib):
     t = np.isin(row, tiny)
     assert (err[t] <= 16.0 * n * 2.0**-53 * mag[t]).all()
     assert np.nanmax(err) < 16.0 * n * 2.0**-53 * np.abs(A).sum(axis=1).max()
+
+
+def _large_inverse_matrix(n, scale, seed):
+    """A = L U whose unit-lower L has diagonal blocks with large inverses: entries uniform on
+    [-scale, scale] within the first 256 columns, small ones beyond; U with a heavy
+    diagonal, so that the pivots are the diagonal."""
+    r = np.random.default_rng(seed)
+    L = np.tril(r.uniform(-1, 1, (n, n)), -1)
+    L[:, :256] *= scale
+    L[:, 256:] *= 0.02
+    U = np.triu(r.uniform(-0.5, 0.5, (n, n)), 1) + np.diag(r.uniform(1, 2, n))
+    return np.asfortranarray((L + np.eye(n)) @ U)
+
+
+@pytest.mark.parametrize("lookahead", [1, 0])
+@pytest.mark.parametrize("n,nb,scale", [(1700, 64, 0.5), (1700, 256, 0.9), (2100, 320, 0.9)])
+def test_u12_with_a_large_inverse(sl, orc, ctx, n, nb, scale, lookahead):
+    """A block whose inv(L11) is large has U12 formed by substitution: the factors keep the
+    tester's bound, which the product with the inverse misses by many orders."""
+    A0 = _large_inverse_matrix(n, scale, n)
+    B0 = np.asfortranarray(orc.matgen(n, 2, 200, kind=1))
+    r0 = _routes(sl)
+    sl.lib().sl1x1_set_lookahead(lookahead)
+    try:
+        info, LU, rel, X = run_pdgesv(sl, ctx, A0, B0, nb)
+    finally:
+        sl.lib().sl1x1_set_lookahead(1)
+    assert info == 0
+    assert _routes(sl) > r0
+    assert orc.fresid(LU, rel, A0) < RESID_THRESH
+    assert orc.sresid(A0, B0, X) < RESID_THRESH
