@@ -212,11 +212,12 @@ int factor_nb(int m, int n, int nb) {
 
 // Grows a sliced-product scratch buffer; a new one starts with its balancing
 // words zeroed (the memory may hold anything, including words that look like
-// a later epoch's).
+// a later epoch's). It is told by its size: it may come back at the old one's
+// address, and another thread of the program may have had that memory meanwhile.
 static cudaError_t grow_oz(unsigned char** p, size_t* cap, size_t need) {
-  const unsigned char* old = *p;
+  const size_t old = *cap;
   cudaError_t e = grow(p, cap, need);
-  if (e == cudaSuccess && *p != old)
+  if (e == cudaSuccess && *cap != old)
     e = cudaMemset(*p, 0, *cap < (size_t)sl::kOzKinfoBytes ? *cap : (size_t)sl::kOzKinfoBytes);
   return e;
 }
