@@ -574,6 +574,51 @@ __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
+// What all CTAs send one of them per column.
+template <typename T>
+__host__ __device__ constexpr uint32_t panel_column_bytes(int CS) {
+  return (uint32_t)(CS * (16 + (sizeof(T) == 8 ? 8 : 0) + PW * sizeof(T)));
+}
+
+// After a give-up, by all threads of CTA b (sent: what panel_cluster_kernel keeps in
+// s_sent, the same on every CTA): its first warp sends the column that others have
+// begun and it has not, and the CTA waits for all that it was sent.
+template <typename T>
+__device__ __noinline__ void panel_cluster_finish(const int* sent, int CS, int b, uint32_t bar0, uint32_t in0) {
+  const int lane = threadIdx.x & 31;
+  int most = 0;
+  for (int q = 0; q < CS; ++q) most = max(most, sent[q]);
+  if (threadIdx.x < 32)
+    for (int c = sent[b]; c < most; ++c) {
+      const uint32_t bar = bar0 + 8 * (c % 3);
+      const uint32_t slot = in0 + (uint32_t)((c % 3 * CMAXG + b) * sizeof(PanelInbox<T>));
+      if (lane == 0)
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(panel_column_bytes<T>(CS))
+                     : "memory");
+      // (zeros, in pieces of 8 bytes: key and label, reciprocal, row)
+      for (int q = 0; q < CS; ++q) {
+        constexpr int kHead = sizeof(T) == 8 ? 3 : 2;
+        for (int i = lane; i < kHead + (int)(PW * sizeof(T) / 8); i += 32)
+          asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(
+                           cluster_addr(slot + 8 * (i < kHead ? i : i - kHead + 4), q)),
+                       "l"(0LL), "r"(cluster_addr(bar, q))
+                       : "memory");
+      }
+    }
+  __syncthreads();
+  for (int c = max(0, most - 3); c < most; ++c)
+    for (long long spins = 0; spins < kSpinLimit; ++spins) {
+      uint32_t done;
+      asm volatile(
+          "{\n .reg .pred p;\n mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+          " selp.u32 %0, 1, 0, p;\n}\n"
+          : "=r"(done)
+          : "r"(bar0 + 8 * (c % 3)), "r"((uint32_t)((c / 3) & 1))
+          : "memory");
+      if (done) break;
+    }
+}
+
 // NTR row threads and the reciprocal's warp; a row thread has at most one row (rpc *
 // tpr <= NTR), whose label stays in a register.
 template <typename T, int NTR>
@@ -589,7 +634,8 @@ panel_cluster_kernel(T* A, long long lda, int m, int r0, int c0, int w, int rpc,
   __shared__ long long s_wk[2][NW];
   __shared__ int s_wr[2][NW], s_wl[2][NW];
   __shared__ int s_fail[2];       // a wait gave up, by column parity
-  __shared__ int s_sent[CMAXG];   // 2 x columns each CTA has sent, + 1 if it gave up
+  __shared__ int s_sent[CMAXG];   // columns each CTA has sent
+  __shared__ int s_any;           // some CTA gave up
 
   const int CS = gridDim.x, b = blockIdx.x, tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
@@ -600,9 +646,9 @@ panel_cluster_kernel(T* A, long long lda, int m, int r0, int c0, int w, int rpc,
   const int nr = max(0, min(rpc, R - lo));
   const uint32_t bar0 = (uint32_t)__cvta_generic_to_shared(s_bar);
   const uint32_t in0 = (uint32_t)__cvta_generic_to_shared(inbox);
-  if (tid < CMAXG) s_sent[tid] = 2 * kw;
+  if (tid < CMAXG) s_sent[tid] = kw;
   if (tid == 0) {
-    s_fail[0] = s_fail[1] = 0;
+    s_fail[0] = s_fail[1] = s_any = 0;
     for (int i = 0; i < 3; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0 + 8 * i));
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -662,71 +708,21 @@ panel_cluster_kernel(T* A, long long lda, int m, int r0, int c0, int w, int rpc,
     row[j] = fma(-l, u, v);
   };
 
-  // column c of a CTA: bytes that each CTA receives from all of them
-  const uint32_t col_bytes = (uint32_t)(CS * (16 + (sizeof(T) == 8 ? 8 : 0) + PW * sizeof(T)));
-  auto expect_column = [&](int c) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar0 + 8 * (c % 3)), "r"(col_bytes)
-                 : "memory");
-  };
-  // one warp sends this CTA's candidate of column c (its key, label and row) to every
-  // CTA's inbox, and for FP64 one warp the reciprocal of its magnitude
-  auto send_candidate = [&](int c, long long ckey, long long clabel, T v) {
-    const int buf = c % 3;
-    const uint32_t slot = in0 + (uint32_t)((buf * CMAXG + b) * sizeof(PanelInbox<T>));
-    if (lane < CS)
-      asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];" ::"r"(
-                       cluster_addr(slot, lane)),
-                   "l"(ckey), "l"(clabel), "r"(cluster_addr(bar0 + 8 * buf, lane))
-                   : "memory");
-    const uint32_t mine = slot + 32 + (uint32_t)(lane * sizeof(T));
-    for (int q = 0; q < CS; ++q) {
-      const uint32_t dst = cluster_addr(mine, q), bar = cluster_addr(bar0 + 8 * buf, q);
-      if constexpr (sizeof(T) == 8)
-        asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(dst),
-                     "l"(__double_as_longlong(v)), "r"(bar)
-                     : "memory");
-      else
-        asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(dst),
-                     "r"(__float_as_uint(v)), "r"(bar)
-                     : "memory");
-    }
-  };
-  auto send_reciprocal = [&](int c, double ra) {
-    const int buf = c % 3;
-    const uint32_t slot = in0 + (uint32_t)((buf * CMAXG + b) * sizeof(PanelInbox<T>));
-    if (lane < CS)
-      asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(
-                       cluster_addr(slot + 16, lane)),
-                   "l"(__double_as_longlong(ra)), "r"(cluster_addr(bar0 + 8 * buf, lane))
-                   : "memory");
-  };
-  // at most `polls` looks at whether column c of every CTA is here
-  auto column_here = [&](int c, long long polls) {
-    for (long long spins = 0; spins < polls; ++spins) {
-      uint32_t done;
-      asm volatile(
-          "{\n .reg .pred p;\n mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
-          " selp.u32 %0, 1, 0, p;\n}\n"
-          : "=r"(done)
-          : "r"(bar0 + 8 * (c % 3)), "r"((uint32_t)((c / 3) & 1))
-          : "memory");
-      if (done) return true;
-    }
-    return false;
-  };
-
   const T* Uprev = nullptr;  // pivot row of column k-1
   int k = 0;                 // columns sent
   for (; k < kw; ++k) {
     const int buf = k % 3, par = k & 1;
     __syncthreads();
-    if (k > 0 && s_fail[par ^ 1]) break;
+    if (s_fail[par ^ 1]) break;
     // --- this CTA's candidate, into every CTA's inbox ---
     long long key = lane < NW ? s_wk[par][lane] : -3;
     int label = lane < NW ? s_wr[par][lane] : INT_MAX;
     const int cw = warp_best(key, label);
     const int lrow = s_wl[par][cw];
-    if (tid == 0) expect_column(k);
+    if (tid == 0)
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar0 + 8 * buf),
+                   "r"(panel_column_bytes<T>(CS))
+                   : "memory");
     if (warp == cw) {
       // the candidate row with column k-1's update of its columns beyond k
       T v = (T)0;
@@ -734,7 +730,26 @@ panel_cluster_kernel(T* A, long long lda, int m, int r0, int c0, int w, int rpc,
         v = tile[lrow * PLD + lane];
         if (k > 0 && lane > k) v = fma(-tile[lrow * PLD + k - 1], Uprev[lane], v);
       }
-      send_candidate(k, s_wk[par][cw], s_wr[par][cw], v);
+      const uint32_t slot = in0 + (uint32_t)((buf * CMAXG + b) * sizeof(PanelInbox<T>));
+      const long long ck = s_wk[par][cw];
+      const long long cl = s_wr[par][cw];
+      if (lane < CS)
+        asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];" ::"r"(
+                         cluster_addr(slot, lane)),
+                     "l"(ck), "l"(cl), "r"(cluster_addr(bar0 + 8 * buf, lane))
+                     : "memory");
+      const uint32_t mine = slot + 32 + (uint32_t)(lane * sizeof(T));
+      for (int q = 0; q < CS; ++q) {
+        const uint32_t dst = cluster_addr(mine, q), bar = cluster_addr(bar0 + 8 * buf, q);
+        if constexpr (sizeof(T) == 8)
+          asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(dst),
+                       "l"(__double_as_longlong(v)), "r"(bar)
+                       : "memory");
+        else
+          asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(dst),
+                       "r"(__float_as_uint(v)), "r"(bar)
+                       : "memory");
+      }
       __syncwarp();  // (the row is read before its owner goes on)
     }
     if (exch) {
@@ -742,14 +757,31 @@ panel_cluster_kernel(T* A, long long lda, int m, int r0, int c0, int w, int rpc,
         // 1/|candidate| on the integer pipe while the rows are updated: 450
         // cycles that every thread would otherwise wait for after the exchange
         const unsigned long long kb = (unsigned long long)s_wk[par][cw];
-        send_reciprocal(k, kb - 1ULL < 0x7FEFFFFFFFFFFFFFULL ? recip_bits(kb) : 0.0);
+        const double ra = kb - 1ULL < 0x7FEFFFFFFFFFFFFFULL ? recip_bits(kb) : 0.0;
+        const uint32_t slot = in0 + (uint32_t)((buf * CMAXG + b) * sizeof(PanelInbox<T>));
+        if (lane < CS)
+          asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(
+                           cluster_addr(slot + 16, lane)),
+                       "l"(__double_as_longlong(ra)), "r"(cluster_addr(bar0 + 8 * buf, lane))
+                       : "memory");
       }
     } else if (k > 0) {
       finish_update(k - 1, Uprev);
     }
     // --- every CTA's candidate is here: the winner, U(k, :) and 1/pivot ---
-    // (a poll here takes an eighth of one in L2)
-    if (!__all_sync(0xffffffffu, column_here(k, 8 * spin_limit))) {
+    bool ok = false;
+    for (long long spins = 0; spins < 8 * spin_limit; ++spins) {  // (a poll here takes an eighth of one in L2)
+      uint32_t done;
+      asm volatile(
+          "{\n .reg .pred p;\n mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+          " selp.u32 %0, 1, 0, p;\n}\n"
+          : "=r"(done)
+          : "r"(bar0 + 8 * buf), "r"((uint32_t)((k / 3) & 1))
+          : "memory");
+      if (done) { ok = true; break; }
+    }
+    ok = __all_sync(0xffffffffu, ok);
+    if (!ok) {
       if (lane == 0) {
         atomicExch(status, (int)kFlagTimeout);
         s_fail[par] = 1;
@@ -808,11 +840,16 @@ panel_cluster_kernel(T* A, long long lda, int m, int r0, int c0, int w, int rpc,
     // pivots from the first one that was not chosen become the diagonal rows
     if (b == 0)
       for (int q = max(k - 1, 0) + tid; q < kw; q += NTR + 32) ipiv[c0 + q] = r0 + q;
-    if (tid < CS)
+    if (tid < CS) {
       asm volatile("st.relaxed.cluster.shared::cluster.b32 [%0], %1;" ::"r"(
                        cluster_addr((uint32_t)__cvta_generic_to_shared(s_sent) + 4 * b, tid)),
-                   "r"(2 * k + 1)
+                   "r"(k)
                    : "memory");
+      asm volatile("st.relaxed.cluster.shared::cluster.b32 [%0], %1;" ::"r"(
+                       cluster_addr((uint32_t)__cvta_generic_to_shared(&s_any), tid)),
+                   "r"(1)
+                   : "memory");
+    }
   } else {
     if (kw > 0) finish_update(kw - 1, Uprev);
     if (part == 0 && row0 < nr) lab[row0] = mylab;
@@ -832,22 +869,8 @@ panel_cluster_kernel(T* A, long long lda, int m, int r0, int c0, int w, int rpc,
     }
   }
   cluster_sync();
-  int most = 0, gave_up = 0;
-  for (int q = 0; q < CS; ++q) {
-    most = max(most, s_sent[q] >> 1);
-    gave_up |= s_sent[q] & 1;
-  }
-  if (!gave_up) return;  // every CTA has received all columns
-  // (every CTA reads the same counts) complete what was begun, and wait for what this
-  // CTA was sent before its shared memory goes
-  if (warp == 0)
-    for (int c = s_sent[b] >> 1; c < most; ++c) {
-      if (lane == 0) expect_column(c);
-      send_candidate(c, 0, 0, (T)0);
-      if constexpr (sizeof(T) == 8) send_reciprocal(c, 0.0);
-    }
-  __syncthreads();
-  for (int c = max(0, most - 3); c < most; ++c) column_here(c, kSpinLimit);
+  if (!*(volatile int*)&s_any) return;  // every CTA has received all columns
+  panel_cluster_finish<T>(s_sent, CS, b, bar0, in0);
   cluster_sync();
 }
 
