@@ -1726,6 +1726,50 @@ gemm_skinny_kernel(int m, int n, int k, T alpha, const T* __restrict__ A, long l
 
 // ------------------------------------------------------------ launch helpers
 
+// Threads of the widest one-cluster panel (FP64 rows per CTA never pass PTR), and its
+// rows per CTA at most.
+template <typename T>
+constexpr int kClusterThreads = sizeof(T) == 4 ? 2 * PTR : PTR;
+template <typename T>
+inline int panel_cluster_rows_of() { return sizeof(T) == 4 ? 512 : panel_cluster_rows(); }
+template <typename T>
+inline size_t panel_cluster_smem(int rpc) {
+  return panel_inbox_bytes<T>() + (sizeof(T) * PLD + sizeof(int)) * (size_t)rpc;
+}
+
+// Prepares the one-cluster panel's kernels, once; whether the device gives a cluster of
+// CMAXG of them room (a part of a GPU may not: the other form runs there).
+template <typename T>
+inline bool panel_cluster_fits() {
+  static const bool fits = [] {
+    const void* kerns[] = {(const void*)panel_cluster_kernel<T, PTR>,
+                           (const void*)panel_cluster_kernel<T, kClusterThreads<T>>};
+    for (const void* f : kerns)
+      if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess ||
+          cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+      }
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute la[1];
+    la[0].id = cudaLaunchAttributeClusterDimension;
+    la[0].val.clusterDim.x = CMAXG;
+    la[0].val.clusterDim.y = la[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(CMAXG);
+    cfg.blockDim = dim3(kClusterThreads<T> + 32);
+    cfg.dynamicSmemBytes = panel_cluster_smem<T>(panel_cluster_rows_of<T>());
+    cfg.attrs = la;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kerns[1], &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    return n > 0;
+  }();
+  return fits;
+}
+
 template <typename T>
 inline cudaError_t launch_panel(T* A, long long lda, int m, int r0, int c0, int w, int* ipiv,
                                 const LuWork& ws, cudaStream_t s, bool after_kernel = false) {
@@ -1733,22 +1777,12 @@ inline cudaError_t launch_panel(T* A, long long lda, int m, int r0, int c0, int 
   // One cluster (16 CTAs at most, of 32 rows at least) while its rows stay
   // within what its SMs' FP64 units do in a column's time. (The tuning knobs of
   // the row slices and CTAs ask for the other form.)
-  const int cl_rows = sizeof(T) == 4 ? 512 : panel_cluster_rows();
-  if (panel_min_rows() == 0 && panel_ctas() == 64 && R <= CMAXG * cl_rows && w > 0) {
+  if (panel_min_rows() == 0 && panel_ctas() == 64 && R <= CMAXG * panel_cluster_rows_of<T>() && w > 0 &&
+      panel_cluster_fits<T>()) {
     int cs = 1;
     while (cs < CMAXG && R > 32 * cs) cs *= 2;
     int crpc = ((R + cs - 1) / cs + 7) & ~7;
-    const size_t csmem = panel_inbox_bytes<T>() + (sizeof(T) * PLD + sizeof(int)) * (size_t)crpc;
-    constexpr int kWide = sizeof(T) == 4 ? 2 * PTR : PTR;  // (FP64 rows per CTA never pass PTR)
-    static const cudaError_t at = [] {
-      for (const void* f : {(const void*)panel_cluster_kernel<T, PTR>, (const void*)panel_cluster_kernel<T, kWide>}) {
-        cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        if (e != cudaSuccess) return e;
-      }
-      return cudaSuccess;
-    }();
-    SL_TRY(at);
+    const size_t csmem = panel_cluster_smem<T>(crpc);
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute la[2];
     la[0].id = cudaLaunchAttributeClusterDimension;
@@ -1757,7 +1791,7 @@ inline cudaError_t launch_panel(T* A, long long lda, int m, int r0, int c0, int 
     la[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // (see launch_after)
     la[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.gridDim = dim3(cs);
-    const int ntr = crpc > PTR ? kWide : PTR;
+    const int ntr = crpc > PTR ? kClusterThreads<T> : PTR;
     cfg.blockDim = dim3(ntr + 32);
     cfg.dynamicSmemBytes = csmem;
     cfg.stream = s;
@@ -1765,7 +1799,7 @@ inline cudaError_t launch_panel(T* A, long long lda, int m, int r0, int c0, int 
     cfg.numAttrs = after_kernel ? 2 : 1;
     int ctpr = crpc > PTR / 4 ? 1 : (crpc > PTR / 8 ? 2 : 4);
     count_launches(1);
-    auto kern = ntr == PTR ? panel_cluster_kernel<T, PTR> : panel_cluster_kernel<T, kWide>;
+    auto kern = ntr == PTR ? panel_cluster_kernel<T, PTR> : panel_cluster_kernel<T, kClusterThreads<T>>;
     return cudaLaunchKernelEx(&cfg, kern, A, lda, m, r0, c0, w, crpc, ipiv, ws.info_col, ws.status,
                               spin_limit(), ctpr);
   }
