@@ -211,3 +211,59 @@ def test_u12_with_a_large_inverse(sl, orc, ctx, n, nb, scale, lookahead):
     assert _routes(sl) > r0
     assert orc.fresid(LU, rel, A0) < RESID_THRESH
     assert orc.sresid(A0, B0, X) < RESID_THRESH
+
+
+# Square matrices of up to 1536 columns are one panel whatever NB is: the orders below go
+# through the blocked form too (256-wide panels with the look-ahead, U12 through the inverse
+# of L11 balanced by A12's rows, updates of K = 256, and a last panel of up to 1024).
+@pytest.mark.parametrize("kind", ["rows60", "cols60", "both300", "rows_smooth", "dominant",
+                                  "diag_d"])
+@pytest.mark.parametrize("n,nb", [(1600, 64), (2100, 256)])
+def test_badly_scaled_parity_in_blocks(sl, orc, ctx, kind, n, nb):
+    A0 = graded(orc, n, kind)
+    B0 = np.asfortranarray(orc.matgen(n, 2, 200, kind=1))
+    info, LU, rel, X = run_pdgesv(sl, ctx, A0, B0, nb)
+    assert info == 0
+    bad, ties = compare_ipiv(orc, A0, rel, nb)
+    assert bad == 0, f"IPIV differs outside near-ties (ties logged: {ties})"
+    assert orc.fresid(LU, rel, A0) < RESID_THRESH
+    assert orc.sresid(A0, B0, X) < RESID_THRESH
+
+
+def test_budget_sends_a_blocks_update_to_fp64(sl, orc, ctx):
+    """The spike at the end of the first block of 256: the update of K = 256 by it. (Row 7's
+    entry 64: after 255 steps other rows' entries reach 4.)"""
+    n, nb = 1700, 256
+    A0 = spike_matrix(orc, n, nb, j0=1200)
+    A0[7, nb - 1] = 64.0
+    B0 = np.asfortranarray(orc.matgen(n, 1, 200, kind=1))
+    r0 = _routes(sl)
+    info, LU, rel, X = run_pdgesv(sl, ctx, A0, B0, nb)
+    assert info == 0
+    assert _routes(sl) > r0
+    bad, ties = compare_ipiv(orc, A0, rel, nb)
+    assert bad == 0, f"IPIV differs outside near-ties (ties logged: {ties})"
+    assert orc.fresid(LU, rel, A0) < RESID_THRESH
+    assert orc.sresid(A0, B0, X) < RESID_THRESH
+    LUo = np.asfortranarray(A0.copy())
+    orc.pdgetrf(n, n, LUo, nb=nb)
+    scale = np.max(np.abs(LUo), axis=1, keepdims=True)
+    assert np.max(np.abs(LU - LUo) / scale) < 1e-9
+
+
+@pytest.mark.parametrize("kind", ["rows60", "both300"])
+def test_graded_modes_agree_in_blocks(sl, orc, ctx, kind):
+    n, nb = 1700, 128
+    A0 = graded(orc, n, kind)
+    B0 = np.asfortranarray(orc.matgen(n, 1, 200, kind=1))
+    out = {}
+    try:
+        for mode in (0, 1):
+            sl.set_f64_update(mode)
+            out[mode] = run_pdgesv(sl, ctx, A0, B0, nb)
+    finally:
+        sl.set_f64_update(1)
+    np.testing.assert_array_equal(out[0][2], out[1][2])
+    LU0, LU1 = out[0][1], out[1][1]
+    scale = np.maximum(np.max(np.abs(LU0), axis=1, keepdims=True), 1e-300)
+    assert np.max(np.abs(LU0 - LU1) / scale) < 1e-8

@@ -669,3 +669,33 @@ def test_tail_as_one_panel_edges(sl, gpu_required, m, n):
     low.diagonal().fill_(1.0)
     res = A.T[torch.from_numpy(perm).cuda()] - low @ torch.triu(dA.T[:n])
     assert res.abs().max().item() < 16.0 * m * 2.0**-53 * A.T.abs().sum(dim=1).max().item()
+
+
+@pytest.mark.parametrize("zero", [100, 300, 700, 1650])
+def test_singular_info_in_blocks(sl, orc, ctx, zero):
+    """A zero column in the first, second and third block of 256 and in the last panel."""
+    n, nb = 1700, 64
+    A0, B0 = system(orc, n, 1)
+    A0[:, zero] = 0.0
+    info, LU, rel, X = run_pdgesv(sl, ctx, A0, B0, nb)
+    assert info == zero + 1
+    np.testing.assert_array_equal(X, B0)
+    bad, _ = compare_ipiv(orc, A0, rel, nb)
+    assert bad == 0
+    assert orc.fresid(LU, rel, A0) < RESID_THRESH
+
+
+@pytest.mark.parametrize("col", [400, 1650])
+def test_nan_in_blocks(sl, orc, ctx, col):
+    """A NaN in one column of a matrix factored in blocks leaves the columns before it
+    as they are, pivots and factors, and reaches the columns behind it."""
+    n, nb = 1700, 64
+    A0, B0 = system(orc, n, 1)
+    _, LU0, rel0, _ = run_pdgesv(sl, ctx, A0, B0, nb)
+    A1 = np.asfortranarray(A0.copy())
+    A1[1000, col] = np.nan
+    _, LU1, rel1, X = run_pdgesv(sl, ctx, A1, B0, nb)
+    np.testing.assert_array_equal(rel1[:col], rel0[:col])
+    # (columns of L, in the rows' order at that point: the later pivots permute them)
+    np.testing.assert_allclose(LU1[:col, :col], LU0[:col, :col], rtol=0, atol=1e-9)
+    assert np.isnan(LU1[:, col]).any() and np.isnan(LU1[-1, -1]) and np.isnan(X).any()

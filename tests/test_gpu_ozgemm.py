@@ -330,3 +330,26 @@ def test_fp64_route_with_c_aliasing_b(sl, torch_dev, k):
     assert _routes(sl) == r0 + 1
     got = dB.cpu().numpy().T
     assert _componentwise_ok(got, A, B, B, 1.0, c=1.0) <= 1.0
+
+
+@pytest.mark.parametrize("n,nb", [(1700, 64), (2100, 320)])
+def test_blocked_lu_matches_dmma_pivots(sl, orc, torch_dev, n, nb):
+    """Orders that the sliced mode factors in blocks of 256; the DMMA mode in the caller's
+    (320: more interchanges than the composite form holds)."""
+    torch, dev = torch_dev
+    A = np.random.default_rng(n + nb).uniform(-0.5, 0.5, (n, n))
+    res = {}
+    try:
+        for mode in (0, 1):
+            sl.set_f64_update(mode)
+            dA = torch.from_numpy(np.ascontiguousarray(A.T)).to(dev)
+            piv = torch.zeros(n, dtype=torch.int32, device=dev)
+            torch.cuda.synchronize()
+            assert sl.dgetrf_dev(n, n, dA.data_ptr(), n, piv.data_ptr(), nb) == 0
+            res[mode] = (dA.cpu().numpy().T.copy(), piv.cpu().numpy().copy())
+    finally:
+        sl.set_f64_update(1)
+    np.testing.assert_array_equal(res[0][1], res[1][1])
+    for mode in (0, 1):
+        assert orc.fresid(res[mode][0], res[mode][1], A) < 16.0
+    assert np.max(np.abs(res[0][0] - res[1][0])) < 1e-9
