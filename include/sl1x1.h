@@ -280,7 +280,8 @@ int sl1x1_dgerfs_dev(char trans, int n, int nrhs, const double* dA, long long ld
 void sl1x1_finalize(void);
 /* Block size NB used by the device entry points when nb <= 0 (default 256).
  * With the sliced update the FP64 factorization chooses its own width whatever
- * NB is: the whole matrix up to 1536 columns, 256 columns beyond. */
+ * NB is: the whole matrix for M >= N, N <= 1536 and at most two tiles of 128 x 64
+ * per SM, else 256 columns. */
 void sl1x1_set_default_nb(int nb);
 /* Look-ahead in the factorizations (default on): the next panel is factored
  * on a second stream while the trailing update runs. Same pivots (except
@@ -361,8 +362,9 @@ void sl1x1_set_lowp_stages(int stages);
  * SRC/pdgetrf.f:288-290): 1 (default) = the product formed exactly on the
  * BF16 tensor cores (tcgen05) from 8-bit integer slices of the operands (7
  * balanced base-256 digits, row and column power-of-two scales, the leading
- * diagonals of the slice products summed exactly as integers), accurate to a
- * few units of 2^-53 of max|L21(i,:)| max|U12(:,j)| and independent of the
+ * diagonals of the slice products summed as integers), accurate to a few
+ * units of 2^-53 of max|L21(i,:)| max|U12(:,j)| on operands without a pattern,
+ * to 2^-45.4 of it (per 256 columns) on any, and independent of the
  * summation order; 0 =
  * FP64 DMMA (mma.sync m16n8k4). The sliced form needs device scratch of about
  * 4 KB per row plus 4 KB per column of the matrix; where it cannot be had

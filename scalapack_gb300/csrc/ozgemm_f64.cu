@@ -12,7 +12,7 @@
 // column j of B likewise with 2^-f_j and b_t. BF16 holds every such digit exactly
 // (8 significant bits). Balanced digits carry 8 bits a slice where truncated ones
 // of the same exactness carry 7: 7 slices and 28 products instead of 8 and 36,
-// with the same 2^-56 of the scale kept and no bias.
+// with the same 2^-56 of the scale kept.
 //
 // Exact products. For K <= 256, sum_k a_s b_t is an integer of magnitude at
 // most 256 * 128^2 = 2^22: up to four such products sum exactly in FP32, in
@@ -22,8 +22,9 @@
 // Each diagonal d = 2..8 has its own TMEM accumulator (7 x 64 columns). d <= 5
 // holds at most 4 products: exact; d = 6..8 hold 5 to 7, exact unless their sum
 // passes 2^24, which takes most of the 1280 to 1792 terms at full magnitude with
-// one sign; d >= 9 is dropped: 6 products of weight 2^-70, whose balanced digits
-// have no common sign. 28 slice products, issued as 10 instructions per 16-wide
+// one sign (constant rows of 254/255 do that; the FP32 rounding is then 2^-24 of terms
+// 2^-40 below the scales' largest sum); d >= 9 is dropped: at most 6 256 128^2 2^-70,
+// 2^-45.4, of 2^(e_i + f_j). 28 slice products, issued as 10 instructions per 16-wide
 // k step: A slice s against B slices t = 0..6-s (consecutive in shared memory)
 // into accumulators s..6 (consecutive in TMEM) in groups of up to 4 (N up to
 // 256).
@@ -36,9 +37,13 @@
 // multiplies doubles at 2 lanes per cycle and SM, so a conversion, a
 // multiplication and an fma per element would take as long as the tile's
 // products, and a 64-bit conversion before the accumulators are released would
-// hold the products up. The result is within a few units of 2^-53 of
-// 2^(e_i + f_j) of the exact product, and independent of the accumulation order
-// (run to run identical). Rows or columns holding Inf or NaN give NaN in their
+// hold the products up. The result is within 2^-45.4 of 2^(e_i + f_j) of the exact
+// product (about K/1.3 units of 2^-53, as an FP64 GEMM's bound of K units), reached
+// where all low digits have one sign: 2^-46.1 for constant operands of 0.1, 2^-45.4
+// for one large entry among small ones with that pattern, where a GEMM's actual error
+// is below 2^-50; on operands without a pattern it is a few units of 2^-53. (8
+// truncated slices and 36 products: 2^-45.2.) It is independent of the accumulation
+// order (run to run identical). Rows or columns holding Inf or NaN give NaN in their
 // row or column of C.
 //
 // Balancing along k. A B = (A 2^-d)(2^d B) for any integers d_k, so the

@@ -50,3 +50,31 @@ def test_seven_slice_product_error():
         worst = max(worst, abs(float(got - exact)))
         assert abs(sum(p * 2.0 ** (56 - 8 * d) for d, p in P.items())) < 2.0**63
     assert worst < 4 * 2.0**-52
+
+
+def _seven_slice_error(a, b):
+    """|kept products - exact| of two vectors whose scales are 1, in exact arithmetic."""
+    from fractions import Fraction
+
+    da, db = [_balanced_digits(float(v), 0)[0] for v in a], [_balanced_digits(float(v), 0)[0] for v in b]
+    got = sum(Fraction(sum(x[s - 1] * y[d - s - 1] for x, y in zip(da, db) for s in range(max(1, d - 7), min(7, d - 1) + 1)))
+              * Fraction(2) ** (2 - 8 * d) for d in range(2, 9))
+    return abs(float(got - sum(Fraction(float(x)) * Fraction(float(y)) for x, y in zip(a, b))))
+
+
+@pytest.mark.parametrize("kind", ["constant", "one large", "254/255"])
+def test_seven_slice_product_worst_case(kind):
+    """Operands with a pattern: the dropped products are at most 6 256 128^2 2^-70 (d = 9) and
+    1/300 of that beyond (d = 10 .. 14: 5, 4, .. products, each 2^-8 further down), the
+    cuts 256 2^-55. All three are far above the few units of random operands."""
+    K = 256
+    if kind == "constant":
+        a = np.full(K, 0.8)  # 0.1 against its own scale
+    elif kind == "one large":
+        a = np.full(K, float.fromhex("0x1.fdfdfdfdfdfcp-9"))
+        a[0] = 0.75
+    else:
+        a = np.full(K, 254.0 / 255.0)
+    err = _seven_slice_error(a, a)
+    assert err <= 6 * K * 128**2 * 2.0**-70 * (1 + 1 / 300) + K * 2.0**-55
+    assert err > 2.0**-47
