@@ -325,12 +325,6 @@ __device__ __forceinline__ void factor_system(T* W, int n, int ncols, int* ipiv,
   __syncthreads();
 }
 
-// x / d from r = 1/d, rounded like the division (one correction step).
-__device__ __forceinline__ double div_by(double x, double d, double r) {
-  const double q = x * r;
-  const double f = fma(fma(-d, q, x), r, q);
-  return (f - f == 0.0) ? f : x / d;  // (infinities, zeros and NaN divide)
-}
 __device__ __forceinline__ float div_by(float x, float d, float) { return x / d; }
 
 // Triangular solve with the unit-lower L (LOWER) or the upper U of the factors

@@ -111,10 +111,7 @@ small_gesv_kernel(int n, int nrhs, double* A, long long lda, double* B, long lon
   for (int r = warp; r < nrhs; r += 4) {
     double x = lane < n ? s_Y[r * 33 + lane] : 0.0;
     for (int k = n - 1; k >= 0; --k) {
-      // x / d to nearest from 1/d (one correction; what is not finite divides)
-      const double q0 = x * rd, f = fma(fma(-d, q0, x), rd, q0);
-      const bool fin = ((__double2hiint(f) >> 20) & 0x7ff) != 0x7ff;
-      if (lane == k) x = fin ? f : x / d;
+      if (lane == k) x = div_by(x, d, rd);
       const double xk = __shfl_sync(0xffffffffu, x, k);
       if (lane < k) x = fma(-s_U[k * 33 + lane], xk, x);
     }

@@ -162,3 +162,41 @@ def test_batched_panel_edges(sl, orc, gpu_required, mode, orders):
         assert info[i] == 0
         assert orc.sresid(A, B, X[i]) < 16.0  # the tester's bound
     plan.close()
+
+
+def test_one_by_one_systems_divide(sl, gpu_required):
+    """The backward substitution's quotient from the diagonal's reciprocal: the rounded one
+    over random and special significands (all ones, powers of two, neighbours of 1), and
+    within one unit in the last place where remainders or reciprocals are subnormal. As
+    one-by-one systems of a plan and of PDGESV."""
+    import torch
+
+    rng = np.random.default_rng(11)
+    a = rng.uniform(1, 2, 512) * np.exp2(rng.integers(-300, 301, 512))
+    a[:6] = [1.0, 2.0 - 2.0**-52, 1.0 + 2.0**-52, 0.5, 3.0, 1.0 - 2.0**-53]
+    b = rng.uniform(1, 2, (512, 8)) * np.exp2(rng.integers(-300, 301, (512, 8)))
+    b[:6] = rng.uniform(1, 2, (6, 8))
+    b[:, 0] = a
+    a[::3] *= -1
+    edge_a = np.array([2.0**1023, 1.7e308, 2.0**-1022, 5e-324 * 12345, 1.0, 3.0, 2.0**1000, 2.0**-500])
+    edge_b = np.array([[1.0, 1.5e308, 2.0**-1000 * 1.7, 3e-310, 1.1e-300, 2.0**-1022, 1.2e-308, 7.0 * 5e-324]]).repeat(8, 0)
+    for A, B, ulps in ((a, b, 0), (edge_a, edge_b, 1)):
+        with np.errstate(over="ignore", under="ignore"):
+            want = B / A[:, None]
+        ok = np.isfinite(want)
+        systems = [(np.full((1, 1), v, order="F"), np.asfortranarray(w[None, :])) for v, w in zip(A, B)]
+        p = Plan(sl, torch, systems, mode=0, autotune=0)
+        p.run()
+        torch.cuda.synchronize()
+        got = np.array([x.cpu().numpy().reshape(-1) for x in p.dX])
+        p.close()
+        assert (np.abs(got[ok] - want[ok]) <= ulps * np.spacing(np.abs(want[ok]))).all()
+        assert np.array_equal(np.isfinite(got), ok)
+        dA, dB = torch.from_numpy(A.copy()).cuda(), torch.from_numpy(B.copy()).cuda()
+        ip = torch.zeros(1, dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        for i in range(0, len(A), 1 if ulps else 16):
+            assert sl.dgesv_dev(1, 8, dA.data_ptr() + 8 * i, 1, ip.data_ptr(), dB.data_ptr() + 64 * i, 1) == 0
+            x = dB[i].cpu().numpy()
+            x, w = x[ok[i]], want[i][ok[i]]
+            assert (np.abs(x - w) <= ulps * np.spacing(np.abs(w))).all()
