@@ -451,7 +451,8 @@ __device__ __forceinline__ double residual_system(const double* A, int lda, int 
     if (lane < nrhs) {
       const double rn = __longlong_as_double((long long)s_rm[lane]);
       rmax[lane] = rn;
-      v = rn / (__longlong_as_double((long long)s_xm[lane]) * anorm * ldexp(1.0, -53) * n);
+      // (a zero right-hand side and its zero solution are exact, not 0 / 0)
+      v = rn == 0.0 ? 0.0 : rn / (__longlong_as_double((long long)s_xm[lane]) * anorm * ldexp(1.0, -53) * n);
     }
     const unsigned long long w = warp_max64(mag_key(v));
     if (lane == 0) s_worst = __longlong_as_double((long long)w);

@@ -200,3 +200,28 @@ def test_one_by_one_systems_divide(sl, gpu_required):
             x = dB[i].cpu().numpy()
             x, w = x[ok[i]], want[i][ok[i]]
             assert (np.abs(x - w) <= ulps * np.spacing(np.abs(w))).all()
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+def test_zero_right_hand_sides(sl, orc, gpu_required, mode):
+    """Zero columns first, in the middle, last and throughout: zero solutions, finite
+    residuals of the others, and no system sent to the FP64 pass for them."""
+    import torch
+
+    rng = np.random.default_rng(21)
+    systems = make_batch(rng, 8, nmin=20, nmax=150, rmax=1)
+    zeros = [[0], [2], [4], [0, 4], [1, 2, 3], [0, 1, 2, 3, 4], [0, 1, 2, 3], []]
+    systems = [(A + np.eye(len(A)) * 4, np.asfortranarray(rng.uniform(-0.5, 0.5, (len(A), 5)))) for A, _ in systems]
+    for (_, B), z in zip(systems, zeros):
+        B[:, z] = 0.0
+    systems = [(np.asfortranarray(A), B) for A, B in systems]
+    plan = Plan(sl, torch, systems, mode)
+    info, its, sr, X = plan.run()
+    plan.close()
+    for i, ((A, B), z) in enumerate(zip(systems, zeros)):
+        assert info[i] == 0 and np.isfinite(sr[i]) and sr[i] < 16.0
+        assert its[i] >= 1 if mode == 1 else its[i] == 0
+        assert (X[i][:, z] == 0.0).all()
+        keep = [c for c in range(5) if c not in z]
+        if keep:
+            assert orc.sresid(A, np.asfortranarray(B[:, keep]), np.asfortranarray(X[i][:, keep])) < 16.0
