@@ -848,14 +848,14 @@ int sl1x1_dgesv_ir_dev(int n, int nrhs, double* dA, long long ldda, int* dipiv, 
                           opt, &st, w, mw, s);
   if (e == cudaErrorInvalidValue) return -30000;
   if (e != cudaSuccess) return cuda_info(e);
-  if (st.fell_back) {  // the FP64 factorization and solve
-    const int r = take_status(s);
-    if (r != 0) return r;
-  }
   if (stats) {
     stats[0] = st.classical; stats[1] = st.gmres_outer; stats[2] = st.gmres_inner;
     stats[3] = st.fell_back ? (st.gave_up ? 2 : 1) : 0; stats[4] = st.sresid; stats[5] = st.anorm;
     stats[6] = st.factor_ms; stats[7] = st.refine_ms;
+  }
+  if (st.fell_back) {  // the FP64 factorization and solve
+    const int r = take_status(s);
+    if (r != 0) return r;
   }
   if (st.dev_status) return -20000 - st.dev_status;
   if (iter) *iter = st.fell_back ? (st.gmres_outer > 0 || st.classical > 0 ? -3 : -1)
