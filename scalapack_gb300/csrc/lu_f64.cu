@@ -62,6 +62,11 @@ static int g_panel_ctas = 64;  // CTAs a panel's rows are spread over (before th
 // where the products are what takes the time. PDGETRF, ms, one / two: N = 4096 13.2 /
 // 14.0, 6001 x 3007 11.1 / 11.7, N = 8192 31.7 / 32.7, N = 12000 61.6 / 62.6; 20000 x
 // 4000 28.2 / 27.4, 30000 x 1000 8.2 / 7.6.
+// One rounds C once per 32 columns inside a panel, two once per 64: where the diagonal is
+// heavy and the updates small beside it the factors' error is up to 8 % larger (6001 x
+// 3007 2.94e-16 / 2.72e-16 of their norm, N = 8192 3.86 / 3.76, N = 600 4.43 / 4.40); on
+// uniform matrices it is the same to 1 % (N = 4096 3.95e-13 / 3.93e-13) or smaller (N = 600
+// 1.91e-14 / 2.03e-14).
 constexpr int kDeepPanelRows = 12000;
 static int g_panel_ib = 0;
 void set_panel_ib(int ib) { g_panel_ib = ib < 1 ? 0 : (ib > 8 ? 8 : ib); }
@@ -446,7 +451,10 @@ static cudaError_t step0_by_chunks(int m, int n, double* dA, long long ldda, int
 // launches of a block beside its panel cost more than the wider products), their
 // interchanges applied to the `left` columns before them by the in-panel steps. In us,
 // without / with: N = 1600 4519 / 4229, N = 2000 5746 / 5454 (up to 1536 columns: 5510),
-// N = 3000 9198 / 8923, N = 4096 13210 / 13148, N = 8192 no difference.
+// N = 3000 9198 / 8923, N = 4096 13210 / 13148, N = 8192 no difference. Its columns'
+// updates are rounded once per 32 columns instead of once per 256: error of the factors
+// with a heavy diagonal 2 % larger (N = 2000 5.00e-16 / 4.91e-16), of uniform ones 1 to 6 %
+// smaller (1.56e-13 / 1.65e-13).
 static bool one_panel_tail(int m, int n, int left) {
   return n <= 1024 && left <= 4096 && ((m + 127LL) / 128) * ((n + 63) / 64) <= 2LL * num_sms();
 }
