@@ -287,3 +287,14 @@ def test_solve_that_gives_up_is_reported_by_every_caller(sl, orc, ctx):
             sl.lib().sl1x1_debug_set_spin_limit(-1)
         info, err = call()
         assert info == 0 and err < 1e-9
+
+
+@pytest.mark.parametrize("polls", [0, 1, 8])
+def test_grid_panel_gives_up(sl, orc, ctx, polls):
+    """The panel that exchanges through L2, asked for by a row-slice setting at an order
+    whose panels are one cluster otherwise."""
+    sl.lib().sl1x1_set_panel_rows(64)
+    try:
+        _recovers(sl, orc, ctx, 700, 1, 64, polls, 4)
+    finally:
+        sl.lib().sl1x1_set_panel_rows(0)

@@ -405,6 +405,22 @@ def test_solve_with_ill_conditioned_triangles(sl, gpu_required, kind, n, seed, n
     assert (res < RESID_THRESH).all(), res.max()
 
 
+@pytest.mark.parametrize("kind,n,seed", [("uniform", 64, 0), ("uniform", 300, 4), ("lower", 200, 0), ("lower", 400, 0)])
+def test_inverse_of_ill_conditioned_triangles(sl, gpu_required, kind, n, seed):
+    """PDGETRI through the same block steps, below and above 256 (inv(L) as a triangle):
+    each column of the inverse solves its system within the tester's bound."""
+    import torch
+
+    A = _triangle(kind, n, seed)
+    dA = torch.from_numpy(A.T.copy()).cuda()
+    ip = torch.arange(1, n + 1, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    assert sl.lib().sl1x1_dgetri_dev(n, dA.data_ptr(), n, ip.data_ptr(), None) == 0
+    X = dA.T.cpu().numpy()
+    res = np.abs(np.eye(n) - A @ X).max(axis=0) / (np.abs(A).sum(axis=1).max() * np.abs(X).max(axis=0) * n * 2.0**-53)
+    assert (res < RESID_THRESH).all(), res.max()
+
+
 @pytest.mark.parametrize("trans", ["N", "T"])
 @pytest.mark.parametrize("nrhs", [1, 129, 300])
 @pytest.mark.parametrize("n", [20, 90])
