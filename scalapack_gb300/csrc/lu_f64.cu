@@ -215,8 +215,8 @@ static_assert(kDinv64Doubles >= (size_t)kFullInvMax * kFullInvMax, "inverse of L
 // 2^10: 0.5 (substitution 0.04), 2^12: 11, 2^40: 2e8.
 __host__ __device__ inline int inv_cols_blocks(int jb) { return (jb + 1) / 2; }
 __global__ void __launch_bounds__(256)
-unit_lower_inv_cols_kernel(int jb, const double* __restrict__ L, long long ldl, double* X,
-                           int ldx, int* flags, int k1, int k2, const int* __restrict__ ipiv, int* plan) {
+unit_lower_inv_cols_kernel(int jb, const double* L, long long ldl, double* X,
+                           int ldx, int* flags, int k1, int k2, const int* ipiv, int* plan) {
   wait_for_previous();
   if (plan != nullptr && (int)blockIdx.x == inv_cols_blocks(jb)) {
     laswp_plan_block(k1, k2, ipiv, plan);

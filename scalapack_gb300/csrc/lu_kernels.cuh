@@ -983,8 +983,7 @@ laswp_kernel(T* A, long long lda, int k1, int k2, const int* __restrict__ ipiv, 
 // other way), so the cost is npiv shared-memory reads per row, in parallel.
 // The pairs come out in the order of a sequential replay. Computed once per
 // panel, on the panel's stream; laswp_apply_kernel then only moves data.
-static __device__ __noinline__ void laswp_plan_block(int k1, int k2, const int* __restrict__ ipiv,
-                                                    int* plan) {
+static __device__ __noinline__ void laswp_plan_block(int k1, int k2, const int* ipiv, int* plan) {
   __shared__ int s_piv[LSW_MAXP], s_row[2 * LSW_MAXP];
   const int npiv = k2 - k1, tid = threadIdx.x, nt = blockDim.x;
   for (int i = tid; i < npiv; i += nt) s_piv[i] = ipiv[k1 + i];
@@ -1093,7 +1092,7 @@ laswp_apply_kernel(T* A, long long lda, const int* __restrict__ plan, int cb1, i
 constexpr int IPC = 4;  // columns (warps) per CTA
 template <typename T>
 __global__ void __launch_bounds__(32 * IPC)
-inpanel_step_kernel(T* A, long long lda, int k1, int k2, const int* __restrict__ ipiv, int cb1, int ce1,
+inpanel_step_kernel(T* A, long long lda, int k1, int k2, const int* ipiv, int cb1, int ce1,
                     int cb2, int ce2, int nsolve, int kb, OzKeyJob kj) {
   __shared__ T Ls[64 * 64];  // T(i, q) at q*64 + i, rows below the diagonal
   __shared__ int s_piv[32], s_row[64], s_src[64];

@@ -90,8 +90,8 @@ sgemm_simt_kernel(int m, int n, int k, float alpha, const float* __restrict__ A,
 // in different columns).
 constexpr int K32_N = 16;
 __global__ void __launch_bounds__(256)
-sgemm_k32_kernel(int m, int n, int k, float alpha, const float* __restrict__ A, long long lda,
-                 const float* __restrict__ B, long long ldb, float* C, long long ldc) {
+sgemm_k32_kernel(int m, int n, int k, float alpha, const float* A, long long lda,
+                 const float* B, long long ldb, float* C, long long ldc) {
   __shared__ __align__(16) float Bs[32][K32_N];
   const int row = blockIdx.x * 256 + threadIdx.x, n0 = blockIdx.y * K32_N, nc = min(K32_N, n - n0);
   const float* a = A + min(row, m - 1);
